@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(AD_THREADS) attn_decode_kernel(
     __nv_bfloat16* __restrict__ out, float* __restrict__ part_acc, float* __restrict__ part_ml, int Hq, int Hkv,
     int page_size, int window, float scale_log2, int chunk, int S, const int* __restrict__ q_len, int row_limit,
     const int* __restrict__ ctx_len, int* __restrict__ counters, const float* __restrict__ r1p,
-    const float* __restrict__ r2p, const float* __restrict__ sink, AdDiff df) {
+    const float* __restrict__ r2p, const float* __restrict__ sink, AdDiff df, const int* __restrict__ row_list) {
   static_assert(!DIFF || (TMA && !EX && G % 2 == 0), "two score maps: by TMA, no extras");
   constexpr int CH = D / 8, KS = D / 16, NT_O = D / 8, WK = 64;  // WK: keys per warp pass
   extern __shared__ __align__(128) uint8_t smem_dyn[];
@@ -139,7 +139,11 @@ __global__ void __launch_bounds__(AD_THREADS) attn_decode_kernel(
   __shared__ float fin[DIFF ? G * D : 1];                    // DIFF: the maps' results, before they are combined
   hb_pdl_launch();
   HB_TL_MARK(0, 0);
-  const int t = blockIdx.z, h = blockIdx.y;
+  // row_list: the rows this grid is for, where they are a few of the step's (t: the row, tw: its place in the workspace). A step of
+  // a prompt portion and a few decoded rows had a grid over ALL its rows, of which each block read its request's length and
+  // left: some 80,000 blocks in a 2,048-row step behind 2,048 tokens, 71 us a layer more than the grid over the list (measured:
+  // 8 requests of 2,048 + 128 tokens 145.7 -> 136.6 ms, 14 mixed ones at head_dim 128 235.9 -> 214.2 ms).
+  const int tw = blockIdx.z, t = row_list ? __ldg(row_list + tw) : tw, h = blockIdx.y;
   // row_req null: a step of single decode rows, row t being request t (and its position the length its request had):
   // one round trip to memory less before the keys can be asked for
   const int rq = row_req ? row_req[t] : t;
@@ -400,9 +404,9 @@ __global__ void __launch_bounds__(AD_THREADS) attn_decode_kernel(
       a += red_o[(w * G + gg) * D + d] * f;
       l += red_ml[(w * G + gg) * 2 + 1] * f;
     }
-    const size_t head = (size_t)t * Hq + (size_t)h * G + gg;
+    const size_t head = (size_t)tw * Hq + (size_t)h * G + gg;   // in the workspace
     if (whole) {
-      put(head, gg, d, a / l);
+      put((size_t)t * Hq + (size_t)h * G + gg, gg, d, a / l);
     } else if constexpr (CL) {
       cl_acc[i] = a;
       if (d == 0) { cl_ml[gg * 2] = m * 0.6931471805599453f; cl_ml[gg * 2 + 1] = l; }
@@ -458,7 +462,7 @@ __global__ void __launch_bounds__(AD_THREADS) attn_decode_kernel(
   __threadfence();
   __syncthreads();
   if (tid == 0) {
-    int* cnt = counters + (size_t)t * Hkv + h;
+    int* cnt = counters + (size_t)tw * Hkv + h;
     const int last = atomicAdd(cnt, 1) == s_hi - s_lo;
     if (last) *cnt = 0;
     is_last = last;
@@ -476,7 +480,7 @@ __global__ void __launch_bounds__(AD_THREADS) attn_decode_kernel(
     for (int k = 0; k < PER; k++) {
       const int i = i0 + k * AD_THREADS, gg = i / D, d = i - gg * D;
       if (i < G * D) {
-        const size_t head = (size_t)t * Hq + (size_t)h * G + gg;
+        const size_t head = (size_t)tw * Hq + (size_t)h * G + gg;
         const float2* ml = (const float2*)part_ml + head * S + s_lo - s_off;
         const float* pa = part_acc + (head * S + s_lo - s_off) * D + d;
 #pragma unroll
@@ -506,7 +510,7 @@ __global__ void __launch_bounds__(AD_THREADS) attn_decode_kernel(
   } else {
     for (int i = tid; i < G * D; i += AD_THREADS) {
       const int gg = i / D, d = i - gg * D;
-      const size_t head = (size_t)t * Hq + (size_t)h * G + gg;
+      const size_t head = (size_t)tw * Hq + (size_t)h * G + gg;
       const float2* ml = (const float2*)part_ml + head * S + s_lo - s_off;
       const float* pa = part_acc + (head * S + s_lo - s_off) * D + d;
       float m = -INFINITY, a = 0.f, l = 0.f;
@@ -517,7 +521,7 @@ __global__ void __launch_bounds__(AD_THREADS) attn_decode_kernel(
         l += v.y * f;
         a += __ldcg(pa + (size_t)c * D) * f;
       }
-      put(head, gg, d, a / l);
+      put((size_t)t * Hq + (size_t)h * G + gg, gg, d, a / l);
     }
   }
   combine();
@@ -530,7 +534,7 @@ static int launch_decode(int G, dim3 grid, size_t smem, cudaStream_t st, const C
                          const int* bt, int bt_stride, const int* row_req, const int* pos, __nv_bfloat16* out, float* pa,
                          float* pm, int Hq, int Hkv, int page_size, int window, float scale, int chunk, int S,
                          const int* q_len, int row_limit, const int* ctx_len, int* counters, const float* r1, const float* r2,
-                         const float* sink, const AdDiff& df = AdDiff{}) {
+                         const float* sink, const AdDiff& df = AdDiff{}, const int* row_list = nullptr) {
 #define HB_AD_CASE(GG)                                                                                              \
   case GG:                                                                                                          \
     {                                                                                                               \
@@ -543,11 +547,11 @@ static int launch_decode(int G, dim3 grid, size_t smem, cudaStream_t st, const C
     if (CL)                                                                                                         \
       hb_launch_cluster(attn_decode_kernel<D, GG, TMA, RW, KW, SR, CL, EX, DIFF>, grid, AD_THREADS, smem, st, dim3(grid.x, 1, 1), mk, mv, status, \
                         q, kc, vc, bt, bt_stride, row_req, pos, out, pa, pm, Hq, Hkv, page_size, window, scale, chunk, S,    \
-                        q_len, row_limit, ctx_len, counters, r1, r2, sink, df);                                         \
+                        q_len, row_limit, ctx_len, counters, r1, r2, sink, df, row_list);                               \
     else                                                                                                            \
       hb_launch(attn_decode_kernel<D, GG, TMA, RW, KW, SR, CL, EX, DIFF>, grid, AD_THREADS, smem, st, mk, mv, status, q, kc, vc, bt, bt_stride, \
                 row_req, pos, out, pa, pm, Hq, Hkv, page_size, window, scale, chunk, S, q_len, row_limit, ctx_len,  \
-                counters, r1, r2, sink, df);                                                                            \
+                counters, r1, r2, sink, df, row_list);                                                                  \
     return 0;
   if constexpr (DIFF) {
     switch (G) { HB_AD_CASE(2) HB_AD_CASE(4) HB_AD_CASE(6) HB_AD_CASE(8) }
@@ -568,7 +572,8 @@ HB_EXPORT int hb_attn_decode_supported(int Hq, int Hkv, int D) {
 // Partials layout as hb_attn_rows of the core library: workspace = part_acc [T, Hq, S, D] then
 // part_ml [T, Hq, S, 2], S = max_pos / chunk + 1; `counters` are T * Hkv ints that are zero
 // between calls (needed when S > 1). With q_len given, rows of requests whose portion has
-// row_limit rows or more are skipped (the flash kernel computes those). ctx_len (per request,
+// row_limit rows or more are skipped (the flash kernel computes those). row_list (T ints, or null): the
+// rows the call is for, their indices in q, pos, row_req and out; workspace and counters go by the place in the list. ctx_len (per request,
 // or null): the tokens that were in the cache before this step; their keys may be read before
 // the kernel ahead in the stream has ended. row_req null: row t is request t's only row. n_pages: the pages the cache holds (its first
 // extent); status: the word a bounded wait that ran out sets to 1. With both, no window, a chunk
@@ -577,7 +582,7 @@ HB_EXPORT int hb_attn_decode(const void* q, const void* kc, const void* vc, long
                              const int* row_req, const int* pos, void* out, float* workspace, int* counters, int T,
                              int Hq, int Hkv, int D, int page_size, int window, float scale, int chunk, int max_pos,
                              const int* q_len, int row_limit, const int* ctx_len, int* status, const float* r1, const float* r2,
-                             const float* sink, cudaStream_t st) {
+                             const float* sink, const int* row_list, cudaStream_t st) {
   if (T <= 0) return 0;
   if (!hb_attn_decode_supported(Hq, Hkv, D)) HB_FAIL("hb_attn_decode: %d/%d heads of %d are not supported", Hq, Hkv, D);
   if (chunk <= 0 || chunk % 32) HB_FAIL("hb_attn_decode: chunk %d must be a positive multiple of 32", chunk);
@@ -621,7 +626,7 @@ HB_EXPORT int hb_attn_decode(const void* q, const void* kc, const void* vc, long
   const float sl2 = scale * 1.4426950408889634f;
   int r = 1;
 #define HB_AD_ARGS G, grid, smem, st, mk, mv, status, qq, kk, vv, bt, bt_stride, row_req, pos, (__nv_bfloat16*)out, pa, pm, Hq, Hkv, \
-                   page_size, window, sl2, chunk, S, q_len, row_limit, ctx_len, counters, r1, r2, sink
+                   page_size, window, sl2, chunk, S, q_len, row_limit, ctx_len, counters, r1, r2, sink, AdDiff{}, row_list
   // a step of few rows whose chunks fit one cluster: the chunks' partial results meet in distributed shared memory
   const bool cl = tma && S >= 2 && S <= 8 && T <= g_ad_cluster_rows;
   if (r1 || sink) {

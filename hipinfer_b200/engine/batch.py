@@ -49,8 +49,28 @@ class StepBatch:
     max_pos: int = 0              # largest position among the rows
     max_q_len: int = 0
     extra: dict = field(default_factory=dict)  # what a kernel dispatcher derived for this batch (cached per step)
+    short_list: Optional[torch.Tensor] = None  # int32: rows of requests with fewer than SHORT_ROWS rows, in a step with longer ones
     dump: Optional[dict] = None   # debug: planes of the step are recorded here, keyed (order index, name) (parts/planes.py)
     dump_step: int = -1           # the order index the decoder is at
+
+    def short_rows(self, limit: int):
+        """The rows of requests that bring fewer than `limit` rows (int32 on the device; packed with the batch for
+        SHORT_ROWS, else copied once a step), and the largest position among them."""
+        key = ("short_rows", limit)
+        if key not in self.extra:
+            short = [r for r in range(self.n_requests) if self.h_q_len[r] < limit]
+            rows = self.short_list if limit == SHORT_ROWS else None
+            if rows is None:
+                rows = torch.from_numpy(_rows_of(short, self.h_q_start, self.h_q_len)).to(self.tokens.device)
+            self.extra[key] = rows, max(self.h_ctx_len[r] + self.h_q_len[r] - 1 for r in short)
+        return self.extra[key]
+
+
+SHORT_ROWS = 16     # portions of fewer rows are computed row by row (kernels/fast.py: FLASH_MIN_ROWS)
+
+
+def _rows_of(requests, q_start, q_len) -> np.ndarray:
+    return np.concatenate([np.arange(q_start[r], q_start[r] + q_len[r], dtype=np.int32) for r in requests] or [np.zeros(0, np.int32)])
 
 
 def build_step_batch(entries: Sequence[StepEntry], ctx_lens: Sequence[int], state_slots: Sequence[int],
@@ -76,7 +96,8 @@ def build_step_batch(entries: Sequence[StepEntry], ctx_lens: Sequence[int], stat
     if table_widths is not None:
         assert all(w <= tw for w, tw in zip(widths, table_widths)), "a block table is wider than the graph was made for"
         widths = list(table_widths)
-    n_int = 4 * T + 4 * R + W + sum(R * w for w in widths) + n_groups * T
+    short = _rows_of([r for r in range(R) if q_len[r] < SHORT_ROWS], q_start, q_len) if R and max(q_len) >= SHORT_ROWS else np.zeros(0, np.int32)
+    n_int = 4 * T + 4 * R + W + sum(R * w for w in widths) + n_groups * T + len(short)
     host = torch.empty(max(n_int, 1), dtype=torch.int32, pin_memory=torch.device(device).type == "cuda")
     buf = host.numpy()
     off = 0
@@ -109,6 +130,7 @@ def build_step_batch(entries: Sequence[StepEntry], ctx_lens: Sequence[int], stat
         o_bt.append(o)
     o_sm = [put(np.concatenate([np.asarray(slot_maps[r][g], dtype=np.int64) for r in range(R)]) if R else [], T)
             for g in range(n_groups)]
+    o_short = put(short, len(short))
     if static is not None:
         assert static.numel() >= n_int
         static[:n_int].copy_(host[:n_int], non_blocking=True)
@@ -126,4 +148,5 @@ def build_step_batch(entries: Sequence[StepEntry], ctx_lens: Sequence[int], stat
         block_tables=[view(o_bt[g], R * widths[g]).view(R, widths[g]) for g in range(n_groups)],
         slot_maps=[view(o_sm[g], T) for g in range(n_groups)],
         h_q_start=q_start, h_q_len=q_len, h_ctx_len=list(ctx_lens), h_state_slot=list(state_slots),
+        short_list=view(o_short, len(short)) if len(short) else None,
         max_pos=(int(pos.max()) if T else 0) if max_pos is None else max_pos, max_q_len=max(q_len) if q_len else 0)

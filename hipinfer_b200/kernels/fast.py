@@ -25,7 +25,7 @@ _SIGS = {
     "hb_gemm_stream_finish": [_p, _p, _l, _i, _i, _i, _i, _p],
     "hb_add_rmsnorm_slices": [_p, _l, _p, _i, _l, _l, _p, _p, _p, _i, _i, _f, _p],
     "hb_rope_kv_slices": [_p, _i, _l, _l, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _p],
-    "hb_attn_decode": [_p, _p, _p, _l, _p, _i, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _f, _i, _i, _p, _i, _p, _p, _p, _p, _p, _p],
+    "hb_attn_decode": [_p, _p, _p, _l, _p, _i, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _f, _i, _i, _p, _i, _p, _p, _p, _p, _p, _p, _p],
     "hb_flash_prefill": [_p, _p, _p, _p, _i, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f, _i, _p],
     "hb_flash_prefill_supported": [_i, _i, _i],
     "hb_flash_prefill_tc": [_p, _p, _p, _l, _p, _i, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _p, _p, _p, _p, _p],
@@ -468,17 +468,18 @@ def _decode_counters(device, n):
 
 def attention_decode(q, k_cache, v_cache, block_table, row_request, positions, out, n_heads, n_kv_heads, head_dim,
                      page_size, window, scale, max_pos, chunk=None, q_len=None, row_limit=0, ctx_len=None, distance=None,
-                     sink=None):
+                     sink=None, row_list=None):
     """The bf16 row-attention kernel itself (see csrc/attention_fast.cu); rows whose keys span several
     chunks are finished inside it. With q_len (int32 per request) rows of requests with row_limit
     rows or more are skipped. row_request None: row t is the only row of request t (a decode-only
     step). ctx_len (int32 per request): the tokens in the cache before this
     step; with it the kernel asks for their keys before the kernel ahead of it has ended, so
-    positions, tables and ctx_len must then be in place before that kernel starts. distance (an ops.DistanceBias) and sink
+    positions, tables and ctx_len must then be in place before that kernel starts. row_list (int32, in place as early): only these
+    rows are computed, the others' places in out are left alone. distance (an ops.DistanceBias) and sink
     (float32 [n_heads]) as in ops.attention_masked."""
     from . import ops
 
-    T = q.shape[0]
+    T = q.shape[0] if row_list is None else row_list.numel()
     chunk = chunk or decode_chunk(head_dim, int(window))
     ws = ops.attention_workspace(T, n_heads, head_dim, max_pos, chunk, q.device)
     cnt = None if ws is None else _decode_counters(q.device, T * n_kv_heads)
@@ -487,7 +488,7 @@ def attention_decode(q, k_cache, v_cache, block_table, row_request, positions, o
           None if ws is None else ws.data_ptr(), None if cnt is None else cnt.data_ptr(), T, n_heads, n_kv_heads,
           head_dim, page_size, int(window), float(scale), chunk, int(max_pos),
           None if q_len is None else q_len.data_ptr(), int(row_limit), None if ctx_len is None else ctx_len.data_ptr(),
-          status_word().data_ptr(), *_extras(distance, sink), _stream())
+          status_word().data_ptr(), *_extras(distance, sink), None if row_list is None else row_list.data_ptr(), _stream())
     return out
 
 
@@ -603,8 +604,11 @@ def attention(q, k_cache, v_cache, batch, group, out, n_heads, n_kv_heads, head_
     if need_rows:
         # a step of single decode rows: row t is request t, which the kernel need not look up
         rows_are_requests = batch.max_q_len == 1 and batch.n_rows == batch.n_requests
+        # beside a portion for the flash kernel: a grid over the few other rows alone, and the chunks of the longest of them
+        listed = use_flash and hasattr(batch, "short_rows")
+        rows, max_pos = batch.short_rows(FLASH_MIN_ROWS) if listed else (None, batch.max_pos)
         attention_decode(q, k_cache, v_cache, bt, None if rows_are_requests else batch.row_request, batch.positions, out, n_heads, n_kv_heads,
-                         head_dim, page_size, window, scale, batch.max_pos,
-                         q_len=batch.req_q_len if use_flash else None, row_limit=FLASH_MIN_ROWS,
-                         ctx_len=batch.req_ctx_len, distance=distance, sink=sink)
+                         head_dim, page_size, window, scale, max_pos,
+                         q_len=batch.req_q_len if use_flash and not listed else None, row_limit=FLASH_MIN_ROWS,
+                         ctx_len=batch.req_ctx_len, distance=distance, sink=sink, row_list=rows)
     return True

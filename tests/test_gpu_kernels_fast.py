@@ -290,6 +290,35 @@ def test_attention_decode_few_and_many_rows_give_the_same_bits(D):
     torch.testing.assert_close(many[t:t + 1].float().cpu().reshape(1, Hq, D), ref, rtol=1e-2, atol=1e-2)
 
 
+@pytest.mark.parametrize("D,lens,most", [(64, [1500, 40, 2300], 0), (128, [700, 300, 33], 1), (64, [100, 513, 64], 8)])
+def test_attention_decode_of_listed_rows(D, lens, most):
+    """A grid over a list of the step's rows gives the bits of the grid over all of them, and leaves the other rows' places
+    alone (`most`: rows up to which the chunks of a row are one cluster; the list has 4 rows, the step 12)."""
+    Hq, Hkv, ps = 8, 2, 16
+    kc, vc, bt, ks, vs = _paged_setup(lens, Hkv, D, ps, torch.bfloat16, 73)
+    rows = [(r, p) for r, n in enumerate(lens) for p in range(n - 4, n)]
+    q = rnd(len(rows), Hq * D, seed=74)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    args = (kc, vc, bt, i32([r for r, _ in rows]), i32([p for _, p in rows]))
+    every = torch.empty(len(rows), Hq * D, dtype=torch.bfloat16, device=DEV)
+    fast().attention_decode(q, *args, every, Hq, Hkv, D, ps, 0, 1 / math.sqrt(D), max(lens) - 1, ctx_len=i32([n - 4 for n in lens]))
+    from hipinfer_b200.kernels import library
+
+    pick = [11, 0, 7, 4]
+    some = torch.full_like(every, 5.0)
+    library.load("fast").hb_attn_decode_set_cluster_rows(most)
+    try:
+        for _ in range(2):      # twice: the counters are left at zero
+            fast().attention_decode(q, *args, some, Hq, Hkv, D, ps, 0, 1 / math.sqrt(D), max(rows[i][1] for i in pick),
+                                    ctx_len=i32([n - 4 for n in lens]), row_list=i32(pick))
+    finally:
+        library.load("fast").hb_attn_decode_set_cluster_rows(8)
+    sync_check()
+    assert torch.equal(some[pick], every[pick])
+    rest = [i for i in range(len(rows)) if i not in pick]
+    assert bool((some[rest] == 5.0).all())
+
+
 def test_attention_decode_rows_that_are_requests():
     """A decode-only step: row t is request t, which the kernel then does not look up: the same bits."""
     Hq, Hkv, D, ps = 8, 2, 64, 16
