@@ -333,108 +333,6 @@ HB_EXPORT int hb_bias_act(const float* x, long ldx, const void* bias, int bias_d
 }
 
 // ---------------------------------------------------------------------------------------
-// Plain matrix product C[M,N] = A[M,K] W[N,K]^T, W row-major with K contiguous as the
-// reference stores weights (src/api.cu:81-83). 64x64 tile, 16 deep, 4x4 outputs per thread,
-// one FFMA chain per output running k = 0..K-1 in order: an output's value does not depend on
-// M, on the tile it lies in, or on anything else in the batch.
-// EPI 0: C = acc;  EPI 1: C += acc (32-bit C: the residual stream);  EPI 2: C += colscale[n] * acc (the same with
-// a scale vector over the output columns, 32-bit or the weight's element type).
-// ---------------------------------------------------------------------------------------
-template <typename TA, typename TW, typename TC, int EPI>
-__global__ void __launch_bounds__(256) gemm_simt_kernel(const TA* __restrict__ A, long lda, const TW* __restrict__ W,
-                                                        long ldw, TC* __restrict__ C, long ldc, int M, int N, int K,
-                                                        const TW* __restrict__ colscale = nullptr) {
-  __shared__ float As[16][68], Ws[16][68];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int m_blk = blockIdx.y * 64, n_blk = blockIdx.x * 64;
-  const int lr = tid >> 2, lk = (tid & 3) * 4;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += 16) {
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int k = k0 + lk + i;
-      As[lk + i][lr] = (m_blk + lr < M && k < K) ? hb_to_float(A[(size_t)(m_blk + lr) * lda + k]) : 0.f;
-      Ws[lk + i][lr] = (n_blk + lr < N && k < K) ? hb_to_float(W[(size_t)(n_blk + lr) * ldw + k]) : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 16; k++) {
-      float a[4], w[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) { a[i] = As[k][ty * 4 + i]; w[i] = Ws[k][tx * 4 + i]; }
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int m = m_blk + ty * 4 + i;
-    if (m >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int n = n_blk + tx * 4 + j;
-      if (n >= N) continue;
-      TC* c = C + (size_t)m * ldc + n;
-      if (EPI == 2) *c = hb_from_float<TC>(__fadd_rn(hb_to_float(*c), __fmul_rn(hb_to_float(colscale[n]), acc[i][j])));
-      else if (EPI == 1) *c = hb_from_float<TC>(hb_to_float(*c) + acc[i][j]);
-      else *c = hb_from_float<TC>(acc[i][j]);
-    }
-  }
-}
-
-template <typename TA, typename TW>
-static int gemm_simt_launch(const void* A, long lda, const void* W, long ldw, void* C, int c_dt, long ldc, int M, int N,
-                            int K, int epi, cudaStream_t s, const void* colscale = nullptr) {
-  dim3 grid((N + 63) / 64, (M + 63) / 64);
-  if (epi == 2) {
-    if (c_dt != HB_F32 || !colscale) HB_FAIL("hb_gemm_simt: the scaled sum needs a 32-bit C and a scale vector");
-    gemm_simt_kernel<TA, TW, float, 2><<<grid, 256, 0, s>>>((const TA*)A, lda, (const TW*)W, ldw, (float*)C, ldc, M, N, K,
-                                                            (const TW*)colscale);
-  } else if (epi == 1) {
-    if (c_dt != HB_F32) HB_FAIL("hb_gemm_simt: accumulating into C needs a 32-bit C");
-    gemm_simt_kernel<TA, TW, float, 1><<<grid, 256, 0, s>>>((const TA*)A, lda, (const TW*)W, ldw, (float*)C, ldc, M, N, K);
-  } else if (c_dt == HB_F32) {
-    gemm_simt_kernel<TA, TW, float, 0><<<grid, 256, 0, s>>>((const TA*)A, lda, (const TW*)W, ldw, (float*)C, ldc, M, N, K);
-  } else if (c_dt == HB_BF16) {
-    gemm_simt_kernel<TA, TW, __nv_bfloat16, 0><<<grid, 256, 0, s>>>((const TA*)A, lda, (const TW*)W, ldw,
-                                                                    (__nv_bfloat16*)C, ldc, M, N, K);
-  } else {
-    HB_FAIL("hb_gemm_simt: unknown C dtype code %d", c_dt);
-  }
-  return 0;
-}
-
-// colscale (epilogue 2 only): N values of the weight's element type.
-HB_EXPORT int hb_gemm_simt_scaled(const void* A, int a_dt, long lda, const void* W, int w_dt, long ldw, float* C, long ldc,
-                                  int M, int N, int K, const void* colscale, cudaStream_t s) {
-  if (M <= 0 || N <= 0) return 0;
-  if (K <= 0) HB_FAIL("hb_gemm_simt_scaled: K must be positive");
-  if ((M + 63) / 64 > 65535) HB_FAIL("hb_gemm_simt_scaled: M = %d is beyond the grid limit", M);
-  int r = -1;
-  HB_DISPATCH_2(a_dt, w_dt, "hb_gemm_simt_scaled",
-                (r = gemm_simt_launch<TA, TB>(A, lda, W, ldw, C, HB_F32, ldc, M, N, K, 2, s, colscale)));
-  if (r) return r;
-  HB_CHECK_LAUNCH("hb_gemm_simt_scaled");
-  return 0;
-}
-
-HB_EXPORT int hb_gemm_simt(const void* A, int a_dt, long lda, const void* W, int w_dt, long ldw, void* C, int c_dt,
-                           long ldc, int M, int N, int K, int epi, cudaStream_t s) {
-  if (M <= 0 || N <= 0) return 0;
-  if (K <= 0) HB_FAIL("hb_gemm_simt: K must be positive");
-  if (epi != 0 && epi != 1) HB_FAIL("hb_gemm_simt: unknown epilogue %d", epi);
-  if ((M + 63) / 64 > 65535) HB_FAIL("hb_gemm_simt: M = %d is beyond the grid limit", M);
-  int r = -1;
-  HB_DISPATCH_2(a_dt, w_dt, "hb_gemm_simt", (r = gemm_simt_launch<TA, TB>(A, lda, W, ldw, C, c_dt, ldc, M, N, K, epi, s)));
-  if (r) return r;
-  HB_CHECK_LAUNCH("hb_gemm_simt");
-  return 0;
-}
-
-// ---------------------------------------------------------------------------------------
 // SwiGLU over a gate/up matrix whose columns are interleaved in groups of `grp`
 // (grp gate columns, grp up columns, ...): act[m, i] = silu(g) * u, silu(g) = g / (1 + e^-g).
 // kind 1: the tanh form of GELU instead of silu, 0.5 g (1 + tanh(sqrt(2/pi) (g + 0.044715 g^3))).
@@ -893,6 +791,132 @@ __global__ void __launch_bounds__(128) attn_rows_kernel(
   }
 }
 
+// The same for heads of at most 128 dimensions (a multiple of 4) in groups of at most GM, with the loads of a key shared by
+// its group: LPK lanes (a power of two) hold a key's dimensions four each, so that a warp's access covers whole rows of the
+// cache, and a key or value element is loaded once for all G heads instead of once a head. A score is the lanes' chains of four
+// added by a butterfly; the values are summed by 128 / LPK groups of threads that take every (128 / LPK)-th key, added group 0
+// first. Both orders depend on the position alone. (No __restrict__ on what the kernel ahead wrote: see gemm_simt.cu.) Bound by the latency of a block's passes over its chunk and, for prompts, by
+// L2 (every row reads its keys again).
+template <typename TQ, typename TC, int GM, int LPK>
+__global__ void __launch_bounds__(128) attn_rows_vec_kernel(
+    const TQ* q, const TC* kc, const TC* vc, const int* __restrict__ bt,
+    int bt_stride, const int* __restrict__ row_req, const int* __restrict__ pos, TQ* out,
+    float* part_acc, float* part_ml, int Hq, int Hkv, int D, int page_size, int window,
+    float scale, int chunk, int S) {
+  constexpr int GROUPS = 128 / LPK, U = 4;      // U: keys of a thread whose loads are in flight together
+  extern __shared__ float smem[];
+  hb_pdl_launch();
+  hb_pdl_wait();
+  const int t = blockIdx.z, h = blockIdx.y, s = blockIdx.x, G = Hq / Hkv;
+  const int p = pos[t];
+  const int lo = window > 0 ? max(0, p - window + 1) : 0;
+  const int s_lo = lo / chunk, s_hi = p / chunk;
+  if (s < s_lo || s > s_hi) return;
+  const int k0 = max(s * chunk, lo), k1 = min((s + 1) * chunk, p + 1), nk = k1 - k0;
+  float* sc = smem;                                // [G][chunk]
+  int* rows = (int*)(sc + G * chunk);              // [chunk] cache row of each key (in rows of D elements of kv head h)
+  float* ml = (float*)(rows + chunk);              // [G][2]
+  float* red = ml + 16;                            // [GROUPS][G][LPK * 4], 16-byte aligned (chunk is a multiple of 32)
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = tid % LPK, grp = tid / LPK, d = sub * 4;
+  const int* table = bt + (size_t)row_req[t] * bt_stride;
+  for (int j = tid; j < nk; j += 128) {
+    const int kp = k0 + j;
+    rows[j] = (table[kp / page_size] * Hkv + h) * page_size + kp % page_size;
+  }
+  float4 qv[GM];
+#pragma unroll
+  for (int g = 0; g < GM; g++) {
+    qv[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (g < G && d < D) {
+      qv[g] = hb_load4(q + ((size_t)t * Hq + (size_t)h * G + g) * D + d);
+      qv[g].x *= scale; qv[g].y *= scale; qv[g].z *= scale; qv[g].w *= scale;
+    }
+  }
+  __syncthreads();
+  for (int j0 = 0; j0 < nk; j0 += GROUPS * U) {    // every lane of a warp takes part in the butterflies
+    float4 kv[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int j = j0 + u * GROUPS + grp;
+      kv[u] = j < nk && d < D ? hb_load4(kc + (size_t)rows[j] * D + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int j = j0 + u * GROUPS + grp;
+#pragma unroll
+      for (int g = 0; g < GM; g++) {
+        if (g < G) {
+          float a = fmaf(qv[g].w, kv[u].w, fmaf(qv[g].z, kv[u].z, fmaf(qv[g].y, kv[u].y, qv[g].x * kv[u].x)));
+#pragma unroll
+          for (int o = LPK / 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+          if (sub == 0 && j < nk) sc[g * chunk + j] = a;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  for (int g = warp; g < G; g += 4) {
+    float m = -INFINITY;
+    for (int j = lane; j < nk; j += 32) m = fmaxf(m, sc[g * chunk + j]);
+    m = hb_warp_max(m);
+    float l = 0.f;
+    for (int j = lane; j < nk; j += 32) {
+      const float e = expf(sc[g * chunk + j] - m);
+      sc[g * chunk + j] = e;
+      l += e;
+    }
+    l = hb_warp_sum(l);
+    if (lane == 0) { ml[2 * g] = m; ml[2 * g + 1] = l; }
+  }
+  __syncthreads();
+  float4 acc[GM];
+#pragma unroll
+  for (int g = 0; g < GM; g++) acc[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (d < D) {
+    for (int j0 = grp; j0 < nk; j0 += GROUPS * U) {
+      float4 vv[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int j = j0 + u * GROUPS;
+        if (j < nk) vv[u] = hb_load4(vc + (size_t)rows[j] * D + d);
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int j = j0 + u * GROUPS;
+        if (j < nk) {
+#pragma unroll
+          for (int g = 0; g < GM; g++) {
+            if (g < G) {
+              const float w = sc[g * chunk + j];
+              acc[g].x = fmaf(w, vv[u].x, acc[g].x); acc[g].y = fmaf(w, vv[u].y, acc[g].y);
+              acc[g].z = fmaf(w, vv[u].z, acc[g].z); acc[g].w = fmaf(w, vv[u].w, acc[g].w);
+            }
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int g = 0; g < GM; g++)
+      if (g < G) *(float4*)(red + ((size_t)grp * G + g) * (LPK * 4) + d) = acc[g];
+  }
+  __syncthreads();
+  const bool whole = s_lo == s_hi;
+  for (int i = tid; i < G * D; i += 128) {
+    const int g = i / D, dd = i - g * D;
+    float a = 0.f;
+#pragma unroll
+    for (int r = 0; r < GROUPS; r++) a += red[((size_t)r * G + g) * (LPK * 4) + dd];
+    const size_t head = (size_t)t * Hq + (size_t)h * G + g;
+    if (whole) out[head * D + dd] = hb_from_float<TQ>(a / ml[2 * g + 1]);
+    else part_acc[(head * S + s) * D + dd] = a;
+  }
+  if (!whole && tid < G) {
+    const size_t head = (size_t)t * Hq + (size_t)h * G + tid;
+    part_ml[(head * S + s) * 2] = ml[2 * tid];
+    part_ml[(head * S + s) * 2 + 1] = ml[2 * tid + 1];
+  }
+}
+
 template <typename TQ>
 __global__ void attn_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
                                   const int* __restrict__ pos, TQ* __restrict__ out, int Hq, int D, int window, int chunk,
@@ -939,6 +963,41 @@ HB_EXPORT int hb_attn_rows(const void* q, int q_dt, const void* kc, const void* 
   float* part_acc = workspace;
   float* part_ml = workspace ? workspace + (size_t)T * Hq * S * D : nullptr;
   dim3 grid(S, Hkv, T);
+  // the row numbers of the vector kernel are 32-bit: a cache of 2^31 rows of a head has 64 GB a layer even at head_dim 16
+  const bool vec = (D & 3) == 0 && D <= 128 && G <= 8 && !(((uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc) & 15);
+  const size_t smem_v = ((size_t)G * chunk + chunk + 16 + (size_t)512 * G) * sizeof(float);
+  if (vec && smem_v <= 200 * 1024) {
+    cudaError_t e = cudaSuccess;
+#define HB_AR_RUN(GM, LPK)                                                                                                       \
+  do {                                                                                                                           \
+    auto kern = attn_rows_vec_kernel<TA, TA, GM, LPK>;                                                                           \
+    if (smem_v > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(200 * 1024));      \
+    if (e == cudaSuccess)                                                                                                        \
+      e = hb_launch(kern, grid, 128, smem_v, s, (const TA*)q, (const TA*)kc, (const TA*)vc, bt, bt_stride, row_req, pos, (TA*)out, \
+                    part_acc, part_ml, Hq, Hkv, D, page_size, window, scale, chunk, S);                                          \
+  } while (0)
+#define HB_AR_LPK(GM)                      \
+  do {                                     \
+    if (D <= 16) HB_AR_RUN(GM, 4);         \
+    else if (D <= 32) HB_AR_RUN(GM, 8);    \
+    else if (D <= 64) HB_AR_RUN(GM, 16);   \
+    else HB_AR_RUN(GM, 32);                \
+  } while (0)
+    HB_DISPATCH_1(q_dt, "hb_attn_rows", {
+      if (G == 1) HB_AR_LPK(1);
+      else if (G == 2) HB_AR_LPK(2);
+      else if (G <= 4) HB_AR_LPK(4);
+      else HB_AR_LPK(8);
+      if (e != cudaSuccess) HB_FAIL("hb_attn_rows: %s", cudaGetErrorString(e));
+      if (S > 1)
+        hb_launch(attn_merge_kernel<TA>, dim3(Hq, T), 64, 0, s, (const float*)part_acc, (const float*)part_ml, pos, (TA*)out, Hq, D, window,
+                  chunk, S, (const int*)nullptr, (const int*)nullptr, 0);
+    });
+#undef HB_AR_LPK
+#undef HB_AR_RUN
+    HB_CHECK_LAUNCH("hb_attn_rows");
+    return 0;
+  }
   HB_DISPATCH_1(q_dt, "hb_attn_rows", {
     auto kern = attn_rows_kernel<TA, TA>;
     if (smem > 48 * 1024) {

@@ -23,7 +23,7 @@ _SIGS = {
     "core": {
         "hb_embed": [_p, _i, _p, _p, _i, _i, _p],
         "hb_rmsnorm": [_p, _p, _i, _p, _i, _p, _i, _i, _f, _p],
-        "hb_gemm_simt": [_p, _i, _l, _p, _i, _l, _p, _i, _l, _i, _i, _i, _i, _p],
+        "hb_gemm_simt": [_p, _i, _l, _p, _i, _l, _p, _i, _l, _i, _i, _i, _i, _p, _p],
         "hb_swiglu": [_p, _i, _l, _p, _i, _l, _i, _i, _i, _p],
         "hb_rope_table": [_p, _p, _i, _i, C.c_double, _p],
         "hb_rope_kv": [_p, _i, _l, _p, _p, _p, _p, _i, _p, _p, _i, _i, _i, _i, _i, _i, _i, _p],
@@ -43,7 +43,7 @@ _SIGS = {
         "hb_scale_add": [_p, _p, _l, _p, _i, _i, _i, _p],
         "hb_bias_act": [_p, _l, _p, _i, _p, _i, _l, _i, _i, _i, _p],
         "hb_qkv_bias_store": [_p, _l, _p, _p, _p, _i, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _p],
-        "hb_gemm_simt_scaled": [_p, _i, _l, _p, _i, _l, _p, _l, _i, _i, _i, _p, _p],
+        "hb_gemm_simt_scaled": [_p, _i, _l, _p, _i, _l, _p, _l, _i, _i, _i, _p, _p, _p],
     },
     "seqmix": {
         "hb_attn_masked": [_p, _i, _l, _p, _l, _p, _l, _i, _p, _i, _p, _p, _p, _p, _l, _i, _i, _p, _i, _l, _i, _i, _i, _i, _i,
@@ -446,8 +446,20 @@ def gemm_plain(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: 
     N = w.shape[0]
     assert w.shape[1] == K and out.shape == (M, N), (a.shape, w.shape, out.shape)
     _call("core", "hb_gemm_simt", a.data_ptr(), _dt(a), a.stride(0), w.data_ptr(), _dt(w), w.stride(0),
-          out.data_ptr(), _dt(out), out.stride(0), M, N, K, 1 if accumulate else 0, _stream())
+          out.data_ptr(), _dt(out), out.stride(0), M, N, K, 1 if accumulate else 0, _ptr(_simt_workspace(M, N, K, out.device)), _stream())
     return out
+
+
+def _simt_workspace(M, N, K, device):
+    """The partial sums of a plain product whose K is split over blocks (None: it is not)."""
+    if M <= 8:          # a few rows never need one (csrc/gemm_simt.cu: SR_ROWS); where their sizes refuse that kernel, unsplit
+        return None
+    lib = library.load("core")
+    lib.hb_gemm_simt_workspace.restype = C.c_long
+    n = lib.hb_gemm_simt_workspace(M, N, K)
+    if n:
+        library.launches[0] += 1     # the kernel that adds the slices
+    return torch.empty(n, dtype=torch.float32, device=device) if n else None
 
 
 def swiglu(gate_up: torch.Tensor, out: torch.Tensor, group: int) -> torch.Tensor:
@@ -686,7 +698,7 @@ def linear_scaled_add(a: torch.Tensor, w: Weight, x: torch.Tensor, scale: torch.
         gemm_plain(a, w.t, y)
         return scale_add(x, y, scale)
     _call("core", "hb_gemm_simt_scaled", a.data_ptr(), _dt(a), a.stride(0), w.t.data_ptr(), _dt(w.t), w.t.stride(0),
-          x.data_ptr(), x.stride(0), M, N, a.shape[1], scale.data_ptr(), _stream())
+          x.data_ptr(), x.stride(0), M, N, a.shape[1], scale.data_ptr(), _ptr(_simt_workspace(M, N, a.shape[1], x.device)), _stream())
     return x
 
 

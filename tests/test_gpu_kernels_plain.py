@@ -1,6 +1,7 @@
 """Each plain kernel alone beside a plain PyTorch float32 statement of the same operation, at
 sizes other than the engine's: widths that are no power of two, odd row counts, head sizes in
 steps of 16, groups of 1, 3, 5."""
+import ctypes
 import math
 
 import pytest
@@ -78,6 +79,40 @@ def test_gemm_plain_row_does_not_depend_on_batch():
         one = torch.empty(1, 90, device=DEV)
         ops().gemm_plain(a[r:r + 1].contiguous(), w, one)
         assert torch.equal(one[0], full[r])
+
+
+@pytest.mark.parametrize("adt,wdt", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32)])
+@pytest.mark.parametrize("N,K", [(40, 512), (129, 520), (2048, 2048), (17, 8192), (33, 1030), (70000, 1024)])
+def test_gemm_plain_slices(adt, wdt, N, K):
+    """K in one to eight slices, through the kernel of a few rows (the sizes it takes), the tiles with the slices in blocks of
+    their own and the tiles that walk them all: against 64 bits, and the same bits for a row whatever kernel ran. The bound is
+    that of chains of K / slices products and a sum of the slices: (depth + 8) 2^-24 sum |a w|, and the result's rounding."""
+    from hipinfer_b200.kernels import library
+
+    M = 70
+    a, w = rnd(M, K, dtype=adt, seed=31), rnd(N, K, dtype=wdt, seed=32, scale=0.1)
+    ad, wd = a.double(), w.double()
+    bound = (max(512, -(-K // 8)) + 64 + 8) * 2.0 ** -24 * (ad.abs() @ wd.abs().T)
+    full = torch.full((M + 1, N), 7.0, device=DEV)
+    ops().gemm_plain(a, w, full[:M])
+    assert bool(((full[:M].double() - ad @ wd.T).abs() <= bound).all()) and bool((full[M] == 7.0).all())
+    for rows in ([0], [5, 69, 64], list(range(8)), list(range(60, 69))):
+        few = torch.empty(len(rows), N, device=DEV)
+        ops().gemm_plain(a[rows].contiguous(), w, few)
+        assert torch.equal(few, full[rows]), rows
+    # without a workspace the same product is not split over blocks
+    whole = torch.empty(M, N, device=DEV)
+    dt = {torch.float32: 0, torch.bfloat16: 1}
+    assert library.load("core").hb_gemm_simt(*[ctypes.c_void_p(a.data_ptr()), dt[adt], ctypes.c_long(K), ctypes.c_void_p(w.data_ptr()), dt[wdt],
+                                               ctypes.c_long(K), ctypes.c_void_p(whole.data_ptr()), 0, ctypes.c_long(N), M, N, K, 0, None,
+                                               ctypes.c_void_p(library.current_stream())]) == 0
+    assert torch.equal(whole, full[:M])
+    acc = rnd(M, N, seed=33)
+    want = acc + full[:M]
+    few = acc[3:6].clone()
+    ops().gemm_plain(a, w, acc, accumulate=True)
+    ops().gemm_plain(a[3:6].contiguous(), w, few, accumulate=True)
+    assert torch.equal(acc, want) and torch.equal(few, want[3:6])
 
 
 @pytest.mark.parametrize("idt", DT)
