@@ -24,14 +24,18 @@ enum { ST_F32 = 0, ST_BF16 = 1, ST_ADD_F32 = 2, ST_SWIGLU_BF16 = 3, ST_SLICES = 
 #define ST_IS_GLU(e) ((e) == ST_SWIGLU_BF16 || (e) == ST_GEGLU_BF16)
 constexpr int ST_ROWS = 128, ST_BK = 64, ST_W_BYTES = ST_ROWS * ST_BK * 2;
 
-// DEEP: the pipeline of a product that is not split along K (many column blocks): six stages,
-// two CTAs per SM; otherwise four (three for 64 tokens) and three CTAs per SM.
+// The stages of a product split along K: as many as let three CTAs lie on an SM, which the split is made for (with four
+// of 20 KB for 32 tokens only two did, and a product ran in two rounds: 20 rows of the 8B layer sizes took 19.2 us a product,
+// 10.6 us with three). DEEP: six stages and two CTAs per SM, for the unsplit products of up to 16 tokens (at one token the
+// persistent kernel below is slower: 88 us against 81 for a head of 128,256 x 2,048; its blocks are dealt out beforehand, these
+// as SMs come free).
 template <int NT, bool DEEP> struct StreamCfg {
   static constexpr int STAGE = ST_W_BYTES + NT * ST_BK * 2;
-  static constexpr int STAGES = DEEP ? (NT <= 32 ? 6 : 4) : (NT <= 32 ? 4 : 3);
+  static constexpr int STAGES = DEEP ? 6 : NT <= 16 ? 4 : 3;
   static constexpr int BAR = STAGES * STAGE;
   static constexpr int TOTAL = BAR + 256 + 1024;
   static constexpr int TMEM_COLS = NT < 32 ? 32 : NT;
+  static_assert((DEEP ? 2 : 3) * (TOTAL + 1024) <= 228 * 1024, "the CTAs an SM that the stages are chosen for");
 };
 
 __device__ __forceinline__ void stream_store(int epi, void* C, long ldc, int m, int n, int N, float v, float v_up, bool lower_half) {
@@ -205,6 +209,132 @@ __global__ void __launch_bounds__(192) gemm_stream_kernel(const __grid_constant_
   if (threadIdx.x == 0) counters[nb] = 0;
 }
 
+// A product of so many column blocks that K is not split (a head, a wide gate/up): one persistent CTA an SM walks the blocks
+// b, b + gridDim.x, .. . Its ring of weight tiles runs on from one block to the next, and the accumulator is double-buffered in
+// tensor memory, so neither the start of a block nor its write-back (64 tokens: 32 KB in pieces of 128 bytes) leaves HBM idle; one
+// CTA a block, two or fewer an SM at a time, paid for both at each of them. Every weight byte is read once, the few activation
+// rows once a block from L2. Measured inside decode steps:
+// 28,672 x 4,096 and 128,256 x 4,096 at 20 tokens 86 -> 58 us a product on average, 128,256 x 2,048 at 64 280 -> 116 us.
+template <int NT> struct PersistCfg {
+  static constexpr int STAGE = ST_W_BYTES + NT * ST_BK * 2;
+  static constexpr int STAGES = NT == 32 ? 10 : 8;      // 205 and 197 KB
+  static constexpr int BAR = STAGES * STAGE;
+  static constexpr int TOTAL = BAR + 512 + 1024;
+  static constexpr int TMEM_COLS = 2 * NT;
+};
+
+template <int NT>
+__global__ void __launch_bounds__(192, 1) gemm_stream_persist_kernel(const __grid_constant__ CUtensorMap map_w,
+                                                                     const __grid_constant__ CUtensorMap map_x, void* C, long ldc,
+                                                                     int M, int N, int K, int epi, int* status) {
+  using S = PersistCfg<NT>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t* full = (uint64_t*)(smem + S::BAR);
+  uint64_t* empty = full + S::STAGES;
+  uint64_t* tmem_full = empty + S::STAGES;
+  uint64_t* tmem_empty = tmem_full + 2;
+  uint32_t* tmem_slot = (uint32_t*)(tmem_empty + 2);
+  volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+
+  hb_pdl_launch();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n_blocks = (N + ST_ROWS - 1) / ST_ROWS, num_kb = (K + ST_BK - 1) / ST_BK;
+  const int mine = (n_blocks - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x, total = mine * num_kb;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S::STAGES; s++) { hb_mbar_init(&full[s], 1); hb_mbar_init(&empty[s], 1); }
+    for (int b = 0; b < 2; b++) { hb_mbar_init(&tmem_full[b], 1); hb_mbar_init(&tmem_empty[b], 4); }
+    *abort_flag = 0;
+    hb_fence_barrier_init();
+  }
+  if (warp == 5) {
+    hb_tmem_alloc(tmem_slot, S::TMEM_COLS);
+    hb_tmem_relinquish();
+  }
+  if (warp == 4 && lane == 0) { hb_tma_prefetch_desc(&map_w); hb_tma_prefetch_desc(&map_x); }
+  hb_tc_fence_before();
+  __syncthreads();
+  hb_tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 4) {
+    if (lane == 0) {  // ---------------- TMA producer; the ring's first weight tiles do not wait for the kernel ahead
+      const int pre = total < S::STAGES ? total : S::STAGES;
+      for (int it = 0; it < pre; it++) {
+        hb_mbar_expect_tx(&full[it], S::STAGE);
+        hb_tma_load_2d(smem + it * S::STAGE, &map_w, &full[it], it % num_kb * ST_BK, (int)(blockIdx.x + it / num_kb * gridDim.x) * ST_ROWS);
+      }
+      hb_pdl_wait();
+      for (int it = 0; it < pre; it++)
+        hb_tma_load_2d(smem + it * S::STAGE + ST_W_BYTES, &map_x, &full[it], it % num_kb * ST_BK, 0);
+      int kb = pre % num_kb, nb = blockIdx.x + pre / num_kb * gridDim.x;
+      for (int it = pre; it < total; it++) {
+        const uint32_t s = it % S::STAGES, ph = (it / S::STAGES) & 1;
+        if (!hb_mbar_wait(&empty[s], ph ^ 1, abort_flag)) break;
+        hb_mbar_expect_tx(&full[s], S::STAGE);
+        hb_tma_load_2d(smem + s * S::STAGE, &map_w, &full[s], kb * ST_BK, nb * ST_ROWS);
+        hb_tma_load_2d(smem + s * S::STAGE + ST_W_BYTES, &map_x, &full[s], kb * ST_BK, 0);
+        if (++kb == num_kb) { kb = 0; nb += gridDim.x; }
+      }
+    }
+  } else if (warp == 5) {
+    if (lane == 0) {  // ---------------- MMA issuer
+      constexpr uint32_t idesc = hb_umma_idesc_bf16(ST_ROWS, NT);
+      uint32_t it = 0;
+      bool ok = true;
+      for (int i = 0; i < mine && ok; i++) {
+        const uint32_t buf = i & 1, aph = (i >> 1) & 1;
+        if (!hb_mbar_wait(&tmem_empty[buf], aph ^ 1, abort_flag)) break;
+        hb_tc_fence_after();
+        for (int kb = 0; kb < num_kb; kb++, it++) {
+          const uint32_t s = it % S::STAGES, ph = (it / S::STAGES) & 1;
+          if (!hb_mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
+          hb_tc_fence_after();
+          const uint64_t dw = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE));
+          const uint64_t dx = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE + ST_W_BYTES));
+#pragma unroll
+          for (int k = 0; k < ST_BK / 16; k++) hb_umma_bf16(tmem_base + buf * NT, dw + 2 * k, dx + 2 * k, idesc, (kb | k) != 0);
+          hb_umma_commit(&empty[s]);
+        }
+        if (ok) hb_umma_commit(&tmem_full[buf]);
+      }
+    }
+  } else {  // ---------------- epilogue warps: lane = output column, v[m] = token m
+    hb_pdl_wait();  // before the first access to memory that earlier kernels wrote or still read
+    for (int i = 0; i < mine; i++) {
+      const uint32_t buf = i & 1, aph = (i >> 1) & 1;
+      if (!hb_mbar_wait(&tmem_full[buf], aph, abort_flag)) break;
+      hb_tc_fence_after();
+      float v[NT];
+#pragma unroll
+      for (int c = 0; c < NT / 16; c++) hb_tmem_ld16(tmem_base + ((uint32_t)(warp * 32) << 16) + buf * NT + c * 16, v + 16 * c);
+      hb_tc_fence_before();
+      __syncwarp();
+      if (lane == 0) hb_mbar_arrive(&tmem_empty[buf]);
+      const int n = (int)(blockIdx.x + i * gridDim.x) * ST_ROWS + warp * 32 + lane;
+#pragma unroll
+      for (int m = 0; m < NT; m++) {
+        if (m < M) {
+          const float up = __shfl_down_sync(0xffffffffu, v[m], 16);
+          stream_store(epi, C, ldc, m, n, N, v[m], up, (lane & 16) == 0);
+        }
+      }
+    }
+  }
+
+  hb_tc_fence_before();
+  __syncthreads();
+  if (*abort_flag) {
+    if (threadIdx.x == 0) atomicExch(status, 1);
+    __nanosleep(100000);   // let copies that may still be in flight land before the shared memory is given up
+  }
+  if (warp == 5) {
+    __syncwarp();
+    hb_tmem_dealloc(tmem_base, S::TMEM_COLS);
+  }
+}
+
 // The slices' partial sums added in slice order and the epilogue applied, four columns per thread,
 // over the whole output at once. With many token rows this is much more work than one CTA per
 // column block should do at the end of the product kernel, so it runs as a kernel of its own.
@@ -276,6 +406,29 @@ HB_EXPORT int hb_gemm_stream_plan(int N, int K, int* kslice, int* ksplit, long* 
   return 0;
 }
 
+// K unsplit, more than 16 tokens: see gemm_stream_persist_kernel.
+template <int NT>
+static int launch_stream_whole(const CUtensorMap& mw, const CUtensorMap& mx, void* C, long ldc, int M, int N, int K, int n_blocks,
+                               int epi, int* status, cudaStream_t s) {
+  using S = PersistCfg<NT>;
+  auto kern = gemm_stream_persist_kernel<NT>;
+  static bool configured[64] = {};      // the attribute belongs to a device: set once on each
+  static int sms[64] = {};
+  int dev = 0, n_sm = 148;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !configured[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) HB_FAIL("hb_gemm_stream: %s", cudaGetErrorString(e));
+    if (dev >= 0 && dev < 64) { sms[dev] = n_sm; configured[dev] = true; }
+  } else {
+    n_sm = sms[dev];
+  }
+  cudaError_t e = hb_launch(kern, n_blocks < n_sm ? n_blocks : n_sm, 192, S::TOTAL, s, mw, mx, C, ldc, M, N, K, epi, status);
+  if (e != cudaSuccess) HB_FAIL("hb_gemm_stream: %s", cudaGetErrorString(e));
+  return 0;
+}
+
 template <int NT, bool DEEP>
 static int launch_stream(const CUtensorMap& mw, const CUtensorMap& mx, void* C, long ldc, int M, int N, int K, int kslice,
                          int ksplit, int n_blocks, float* ws, int* counters, int epi, int* status, cudaStream_t s) {
@@ -329,10 +482,10 @@ HB_EXPORT int hb_gemm_stream(const void* A, long lda, const void* W, long ldw, v
   if (hb_make_tensor_map_bf16(&mx, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, (uint32_t)NT)) return -1;
   int r;
 #define HB_ST_ARGS mw, mx, C, ldc, M, N, K, kslice, ksplit, n_blocks, ws, counters, epi, status, s
-  if (ksplit == 1) {
+  if (ksplit == 1 && epi != ST_SLICES) {
     if (NT == 16) r = launch_stream<16, true>(HB_ST_ARGS);
-    else if (NT == 32) r = launch_stream<32, true>(HB_ST_ARGS);
-    else r = launch_stream<64, true>(HB_ST_ARGS);
+    else if (NT == 32) r = launch_stream_whole<32>(mw, mx, C, ldc, M, N, K, n_blocks, epi, status, s);
+    else r = launch_stream_whole<64>(mw, mx, C, ldc, M, N, K, n_blocks, epi, status, s);
   } else {
     if (NT == 16) r = launch_stream<16, false>(HB_ST_ARGS);
     else if (NT == 32) r = launch_stream<32, false>(HB_ST_ARGS);
