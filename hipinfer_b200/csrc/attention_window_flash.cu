@@ -263,6 +263,8 @@ struct WinRowsArgs {
   float* part;           // [T][G][splits][2 maps][H/G][E + 2]
   int* arrived;          // [T][G], zero before and after
   int splits;
+  const int* row_list;   // the rows this call is for (indices in q, pos, row_req and out; part and arrived go by the place in the list), or null: all T
+  const int* ctx_len;    // per request, or null: tokens in the cache before this step; tiles wholly of those are read before the wait
 };
 
 template <int D, int E>
@@ -271,9 +273,12 @@ __global__ void __launch_bounds__(WF_THREADS, 3) attn_window_rows_mma_kernel(Win
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ int last;
   hb_pdl_launch();
-  hb_pdl_wait();
-  const int g_kv = blockIdx.x, row = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  if (A.q_len && A.q_len[A.row_req[row]] >= A.row_limit) return;
+  const int g_kv = blockIdx.x, rw = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int row = A.row_list ? A.row_list[rw] : rw, rq = A.row_req[row];
+  if (A.q_len && A.q_len[rq] >= A.row_limit) {
+    if ((blockIdx.x | blockIdx.y | blockIdx.z) == 0) hb_pdl_wait();     // the grid never ends before the one ahead of it
+    return;
+  }
   const int H = A.H, G = A.G, HG = H / G, window = A.window;
   const int p = A.pos[row];
   const int lo = window > 0 ? max(0, p - window + 1) : 0;
@@ -282,9 +287,9 @@ __global__ void __launch_bounds__(WF_THREADS, 3) attn_window_rows_mma_kernel(Win
   const int win0 = max(first_win_tile, last_keep_tile + 1), n_vis = (last_keep_tile + 1) + (last_tile - win0 + 1);
   const int n_splits = (n_vis + RM_SPLIT_TILES - 1) / RM_SPLIT_TILES;
   const int ord0 = blockIdx.z * RM_SPLIT_TILES, ord1 = min(n_vis, ord0 + RM_SPLIT_TILES);
-  if (ord0 >= n_vis) return;
+  if (ord0 >= n_vis) return;                       // (split 0 always has a tile)
   auto tile_of = [&](int ord) { return ord <= last_keep_tile ? ord : win0 + (ord - (last_keep_tile + 1)); };
-  const int* table = A.bt + (size_t)A.row_req[row] * A.bt_stride;
+  const int* table = A.bt + (size_t)rq * A.bt_stride;
   const uint32_t sQ = hb_smem_u32(smem), sK = sQ + 16 * QW * 2, sV = sK + RM_SPLIT_TILES * KTILE;
   int* rowoff = (int*)(smem + 16 * QW * 2 + RM_SPLIT_TILES * (KTILE + VTILE));      // [RM_SPLIT_TILES][64]: a key's row in the planes, -1: not visible
   const int n_tiles = ord1 - ord0;
@@ -295,19 +300,28 @@ __global__ void __launch_bounds__(WF_THREADS, 3) attn_window_rows_mma_kernel(Win
     const bool vis = kp <= p && (kp >= lo || kp < keep);
     rowoff[i] = vis ? (table[kp / A.page_size] * G + g_kv) * A.page_size + kp % A.page_size : -1;
   }
+  __syncthreads();
+  // ALL tiles of the split are asked for at once: their trips to memory overlap, the walk then waits once. Tiles of earlier steps'
+  // keys do not wait for the kernel ahead.
+  auto load_tile = [&](int s_) {
+    constexpr int CK = QW / 8, CA = QW / 8 + E / 8;
+    for (int i = tid; i < WF_BKV * CA; i += WF_THREADS) {
+      const int r = i / CA, c = i - r * CA, off = rowoff[s_ * WF_BKV + r];
+      const uint32_t dst = c < CK ? sK + s_ * KTILE + wf_swz(r, c, QW * 2) : sV + s_ * VTILE + wf_swz(r, c - CK, E * 2);
+      if (off >= 0) hb_cp_async16(dst, c < CK ? A.kc + (size_t)off * QW + c * 8 : A.vc + (size_t)off * E + (c - CK) * 8);
+      else asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "r"(0u) : "memory");
+    }
+  };
+  const int old = A.ctx_len ? A.ctx_len[rq] : 0;
+  for (int s_ = 0; s_ < n_tiles; s_++)
+    if ((tile_of(ord0 + s_) + 1) * WF_BKV <= old) load_tile(s_);
+  hb_pdl_wait();
+  for (int s_ = 0; s_ < n_tiles; s_++)
+    if ((tile_of(ord0 + s_) + 1) * WF_BKV > old) load_tile(s_);
   for (int i = tid; i < 16 * (QW / 8); i += WF_THREADS) {      // the group's heads as rows 0 .. HG-1, the rest zero
     const int r = i / (QW / 8), c = i - r * (QW / 8);
     const uint32_t dst = sQ + wf_swz(r, c, QW * 2);
     if (r < HG) hb_cp_async16(dst, A.q + ((size_t)row * H + (size_t)g_kv * HG + r) * QW + c * 8);
-    else asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "r"(0u) : "memory");
-  }
-  __syncthreads();
-  // ALL tiles of the split are asked for at once: their trips to memory overlap, the walk then waits once
-  for (int i = tid; i < n_tiles * WF_BKV * (QW / 8 + E / 8); i += WF_THREADS) {
-    constexpr int CK = QW / 8, CA = QW / 8 + E / 8;
-    const int kr = i / CA, c = i - kr * CA, s_ = kr / WF_BKV, r = kr & (WF_BKV - 1), off = rowoff[kr];
-    const uint32_t dst = c < CK ? sK + s_ * KTILE + wf_swz(r, c, QW * 2) : sV + s_ * VTILE + wf_swz(r, c - CK, E * 2);
-    if (off >= 0) hb_cp_async16(dst, c < CK ? A.kc + (size_t)off * QW + c * 8 : A.vc + (size_t)off * E + (c - CK) * 8);
     else asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "r"(0u) : "memory");
   }
   hb_cp_async_commit();
@@ -457,7 +471,7 @@ __global__ void __launch_bounds__(WF_THREADS, 3) attn_window_rows_mma_kernel(Win
     __syncthreads();             // (the join of the splits below takes the same memory)
   }
   if (n_splits > 1) {
-    const size_t slot = ((size_t)row * G + g_kv) * A.splits;
+    const size_t slot = ((size_t)rw * G + g_kv) * A.splits;
     if (warp == 0) {
       float* mine = A.part + (slot + blockIdx.z) * 2 * HG * (E + 2);
 #pragma unroll
@@ -480,9 +494,9 @@ __global__ void __launch_bounds__(WF_THREADS, 3) attn_window_rows_mma_kernel(Win
     __threadfence();
     __syncthreads();
     if (tid == 0) {
-      const int seen = atomicAdd(A.arrived + (size_t)row * G + g_kv, 1);
+      const int seen = atomicAdd(A.arrived + (size_t)rw * G + g_kv, 1);
       last = seen == n_splits - 1;
-      if (last) A.arrived[(size_t)row * G + g_kv] = 0;
+      if (last) A.arrived[(size_t)rw * G + g_kv] = 0;
     }
     __syncthreads();
     if (!last) return;
@@ -625,7 +639,8 @@ HB_EXPORT int hb_attn_window_rows_mma(const void* q, const void* kc, const void*
                                       const int* row_req, const int* pos, const float* gate, long ld_gate, int gate_off,
                                       void* out, int T, int H, int G, int D, int E, int page_size, int window, int keep_first,
                                       float scale, float lambda, float post, float eps, const int* q_len, int row_limit,
-                                      float* part, long part_floats, int* arrived, int max_pos, cudaStream_t s) {
+                                      float* part, long part_floats, int* arrived, int max_pos, const int* row_list, const int* ctx_len,
+                                      cudaStream_t s) {
   if (T <= 0) return 0;
   if (!hb_attn_window_rows_mma_supported(H, G, D, E, 2)) HB_FAIL("hb_attn_window_rows_mma: %d/%d heads of %d/%d are not supported", H, G, D, E);
   if (T > 65535) HB_FAIL("hb_attn_window_rows_mma: %d rows are beyond the grid limit", T);
@@ -636,7 +651,7 @@ HB_EXPORT int hb_attn_window_rows_mma(const void* q, const void* kc, const void*
   if (splits > 65535) HB_FAIL("hb_attn_window_rows_mma: %d key splits are beyond the grid limit", splits);
   WinRowsArgs A{(const __nv_bfloat16*)q, (const __nv_bfloat16*)kc, (const __nv_bfloat16*)vc, bt, bt_stride, row_req, pos, gate, ld_gate,
                 gate_off, (__nv_bfloat16*)out, H, G, page_size, window, keep_first, scale * 1.4426950408889634f, lambda, post, eps,
-                q_len, row_limit, part, arrived, splits};
+                q_len, row_limit, part, arrived, splits, row_list, ctx_len};
   const dim3 grid(G, T, splits);
   int r = -1;
   if (D == 32 && E == 64) r = rm_launch<32, 64>(A, grid, s);

@@ -140,14 +140,147 @@ __global__ void __launch_bounds__(HL_THREADS) heads_linear_kernel(const float* _
   }
 }
 
+// The same for N a multiple of 8 and rows of the weight on 16-byte boundaries: a warp owns HV_ROWS rows, one head and eight output
+// columns, its lanes the k's lane, lane + 32, ..: a lane's loads of the weight are 16 bytes each, eight of them in flight, and
+// asked for before the wait for the kernel ahead. The lanes' sums meet by a transposing butterfly that leaves lane l the sum
+// of (row l / 8, column l % 8): 31 shuffles for 32 sums, no shared memory, no barrier. Bound by latency: the weight of a head is
+// 32 KB (4 rows, 32 heads of 256 x 64: 13.5 us with two-byte loads of one k after the other, 4.4 now). row_list: the rows the
+// call is for (indices in a, out, gate and pos), or null: all T. What the kernel ahead wrote (a, the gate) has no __restrict__.
+constexpr int HV_ROWS = 4, HV_K = 8;
+struct HeadsVec {
+  const float* a; long lda, a_head;
+  const void* wt;
+  void* out; long ldo, o_head;
+  int T, K, N;
+  const float* gate; long ld_gate;
+  int gate_off, tail, rot;
+  const int* pos; const float2* table;
+  const int *row_list, *row_req, *q_len;
+  int row_limit, pairing, gate_per_head;
+};
+
+template <typename TW> __device__ __forceinline__ void hv_load8(const TW* p, float* v);
+template <> __device__ __forceinline__ void hv_load8<float>(const float* p, float* v) {
+  *(float4*)v = *(const float4*)p;
+  *(float4*)(v + 4) = *(const float4*)(p + 4);
+}
+template <> __device__ __forceinline__ void hv_load8<__nv_bfloat16>(const __nv_bfloat16* p, float* v) {
+  const uint4 r = *(const uint4*)p;
+  const uint32_t u[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    v[2 * i] = __uint_as_float(u[i] << 16);
+    v[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
+  }
+}
+
+template <typename TW, typename TO>
+__global__ void __launch_bounds__(256) heads_linear_vec_kernel(HeadsVec A) {
+  hb_pdl_launch();
+  const int h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i0 = blockIdx.z * HV_ROWS;
+  const int n0 = (blockIdx.x * 8 + warp) * 8, K = A.K, N = A.N;
+  const bool tail_block = (int)blockIdx.x * 64 >= N;
+  int row[HV_ROWS];
+  bool on[HV_ROWS], any = false;
+#pragma unroll
+  for (int r = 0; r < HV_ROWS; r++) {
+    on[r] = i0 + r < A.T;
+    row[r] = on[r] ? (A.row_list ? A.row_list[i0 + r] : i0 + r) : 0;
+    if (on[r] && A.q_len && A.q_len[A.row_req[row[r]]] >= A.row_limit) on[r] = false;
+    any |= on[r];
+  }
+  if (!any || (!tail_block && n0 >= N)) {
+    if ((blockIdx.x | blockIdx.y | blockIdx.z) == 0) hb_pdl_wait();      // the grid never ends before the one ahead of it
+    return;
+  }
+  if (tail_block) {                       // the rotated columns behind the product's
+    hb_pdl_wait();
+    const int half = A.rot >> 1;
+#pragma unroll
+    for (int r = 0; r < HV_ROWS; r++) {
+      if (!on[r]) continue;
+      const float* src = A.a + (size_t)row[r] * A.lda + (size_t)h * A.a_head + K;
+      for (int j = threadIdx.x; j < A.tail; j += 256) {
+        float y = src[j];
+        if (j < A.rot) {
+          const int i = A.pairing ? j >> 1 : (j < half ? j : j - half);
+          const bool second = A.pairing ? (j & 1) : (j >= half);
+          const float2 c = A.table[(size_t)A.pos[row[r]] * half + i];
+          const float u = src[A.pairing ? 2 * i : i], v = src[A.pairing ? 2 * i + 1 : i + half];
+          y = second ? __fadd_rn(__fmul_rn(v, c.x), __fmul_rn(u, c.y)) : __fsub_rn(__fmul_rn(u, c.x), __fmul_rn(v, c.y));
+        }
+        ((TO*)A.out)[(size_t)row[r] * A.ldo + (size_t)h * A.o_head + N + j] = hb_from_float<TO>(y);
+      }
+    }
+    return;
+  }
+  const TW* w = (const TW*)A.wt + (size_t)h * K * N + n0;
+  float acc[HV_ROWS * 8];
+#pragma unroll
+  for (int i = 0; i < HV_ROWS * 8; i++) acc[i] = 0.f;
+  for (int k0 = 0; k0 < K; k0 += 32 * HV_K) {
+    float wv[HV_K][8];
+#pragma unroll
+    for (int i = 0; i < HV_K; i++) {
+      const int k = k0 + i * 32 + lane;
+      if (k < K) hv_load8<TW>(w + (size_t)k * N, wv[i]);
+    }
+    if (k0 == 0) hb_pdl_wait();
+    float av[HV_ROWS][HV_K];
+#pragma unroll
+    for (int r = 0; r < HV_ROWS; r++)
+#pragma unroll
+      for (int i = 0; i < HV_K; i++) {
+        const int k = k0 + i * 32 + lane;
+        av[r][i] = on[r] && k < K ? A.a[(size_t)row[r] * A.lda + (size_t)h * A.a_head + k] : 0.f;
+      }
+#pragma unroll
+    for (int i = 0; i < HV_K; i++)
+      if (k0 + i * 32 + lane < K)
+#pragma unroll
+        for (int r = 0; r < HV_ROWS; r++)
+#pragma unroll
+          for (int c = 0; c < 8; c++) acc[r * 8 + c] = fmaf(av[r][i], wv[i][c], acc[r * 8 + c]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {      // after the step of o a lane keeps the sums whose bit o is its own
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < 16; i++)
+      if (i < o) {
+        const float send = up ? acc[i] : acc[i + o], kept = up ? acc[i + o] : acc[i];
+        acc[i] = kept + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+  }
+  const int r = lane >> 3, n = n0 + (lane & 7);
+  bool mine = false;
+  int t = 0;
+#pragma unroll
+  for (int i = 0; i < HV_ROWS; i++)
+    if (i == r) { mine = on[i]; t = row[i]; }
+  if (!mine) return;
+  float y = acc[0];
+  if (A.gate) y *= 1.f / (1.f + expf(-A.gate[(size_t)t * A.ld_gate + A.gate_off + (A.gate_per_head ? (size_t)h : (size_t)h * N + n)]));
+  ((TO*)A.out)[(size_t)t * A.ldo + (size_t)h * A.o_head + n] = hb_from_float<TO>(y);
+}
+
 // a float32 [T][lda], head h's K (+ tail) inputs at column h * a_head; wt [H][K][N]; out [T][ldo], head h's N (+ tail)
 // outputs at column h * o_head.
 HB_EXPORT int hb_heads_linear(const float* a, long lda, long a_head, const void* wt, int w_dt, void* out, int o_dt, long ldo,
                               long o_head, int T, int H, int K, int N, const float* gate, long ld_gate, int gate_off, int tail,
                               int rot, const int* pos, const void* table, const int* row_req, const int* q_len, int row_limit,
-                              int pairing, int gate_per_head, cudaStream_t s) {
+                              int pairing, int gate_per_head, const int* row_list, cudaStream_t s) {
   if (T <= 0 || H <= 0) return 0;
   if (tail && (!pos || !table || rot > tail || (rot & 1))) HB_FAIL("hb_heads_linear: a rotated tail needs positions and a table");
+  if (N % 8 == 0 && ((uintptr_t)wt & 15) == 0 && H <= 65535 && (T + HV_ROWS - 1) / HV_ROWS <= 65535) {     // (a row of 8 is 16 or 32 bytes)
+    const HeadsVec A{a, lda, a_head, wt, out, ldo, o_head, T, K, N, gate, ld_gate, gate_off, tail, rot, pos, (const float2*)table, row_list,
+                     row_req, q_len, row_limit, pairing, gate_per_head};
+    const dim3 grid((N + 63) / 64 + (tail ? 1 : 0), H, (T + HV_ROWS - 1) / HV_ROWS);
+    HB_DISPATCH_2(w_dt, o_dt, "hb_heads_linear", (hb_launch(heads_linear_vec_kernel<TA, TB>, grid, 256, 0, s, A)));
+    HB_CHECK_LAUNCH("hb_heads_linear");
+    return 0;
+  }
+  if (row_list) HB_FAIL("hb_heads_linear: a list of rows wants outputs in multiples of 8 and a weight on a 16-byte boundary");
   const size_t smem = ((size_t)HL_TM * (K + tail) + (size_t)HL_KZ * HL_TM * HL_TN) * sizeof(float);
   if (smem > 96 * 1024) HB_FAIL("hb_heads_linear: K = %d is too wide", K);
   if ((T + HL_TM - 1) / HL_TM > 65535 || H > 65535) HB_FAIL("hb_heads_linear: the grid is too large");

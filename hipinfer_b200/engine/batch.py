@@ -62,7 +62,7 @@ class StepBatch:
             rows = self.short_list if limit == SHORT_ROWS else None
             if rows is None:
                 rows = torch.from_numpy(_rows_of(short, self.h_q_start, self.h_q_len)).to(self.tokens.device)
-            self.extra[key] = rows, max(self.h_ctx_len[r] + self.h_q_len[r] - 1 for r in short)
+            self.extra[key] = rows, max((self.h_ctx_len[r] + self.h_q_len[r] - 1 for r in short), default=0)
         return self.extra[key]
 
 

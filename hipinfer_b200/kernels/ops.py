@@ -49,12 +49,12 @@ _SIGS = {
         "hb_attn_masked": [_p, _i, _l, _p, _l, _p, _l, _i, _p, _i, _p, _p, _p, _p, _l, _i, _i, _p, _i, _l, _i, _i, _i, _i, _i,
                            _i, _i, _i, _i, _i, _f, _p, _i, _p, _l, _p, _i, _p, _p, _p],
         "hb_latent_prepare": [_p, _l, _i, _i, _i, _p, _p, _i, _p, _p, _p, _i, _f, _p, _p, _i, _i, _i, _i, _i, _i, _i, _p],
-        "hb_heads_linear": [_p, _l, _l, _p, _i, _p, _i, _l, _l, _i, _i, _i, _i, _p, _l, _i, _i, _i, _p, _p, _p, _p, _i, _i, _i, _p],
+        "hb_heads_linear": [_p, _l, _l, _p, _i, _p, _i, _l, _l, _i, _i, _i, _i, _p, _l, _i, _i, _i, _p, _p, _p, _p, _i, _i, _i, _p, _p],
         "hb_gather_rows": [_p, _i, _p, _p, _i, _i, _i, _p],
         "hb_attn_masked_flash_supported": [_i, _i],
         "hb_attn_masked_heads_supported": [_i, _i, _i, _i, _i],
         "hb_attn_masked_heads": [_p, _l, _p, _l, _l, _l, _p, _l, _l, _l, _i, _p, _i, _p, _p, _p, _p, _l, _i, _i, _p, _i, _l, _i, _i,
-                                 _i, _i, _i, _i, _i, _i, _i, _i, _f, _p, _i, _p, _l, _i, _p, _p, _p],
+                                 _i, _i, _i, _i, _i, _i, _i, _i, _f, _p, _i, _p, _l, _i, _p, _p, _p, _p, _p],
         "hb_attn_masked_flash": [_p, _l, _p, _l, _l, _l, _p, _l, _l, _l, _p, _i, _p, _p, _p, _i, _i, _i, _i, _p, _p, _l, _i, _i, _p,
                                  _i, _l, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _p, _p, _p],
         "hb_gla": [_p, _l, _i, _i, _i, _i, _p, _l, _p, _p, _i, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _f, _f, _p],
@@ -104,7 +104,7 @@ _SIGS = {
         "hb_attn_window_flash_supported": [_i, _i, _i, _i, _i],
         "hb_attn_window_rows_mma_supported": [_i, _i, _i, _i, _i],
         "hb_attn_window_rows_mma": [_p, _p, _p, _p, _i, _p, _p, _p, _l, _i, _p, _i, _i, _i, _i, _i, _i, _i, _i, _f, _f, _f, _f,
-                                    _p, _i, _p, _l, _p, _i, _p],
+                                    _p, _i, _p, _l, _p, _i, _p, _p, _p],
     },
 }
 _fn_cache = {}
@@ -391,6 +391,10 @@ def attention_window(q, k_cache, v_cache, batch, group: int, out, n_heads: int, 
     if (maps == 2 and norm and q.dtype == torch.bfloat16 and not fast.PLAIN_ONLY and not force_plain and not force_simt
             and _fn("mixers", "hb_attn_window_rows_mma_supported")(n_heads, n_kv_heads, dim, vdim, maps) == 1):
         # the heads of a kv head as the rows of a warp MMA tile
+        rows = None
+        if flash and hasattr(batch, "short_rows"):     # beside portions for the flash kernel: a grid over the other rows alone
+            (rows, max_pos), q_len_ptr = batch.short_rows(WINDOW_FLASH_MIN_ROWS), None
+            T = rows.numel()
         n_ws = lib.hb_attn_window_rows_mma_workspace(T, n_heads, n_kv_heads, vdim, int(window), int(keep_first), max_pos)
         ws = torch.empty(n_ws, dtype=torch.float32, device=q.device) if n_ws else None
         arrived = fast._decode_counters(q.device, T * n_kv_heads) if n_ws else None
@@ -398,7 +402,7 @@ def attention_window(q, k_cache, v_cache, batch, group: int, out, n_heads: int, 
               bt.stride(0), batch.row_request.data_ptr(), batch.positions.data_ptr(), _ptr(gate), gate_ld, int(gate_offset),
               out.data_ptr(), T, n_heads, n_kv_heads, dim, vdim, page_size, int(window), int(keep_first), float(scale),
               float(lam), float(post), float(eps), q_len_ptr, WINDOW_FLASH_MIN_ROWS, _ptr(ws), n_ws, _ptr(arrived), max_pos,
-              _stream())
+              _ptr(rows), _ptr(getattr(batch, "req_ctx_len", None)), _stream())
         return out
     n_ws = 0 if (q.dtype != torch.bfloat16 or force_plain) else lib.hb_attn_window_workspace(
         T, n_heads, n_kv_heads, vdim, maps, int(window), int(keep_first), max_pos)
@@ -1034,6 +1038,12 @@ def attention_masked(q, k_cache, v_cache, batch, group: int, out, n_heads: int, 
         # the heads of a kv head as the rows of warp MMA tiles: a key tile is read once for all of them
         lib.hb_attn_masked_heads_workspace.restype = C.c_long
         lib.hb_attn_masked_heads_workspace.argtypes = [_i] * 9
+        rows = None
+        if limit and hasattr(batch, "short_rows"):     # beside portions for another kernel: a grid over the other rows alone
+            rows, max_pos = batch.short_rows(limit)
+            T = rows.numel()
+            if T == 0:
+                return out
         n_ws = lib.hb_attn_masked_heads_workspace(T, n_heads, n_kv_heads, vdim, m, int(window), int(keep_first), int(chunk), max_pos)
         ws = torch.empty(n_ws, dtype=torch.float32, device=q.device) if n_ws else None
         _call("seqmix", "hb_attn_masked_heads", q.data_ptr(), q.stride(0), k_cache.data_ptr(), n_kv_heads * page_size * kw,
@@ -1041,8 +1051,8 @@ def attention_masked(q, k_cache, v_cache, batch, group: int, out, n_heads: int, 
               bt.data_ptr(), bt.stride(0), batch.row_request.data_ptr(), batch.positions.data_ptr(), _ptr(sink), _ptr(gate),
               gate.stride(0) if gate is not None else 0, int(gate_offset), (2 if gate_per_head else 1) if gate is not None else 0,
               out.data_ptr(), _dt(out), out.stride(0), T, n_heads, n_kv_heads, dim, vdim, page_size, m, int(window),
-              int(keep_first), int(chunk), float(scale), batch.req_q_len.data_ptr() if limit else None, limit, _ptr(ws), n_ws,
-              max_pos, _ptr(r1), _ptr(r2), _stream())
+              int(keep_first), int(chunk), float(scale), batch.req_q_len.data_ptr() if limit and rows is None else None, limit, _ptr(ws),
+              n_ws, max_pos, _ptr(r1), _ptr(r2), _ptr(rows), _ptr(getattr(batch, "req_ctx_len", None)), _stream())
         return out
     n_ws = lib.hb_attn_masked_workspace(T, n_heads, n_kv_heads, dim, vdim, m, int(window), int(keep_first), int(chunk), max_pos)
     ws = arrived = None
@@ -1099,11 +1109,18 @@ def heads_linear(a: torch.Tensor, a_head: int, wt: torch.Tensor, out: torch.Tens
     assert a.dtype == torch.float32 and wt.is_contiguous() and out.shape[0] == T
     if gate is not None:
         assert gate.dtype == torch.float32 and gate.stride(1) == 1
+    rows = None
+    if row_limit and N % 8 == 0 and wt.data_ptr() % 16 == 0 and hasattr(batch, "short_rows"):
+        rows = batch.short_rows(row_limit)[0]      # a grid over the rows that are meant
+        T = rows.numel()
+        if T == 0:
+            return out
     _call("seqmix", "hb_heads_linear", a.data_ptr(), a.stride(0), int(a_head), wt.data_ptr(), _dt(wt), out.data_ptr(),
           _dt(out), out.stride(0), int(o_head), T, H, K, N, _ptr(gate), gate.stride(0) if gate is not None else 0,
           int(gate_offset), int(tail), int(rot), _ptr(positions), _ptr(table),
-          batch.row_request.data_ptr() if row_limit else None, batch.req_q_len.data_ptr() if row_limit else None, int(row_limit),
-          PAIRINGS[pairing], 1 if gate_per_head else 0, _stream())
+          batch.row_request.data_ptr() if row_limit and rows is None else None,
+          batch.req_q_len.data_ptr() if row_limit and rows is None else None, int(row_limit),
+          PAIRINGS[pairing], 1 if gate_per_head else 0, _ptr(rows), _stream())
     return out
 
 

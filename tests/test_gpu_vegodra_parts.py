@@ -401,3 +401,67 @@ def test_single_rows_whose_values_are_a_prefix_of_the_key_rows(H, D, E):
             kk = keys[r].to(dtype).double()
             want = _attend_plain(q[t].to(dtype).double().view(H, D), kk, kk[..., :E], p, H, 1, scale, "causal", 0, 0, 0, None, None, False)
             close(out[t], want, dtype, f"row {t} (request {r}, position {p}, plain kernel {plain_kernel})")
+
+
+@pytest.mark.parametrize("H,G,D,E,mask,window,chunk", [(32, 1, 288, 256, "causal", 0, 0), (8, 2, 64, 64, "window", 200, 0), (6, 2, 32, 48, "chunk", 0, 512)])
+def test_single_rows_of_a_list_and_keys_read_ahead(H, G, D, E, mask, window, chunk):
+    """The row kernel over a list of the step's rows, with the requests' earlier lengths known (whole tiles of earlier keys are
+    then read before the kernel ahead has ended): the bits of the call over all rows, the other rows' places untouched. 1, 8
+    and 9 tiles of 64 keys: one cluster of tiles, a full one, two."""
+    from hipinfer_b200.kernels import ops
+
+    dtype, ps = torch.bfloat16, 16
+    lens = [530, 70, 512, 64]
+    alias = G == 1
+    keys = [rnd(n, G, D, seed=10 + r) for r, n in enumerate(lens)]
+    kc, vc, bt = _paged(keys, [k[..., :E] if alias else rnd(n, G, E, seed=20 + r) for r, (k, n) in enumerate(zip(keys, lens))], ps, dtype,
+                        seed=3, **(dict(alias=True) if alias else {}))
+    rows = [(r, p) for r, n in enumerate(lens) for p in (n - 3, n - 2, n - 1)]
+    q = rnd(len(rows), H * D, seed=5).to(dtype).to(DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    common = dict(block_tables=[bt], row_request=i32([r for r, _ in rows]), positions=i32([p for _, p in rows]), max_pos=max(lens) - 1)
+    args = (kc, kc if alias else vc)
+    every = torch.empty(len(rows), H * E, dtype=torch.float32, device=DEV)
+    ops.attention_masked(q, *args, SimpleNamespace(**common), 0, every, H, G, D, E, ps, D ** -0.5, mask, window, 0, chunk)
+    pick = [11, 0, 7, 4, 2]
+    some = torch.full_like(every, 5.0)
+    listed = SimpleNamespace(**common, req_ctx_len=i32([n - 3 for n in lens]), req_q_len=i32([3] * 4),
+                             short_rows=lambda limit: (i32(pick), max(rows[i][1] for i in pick)))
+    ops.attention_masked(q, *args, listed, 0, some, H, G, D, E, ps, D ** -0.5, mask, window, 0, chunk, row_limit=16)
+    assert torch.equal(some[pick], every[pick])
+    rest = [i for i in range(len(rows)) if i not in pick]
+    assert bool((some[rest] == 5.0).all())
+
+
+@pytest.mark.parametrize("wdt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,K,N,tail,T", [(32, 256, 64, 0, 4), (4, 64, 256, 32, 5), (3, 300, 40, 8, 1), (2, 33, 8, 0, 9), (5, 520, 72, 0, 3)])
+def test_heads_linear_of_all_and_of_listed_rows(wdt, H, K, N, tail, T):
+    """Per-head products of 32-bit rows with outputs in multiples of 8: k in several rounds of the lanes and ragged ends of it,
+    columns beyond a block's 64, a gate per element, a rotated tail. The bound: 32-bit sums of K products and a sigmoid."""
+    from hipinfer_b200.kernels import ops
+
+    a, w = rnd(T, H * (K + tail), seed=41), rnd(H, K, N, seed=42, scale=0.1).to(wdt)
+    gate = rnd(T, 3 + H * N, seed=43)
+    table = torch.stack([torch.cos(rnd(50, max(tail // 2, 1), seed=44)), torch.sin(rnd(50, max(tail // 2, 1), seed=44))], -1).contiguous()
+    pos = torch.arange(T, dtype=torch.int32) * 3
+    out = torch.empty(T, H * (N + tail), device=DEV)
+    kw = dict(gate=gate.to(DEV), gate_offset=3)
+    if tail:
+        kw.update(tail=tail, rot=tail, positions=pos.to(DEV), table=table.to(DEV))
+    ops.heads_linear(a.to(DEV), K + tail, w.to(DEV), out, N + tail, **kw)
+    ad, wd = a.double().view(T, H, K + tail), w.double()
+    plain = torch.einsum("thk,hkn->thn", ad[..., :K], wd)
+    bound = (K + 16) * 2.0 ** -24 * torch.einsum("thk,hkn->thn", ad[..., :K].abs(), wd.abs()) + 1e-6 * plain.abs()
+    got = out.double().cpu().view(T, H, N + tail)
+    assert bool(((got[..., :N] - plain * torch.sigmoid(gate[:, 3:].double().view(T, H, N))).abs() <= bound + 1e-12).all())
+    if tail:
+        u, v = ad[..., K::2], ad[..., K + 1::2]
+        c, s = table[pos.long()][:, None, :, 0].double(), table[pos.long()][:, None, :, 1].double()
+        want = torch.stack([u * c - v * s, v * c + u * s], -1).flatten(-2)
+        torch.testing.assert_close(got[..., N:], want, rtol=1e-5, atol=1e-6)
+    pick = [T - 1] + ([0] if T > 1 else [])
+    some = torch.full_like(out, 5.0)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    batch = SimpleNamespace(row_request=i32([0] * T), req_q_len=i32([T]), short_rows=lambda limit: (i32(pick), 0))
+    ops.heads_linear(a.to(DEV), K + tail, w.to(DEV), some, N + tail, batch=batch, row_limit=16, **kw)
+    assert torch.equal(some[pick], out[pick]) and bool((some[[t for t in range(T) if t not in pick]] == 5.0).all())
