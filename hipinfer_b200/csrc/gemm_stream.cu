@@ -497,18 +497,17 @@ HB_EXPORT int hb_gemm_stream(const void* A, long lda, const void* W, long ldw, v
   return 0;
 }
 
-// Finish a product that was left as slices (epi 4): C per `epi` (0 to 3) from ws, for the same M, N, K.
-HB_EXPORT int hb_gemm_stream_finish(const float* ws, void* C, long ldc, int M, int N, int K, int epi, cudaStream_t s) {
+// Finish a product that was left as ksplit slices (hb_gemm_stream's epi 4, hb_gemm_tc_slices): C per `epi` (0 to 3 and 5 to 7) from
+// ws[slice][slice_rows][row_stride].
+HB_EXPORT int hb_slices_finish(const float* ws, void* C, long ldc, int M, int N, int row_stride, int slice_rows, int ksplit, int epi,
+                               cudaStream_t s) {
   if (M <= 0 || N <= 0) return 0;
-  if (epi < 0 || (epi > 3 && epi != ST_GEGLU_BF16 && epi != ST_GELU_BF16 && epi != ST_RELU2_BF16)) HB_FAIL("hb_gemm_stream_finish: unknown epilogue %d", epi);
-  int kslice, ksplit, n_blocks;
-  long per_token;
-  hb_gemm_stream_plan(N, K, &kslice, &ksplit, &per_token, &n_blocks);
-  const int NT = M <= 16 ? 16 : M <= 32 ? 32 : 64, NP = n_blocks * ST_ROWS;
-  const long items = (long)M * (NP / 4);
-  cudaError_t e = hb_launch(stream_reduce_kernel, (unsigned)((items + 255) / 256), 256, 0, s, ws, C, ldc, M, N, NP, NT,
+  if (epi < 0 || (epi > 3 && epi != ST_GEGLU_BF16 && epi != ST_GELU_BF16 && epi != ST_RELU2_BF16)) HB_FAIL("hb_slices_finish: unknown epilogue %d", epi);
+  if (row_stride < N || (row_stride & 3) || slice_rows < M || ksplit < 1) HB_FAIL("hb_slices_finish: %d slices of %d rows of %d", ksplit, slice_rows, row_stride);
+  const long items = (long)M * (row_stride / 4);
+  cudaError_t e = hb_launch(stream_reduce_kernel, (unsigned)((items + 255) / 256), 256, 0, s, ws, C, ldc, M, N, row_stride, slice_rows,
                             ksplit, epi);
-  if (e != cudaSuccess) HB_FAIL("hb_gemm_stream_finish: %s", cudaGetErrorString(e));
+  if (e != cudaSuccess) HB_FAIL("hb_slices_finish: %s", cudaGetErrorString(e));
   return 0;
 }
 

@@ -344,6 +344,11 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
 // of both CTAs; the loaders of both CTAs count their bytes on the even CTA's barriers; the odd
 // CTA's epilogue warps free the accumulator by arriving on the even CTA's barrier. Results
 // leave through the TMA-store epilogue. K runs in blocks of 64 in ascending order as above.
+//
+// splits > 1: the tiles are walked once per slice of kbs K blocks, and slice i's sums go to rows [i * slice_rows, ..) of C (fp32):
+// a product of so few tiles that most SMs would have none. The alternative, narrower tiles, fills the SMs but reads more
+// operand bytes per product, and at 96 CTAs of 128 x 128 tiles it is L2 that bounds it (512 x 3,072 by 3,072 and by 8,192: 62
+// us for both together; three slices of 256 x 256 tiles 35 us, and the norm that reads the sums next adds the slices).
 // ---------------------------------------------------------------------------------------
 template <int STAGES>
 struct PairSmem {
@@ -357,7 +362,7 @@ template <int STAGES, int EPI>
 __global__ void __launch_bounds__(192, 1) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a,
                                                               const __grid_constant__ CUtensorMap map_w,
                                                               const __grid_constant__ CUtensorMap map_c, int M, int N, int K,
-                                                              int* status) {
+                                                              int* status, int splits, int kbs, int slice_rows) {
   using S = PairSmem<STAGES>;
   constexpr int BN = 256;
   extern __shared__ uint8_t smem_raw[];
@@ -373,7 +378,7 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_pair_kernel(const __grid_const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = hb_cluster_ctarank();                 // 0: issues the MMAs, owns the barriers the loads count on
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
-  const int m_tiles = (M + 255) / 256, n_tiles = (N + BN - 1) / BN, num_tiles = m_tiles * n_tiles;
+  const int m_tiles = (M + 255) / 256, n_tiles = (N + BN - 1) / BN, num_tiles = m_tiles * n_tiles, units = num_tiles * splits;
   const int num_kb = (K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
@@ -398,9 +403,10 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_pair_kernel(const __grid_const
     if (lane == 0) {  // ---------------- TMA producer of this CTA's halves
       uint32_t it = 0;
       bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += n_pairs) {
+      for (int u = pair; u < units && ok; u += n_pairs) {
+        const int tile = u % num_tiles, kb0 = u / num_tiles * kbs, kb1 = min(num_kb, kb0 + kbs);
         const int m0 = (tile % m_tiles) * 256 + rank * 128, n0 = (tile / m_tiles) * BN + rank * 128;
-        for (int kb = 0; kb < num_kb; kb++, it++) {
+        for (int kb = kb0; kb < kb1; kb++, it++) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
           if (!hb_mbar_wait(&empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
           if (rank == 0) hb_mbar_expect_tx(&full[s], 2 * S::STAGE_BYTES);   // both CTAs' bytes
@@ -418,19 +424,20 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_pair_kernel(const __grid_const
       constexpr uint32_t idesc = hb_umma_idesc_bf16(256, BN);
       uint32_t it = 0, tile_i = 0;
       bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += n_pairs, tile_i++) {
+      for (int u = pair; u < units && ok; u += n_pairs, tile_i++) {
+        const int kb0 = u / num_tiles * kbs, kb1 = min(num_kb, kb0 + kbs);
         const uint32_t buf = tile_i & 1, aph = (tile_i >> 1) & 1;
         if (!hb_mbar_wait(&tmem_empty[buf], aph ^ 1, abort_flag)) break;
         hb_tc_fence_after();
         const uint32_t d = tmem_base + buf * BN;
-        for (int kb = 0; kb < num_kb; kb++, it++) {
+        for (int kb = kb0; kb < kb1; kb++, it++) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
           if (!hb_mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
           hb_tc_fence_after();
           const uint64_t da = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE_BYTES));
           const uint64_t db = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE_BYTES + S::A_BYTES));
 #pragma unroll
-          for (int k = 0; k < BK / 16; k++) hb_umma_bf16_pair(d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+          for (int k = 0; k < BK / 16; k++) hb_umma_bf16_pair(d, da + 2 * k, db + 2 * k, idesc, kb != kb0 || k != 0);
           hb_umma_commit_pair(&empty[s]);
         }
         if (ok) hb_umma_commit_pair(&tmem_full[buf]);
@@ -438,8 +445,8 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_pair_kernel(const __grid_const
     }
   } else {  // ---------------- epilogue warps 0..3: this CTA's 128 rows of the tile
     uint32_t tile_i = 0;
-    for (int tile = pair; tile < num_tiles; tile += n_pairs, tile_i++) {
-      const int m0 = (tile % m_tiles) * 256 + rank * 128, n0 = (tile / m_tiles) * BN;
+    for (int u = pair; u < units; u += n_pairs, tile_i++) {
+      const int tile = u % num_tiles, m0 = (tile % m_tiles) * 256 + rank * 128 + u / num_tiles * slice_rows, n0 = (tile / m_tiles) * BN;
       const uint32_t buf = tile_i & 1, aph = (tile_i >> 1) & 1;
       if (!hb_mbar_wait(&tmem_full[buf], aph, abort_flag)) break;
       hb_tc_fence_after();
@@ -575,15 +582,16 @@ static int launch_gemm_tc(const CUtensorMap& ma, const CUtensorMap& mw, void* C,
 }
 
 // The CTA-pair kernel: C must be addressable by TMA stores (16-byte aligned base and rows).
+// splits > 1 (EPI_F32): C has splits * slice_rows rows.
 template <int EPI>
 static int launch_gemm_pair(const CUtensorMap& ma, const void* W, long ldw, void* C, long ldc, int M, int N, int K, int* status,
-                            cudaStream_t s) {
+                            cudaStream_t s, int splits = 1, int kbs = 1 << 30, int slice_rows = 0) {
   using S = PairSmem<6>;
   CUtensorMap mw, mc;
   if (hb_make_tensor_map_bf16(&mw, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, 128)) return -1;
   if (EPI == EPI_F32 || EPI == EPI_ADD_F32) {
     if (((uintptr_t)C & 15) || (ldc & 3)) HB_FAIL("hb_gemm_tc: the CTA-pair kernel needs a 16-byte aligned C");
-    if (hb_make_tensor_map_f32_box32(&mc, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc)) return -1;
+    if (hb_make_tensor_map_f32_box32(&mc, C, splits > 1 ? (uint64_t)splits * slice_rows : (uint64_t)M, (uint64_t)N, (uint64_t)ldc)) return -1;
   } else {
     if (((uintptr_t)C & 15) || (ldc & 7)) HB_FAIL("hb_gemm_tc: the CTA-pair kernel needs a 16-byte aligned C");
     const uint64_t cols = EPI_IS_GLU(EPI) ? (uint64_t)N / 2 : (uint64_t)N;
@@ -596,8 +604,9 @@ static int launch_gemm_pair(const CUtensorMap& ma, const void* W, long ldw, void
     if (e != cudaSuccess) HB_FAIL("hb_gemm_tc: %s", cudaGetErrorString(e));
     configured = true;
   }
-  const int tiles = ((M + 255) / 256) * ((N + 255) / 256), pairs = tiles < sm_count() / 2 ? tiles : sm_count() / 2;
-  cudaError_t e = hb_launch_cluster(kern, dim3(2 * pairs), 192, S::TOTAL, s, dim3(2, 1, 1), ma, mw, mc, M, N, K, status);
+  const int tiles = ((M + 255) / 256) * ((N + 255) / 256) * splits, pairs = tiles < sm_count() / 2 ? tiles : sm_count() / 2;
+  cudaError_t e = hb_launch_cluster(kern, dim3(2 * pairs), 192, S::TOTAL, s, dim3(2, 1, 1), ma, mw, mc, M, N, K, status, splits,
+                                    splits > 1 ? kbs : (K + BK - 1) / BK, slice_rows);
   if (e != cudaSuccess) HB_FAIL("hb_gemm_tc: %s", cudaGetErrorString(e));
   return 0;
 }
@@ -673,6 +682,39 @@ HB_EXPORT int hb_gemm_tc(const void* A, long lda, const void* W, long ldw, void*
                           : launch_gemm_tc<192, 4, EPI_ADD_F32>(ma, mw, C, ldc, M, N, K, status, s);
   if (r) return r;
   HB_CHECK_LAUNCH("hb_gemm_tc");
+  return 0;
+}
+
+// The slices of a product that hb_gemm_tc_slices would split: 0 where it would not. One round of 256 x 256 tiles over the SM pairs
+// has room for sms / 2 / tiles slices; a slice is at least 512 deep, and there are at most 8 (the reader of the sums adds them).
+HB_EXPORT int hb_gemm_tc_splits(int M, int N, int K) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const long tiles = (long)((M + 255) / 256) * ((N + 255) / 256);
+  long n = sm_count() / 2 / tiles;
+  if (n > K / 512) n = K / 512;
+  if (n > 8) n = 8;
+  if (n < 2) return 0;
+  const int num_kb = (K + BK - 1) / BK, kbs = (int)((num_kb + n - 1) / n);
+  return (num_kb + kbs - 1) / kbs;
+}
+
+// A W^T as `splits` (from hb_gemm_tc_splits) K slices: ws[slice][slice_rows][ld], fp32, slice_rows = M rounded up to 256. The rows
+// beyond M of a slice are written too.
+HB_EXPORT int hb_gemm_tc_slices(const void* A, long lda, const void* W, long ldw, float* ws, long ld, long ws_floats, int M, int N, int K,
+                                int splits, int* status, cudaStream_t s) {
+  if (M <= 0 || N <= 0) return 0;
+  if (K <= 0 || (K & 7)) HB_FAIL("hb_gemm_tc_slices: K = %d must be a positive multiple of 8 (16-byte rows for TMA)", K);
+  if (!status) HB_FAIL("hb_gemm_tc_slices: no status word");
+  const int num_kb = (K + BK - 1) / BK, slice_rows = (M + 255) / 256 * 256;
+  if (splits < 2 || splits > num_kb || ld < N) HB_FAIL("hb_gemm_tc_slices: %d slices of %d K blocks, rows of %ld", splits, num_kb, ld);
+  const int kbs = (num_kb + splits - 1) / splits;
+  if ((splits - 1) * kbs >= num_kb) HB_FAIL("hb_gemm_tc_slices: %d K blocks do not make %d slices", num_kb, splits);
+  if (ws_floats < (long)splits * slice_rows * ld) HB_FAIL("hb_gemm_tc_slices: workspace of %ld floats", ws_floats);
+  CUtensorMap ma;
+  if (hb_make_tensor_map_bf16(&ma, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BM)) return -1;
+  const int r = launch_gemm_pair<EPI_F32>(ma, W, ldw, ws, ld, M, N, K, status, s, splits, kbs, slice_rows);
+  if (r) return r;
+  HB_CHECK_LAUNCH("hb_gemm_tc_slices");
   return 0;
 }
 

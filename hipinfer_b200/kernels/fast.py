@@ -22,7 +22,9 @@ _SIGS = {
     "hb_gemm_tc_grouped": [_p, _l, _p, _i, _i, _i, _p, _p, _l, _l, _i, _p, _p, _i, _i, _p, _p],
     "hb_gemm_stream": [_p, _l, _p, _l, _p, _l, _i, _i, _i, _i, _p, _l, _p, _i, _p, _p],
     "hb_gemm_stream_plan": [_i, _i, _p, _p, _p, _p],
-    "hb_gemm_stream_finish": [_p, _p, _l, _i, _i, _i, _i, _p],
+    "hb_slices_finish": [_p, _p, _l, _i, _i, _i, _i, _i, _i, _p],
+    "hb_gemm_tc_splits": [_i, _i, _i],
+    "hb_gemm_tc_slices": [_p, _l, _p, _l, _p, _l, _l, _i, _i, _i, _i, _p, _p],
     "hb_add_rmsnorm_slices": [_p, _l, _p, _i, _l, _l, _p, _p, _p, _i, _i, _f, _p],
     "hb_rope_kv_slices": [_p, _i, _l, _l, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _p],
     "hb_attn_decode": [_p, _p, _p, _l, _p, _i, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _f, _i, _i, _p, _i, _p, _p, _p, _p, _p, _p, _p],
@@ -46,7 +48,7 @@ _SIGS = {
     "hb_rows_norm_supported": [_i, _i],
 }
 _fns = {}
-_LAUNCHES = {"hb_rows_scaled_qkv_rope": 1, "hb_rows_scaled_swiglu": 1, "hb_rows_norm_qkv_rope": 1, "hb_rows_add": 1, "hb_rows_norm_swiglu": 1, "hb_gemm_tc_rope_kv": 1, "hb_gemm_stream_finish": 1, "hb_add_rmsnorm_slices": 1, "hb_rope_kv_slices": 1, "hb_gemm_tc": 1, "hb_gemm_stream": 1, "hb_attn_decode": 1, "hb_flash_prefill": 1, "hb_flash_prefill_tc": 1, "hb_flash_diff_tc": 1, "hb_attn_diff_decode": 1, "hb_gemm_tc_grouped": 1}
+_LAUNCHES = {"hb_rows_scaled_qkv_rope": 1, "hb_rows_scaled_swiglu": 1, "hb_rows_norm_qkv_rope": 1, "hb_rows_add": 1, "hb_rows_norm_swiglu": 1, "hb_gemm_tc_rope_kv": 1, "hb_slices_finish": 1, "hb_add_rmsnorm_slices": 1, "hb_rope_kv_slices": 1, "hb_gemm_tc": 1, "hb_gemm_tc_slices": 1, "hb_gemm_stream": 1, "hb_attn_decode": 1, "hb_flash_prefill": 1, "hb_flash_prefill_tc": 1, "hb_flash_diff_tc": 1, "hb_attn_diff_decode": 1, "hb_gemm_tc_grouped": 1}
 _status = None
 
 EPI_F32, EPI_BF16, EPI_ADD_F32, EPI_SWIGLU_BF16, EPI_SLICES, EPI_GEGLU_BF16, EPI_GELU_BF16, EPI_RELU2_BF16 = 0, 1, 2, 3, 4, 5, 6, 7
@@ -170,7 +172,7 @@ class Slices:
     """A small product a @ w.T left as the K slices it was computed in: fp32 [ksplit][rows][row_stride]
     in the scratch that all small products share, so it has to be consumed (or finished) before
     the next of them runs; `check()` raises if it was not."""
-    __slots__ = ("ws", "ksplit", "slice_stride", "row_stride", "M", "N", "K", "gen")
+    __slots__ = ("ws", "ksplit", "slice_stride", "row_stride", "M", "N", "K", "gen")      # (slice_stride: rows of a slice x row_stride)
 
     def check(self):
         if self.gen != _scratch_gen[0]:
@@ -196,7 +198,8 @@ def gemm_stream_slices(a, w) -> Slices:
 def finish_slices(sl: Slices, out, epi):
     """out per `epi` (0 to 3) from slices, as the product's own reduction would have left it."""
     sl.check()
-    _call("hb_gemm_stream_finish", sl.ws.data_ptr(), out.data_ptr(), out.stride(0), sl.M, sl.N, sl.K, epi, _stream())
+    _call("hb_slices_finish", sl.ws.data_ptr(), out.data_ptr(), out.stride(0), sl.M, sl.N, sl.row_stride, sl.slice_stride // sl.row_stride,
+          sl.ksplit, epi, _stream())
     return out
 
 
@@ -228,10 +231,31 @@ def rope_kv_slices(sl: Slices, positions, slot_map, table, q_out, k_cache, v_cac
 
 
 def linear_slices(a, w):
-    """a @ w.T as slices when the small-product kernel applies (a few bf16 rows), else None."""
-    if a.shape[0] > STREAM_MAX_ROWS or not _tc_ok(a, w.t):
+    """a @ w.T as slices when it is computed in slices: a few bf16 rows, or more rows of a product whose tiles are too few for the
+    SMs; else None."""
+    if not _tc_ok(a, w.t):
         return None
+    if a.shape[0] > STREAM_MAX_ROWS:
+        return gemm_tc_slices(a, w.t)
     return gemm_stream_slices(a, w.t)
+
+
+def gemm_tc_slices(a, w):
+    """The CTA-pair kernel with K in slices that are left for the consumer (csrc/gemm_tc.cu); None where it would not split."""
+    M, K = a.shape
+    N = w.shape[0]
+    n = _fn("hb_gemm_tc_splits")(M, N, K)
+    if not n:
+        return None
+    rows, ld = -(-M // 256) * 256, -(-N // 32) * 32
+    ws, _ = _stream_scratch(a.device, n * rows * ld, 0)
+    _scratch_gen[0] += 1
+    _call("hb_gemm_tc_slices", a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), ws.data_ptr(), ld, ws.numel(), M, N, K, n,
+          status_word().data_ptr(), _stream())
+    sl = Slices()
+    sl.ws, sl.ksplit, sl.row_stride, sl.slice_stride = ws, n, ld, rows * ld
+    sl.M, sl.N, sl.K, sl.gen = M, N, K, _scratch_gen[0]
+    return sl
 
 
 

@@ -720,3 +720,50 @@ def test_rows_add_prepares_the_next_norm(M, H, I, Hq, Hkv, D):
     scale = max(1.0, float(q2.float().abs().max()))
     for a, b in ((q1, q2), (kc1, kc2), (vc1, vc2)):      # the two round the activations at different places: bf16 rounding apart
         assert float((a.float() - b.float()).abs().max()) < 2e-2 * scale
+
+
+@pytest.mark.parametrize("epi", ["f32", "bf16", "add", "swiglu"])
+@pytest.mark.parametrize("M,N,K", [(17, 19104, 320), (33, 38016, 72), (64, 18944, 64), (32, 96, 200)])
+def test_unsplit_products_of_17_to_64_rows(epi, M, N, K):
+    """The persistent kernel: one, two and three column blocks a CTA (148 SMs x 128 columns), a ragged last block, K of one and of
+    several stages and no multiple of one; every epilogue, against 64 bits. The bound: 32-bit sums of K products, one rounding
+    to bf16 (2^-8) where the result is, and 2^-6 through the gate's exponential."""
+    a, w = rnd(M, K, seed=91), rnd(N, K, seed=92, scale=0.05)
+    ref = a.double() @ w.double().T
+    acc = K * 2.0 ** -23 * (a.double().abs() @ w.double().abs().T)
+    F = fast()
+    if epi == "swiglu":
+        out = F.gemm_stream(a, w, torch.empty(M, N // 2, dtype=torch.bfloat16, device=DEV), F.EPI_SWIGLU_BF16)
+        g, u = ref.view(M, N // 32, 2, 16).unbind(2)
+        want = (torch.nn.functional.silu(g) * u).reshape(M, N // 2)
+        assert bool(((out.double() - want).abs() <= 2.0 ** -6 * want.abs() + 1e-4).all())
+    elif epi == "bf16":
+        out = F.gemm_stream(a, w, torch.empty(M, N, dtype=torch.bfloat16, device=DEV), F.EPI_BF16)
+        assert bool(((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + acc).all())
+    else:
+        out = torch.full((M + 1, N), 7.0, device=DEV)
+        F.gemm_stream(a, w, out[:M], F.EPI_ADD_F32 if epi == "add" else F.EPI_F32)
+        want = ref + (7.0 if epi == "add" else 0.0)
+        assert bool(((out[:M].double() - want).abs() <= acc + 2.0 ** -21).all()) and bool((out[M] == 7.0).all())
+    sync_check()
+
+
+@pytest.mark.parametrize("M,N,K", [(65, 512, 1024), (300, 776, 1600), (512, 3072, 3072), (257, 64, 4104), (130, 2048, 8192)])
+def test_products_of_few_tiles_in_slices(M, N, K):
+    """More rows than the small-product kernels take, too few tiles for the SMs: the product comes as K slices (ragged last slices and
+    tiles, K no multiple of a block's 64), which finish as the product, into an output of its own and into a residual; the bound
+    is that of 32-bit sums of K products. What the unsplit kernel takes stays with it."""
+    a, w = rnd(M, K, seed=81), rnd(N, K, seed=82, scale=0.05)
+    sl = fast().gemm_tc_slices(a, w)
+    assert sl is not None and 2 <= sl.ksplit <= 8
+    out = torch.full((M + 1, N), 7.0, device=DEV)
+    fast().finish_slices(sl, out[:M], fast().EPI_F32)
+    sync_check()
+    ad, wd = a.double(), w.double()
+    bound = K * 2.0 ** -23 * (ad.abs() @ wd.abs().T)
+    assert bool(((out[:M].double() - ad @ wd.T).abs() <= bound).all()) and bool((out[M] == 7.0).all())
+    x = rnd(M, N, seed=83, dtype=torch.float32)
+    want = x + out[:M]
+    fast().finish_slices(fast().gemm_tc_slices(a, w), x, fast().EPI_ADD_F32)
+    assert torch.equal(x, want)
+    assert fast().gemm_tc_slices(rnd(2048, 512, seed=84), rnd(4096, 512, seed=85)) is None
