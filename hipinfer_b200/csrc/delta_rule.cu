@@ -15,7 +15,7 @@
 // and how many tokens comes from device arrays (first row, row count and state slot of each request), so the
 // launch is the same for every batch of as many requests and replays from a CUDA graph.
 //
-//   delta_rule_kernel      four threads share a value channel, each with D / 4 key channels of it in registers; tokens
+//   delta_rule_kernel      four threads share two value channels, each with D / 4 key channels of them in registers; tokens
 //                          in chunks, what does not depend on the state a chunk at a time (D = 32, 64, 128).
 //   delta_rule_any_kernel  any D: the state in shared memory, a thread per value channel.
 #include "common.cuh"
@@ -104,191 +104,210 @@ __global__ void delta_rule_any_kernel(DeltaArgs A) {
   if (on) for (int i = 0; i < D; i++) Sg[i * D + j] = S[i * D + j];
 }
 
-// TPC threads per value channel, NR key channels each: D = TPC * NR, blockDim = D * TPC. Thread (q, j) holds
-// S[q * NR + i][j], i < NR, in registers; the TPC parts of a sum over key channels meet in shared memory.
+// A thread holds S[q * NR + i][j], i < NR, of two neighbouring value channels j in registers; the four threads q of a channel
+// pair (D = 4 NR) are neighbouring lanes, so the parts of u^T S meet by two shuffles and no thread waits for another warp while
+// the state walks. Two channels a thread halve the reads of the token's vectors, which (with a barrier a token before that)
+// bounded the walk: one read of 16 bytes serves 8 products instead of 4.
 //
-// The tokens go by in chunks of DR_CH. What does not depend on the state is done for a whole chunk at once, a warp per
-// token: the unit key (one warp sum), decay and removal rate (expf), into shared memory; the raw values of the NEXT
-// chunk are already on their way from global memory while the state walks through this one. The walk itself then
-// costs, per token, 4 NR fused multiply-adds a thread, broadcast reads of the token's vectors and ONE barrier (for
-// u^T S, whose parts must meet before the state moves; the parts of the output meet after the chunk). The head norm
-// and the gate of the chunk's outputs are again a warp per token.
-constexpr int DR_CH = 16;
+// The tokens go by in chunks of DR_CH, and the block's warps have two jobs. The first D / 16 warps WALK the state through the
+// chunk at hand: per token 10 NR multiply-adds a thread and its share of the reads. DR_HELP further warps make, meanwhile, what does
+// not depend on the state for the chunk after it, a warp per token (the unit key, decay and removal rate: a warp sum and two
+// expf), and finish the chunk before it (the parts of the outputs added, head norm, gate). The raw values of the chunk after next
+// are then already on their way from global memory. One barrier a chunk. With one job after the other in the same warps the
+// walk stands still meanwhile (32 heads of 64, two requests, 2,048 tokens: 598 us, and 556 without the barrier a
+// token; 551 us with the helpers: the walk itself is what is left).
+constexpr int DR_CH = 16, DR_Q = 4, DR_HELP = 4;
 
-template <typename TW, typename TO, int NR, int TPC>
-__global__ void __launch_bounds__(NR * TPC * TPC, (NR * TPC * TPC <= 256 ? 2 : 1)) delta_rule_kernel(DeltaArgs A) {
-  constexpr int D = NR * TPC, NT = D * TPC, NW = NT / 32, TPW = DR_CH / NW, CPL = D / 32;
-  static_assert(TPW >= 1 && TPW * NW == DR_CH && CPL >= 1 && NR % 4 == 0, "chunk, warps and head size must fit");
-  extern __shared__ __align__(16) float dr_smem[];
-  float* vr = dr_smem;                 // [DR_CH][D] each
-  float* vw = vr + DR_CH * D;
-  float* vau = vw + DR_CH * D;
-  float* vk = vau + DR_CH * D;
-  float* vu = vk + DR_CH * D;
-  float* vv = vu + DR_CH * D;
-  float* vo = vv + DR_CH * D;          // [DR_CH][TPC][D]: the parts of a token's outputs, summed when the chunk is done
-  float* xs = vo + DR_CH * TPC * D;    // [2][TPC][D]: the parts of u^T S of the token at hand (two buffers, one barrier a token)
+template <typename TW, typename TO, int NR>
+__global__ void __launch_bounds__(2 * DR_Q * NR + 32 * DR_HELP, 1) delta_rule_kernel(DeltaArgs A) {
+  constexpr int D = NR * DR_Q, WALKERS = D / 2 * DR_Q, TPW = DR_CH / DR_HELP, CPL = D / 32;
+  static_assert(WALKERS % 32 == 0 && TPW * DR_HELP == DR_CH && CPL >= 1 && NR % 4 == 0, "chunk, warps and head size must fit");
+  // a vector lies in four parts of NR + 4: the lanes of a warp read four places at once, of banks of their own; the rows of the
+  // output's parts are D + 8 apart for the same reason
+  constexpr int SEG = NR + 4, VS = DR_Q * SEG, OS = D + 8, VEC = DR_CH * VS, IN = 5 * VEC + DR_CH * D, OUT = DR_CH * DR_Q * OS;
+  extern __shared__ __align__(16) float dr_smem[];     // [2] inputs of a chunk (r, w, au, k, u [DR_CH][VS] each, v [DR_CH][D]), [2] outputs
   hb_pdl_launch();
   hb_pdl_wait();
-  // a warp's lanes are 32 value channels j with the SAME part q of the key channels: what they read of the token's
-  // vectors is one address for the whole warp (a broadcast, one pass through shared memory)
-  const int h = blockIdx.x, req = blockIdx.y, tid = threadIdx.x, q = tid / D, j = tid % D, lane = tid & 31, warp = tid >> 5;
-  float* Sg = A.state + ((size_t)A.slot[req] * A.heads + h) * D * D;
-  float S[NR];
-#pragma unroll
-  for (int i = 0; i < NR; i++) S[i] = Sg[(q * NR + i) * D + j];
-  const int t0 = A.q_start[req], n = A.q_len[req];
-  const TW* wb = (const TW*)A.w_bias, *ab = (const TW*)A.a_bias, *nwt = (const TW*)A.norm_w;
+  const int h = blockIdx.x, req = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
+  const int t0 = A.q_start[req], n = A.q_len[req], chunks = (n + DR_CH - 1) / DR_CH;
   const int hc = h * D;
-
-  // raw values of a chunk's tokens: warp `warp` takes tokens warp, warp + NW, ..; a lane channels lane, lane + 32, ..
-  float pre[TPW][CPL][5];              // k, r, v, a_raw, w_raw
-  float gate[TPW][CPL];                // the gate's raw values of the chunk being walked (asked for before the walk)
-  float cab[CPL], cwb[CPL], cnw[CPL];  // this lane's channels of the two biases and the norm weight
+  if (tid >= WALKERS) {                  // ---------------- the helpers
+    const int warp = (tid - WALKERS) >> 5;
+    const TW* wb = (const TW*)A.w_bias, *ab = (const TW*)A.a_bias, *nwt = (const TW*)A.norm_w;
+    // raw values of a chunk's tokens: a warp takes tokens warp, warp + DR_HELP, ..; a lane channels lane, lane + 32, ..
+    float pre[TPW][CPL][5];              // k, r, v, a_raw, w_raw
+    float gate[TPW][CPL];                // the gate's raw values of the chunk to be finished next
+    float cab[CPL], cwb[CPL], cnw[CPL];  // this lane's channels of the two biases and the norm weight
 #pragma unroll
-  for (int y = 0; y < CPL; y++) {
-    cab[y] = hb_to_float(ab[hc + lane + 32 * y]);
-    cwb[y] = hb_to_float(wb[hc + lane + 32 * y]);
-    cnw[y] = hb_to_float(nwt[hc + lane + 32 * y]);
-  }
-  auto fetch_gate = [&](int base) {
-#pragma unroll
-    for (int x = 0; x < TPW; x++) {
-      const int tt = warp + x * NW;
-      if (base + tt < n) {
-        const float* row = A.proj + (size_t)(t0 + base + tt) * A.ld;
-#pragma unroll
-        for (int y = 0; y < CPL; y++) gate[x][y] = row[A.g_off + hc + lane + 32 * y];
-      }
+    for (int y = 0; y < CPL; y++) {
+      cab[y] = hb_to_float(ab[hc + lane + 32 * y]);
+      cwb[y] = hb_to_float(wb[hc + lane + 32 * y]);
+      cnw[y] = hb_to_float(nwt[hc + lane + 32 * y]);
     }
-  };
-  auto fetch = [&](int base) {
+    auto fetch_gate = [&](int base) {
 #pragma unroll
-    for (int x = 0; x < TPW; x++) {
-      const int tt = warp + x * NW;
-      if (base + tt < n) {
-        const float* row = A.proj + (size_t)(t0 + base + tt) * A.ld;
-        const float* wrow = A.w_raw + (size_t)(t0 + base + tt) * A.ldw;
+      for (int x = 0; x < TPW; x++) {
+        const int tt = warp + x * DR_HELP;
+        if (base + tt < n) {
+          const float* row = A.proj + (size_t)(t0 + base + tt) * A.ld;
 #pragma unroll
-        for (int y = 0; y < CPL; y++) {
-          const int c = hc + lane + 32 * y;
-          pre[x][y][0] = row[A.k_off + c];
-          pre[x][y][1] = row[A.r_off + c];
-          pre[x][y][2] = row[A.v_off + c];
-          pre[x][y][3] = row[A.a_off + c];
-          pre[x][y][4] = wrow[c];
+          for (int y = 0; y < CPL; y++) gate[x][y] = row[A.g_off + hc + lane + 32 * y];
         }
       }
-    }
-  };
-  fetch(0);
-  for (int base = 0; base < n; base += DR_CH) {
-    // the chunk's vectors into shared memory
+    };
+    auto fetch = [&](int base) {
 #pragma unroll
-    for (int x = 0; x < TPW; x++) {
-      const int tt = warp + x * NW;
-      if (base + tt < n) {                                   // (uniform over the warp)
-        float kk = 0.f;
+      for (int x = 0; x < TPW; x++) {
+        const int tt = warp + x * DR_HELP;
+        if (base + tt < n) {
+          const float* row = A.proj + (size_t)(t0 + base + tt) * A.ld;
+          const float* wrow = A.w_raw + (size_t)(t0 + base + tt) * A.ldw;
 #pragma unroll
-        for (int y = 0; y < CPL; y++) kk = fmaf(pre[x][y][0], pre[x][y][0], kk);
-        kk = hb_warp_sum(kk);
-        const float inv = 1.f / sqrtf(kk + A.unit_eps);
-#pragma unroll
-        for (int y = 0; y < CPL; y++) {
-          const int cl = lane + 32 * y;
-          const float kj = pre[x][y][0], uj = kj * inv;
-          vk[tt * D + cl] = kj;
-          vu[tt * D + cl] = uj;
-          vr[tt * D + cl] = pre[x][y][1];
-          vv[tt * D + cl] = pre[x][y][2];
-          vau[tt * D + cl] = sigmoidf_(pre[x][y][3] + cab[y]) * uj;
-          vw[tt * D + cl] = expf(-A.decay_scale * sigmoidf_(pre[x][y][4] + cwb[y]));
+          for (int y = 0; y < CPL; y++) {
+            const int c = hc + lane + 32 * y;
+            pre[x][y][0] = row[A.k_off + c];
+            pre[x][y][1] = row[A.r_off + c];
+            pre[x][y][2] = row[A.v_off + c];
+            pre[x][y][3] = row[A.a_off + c];
+            pre[x][y][4] = wrow[c];
+          }
         }
       }
-    }
+    };
+    auto prepare = [&](int c) {          // the fetched chunk's vectors into shared memory
+      float* vr = dr_smem + (c & 1) * IN, *vw = vr + VEC, *vau = vw + VEC, *vk = vau + VEC, *vu = vk + VEC, *vv = vu + VEC;
+#pragma unroll
+      for (int x = 0; x < TPW; x++) {
+        const int tt = warp + x * DR_HELP;
+        if (c * DR_CH + tt < n) {                            // (uniform over the warp)
+          float kk = 0.f;
+#pragma unroll
+          for (int y = 0; y < CPL; y++) kk = fmaf(pre[x][y][0], pre[x][y][0], kk);
+          kk = hb_warp_sum(kk);
+          const float inv = 1.f / sqrtf(kk + A.unit_eps);
+#pragma unroll
+          for (int y = 0; y < CPL; y++) {
+            const int cl = lane + 32 * y, at = tt * VS + cl / NR * SEG + cl % NR;
+            const float kj = pre[x][y][0], uj = kj * inv;
+            vk[at] = kj;
+            vu[at] = uj;
+            vr[at] = pre[x][y][1];
+            vv[tt * D + cl] = pre[x][y][2];
+            vau[at] = sigmoidf_(pre[x][y][3] + cab[y]) * uj;
+            vw[at] = expf(-A.decay_scale * sigmoidf_(pre[x][y][4] + cwb[y]));
+          }
+        }
+      }
+    };
+    auto finish = [&](int c) {           // a walked chunk's outputs: head norm, weight and gate
+      const float* vo = dr_smem + 2 * IN + (c & 1) * OUT;
+#pragma unroll
+      for (int x = 0; x < TPW; x++) {
+        const int tt = warp + x * DR_HELP;
+        if (c * DR_CH + tt < n) {
+          float ov[CPL], oo = 0.f;
+#pragma unroll
+          for (int y = 0; y < CPL; y++) {
+            ov[y] = vo[tt * DR_Q * OS + lane + 32 * y];
+#pragma unroll
+            for (int qq = 1; qq < DR_Q; qq++) ov[y] += vo[(tt * DR_Q + qq) * OS + lane + 32 * y];
+            oo = fmaf(ov[y], ov[y], oo);
+          }
+          oo = hb_warp_sum(oo);
+          const float f = rsqrtf(oo / (float)D + A.eps);
+          const size_t t = (size_t)(t0 + c * DR_CH + tt);
+#pragma unroll
+          for (int y = 0; y < CPL; y++) {
+            const int cc = hc + lane + 32 * y;
+            ((TO*)A.out)[t * A.heads * D + cc] = hb_from_float<TO>(ov[y] * f * cnw[y] * sigmoidf_(gate[x][y]));
+          }
+        }
+      }
+    };
+    fetch(0);
+    prepare(0);
+    fetch(DR_CH);
     __syncthreads();
-    fetch_gate(base);                                        // both in flight during the walk
-    if (base + DR_CH < n) fetch(base + DR_CH);
-    const int m = min(DR_CH, n - base);
-    for (int tt = 0; tt < m; tt++) {
-      // (heads of up to 64) all of the token's vectors are asked for at once: one wait for shared memory a token
-      constexpr bool HOIST = NR <= 16;
-      const float4* up = (const float4*)(vu + tt * D + q * NR);
-      const float4* kp = (const float4*)(vk + tt * D + q * NR);
-      const float4* wp = (const float4*)(vw + tt * D + q * NR);
-      const float4* ap = (const float4*)(vau + tt * D + q * NR);
-      const float4* rp = (const float4*)(vr + tt * D + q * NR);
-      float4 u[HOIST ? NR / 4 : 1], k[HOIST ? NR / 4 : 1], w[HOIST ? NR / 4 : 1], a[HOIST ? NR / 4 : 1], r[HOIST ? NR / 4 : 1];
-      if (HOIST) {
-#pragma unroll
-        for (int i = 0; i < NR / 4; i++) { u[i] = up[i]; k[i] = kp[i]; w[i] = wp[i]; a[i] = ap[i]; r[i] = rp[i]; }
+    for (int c = 0; c < chunks; c++) {
+      if (c > 0) finish(c - 1);
+      fetch_gate(c * DR_CH);
+      if (c + 1 < chunks) {
+        prepare(c + 1);
+        fetch((c + 2) * DR_CH);
       }
-      const float vj = vv[tt * D + j];
-      float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-#pragma unroll
-      for (int i = 0; i < NR / 4; i++) {
-        const float4 uu = HOIST ? u[i] : up[i];
-        s0 = fmaf(uu.x, S[4 * i], s0); s1 = fmaf(uu.y, S[4 * i + 1], s1);
-        s2 = fmaf(uu.z, S[4 * i + 2], s2); s3 = fmaf(uu.w, S[4 * i + 3], s3);
-      }
-      float* x = xs + (tt & 1) * TPC * D;
-      x[q * D + j] = (s0 + s1) + (s2 + s3);
       __syncthreads();
-      float sa = x[j];
+    }
+    if (chunks > 0) finish(chunks - 1);
+    return;
+  }
+  // ---------------- the walkers
+  const int q = lane & 3, j = (tid >> 2) * 2;
+  float* Sg = A.state + ((size_t)A.slot[req] * A.heads + h) * D * D;
+  float S[NR][2];
 #pragma unroll
-      for (int qq = 1; qq < TPC; qq++) sa += x[qq * D + j];
-      float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
+  for (int i = 0; i < NR; i++) {
+    const float2 v = *(const float2*)(Sg + (q * NR + i) * D + j);
+    S[i][0] = v.x;
+    S[i][1] = v.y;
+  }
+  __syncthreads();
+  for (int ch = 0; ch < chunks; ch++) {
+    const float* vr = dr_smem + (ch & 1) * IN, *vw = vr + VEC, *vau = vw + VEC, *vk = vau + VEC, *vu = vk + VEC, *vv = vu + VEC;
+    float* vo = dr_smem + 2 * IN + (ch & 1) * OUT;
+    const int m = min(DR_CH, n - ch * DR_CH);
+    for (int tt = 0; tt < m; tt++) {
+      const int at = tt * VS + q * SEG;
+      float4 u[NR / 4];
+#pragma unroll
+      for (int i = 0; i < NR / 4; i++) u[i] = *(const float4*)(vu + at + 4 * i);
+      const float2 v2 = *(const float2*)(vv + tt * D + j);
+      const float vj[2] = {v2.x, v2.y};
+      float sa[2];
+#pragma unroll
+      for (int c = 0; c < 2; c++) {
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+        for (int i = 0; i < NR / 4; i++) {
+          s0 = fmaf(u[i].x, S[4 * i][c], s0); s1 = fmaf(u[i].y, S[4 * i + 1][c], s1);
+          s2 = fmaf(u[i].z, S[4 * i + 2][c], s2); s3 = fmaf(u[i].w, S[4 * i + 3][c], s3);
+        }
+        sa[c] = (s0 + s1) + (s2 + s3);
+      }
+#pragma unroll
+      for (int o = 1; o < DR_Q; o <<= 1)
+#pragma unroll
+        for (int c = 0; c < 2; c++) sa[c] += __shfl_xor_sync(0xffffffffu, sa[c], o);
+      float o[2][4] = {};
 #pragma unroll
       for (int i = 0; i < NR / 4; i++) {
-        const float4 kk = HOIST ? k[i] : kp[i], ww = HOIST ? w[i] : wp[i], aa = HOIST ? a[i] : ap[i], rr = HOIST ? r[i] : rp[i];
-        S[4 * i] = fmaf(kk.x, vj, fmaf(ww.x, S[4 * i], -aa.x * sa));             o0 = fmaf(S[4 * i], rr.x, o0);
-        S[4 * i + 1] = fmaf(kk.y, vj, fmaf(ww.y, S[4 * i + 1], -aa.y * sa));     o1 = fmaf(S[4 * i + 1], rr.y, o1);
-        S[4 * i + 2] = fmaf(kk.z, vj, fmaf(ww.z, S[4 * i + 2], -aa.z * sa));     o2 = fmaf(S[4 * i + 2], rr.z, o2);
-        S[4 * i + 3] = fmaf(kk.w, vj, fmaf(ww.w, S[4 * i + 3], -aa.w * sa));     o3 = fmaf(S[4 * i + 3], rr.w, o3);
+        const float4 kk = *(const float4*)(vk + at + 4 * i), ww = *(const float4*)(vw + at + 4 * i);
+        const float4 aa = *(const float4*)(vau + at + 4 * i), rr = *(const float4*)(vr + at + 4 * i);
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+          S[4 * i][c] = fmaf(kk.x, vj[c], fmaf(ww.x, S[4 * i][c], -aa.x * sa[c]));             o[c][0] = fmaf(S[4 * i][c], rr.x, o[c][0]);
+          S[4 * i + 1][c] = fmaf(kk.y, vj[c], fmaf(ww.y, S[4 * i + 1][c], -aa.y * sa[c]));     o[c][1] = fmaf(S[4 * i + 1][c], rr.y, o[c][1]);
+          S[4 * i + 2][c] = fmaf(kk.z, vj[c], fmaf(ww.z, S[4 * i + 2][c], -aa.z * sa[c]));     o[c][2] = fmaf(S[4 * i + 2][c], rr.z, o[c][2]);
+          S[4 * i + 3][c] = fmaf(kk.w, vj[c], fmaf(ww.w, S[4 * i + 3][c], -aa.w * sa[c]));     o[c][3] = fmaf(S[4 * i + 3][c], rr.w, o[c][3]);
+        }
       }
-      vo[(tt * TPC + q) * D + j] = (o0 + o1) + (o2 + o3);
+      *(float2*)(vo + (tt * DR_Q + q) * OS + j) = make_float2((o[0][0] + o[0][1]) + (o[0][2] + o[0][3]), (o[1][0] + o[1][1]) + (o[1][2] + o[1][3]));
     }
     __syncthreads();
-    // the chunk's outputs: head norm, weight and gate, a warp per token
-#pragma unroll
-    for (int x = 0; x < TPW; x++) {
-      const int tt = warp + x * NW;
-      if (base + tt < n) {
-        float ov[CPL], oo = 0.f;
-#pragma unroll
-        for (int y = 0; y < CPL; y++) {
-          ov[y] = vo[tt * TPC * D + lane + 32 * y];
-#pragma unroll
-          for (int qq = 1; qq < TPC; qq++) ov[y] += vo[(tt * TPC + qq) * D + lane + 32 * y];
-          oo = fmaf(ov[y], ov[y], oo);
-        }
-        oo = hb_warp_sum(oo);
-        const float f = rsqrtf(oo / (float)D + A.eps);
-        const size_t t = (size_t)(t0 + base + tt);
-#pragma unroll
-        for (int y = 0; y < CPL; y++) {
-          const int c = hc + lane + 32 * y;
-          ((TO*)A.out)[t * A.heads * D + c] = hb_from_float<TO>(ov[y] * f * cnw[y] * sigmoidf_(gate[x][y]));
-        }
-      }
-    }
   }
 #pragma unroll
-  for (int i = 0; i < NR; i++) Sg[(q * NR + i) * D + j] = S[i];
+  for (int i = 0; i < NR; i++) *(float2*)(Sg + (q * NR + i) * D + j) = make_float2(S[i][0], S[i][1]);
 }
 
-template <typename TW, typename TO, int NR, int TPC>
+template <typename TW, typename TO, int NR>
 static int delta_rule_launch_reg(const DeltaArgs& A, dim3 grid, cudaStream_t s) {
-  constexpr int D = NR * TPC;
-  const size_t smem = ((size_t)(6 + TPC) * DR_CH * D + 2 * TPC * D) * sizeof(float);
-  auto kern = delta_rule_kernel<TW, TO, NR, TPC>;
-  static bool configured = false;
-  if (!configured && smem > 48 * 1024) {
+  constexpr int D = NR * DR_Q;
+  const size_t smem = 2 * ((size_t)5 * DR_CH * DR_Q * (NR + 4) + DR_CH * D + (size_t)DR_CH * DR_Q * (D + 8)) * sizeof(float);
+  auto kern = delta_rule_kernel<TW, TO, NR>;
+  if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) HB_FAIL("hb_delta_rule: %s", cudaGetErrorString(e));
-    configured = true;
   }
-  hb_launch(kern, grid, D * TPC, smem, s, A);
+  hb_launch(kern, grid, 2 * D + 32 * DR_HELP, smem, s, A);
   return 0;
 }
 
@@ -296,9 +315,9 @@ template <typename TW, typename TO>
 static int delta_rule_launch(const DeltaArgs& A, int R, cudaStream_t s) {
   const dim3 grid(A.heads, R);
   switch (A.D) {
-    case 32: return delta_rule_launch_reg<TW, TO, 8, 4>(A, grid, s);
-    case 64: return delta_rule_launch_reg<TW, TO, 16, 4>(A, grid, s);
-    case 128: return delta_rule_launch_reg<TW, TO, 32, 4>(A, grid, s);
+    case 32: return delta_rule_launch_reg<TW, TO, 8>(A, grid, s);
+    case 64: return delta_rule_launch_reg<TW, TO, 16>(A, grid, s);
+    case 128: return delta_rule_launch_reg<TW, TO, 32>(A, grid, s);
     default: break;
   }
   const int threads = (A.D + 31) / 32 * 32;
