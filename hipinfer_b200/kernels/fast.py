@@ -50,6 +50,7 @@ _SIGS = {
 _fns = {}
 _LAUNCHES = {"hb_rows_scaled_qkv_rope": 1, "hb_rows_scaled_swiglu": 1, "hb_rows_norm_qkv_rope": 1, "hb_rows_add": 1, "hb_rows_norm_swiglu": 1, "hb_gemm_tc_rope_kv": 1, "hb_slices_finish": 1, "hb_add_rmsnorm_slices": 1, "hb_rope_kv_slices": 1, "hb_gemm_tc": 1, "hb_gemm_tc_slices": 1, "hb_gemm_stream": 1, "hb_attn_decode": 1, "hb_flash_prefill": 1, "hb_flash_prefill_tc": 1, "hb_flash_diff_tc": 1, "hb_attn_diff_decode": 1, "hb_gemm_tc_grouped": 1}
 _status = None
+_status_address = None
 
 EPI_F32, EPI_BF16, EPI_ADD_F32, EPI_SWIGLU_BF16, EPI_SLICES, EPI_GEGLU_BF16, EPI_GELU_BF16, EPI_RELU2_BF16 = 0, 1, 2, 3, 4, 5, 6, 7
 ACT_EPILOGUES = {"gelu": EPI_GELU_BF16, "relu2": EPI_RELU2_BF16}
@@ -87,6 +88,13 @@ def status_word() -> torch.Tensor:
     return _status
 
 
+def _status_ptr() -> int:
+    global _status_address
+    if _status_address is None:
+        _status_address = status_word().data_ptr()
+    return _status_address
+
+
 def check_status() -> None:
     """Call after a synchronisation: raises if a kernel gave up on a wait since the last check."""
     if _status is not None and int(_status[0]) != 0:
@@ -99,12 +107,11 @@ def wait_selftest(polls: int = 4096) -> torch.Tensor:
     `polls` polls, raises the status word, frees its tensor memory and returns. Returns its two result words
     (on the device): [the wait completed, the block's abort flag]. check_status() raises after it."""
     out = torch.zeros(2, dtype=torch.int32, device="cuda")
-    _call("hb_wait_selftest", status_word().data_ptr(), int(polls), out.data_ptr(), _stream())
+    _call("hb_wait_selftest", _status_ptr(), int(polls), out.data_ptr(), _stream())
     return out
 
 
-def _stream():
-    return library.current_stream()
+_stream = library.current_stream
 
 
 def _tc_ok(a, w) -> bool:
@@ -117,7 +124,7 @@ def gemm_tc(a, w, out, epi, tile_n=0):
     M, K = a.shape
     N = w.shape[0]
     _call("hb_gemm_tc", a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), M, N, K,
-          epi, tile_n, status_word().data_ptr(), _stream())
+          epi, tile_n, _status_ptr(), _stream())
     return out
 
 
@@ -164,7 +171,7 @@ def gemm_stream(a, w, out, epi):
     if stream_plan(N, K)[1] > 1 and M >= 8:
         library.launches[0] += 1     # the slices are added by a kernel of its own (counted here, launched by the call below)
     _call("hb_gemm_stream", a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), M, N, K,
-          epi, ws.data_ptr(), ws.numel(), cnt.data_ptr(), cnt.numel(), status_word().data_ptr(), _stream())
+          epi, ws.data_ptr(), ws.numel(), cnt.data_ptr(), cnt.numel(), _status_ptr(), _stream())
     return out
 
 
@@ -188,7 +195,7 @@ def gemm_stream_slices(a, w) -> Slices:
     ws, cnt = _stream_scratch(a.device, per_token * nt, n_blocks)
     _scratch_gen[0] += 1
     _call("hb_gemm_stream", a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), None, 0, M, N, K, EPI_SLICES,
-          ws.data_ptr(), ws.numel(), cnt.data_ptr(), cnt.numel(), status_word().data_ptr(), _stream())
+          ws.data_ptr(), ws.numel(), cnt.data_ptr(), cnt.numel(), _status_ptr(), _stream())
     sl = Slices()
     sl.ws, sl.ksplit, sl.row_stride, sl.slice_stride = ws, ksplit, n_blocks * 128, nt * n_blocks * 128
     sl.M, sl.N, sl.K, sl.gen = M, N, K, _scratch_gen[0]
@@ -251,7 +258,7 @@ def gemm_tc_slices(a, w):
     ws, _ = _stream_scratch(a.device, n * rows * ld, 0)
     _scratch_gen[0] += 1
     _call("hb_gemm_tc_slices", a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), ws.data_ptr(), ld, ws.numel(), M, N, K, n,
-          status_word().data_ptr(), _stream())
+          _status_ptr(), _stream())
     sl = Slices()
     sl.ws, sl.ksplit, sl.row_stride, sl.slice_stride = ws, n, ld, rows * ld
     sl.M, sl.N, sl.K, sl.gen = M, N, K, _scratch_gen[0]
@@ -295,7 +302,7 @@ def linear_rope_kv(a, w, positions, slot_map, table, q_out, k_cache, v_cache, n_
     p = lambda t: None if t is None else t.data_ptr()
     _call("hb_gemm_tc_rope_kv", a.data_ptr(), a.stride(0), w.t.data_ptr(), w.t.stride(0), a.shape[0], a.shape[1],
           positions.data_ptr(), p(slot_map), table.data_ptr(), q_out.data_ptr(), p(k_cache) if slot_map is not None else None,
-          p(v_cache) if slot_map is not None else None, n_heads, n_kv_heads, head_dim, page_size, status_word().data_ptr(),
+          p(v_cache) if slot_map is not None else None, n_heads, n_kv_heads, head_dim, page_size, _status_ptr(),
           _stream())
     return True
 
@@ -329,7 +336,7 @@ def grouped_linear(a, w, offsets, out, src, score, at_output, tile_n=0) -> bool:
     p = lambda t: None if t is None else t.data_ptr()
     _call("hb_gemm_tc_grouped", a.data_ptr(), a.stride(0), w.data_ptr(), E, N, K, offsets.data_ptr(), out.data_ptr(), out.stride(0),
           a.shape[0], EPI_SWIGLU_BF16 if gated else EPI_F32, p(src), p(score), 1 if at_output else 0, int(tile_n),
-          status_word().data_ptr(), _stream())
+          _status_ptr(), _stream())
     return True
 
 
@@ -381,7 +388,7 @@ def rows_norm_qkv_rope(x, norm_w, eps, w, positions, slot_map, table, q_out, k_c
     _call("hb_rows_norm_qkv_rope", x.data_ptr(), x.stride(0), norm_w.data_ptr(), float(eps), w.data_ptr(), w.stride(0),
           x.shape[0], x.shape[1], positions.data_ptr(), p(slot_map), table.data_ptr(), q_out.data_ptr(),
           p(k_cache) if slot_map is not None else None, p(v_cache) if slot_map is not None else None, n_heads, n_kv_heads,
-          head_dim, page_size, status_word().data_ptr(), _stream())
+          head_dim, page_size, _status_ptr(), _stream())
     return True
 
 
@@ -416,7 +423,7 @@ def rows_add(act, w, out, feed: "NormFeed" = None, store: bool = False) -> bool:
     _call("hb_rows_add", act.data_ptr(), act.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), M, w.shape[0],
           K, None if feed is None else feed.weight.data_ptr(), None if feed is None else feed.xb.data_ptr(),
           0 if feed is None else feed.xb.stride(0), None if feed is None else feed.ssq.data_ptr(), 1 if store else 0,
-          status_word().data_ptr(), _stream())
+          _status_ptr(), _stream())
     if feed is not None:
         feed.filled = True
     return True
@@ -442,7 +449,7 @@ def rows_scaled_qkv_rope(feed, M, w, positions, slot_map, table, q_out, k_cache,
     _call("hb_rows_scaled_qkv_rope", feed.xb.data_ptr(), feed.xb.stride(0), feed.ssq.data_ptr(), feed.ssq.shape[0], feed.eps,
           w.data_ptr(), w.stride(0), M, w.shape[1], positions.data_ptr(), p(slot_map), table.data_ptr(), q_out.data_ptr(),
           p(k_cache) if slot_map is not None else None, p(v_cache) if slot_map is not None else None, n_heads, n_kv_heads,
-          head_dim, page_size, status_word().data_ptr(), _stream())
+          head_dim, page_size, _status_ptr(), _stream())
     return True
 
 
@@ -453,7 +460,7 @@ def rows_scaled_swiglu(feed, M, w, act_out, group) -> bool:
         return False
     _call("hb_rows_scaled_swiglu", feed.xb.data_ptr(), feed.xb.stride(0), feed.ssq.data_ptr(), feed.ssq.shape[0], feed.eps,
           w.data_ptr(), w.stride(0), act_out.data_ptr(), act_out.stride(0), M, w.shape[0], w.shape[1],
-          status_word().data_ptr(), _stream())
+          _status_ptr(), _stream())
     return True
 
 
@@ -463,7 +470,7 @@ def rows_norm_swiglu(x, norm_w, eps, w, act_out, group) -> bool:
             or act_out.stride(1) != 1):
         return False
     _call("hb_rows_norm_swiglu", x.data_ptr(), x.stride(0), norm_w.data_ptr(), float(eps), w.data_ptr(), w.stride(0),
-          act_out.data_ptr(), act_out.stride(0), x.shape[0], w.shape[0], x.shape[1], status_word().data_ptr(), _stream())
+          act_out.data_ptr(), act_out.stride(0), x.shape[0], w.shape[0], x.shape[1], _status_ptr(), _stream())
     return True
 
 
@@ -512,7 +519,7 @@ def attention_decode(q, k_cache, v_cache, block_table, row_request, positions, o
           None if ws is None else ws.data_ptr(), None if cnt is None else cnt.data_ptr(), T, n_heads, n_kv_heads,
           head_dim, page_size, int(window), float(scale), chunk, int(max_pos),
           None if q_len is None else q_len.data_ptr(), int(row_limit), None if ctx_len is None else ctx_len.data_ptr(),
-          status_word().data_ptr(), *_extras(distance, sink), None if row_list is None else row_list.data_ptr(), _stream())
+          _status_ptr(), *_extras(distance, sink), None if row_list is None else row_list.data_ptr(), _stream())
     return out
 
 
@@ -547,7 +554,7 @@ def flash_prefill_tc(q, k_cache, v_cache, block_table, q_start, q_len, ctx_len, 
     _call("hb_flash_prefill_tc", q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), k_cache.shape[0],
           block_table.data_ptr(), block_table.stride(0), q_start.data_ptr(), q_len.data_ptr(), ctx_len.data_ptr(),
           out.data_ptr(), q.shape[0], q_len.numel(), int(max_q_len), n_heads, n_kv_heads, head_dim, page_size, int(window),
-          float(scale), int(min_rows), status_word().data_ptr(), *_extras(distance, sink), _stream())
+          float(scale), int(min_rows), _status_ptr(), *_extras(distance, sink), _stream())
     return out
 
 
@@ -568,7 +575,7 @@ def flash_diff_tc(q, k_cache, v_cache, batch, block_table, out, n_heads, n_kv_he
           block_table.stride(0), batch.req_q_start.data_ptr(), batch.req_q_len.data_ptr(), batch.req_ctx_len.data_ptr(),
           None if gate is None else gate.data_ptr(), ld, int(gate_offset), out.data_ptr(), q.shape[0], batch.n_requests,
           batch.max_q_len, n_heads, n_kv_heads, dim, vdim, page_size, int(window), float(scale), float(lam), float(post), float(eps),
-          int(min_rows), status_word().data_ptr(), _stream())
+          int(min_rows), _status_ptr(), _stream())
     return True
 
 
@@ -590,7 +597,7 @@ def attention_diff_decode(q, k_cache, v_cache, batch, block_table, out, n_heads,
           block_table.stride(0), None if rows_are_requests else batch.row_request.data_ptr(), batch.positions.data_ptr(), p(gate),
           0 if gate is None else gate.stride(0), int(gate_offset), out.data_ptr(), p(ws), p(cnt), T, n_heads, n_kv_heads, D, page_size,
           int(window), float(scale), float(lam), float(post), float(eps), int(max_pos), p(q_len), int(row_limit),
-          batch.req_ctx_len.data_ptr(), status_word().data_ptr(), _stream())
+          batch.req_ctx_len.data_ptr(), _status_ptr(), _stream())
     return True
 
 

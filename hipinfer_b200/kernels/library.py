@@ -170,13 +170,21 @@ def build_all(verbose: bool = True) -> List[str]:
     return [build(n, verbose) for n in LIBRARIES]
 
 
+_raw_stream = None
+
+
 def current_stream() -> int:
     """torch's current CUDA stream on the current device, as a raw cudaStream_t. A step launches more than a
     hundred kernels: torch.cuda.current_stream() builds a Stream object each time (several microseconds), the
-    raw accessor does not."""
-    import torch
+    raw accessor (found once) does not."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
 
-    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    if raw is not None:
-        return raw(torch._C._cuda_getDevice())
-    return torch.cuda.current_stream().cuda_stream
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        if raw is not None:
+            device = torch._C._cuda_getDevice
+            _raw_stream = lambda: raw(device())
+        else:
+            _raw_stream = lambda: torch.cuda.current_stream().cuda_stream
+    return _raw_stream()

@@ -14,7 +14,7 @@ from typing import Optional
 
 import torch
 
-from . import library
+from . import fast, library
 
 _DT = {torch.float32: 0, torch.bfloat16: 1}
 _p, _i, _l, _f = C.c_void_p, C.c_int, C.c_long, C.c_float
@@ -145,8 +145,6 @@ def check_device_status() -> None:
     gave up on one of its bounded waits since the last call (its output is not valid), and clears the word.
     It reads one word of pinned host memory. The reference's counterpart: HI_CHECK after its calls
     (src/hip_compat.h:95-97) and the -1 of its entry points (src/api.cu:1827-1839)."""
-    from . import fast
-
     fast.check_status()
 
 
@@ -360,8 +358,6 @@ def attention_window(q, k_cache, v_cache, batch, group: int, out, n_heads: int, 
     gate_ld = gate.stride(0) if gate is not None else 0
     # requests that bring WINDOW_FLASH_MIN_ROWS rows or more go to the tensor-core kernel (bfloat16, two maps, the sizes it
     # takes), the other rows of the step to the row kernel; a decode-only step is the row kernel alone
-    from . import fast
-
     flash = (maps == 2 and norm and q.dtype == torch.bfloat16 and not fast.PLAIN_ONLY and not force_rows
              and getattr(batch, "max_q_len", 0) >= WINDOW_FLASH_MIN_ROWS
              and _fn("mixers", "hb_attn_window_flash_supported")(n_heads, n_kv_heads, dim, vdim, maps) == 1
@@ -424,8 +420,6 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, out: torch.Tensor
     _need_cuda(x, weight, out, rows)
     M, H = out.shape
     if pending is not None:
-        from . import fast
-
         if pending.out is x and pending.accumulate and fast.add_rmsnorm_slices_ok(x, pending.slices, weight, out):
             return fast.add_rmsnorm_slices(x, pending.slices, weight, eps, out, rows)
         pending.finish()
@@ -497,8 +491,6 @@ def rope_kv_write(qkv: torch.Tensor, positions: torch.Tensor, slot_map: Optional
     written yet, its K slices are added here (in the same kernel where that applies)."""
     _need_cuda(qkv, positions, slot_map, table, q_out, k_cache, v_cache)
     if pending is not None:
-        from . import fast
-
         if (pending.out is qkv and not pending.accumulate and rotary_dim == head_dim and head_dim % 8 == 0
                 and q_out.dtype == torch.bfloat16 and q_out.is_contiguous()
                 and (slot_map is None or (k_cache.dtype == torch.bfloat16 and k_cache.is_contiguous() and v_cache.is_contiguous()))):
@@ -525,8 +517,6 @@ def linear_rope_kv_write(a: torch.Tensor, w: "Weight", positions: torch.Tensor, 
                          page_size: int) -> bool:
     """rope_kv_write of a @ w.T in one kernel, where one takes these sizes; False: nothing was done
     (the caller projects, then rotates). The results are the same bits either way."""
-    from . import fast
-
     if not a.is_cuda:
         return False
     return fast.linear_rope_kv(a, w, positions, slot_map, table, q_out, k_cache, v_cache, n_heads, n_kv_heads, head_dim,
@@ -657,8 +647,6 @@ class Weight:
 def linear(a: torch.Tensor, w: Weight, out: torch.Tensor, accumulate: bool = False) -> torch.Tensor:
     """out (+)= a @ w.T. bfloat16 operands go to the tensor-core kernels when those take the
     sizes; everything else to the plain 32-bit kernel."""
-    from . import fast
-
     if fast.linear(a, w, out, accumulate):
         return out
     return gemm_plain(a, w.t, out, accumulate)
@@ -675,8 +663,6 @@ def linear_into_stream(a: torch.Tensor, w: Weight, x: torch.Tensor) -> torch.Ten
 def linear_rows32(a: torch.Tensor, w: Weight, out: torch.Tensor) -> torch.Tensor:
     """out = a @ w.T as 32-bit rows for a 32-bit consumer. For a few bfloat16 rows the whole-K rows kernel (one kernel
     instead of a split-K product and the reduction of its slices); else `linear`."""
-    from . import fast
-
     if (a.is_cuda and a.dtype == torch.bfloat16 and out.dtype == torch.float32 and out.is_contiguous() and a.shape[0] <= fast.ROWS_MAX
             and fast.rows_add(a, w.t, out, store=True)):
         return out
@@ -687,8 +673,6 @@ def linear_scaled_add(a: torch.Tensor, w: Weight, x: torch.Tensor, scale: torch.
     """x[m, n] += scale[n] * (a @ w.T)[m, n]: an output projection times the layer's scale vector, added into the float32
     residual stream. One kernel with the plain product; the tensor-core product leaves its float32 result to a small
     kernel that scales and adds."""
-    from . import fast
-
     M, N = a.shape[0], w.shape[0]
     if fast._tc_ok(a, w.t):
         y = torch.empty(M, N, dtype=torch.float32, device=a.device)
@@ -708,8 +692,6 @@ def linear_scaled_add(a: torch.Tensor, w: Weight, x: torch.Tensor, scale: torch.
 
 def linear_swiglu(a: torch.Tensor, w_gate_up: Weight, act_out: torch.Tensor, group: int) -> torch.Tensor:
     """act_out = swiglu(a @ w_gate_up.T) for a gate/up matrix interleaved in groups of `group` rows."""
-    from . import fast
-
     if fast.linear_swiglu(a, w_gate_up, act_out, group):
         return act_out
     gu = torch.empty(a.shape[0], w_gate_up.shape[0], dtype=torch.float32, device=a.device)
@@ -742,8 +724,6 @@ class LazyNorm:
 
 def lazy_norm_applies(x: torch.Tensor, weight: torch.Tensor, dtype) -> bool:
     """Whether a consumer could fold this norm into its product: a few bf16-path rows on the device."""
-    from . import fast
-
     return (x.is_cuda and dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.dtype == torch.float32
             and x.shape[0] <= fast.ROWS_MAX and not fast.PLAIN_ONLY)
 
@@ -751,8 +731,6 @@ def lazy_norm_applies(x: torch.Tensor, weight: torch.Tensor, dtype) -> bool:
 def norm_linear_rope_kv_write(xn: "LazyNorm", w: "Weight", positions, slot_map, table, q_out, k_cache, v_cache, n_heads,
                               n_kv_heads, head_dim, rotary_dim, page_size) -> bool:
     """rope_kv_write of RMSNorm(x) @ w.T in one kernel for a few rows; False: nothing was done."""
-    from . import fast
-
     if xn.feed is not None and fast.rows_scaled_qkv_rope(xn.feed, xn.x.shape[0], w.t, positions, slot_map, table, q_out, k_cache,
                                                          v_cache, n_heads, n_kv_heads, head_dim, rotary_dim, page_size):
         return True
@@ -762,8 +740,6 @@ def norm_linear_rope_kv_write(xn: "LazyNorm", w: "Weight", positions, slot_map, 
 
 def norm_linear_swiglu(xn: "LazyNorm", w_gate_up: "Weight", act_out: torch.Tensor, group: int) -> bool:
     """act_out = swiglu(RMSNorm(x) @ w_gate_up.T) in one kernel for a few rows; False: nothing was done."""
-    from . import fast
-
     if xn.feed is not None and fast.rows_scaled_swiglu(xn.feed, xn.x.shape[0], w_gate_up.t, act_out, group):
         return True
     return fast.rows_norm_swiglu(xn.x, xn.weight, xn.eps, w_gate_up.t, act_out, group)
@@ -772,15 +748,11 @@ def norm_linear_swiglu(xn: "LazyNorm", w_gate_up: "Weight", act_out: torch.Tenso
 def linear_add_rows(a: torch.Tensor, w: "Weight", out: torch.Tensor, norm_feed=None) -> bool:
     """out += a @ w.T finished in one kernel for a few rows (whole-K stripes, nothing left to add); False: nothing was done.
     norm_feed (a fast.NormFeed of the norm that reads `out` next, or None): the kernel prepares that norm on its way."""
-    from . import fast
-
     return a.is_cuda and a.shape[0] <= fast.ROWS_MAX and fast.rows_add(a, w.t, out, norm_feed)
 
 
 def make_norm_feed(weight: torch.Tensor, eps: float, rows: int):
     """A NormFeed for the norm (weight, eps) over `rows` residual rows, where the rows kernels apply; else None."""
-    from . import fast
-
     return fast.NormFeed(weight, eps, rows) if fast.norm_feed_applies(weight, rows) else None
 
 
@@ -795,8 +767,6 @@ class Pending:
         self.slices, self.out, self.accumulate = slices, out, accumulate
 
     def finish(self):
-        from . import fast
-
         fast.finish_slices(self.slices, self.out, fast.EPI_ADD_F32 if self.accumulate else fast.EPI_F32)
         return self.out
 
@@ -804,8 +774,6 @@ class Pending:
 def linear_deferred(a: torch.Tensor, w: Weight, out: torch.Tensor, accumulate: bool = False) -> Optional[Pending]:
     """out (+)= a @ w.T, with the last step (adding the K slices of a small product) left to the
     consumer where that applies: then a Pending comes back and `out` is not yet written. None: out is done."""
-    from . import fast
-
     if out.dtype == torch.float32 and a.is_cuda:
         sl = fast.linear_slices(a, w)
         if sl is not None:
@@ -816,8 +784,6 @@ def linear_deferred(a: torch.Tensor, w: Weight, out: torch.Tensor, accumulate: b
 
 def attention(q, k_cache, v_cache, batch, group: int, out, n_heads, n_kv_heads, head_dim, page_size, window, scale):
     """Attention of the step's rows over their requests' pages of cache group `group`."""
-    from . import fast
-
     if fast.attention(q, k_cache, v_cache, batch, group, out, n_heads, n_kv_heads, head_dim, page_size, window, scale):
         return out
     return attention_rows(q, k_cache, v_cache, batch.block_tables[group], batch.row_request, batch.positions, out,
@@ -847,16 +813,12 @@ def gated_act(gate_up: torch.Tensor, out: torch.Tensor, group: int, act: str = "
 def linear_gated(a: torch.Tensor, w_gate_up: "Weight", act_out: torch.Tensor, group: int, act: str) -> bool:
     """act_out = act(gate) * up of a @ w_gate_up.T as one kernel (the activation in the product's epilogue) where one
     takes these sizes; False: nothing was done (the caller runs the product, then gated_act)."""
-    from . import fast
-
     return a.is_cuda and fast.linear_gated(a, w_gate_up, act_out, group, act)
 
 
 def linear_act(a: torch.Tensor, w: "Weight", out: torch.Tensor, act: str) -> torch.Tensor:
     """out = act(a @ w.T), act "gelu" (the exact form) or "relu2" (the square of relu): the activation in the product's epilogue where one takes these
     sizes, else the product's 32-bit rows through `bias_act`."""
-    from . import fast
-
     if a.is_cuda and fast.linear_act(a, w, out, act):
         return out
     z = torch.empty(a.shape[0], w.shape[0], dtype=torch.float32, device=a.device)
@@ -1009,8 +971,6 @@ def attention_masked(q, k_cache, v_cache, batch, group: int, out, n_heads: int, 
     m = MASKS[mask]
     # requests that bring MASKED_FLASH_MIN_ROWS rows or more go to the tensor-core kernel (bfloat16, the sizes it takes),
     # the other rows of the step to the row kernel; a decode-only step is the row kernel alone
-    from . import fast
-
     kw, vw = k_cache.shape[-1], v_cache.shape[-1]
     if (mask == "causal" and gate is None and v_cache is not k_cache and dim == vdim == kw == vw and not force_rows and not force_plain
             and not row_limit and q.dtype == out.dtype == torch.bfloat16 and q.is_contiguous() and out.is_contiguous()
@@ -1057,8 +1017,6 @@ def attention_masked(q, k_cache, v_cache, batch, group: int, out, n_heads: int, 
     n_ws = lib.hb_attn_masked_workspace(T, n_heads, n_kv_heads, dim, vdim, m, int(window), int(keep_first), int(chunk), max_pos)
     ws = arrived = None
     if n_ws:
-        from . import fast
-
         ws = torch.empty(n_ws, dtype=torch.float32, device=q.device)
         arrived = fast._decode_counters(q.device, lib.hb_attn_masked_counters(T, n_heads, n_kv_heads, dim, vdim))
     _call("seqmix", "hb_attn_masked", q.data_ptr(), _dt(q), q.stride(0), k_cache.data_ptr(), k_cache.shape[-1],
@@ -1137,8 +1095,6 @@ def gather_rows(plane: torch.Tensor, table: torch.Tensor, dst: torch.Tensor, n: 
 
 def fast_kernels_on() -> bool:
     """False when the plain kernels are asked for everywhere (HIPINFER_B200_PLAIN=1)."""
-    from . import fast
-
     return not fast.PLAIN_ONLY
 
 
@@ -1377,8 +1333,6 @@ def linear_split32(a: torch.Tensor, w: "Weight", out: torch.Tensor) -> torch.Ten
     """out = a @ w.T for float32 rows a (a view of wider rows is fine) and float32 out. Where the weight is bfloat16 and
     the tensor-core product takes the sizes, a goes in as the sum of two bfloat16 matrices (round(a) and round(a - round(a)))
     through two products added in 32-bit: 16 bits of a's mantissa at tensor-core speed. Else the plain 32-bit product."""
-    from . import fast
-
     _need_cuda(a, out)
     _rows_contiguous(a, "linear_split32 a")
     M, K = a.shape
@@ -1540,8 +1494,6 @@ def moe_sorted_linear(a: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, o
     K], offsets int32 [>= E + 1] on the device; out float32 [rows, N], or bfloat16 [rows, N / 2] = silu(gate) * up over
     16-interleaved weight rows with the pairs' scores (src, score, at_output as in moe_act). Rows beyond the last expert's are left
     alone, nothing is read by the host. For sizes that `moe_sorted_fast` takes."""
-    from . import fast
-
     if not fast.grouped_linear(a, w, offsets, out, src, score, at_output):
         raise KernelError(f"moe_sorted_linear: {tuple(w.shape)} weights are not this kernel's")
     return out
@@ -1549,8 +1501,6 @@ def moe_sorted_linear(a: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, o
 
 def moe_sorted_fast(xn: torch.Tensor, wgu: torch.Tensor, wdown: torch.Tensor) -> bool:
     """Whether moe_sorted_linear takes a routed layer's sizes (16-interleaved gate and up rows): bfloat16, at most 256 experts."""
-    from . import fast
-
     E, F2, W = wgu.shape
     return (xn.is_cuda and not fast.PLAIN_ONLY and xn.dtype == wgu.dtype == wdown.dtype == torch.bfloat16 and E <= 256 and W % 8 == 0
             and F2 % 32 == 0 and E * max(F2, W) < 1 << 31 and (wgu.data_ptr() | wdown.data_ptr()) % 16 == 0)
