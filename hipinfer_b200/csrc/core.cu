@@ -64,8 +64,8 @@ __global__ void rmsnorm_kernel(const float* __restrict__ x, const TW* __restrict
 // (H a multiple of 4, at most 256 * 4 * NV elements). The sum runs over the same per-thread
 // partial sums whatever M is.
 template <typename TW, typename TO, int NV>
-__global__ void __launch_bounds__(256) rmsnorm_vec_kernel(const float* __restrict__ x, const TW* __restrict__ w,
-                                                          TO* __restrict__ y, const int* __restrict__ rows, int H,
+__global__ void __launch_bounds__(256) rmsnorm_vec_kernel(const float* x, const TW* __restrict__ w,      // (x without __restrict__: see gemm_simt.cu)
+                                                          TO* y, const int* __restrict__ rows, int H,
                                                           float eps) {
   __shared__ float sh[32];
   hb_pdl_launch();
@@ -434,9 +434,9 @@ __global__ void rope_kv_kernel(const TI* __restrict__ qkv, long ld, const int* _
 
 // The same four elements at a time (rotary over the whole head, head_dim a multiple of 8).
 template <typename TI, typename TQ, typename TC>
-__global__ void __launch_bounds__(256) rope_kv_vec_kernel(const TI* __restrict__ qkv, long ld, const int* __restrict__ pos,
+__global__ void __launch_bounds__(256) rope_kv_vec_kernel(const TI* qkv, long ld, const int* __restrict__ pos,      // (see gemm_simt.cu)
                                                           const int* __restrict__ slot_map, const float2* __restrict__ table,
-                                                          TQ* __restrict__ q_out, TC* __restrict__ kc, TC* __restrict__ vc,
+                                                          TQ* q_out, TC* kc, TC* vc,
                                                           int Hq, int Hkv, int D, int page_size) {
   hb_pdl_launch();
   hb_pdl_wait();
@@ -918,8 +918,8 @@ __global__ void __launch_bounds__(128) attn_rows_vec_kernel(
 }
 
 template <typename TQ>
-__global__ void attn_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
-                                  const int* __restrict__ pos, TQ* __restrict__ out, int Hq, int D, int window, int chunk,
+__global__ void attn_merge_kernel(const float* part_acc, const float* part_ml,      // (no __restrict__: see gemm_simt.cu)
+                                  const int* __restrict__ pos, TQ* out, int Hq, int D, int window, int chunk,
                                   int S, const int* __restrict__ row_req, const int* __restrict__ q_len, int row_limit) {
   hb_pdl_launch();
   hb_pdl_wait();
