@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(192) gemm_stream_kernel(const __grid_constant_
 #pragma unroll
     for (int c = 0; c < NT / 16; c++) hb_tmem_ld16(tmem_base + ((uint32_t)(warp * 32) << 16) + c * 16, v + 16 * c);
     const int n = n0 + warp * 32 + lane;
-    if (ksplit == 1 && epi != ST_SLICES) {
+    if constexpr (DEEP) {          // unsplit, finished here; the others leave slices
 #pragma unroll
       for (int m = 0; m < NT; m++) {
         if (m < M) {
