@@ -37,7 +37,7 @@ template <int D, bool TMA> __device__ __forceinline__ uint32_t ad_off(int row, i
 // Rows [r_lo, r_hi) of the tile (row r = key k0 + r) by cp.async, page by page: the page
 // numbers of four pages are read first, then every thread copies its 16-byte pieces of them.
 template <int D>
-__device__ __forceinline__ void ad_load_rows(const __nv_bfloat16* __restrict__ kc, const __nv_bfloat16* __restrict__ vc,
+__device__ __forceinline__ void ad_load_rows(const __nv_bfloat16* kc, const __nv_bfloat16* vc,
                                              const int* __restrict__ table, int Hkv, int h, int page_size, int k0,
                                              int r_lo, int r_hi, uint32_t sK, uint32_t sV, int tid) {
   constexpr int CH = D / 8;
@@ -112,12 +112,12 @@ struct AdDiff {
 };
 template <int D, int G, bool TMA, int RW, int KW, int SR, bool CL, bool EX, bool DIFF>
 __global__ void __launch_bounds__(AD_THREADS) attn_decode_kernel(
-    const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, int* __restrict__ status,
-    const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kc, const __nv_bfloat16* __restrict__ vc,
+    const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, int* status,
+    const __nv_bfloat16* q, const __nv_bfloat16* kc, const __nv_bfloat16* vc,
     const int* __restrict__ bt, int bt_stride, const int* __restrict__ row_req, const int* __restrict__ pos,
-    __nv_bfloat16* __restrict__ out, float* __restrict__ part_acc, float* __restrict__ part_ml, int Hq, int Hkv,
+    __nv_bfloat16* __restrict__ out, float* part_acc, float* part_ml, int Hq, int Hkv,
     int page_size, int window, float scale_log2, int chunk, int S, const int* __restrict__ q_len, int row_limit,
-    const int* __restrict__ ctx_len, int* __restrict__ counters, const float* __restrict__ r1p,
+    const int* __restrict__ ctx_len, int* counters, const float* __restrict__ r1p,
     const float* __restrict__ r2p, const float* __restrict__ sink, AdDiff df, const int* __restrict__ row_list) {
   static_assert(!DIFF || (TMA && !EX && G % 2 == 0), "two score maps: by TMA, no extras");
   constexpr int CH = D / 8, KS = D / 16, NT_O = D / 8, WK = 64;  // WK: keys per warp pass

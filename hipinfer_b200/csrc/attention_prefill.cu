@@ -25,7 +25,7 @@ template <int D> __device__ __forceinline__ uint32_t fp_swz(int row, int chunk) 
 // Copies keys [k_base, k_base + 64) of kv head h into a [64][D] swizzled tile; rows outside
 // [k_first, k_last] are zeroed (their pages may have been given back, or not exist yet).
 template <int D>
-__device__ __forceinline__ void fp_load_tile(uint32_t tile, const __nv_bfloat16* __restrict__ cache,
+__device__ __forceinline__ void fp_load_tile(uint32_t tile, const __nv_bfloat16* cache,
                                              const int* __restrict__ table, int Hkv, int h, int page_size, int k_base,
                                              int k_first, int k_last, int tid) {
   constexpr int CH = D / 8;

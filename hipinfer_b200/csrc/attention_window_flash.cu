@@ -40,7 +40,7 @@ struct WinFlashArgs {
 // Rows [k_base, k_base + 64) of a plane whose rows are W elements wide into a swizzled [64][W] tile; a row that no
 // query of the CTA sees is zeroed instead.
 template <int W>
-__device__ __forceinline__ void wf_load_tile(uint32_t tile, const __nv_bfloat16* __restrict__ cache, const int* __restrict__ table,
+__device__ __forceinline__ void wf_load_tile(uint32_t tile, const __nv_bfloat16* cache, const int* __restrict__ table,
                                              int G, int h, int page_size, int k_base, int lo, int keep, int p_last, int tid) {
   constexpr int CH = W / 8;
   for (int i = tid; i < WF_BKV * CH; i += WF_THREADS) {

@@ -123,6 +123,10 @@ __device__ __forceinline__ void hb_tl_mark(unsigned long long* buf, int id, int 
 // earlier kernel wrote or still reads; only work on constants (weights, its own shared memory,
 // barriers, tensor memory) may come before the wait. hb_pdl_wait() returns when the preceding
 // kernel has finished and its writes are visible. With g_hb_pdl == 0 launches are ordinary.
+// What an earlier kernel wrote or still writes is reached through pointers WITHOUT __restrict__ (and never through ld.global.nc): the
+// qualifier promises that nobody else writes that memory while the kernel runs, and a load that the compiler may take for
+// constant can move ahead of hb_pdl_wait(). One did (a norm behind a split product: logits changed from run to run). It
+// stays on weights, tables, the step's packed input and outputs that the kernel never reads (tests/test_launch_rules.py).
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void hb_pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void hb_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

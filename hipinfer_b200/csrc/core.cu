@@ -27,7 +27,7 @@ HB_EXPORT void hb_set_pdl(int on) { g_hb_pdl = on; }
 // Embedding: out[i, :] = table[tok[i], :] into the 32-bit residual stream.
 // ---------------------------------------------------------------------------------------
 template <typename TE>
-__global__ void embed_kernel(const TE* __restrict__ table, const int* __restrict__ tok, float* __restrict__ out, int H) {
+__global__ void embed_kernel(const TE* __restrict__ table, const int* tok, float* __restrict__ out, int H) {
   hb_pdl_launch();
   hb_pdl_wait();
   const TE* src = table + (size_t)tok[blockIdx.x] * H;
@@ -64,7 +64,7 @@ __global__ void rmsnorm_kernel(const float* __restrict__ x, const TW* __restrict
 // (H a multiple of 4, at most 256 * 4 * NV elements). The sum runs over the same per-thread
 // partial sums whatever M is.
 template <typename TW, typename TO, int NV>
-__global__ void __launch_bounds__(256) rmsnorm_vec_kernel(const float* x, const TW* __restrict__ w,      // (x without __restrict__: see gemm_simt.cu)
+__global__ void __launch_bounds__(256) rmsnorm_vec_kernel(const float* x, const TW* __restrict__ w,
                                                           TO* y, const int* __restrict__ rows, int H,
                                                           float eps) {
   __shared__ float sh[32];
@@ -121,7 +121,7 @@ HB_EXPORT int hb_rmsnorm(const float* x, const void* w, int w_dt, void* y, int y
 // (ptab null: no position vector). The product and the sum are 32-bit.
 // ---------------------------------------------------------------------------------------
 template <typename TE>
-__global__ void embed_pos_kernel(const TE* __restrict__ table, const TE* __restrict__ ptab, const int* __restrict__ tok,
+__global__ void embed_pos_kernel(const TE* __restrict__ table, const TE* __restrict__ ptab, const int* tok,
                                  const int* __restrict__ pos, float* __restrict__ out, int H, float scale) {
   hb_pdl_launch();
   hb_pdl_wait();
@@ -147,7 +147,7 @@ HB_EXPORT int hb_embed_pos(const void* table, const void* ptab, int table_dt, co
 // 32-bit (the mean first, then the squared deviations from it), the result rounded once. `rows` as in RMSNorm.
 // ---------------------------------------------------------------------------------------
 template <typename TW, typename TO>
-__global__ void __launch_bounds__(256) layernorm_kernel(const float* __restrict__ x, const TW* __restrict__ w,
+__global__ void __launch_bounds__(256) layernorm_kernel(const float* x, const TW* __restrict__ w,
                                                         const TW* __restrict__ b, TO* __restrict__ y,
                                                         const int* __restrict__ rows, int H, float eps) {
   __shared__ float sh[32];
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const float* __restrict_
 
 // The same with the row in registers (H a multiple of 4, at most 256 * 4 * NV elements): one read of x.
 template <typename TW, typename TO, int NV>
-__global__ void __launch_bounds__(256) layernorm_vec_kernel(const float* __restrict__ x, const TW* __restrict__ w,
+__global__ void __launch_bounds__(256) layernorm_vec_kernel(const float* x, const TW* __restrict__ w,
                                                             const TW* __restrict__ b, TO* __restrict__ y,
                                                             const int* __restrict__ rows, int H, float eps) {
   __shared__ float sh[32];
@@ -244,7 +244,7 @@ HB_EXPORT int hb_layernorm(const float* x, const void* w, const void* b, int w_d
 // squares (z^2, z^4, z^6) and the combination are 32-bit; the result is rounded once.
 // ---------------------------------------------------------------------------------------
 template <typename TO>
-__global__ void __launch_bounds__(256) polynorm_kernel(const float* __restrict__ z, long ldz, TO* __restrict__ act, long ld,
+__global__ void __launch_bounds__(256) polynorm_kernel(const float* z, long ldz, TO* __restrict__ act, long ld,
                                                        int I, float c1, float c2, float c3, float c0, float eps) {
   __shared__ float sh[32];
   hb_pdl_launch();
@@ -281,7 +281,7 @@ HB_EXPORT int hb_polynorm(const float* z, long ldz, void* act, int act_dt, long 
 // 32-bit residual stream (one product, one sum, both 32-bit).
 // ---------------------------------------------------------------------------------------
 template <typename TS>
-__global__ void scale_add_kernel(float* __restrict__ x, const float* __restrict__ y, long ldy, const TS* __restrict__ scale,
+__global__ void scale_add_kernel(float* x, const float* y, long ldy, const TS* __restrict__ scale,
                                  int M, int H) {
   hb_pdl_launch();
   hb_pdl_wait();
@@ -306,7 +306,7 @@ HB_EXPORT int hb_scale_add(float* x, const float* y, long ldy, const void* scale
 // middle of a low-rank projection pair), 2 the exact GELU, 3 the square of relu.
 // ---------------------------------------------------------------------------------------
 template <typename TB_, typename TO>
-__global__ void bias_act_kernel(const float* __restrict__ x, long ldx, const TB_* __restrict__ bias, TO* __restrict__ y,
+__global__ void bias_act_kernel(const float* x, long ldx, const TB_* __restrict__ bias, TO* __restrict__ y,
                                 long ldy, int M, int n, int act) {
   hb_pdl_launch();
   hb_pdl_wait();
@@ -434,7 +434,7 @@ __global__ void rope_kv_kernel(const TI* __restrict__ qkv, long ld, const int* _
 
 // The same four elements at a time (rotary over the whole head, head_dim a multiple of 8).
 template <typename TI, typename TQ, typename TC>
-__global__ void __launch_bounds__(256) rope_kv_vec_kernel(const TI* qkv, long ld, const int* __restrict__ pos,      // (see gemm_simt.cu)
+__global__ void __launch_bounds__(256) rope_kv_vec_kernel(const TI* qkv, long ld, const int* __restrict__ pos,
                                                           const int* __restrict__ slot_map, const float2* __restrict__ table,
                                                           TQ* q_out, TC* kc, TC* vc,
                                                           int Hq, int Hkv, int D, int page_size) {
@@ -512,7 +512,7 @@ __device__ __forceinline__ size_t rn_key_row(int kh, int G, int maps, size_t pag
 }
 
 template <typename TQ, typename TW>
-__global__ void __launch_bounds__(256) rope_norm_store_kernel(const float* __restrict__ proj, long ld, int q_off, int k_off,
+__global__ void __launch_bounds__(256) rope_norm_store_kernel(const float* proj, long ld, int q_off, int k_off,
                                                               int v_off, const int* __restrict__ pos,
                                                               const int* __restrict__ slot_map,
                                                               const float2* __restrict__ table, int rot, int rot_off,
@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(256) rope_norm_store_kernel(const float* __res
 // Rotation and cache write alone (no norm, no temperature; halves paired from dimension 0 on), four columns an access: a
 // thread turns four pairs, or copies four columns that pass unchanged, or four values. The same products and sums.
 template <typename TQ>
-__global__ void __launch_bounds__(256) rope_store_vec_kernel(const float* __restrict__ proj, long ld, int q_off, int k_off, int v_off,
+__global__ void __launch_bounds__(256) rope_store_vec_kernel(const float* proj, long ld, int q_off, int k_off, int v_off,
                                                              const int* __restrict__ pos, const int* __restrict__ slot_map,
                                                              const float2* __restrict__ table, int rot, TQ* __restrict__ q_out,
                                                              TQ* __restrict__ kc, TQ* __restrict__ vc, int H, int G, int D, int E,
@@ -677,7 +677,7 @@ HB_EXPORT int hb_rope_norm_store(const float* proj, long ld, int q_off, int k_of
 // rounded once. No slot map (a layer that reads another layer's cache): the row is q alone.
 // ---------------------------------------------------------------------------------------
 template <typename TB_, typename TQ>
-__global__ void __launch_bounds__(256) qkv_bias_store_kernel(const float* __restrict__ qkv, long ld, const TB_* __restrict__ bq,
+__global__ void __launch_bounds__(256) qkv_bias_store_kernel(const float* qkv, long ld, const TB_* __restrict__ bq,
                                                              const TB_* __restrict__ bk, const TB_* __restrict__ bv,
                                                              const int* __restrict__ slot_map, TQ* __restrict__ q_out,
                                                              TQ* __restrict__ kc, TQ* __restrict__ vc, int nq, int G, int kw,
@@ -795,7 +795,7 @@ __global__ void __launch_bounds__(128) attn_rows_kernel(
 // its group: LPK lanes (a power of two) hold a key's dimensions four each, so that a warp's access covers whole rows of the
 // cache, and a key or value element is loaded once for all G heads instead of once a head. A score is the lanes' chains of four
 // added by a butterfly; the values are summed by 128 / LPK groups of threads that take every (128 / LPK)-th key, added group 0
-// first. Both orders depend on the position alone. (No __restrict__ on what the kernel ahead wrote: see gemm_simt.cu.) Bound by the latency of a block's passes over its chunk and, for prompts, by
+// first. Both orders depend on the position alone. Bound by the latency of a block's passes over its chunk and, for prompts, by
 // L2 (every row reads its keys again).
 template <typename TQ, typename TC, int GM, int LPK>
 __global__ void __launch_bounds__(128) attn_rows_vec_kernel(
@@ -918,7 +918,7 @@ __global__ void __launch_bounds__(128) attn_rows_vec_kernel(
 }
 
 template <typename TQ>
-__global__ void attn_merge_kernel(const float* part_acc, const float* part_ml,      // (no __restrict__: see gemm_simt.cu)
+__global__ void attn_merge_kernel(const float* part_acc, const float* part_ml,
                                   const int* __restrict__ pos, TQ* out, int Hq, int D, int window, int chunk,
                                   int S, const int* __restrict__ row_req, const int* __restrict__ q_len, int row_limit) {
   hb_pdl_launch();
@@ -1088,10 +1088,10 @@ __device__ __forceinline__ float sample_uniform(uint32_t seed, uint32_t position
 // the slice's best key meets the others' in best[row] by an atomic maximum (the order of the arrivals does not matter: the
 // keys are totally ordered), and the block that arrives last writes the row's index and leaves best[row] and count[row]
 // zero for the next call: no second kernel.
-__global__ void __launch_bounds__(1024) sample_slice_kernel(const float* __restrict__ logits, long ld, int V, int slice,
+__global__ void __launch_bounds__(1024) sample_slice_kernel(const float* logits, long ld, int V, int slice,
                                                             const float* __restrict__ temperature,
                                                             const uint32_t* __restrict__ seed, const int* __restrict__ position,
-                                                            unsigned long long* __restrict__ best, int* __restrict__ count,
+                                                            unsigned long long* best, int* count,
                                                             int* __restrict__ out) {
   __shared__ unsigned long long sh[32];
   hb_pdl_launch();
@@ -1153,7 +1153,7 @@ HB_EXPORT int hb_sample(const float* logits, long ld, int rows, int V, const flo
 // tokens[i] = src[map[i]] where map[i] >= 0: rows of a step whose token was sampled on the
 // device by the step before and has not been to the host.
 // ---------------------------------------------------------------------------------------
-__global__ void feed_tokens_kernel(int* __restrict__ tokens, const int* __restrict__ src, const int* __restrict__ map, int n) {
+__global__ void feed_tokens_kernel(int* tokens, const int* src, const int* __restrict__ map, int n) {
   hb_pdl_launch();
   hb_pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

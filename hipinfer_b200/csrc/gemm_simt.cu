@@ -14,9 +14,6 @@
 //                      products of so few tiles that whole-K blocks would leave SMs idle.
 // EPI 0: C = sum;  EPI 1: C += sum (32-bit C: the residual stream);  EPI 2: C += colscale[n] * sum (the same with a scale
 // vector over the output columns, of the weight's element type).
-//
-// What an earlier kernel wrote (A, C, the partial sums) is read through pointers without __restrict__: a load that the compiler
-// may take for constant can be moved ahead of hb_pdl_wait() or be served from a line cached before it.
 #include "tc_common.cuh"
 
 constexpr int SM_TM = 64, SM_TN = 128, SM_TK = 16, SM_MAX_SLICES = 8, SM_MIN_SLICE = 512;

@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(192, 1) gemm_stream_persist_kernel(const __gri
 // The slices' partial sums added in slice order and the epilogue applied, four columns per thread,
 // over the whole output at once. With many token rows this is much more work than one CTA per
 // column block should do at the end of the product kernel, so it runs as a kernel of its own.
-__global__ void __launch_bounds__(256) stream_reduce_kernel(const float* __restrict__ ws, void* C, long ldc, int M, int N,
+__global__ void __launch_bounds__(256) stream_reduce_kernel(const float* ws, void* C, long ldc, int M, int N,
                                                             int NP, int NT, int ksplit, int epi) {
   hb_pdl_launch();
   HB_TL_MARK(5, 0);

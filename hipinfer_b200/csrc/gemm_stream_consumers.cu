@@ -16,7 +16,7 @@ HB_TL_DEFINE(consumers)
 // round trips to L2, and every round trip saved is most of a microsecond).
 constexpr int SL_MAX = 16;
 template <int SLM = SL_MAX>
-__device__ __forceinline__ float4 slices_sum4(const float* __restrict__ p, int ksplit, long slice_stride) {
+__device__ __forceinline__ float4 slices_sum4(const float* p, int ksplit, long slice_stride) {
   float4 a[SLM];
 #pragma unroll
   for (int j = 0; j < SLM; j++)
@@ -38,7 +38,7 @@ __device__ __forceinline__ float4 slices_sum4(const float* __restrict__ p, int k
 // SLM: the slices whose loads are in flight together: with four a thread needs half the registers and two blocks lie on an SM, which a
 // portion's hundreds of rows want (512 rows of 3,072 from three slices: 14.0 us with sixteen, 10.7 with four).
 template <int NV, int SLM>
-__global__ void __launch_bounds__(512) add_rmsnorm_slices_kernel(float* __restrict__ x, long ldx, const float* __restrict__ ws,
+__global__ void __launch_bounds__(512) add_rmsnorm_slices_kernel(float* x, long ldx, const float* ws,
                                                                  int ksplit, long slice_stride, long row_stride,
                                                                  const __nv_bfloat16* __restrict__ w,
                                                                  __nv_bfloat16* __restrict__ y, const int* __restrict__ rows,
@@ -68,10 +68,14 @@ __global__ void __launch_bounds__(512) add_rmsnorm_slices_kernel(float* __restri
     if (c < nvec) {
       const float4 o = hb_load4(xr + 4 * c), a = slices_sum4<SLM>(pr + 4 * c, ksplit, slice_stride);
       v[i] = make_float4(o.x + a.x, o.y + a.y, o.z + a.z, o.w + a.w);
-      if (!rows) hb_store4(xr + 4 * c, v[i]);
     }
     ss = fmaf(v[i].x, v[i].x, ss); ss = fmaf(v[i].y, v[i].y, ss);
     ss = fmaf(v[i].z, v[i].z, ss); ss = fmaf(v[i].w, v[i].w, ss);
+  }
+#pragma unroll
+  for (int i = 0; i < NV; i++) {   // behind all loads: for all the compiler knows x and the slices overlap
+    const int c = threadIdx.x + i * 512;
+    if (c < nvec && !rows) hb_store4(xr + 4 * c, v[i]);
   }
   HB_TL_MARK(tl, 2);
   const float inv = rsqrtf(hb_block_sum(ss, sh) / (float)H + eps);
@@ -112,7 +116,7 @@ HB_EXPORT int hb_add_rmsnorm_slices(float* x, long ldx, const float* ws, int ksp
 // turned by the angle of (pos[t], j) from the table of (cos, sin); q goes to q_out, k and v to
 // the cache at slot_map[t] (a negative slot or no map: nothing is stored). blockIdx.y shares a
 // row's heads among several blocks.
-__global__ void __launch_bounds__(256) rope_kv_slices_kernel(const float* __restrict__ ws, int ksplit, long slice_stride,
+__global__ void __launch_bounds__(256) rope_kv_slices_kernel(const float* ws, int ksplit, long slice_stride,
                                                              long row_stride, const int* __restrict__ pos,
                                                              const int* __restrict__ slot_map,
                                                              const float2* __restrict__ table,

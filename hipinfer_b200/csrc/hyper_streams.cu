@@ -29,7 +29,7 @@ __device__ __forceinline__ void hs_load_coef(StreamCoef& c, int S, const float* 
 }
 
 template <typename TW, typename TO>
-__global__ void __launch_bounds__(HS_THREADS) streams_norm_kernel(const float* __restrict__ x, const int* __restrict__ rows,
+__global__ void __launch_bounds__(HS_THREADS) streams_norm_kernel(const float* x, const int* __restrict__ rows,
                                                                   const float* __restrict__ a, const TW* __restrict__ w,
                                                                   TO* __restrict__ out, int S, int W, float eps) {
   __shared__ float sh[32];
@@ -63,7 +63,7 @@ HB_EXPORT int hb_streams_norm(const float* x, const int* rows, int n_rows, const
   return 0;
 }
 
-__global__ void __launch_bounds__(HS_THREADS) streams_update_kernel(float* __restrict__ x, const float* __restrict__ y,
+__global__ void __launch_bounds__(HS_THREADS) streams_update_kernel(float* x, const float* y,
                                                                     const float* __restrict__ b, const float* __restrict__ M,
                                                                     float m, long T, int S, int W) {
   hb_pdl_launch();
@@ -100,7 +100,7 @@ HB_EXPORT int hb_streams_update(float* x, const float* y, const float* b, const 
 // One block a row: the write-back of the sublayer that has just run, then u and the norm of the one that reads next. The
 // thread that wrote a column reads it back in the second pass, so nothing is exchanged but the sum of squares.
 template <typename TW, typename TO>
-__global__ void __launch_bounds__(HS_THREADS) streams_update_norm_kernel(float* __restrict__ x, const float* __restrict__ y,
+__global__ void __launch_bounds__(HS_THREADS) streams_update_norm_kernel(float* x, const float* y,
                                                                          const float* __restrict__ b, const float* __restrict__ M,
                                                                          float m, const float* __restrict__ a_next,
                                                                          const TW* __restrict__ w_next, TO* __restrict__ out,
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(HS_THREADS) streams_update_norm_kernel(float* 
 constexpr int HS_KEEP = 4;
 
 template <typename TW, typename TO, int S>
-__global__ void __launch_bounds__(HS_THREADS) streams_update_norm_vec_kernel(float* __restrict__ x, const float* __restrict__ y,
+__global__ void __launch_bounds__(HS_THREADS) streams_update_norm_vec_kernel(float* x, const float* y,
                                                                              const float* __restrict__ b, const float* __restrict__ M,
                                                                              float m, const float* __restrict__ a_next,
                                                                              const TW* __restrict__ w_next, TO* __restrict__ out,
@@ -157,7 +157,12 @@ __global__ void __launch_bounds__(HS_THREADS) streams_update_norm_vec_kernel(flo
   hb_pdl_wait();
   const int r = blockIdx.x;
   float* row = x + (size_t)r * S * W;
-  float4 uu[HS_KEEP];
+  float4 uu[HS_KEEP], ys[HS_KEEP];
+#pragma unroll
+  for (int k = 0; k < HS_KEEP; k++) {       // ahead of the stores to x, which for all the compiler knows are to y too
+    const int i = (k * HS_THREADS + threadIdx.x) * 4;
+    ys[k] = i < W ? *(const float4*)(y + (size_t)r * W + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
   float ss = 0.f;
 #pragma unroll
   for (int k = 0; k < HS_KEEP; k++) {
@@ -167,7 +172,7 @@ __global__ void __launch_bounds__(HS_THREADS) streams_update_norm_vec_kernel(flo
       float4 old[S];
 #pragma unroll
       for (int s = 0; s < S; s++) old[s] = *(const float4*)(row + (size_t)s * W + i);
-      const float4 yy = *(const float4*)(y + (size_t)r * W + i);
+      const float4 yy = ys[k];
       float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int to = 0; to < S; to++) {
@@ -227,7 +232,7 @@ HB_EXPORT int hb_streams_update_norm(float* x, const float* y, const float* b, c
   return 0;
 }
 
-__global__ void __launch_bounds__(HS_THREADS) streams_expand_kernel(const float* __restrict__ x, float* __restrict__ xs, long T,
+__global__ void __launch_bounds__(HS_THREADS) streams_expand_kernel(const float* x, float* __restrict__ xs, long T,
                                                                     int S, int W) {
   hb_pdl_launch();
   hb_pdl_wait();
@@ -266,7 +271,7 @@ __device__ __forceinline__ float glu_one(float g, float u, int kind, float limit
 }
 
 template <typename TW, typename TO>
-__global__ void __launch_bounds__(256) glu_bias_kernel(const float* __restrict__ gu, long ld, const TW* __restrict__ bias,
+__global__ void __launch_bounds__(256) glu_bias_kernel(const float* gu, long ld, const TW* __restrict__ bias,
                                                        TO* __restrict__ out, long ldo, long M, int I, int group, int kind,
                                                        float limit, float alpha) {
   hb_pdl_launch();
@@ -288,7 +293,7 @@ __global__ void __launch_bounds__(256) glu_bias_kernel(const float* __restrict__
 // Four output columns a thread (groups that are multiples of four, 16-byte aligned rows): the same values, fewer and
 // wider loads and stores.
 template <typename TW, typename TO>
-__global__ void __launch_bounds__(256) glu_bias_vec_kernel(const float* __restrict__ gu, long ld, const TW* __restrict__ bias,
+__global__ void __launch_bounds__(256) glu_bias_vec_kernel(const float* gu, long ld, const TW* __restrict__ bias,
                                                            TO* __restrict__ out, long ldo, long M, int I, int group, int kind,
                                                            float limit, float alpha) {
   hb_pdl_launch();
@@ -334,7 +339,7 @@ HB_EXPORT int hb_glu_bias(const float* gu, long ld, const void* bias, int b_dt, 
 
 // x[m][n] = x[m][n] * scale (+ bias[n]): the scaled logits; a projection's bias
 template <typename TW>
-__global__ void __launch_bounds__(256) scale_bias_rows_kernel(float* __restrict__ x, long ld, const TW* __restrict__ bias,
+__global__ void __launch_bounds__(256) scale_bias_rows_kernel(float* x, long ld, const TW* __restrict__ bias,
                                                               float scale, long M, int N) {
   hb_pdl_launch();
   hb_pdl_wait();

@@ -17,7 +17,7 @@
 #include "common.cuh"
 
 template <typename TW, typename TO>
-__global__ void __launch_bounds__(256) latent_prepare_kernel(const float* __restrict__ proj, long ld, int cq_off, int c_off,
+__global__ void __launch_bounds__(256) latent_prepare_kernel(const float* proj, long ld, int cq_off, int c_off,
                                                              int kr_off, const TW* __restrict__ wq, const TW* __restrict__ wc,
                                                              const int* __restrict__ pos, const int* __restrict__ slot_map,
                                                              const float2* __restrict__ table, int rot, float eps,
@@ -71,10 +71,10 @@ constexpr int HL_TM = 8, HL_THREADS = 128, HL_TN = 32, HL_KZ = HL_THREADS / HL_T
 // k, summed in a fixed order (slice 0 .. HL_KZ - 1) through shared memory: few rows still fill the machine, and a
 // thread's loads of the weight are independent of one another.
 template <typename TW, typename TO>
-__global__ void __launch_bounds__(HL_THREADS) heads_linear_kernel(const float* __restrict__ a, long lda, long a_head,
+__global__ void __launch_bounds__(HL_THREADS) heads_linear_kernel(const float* a, long lda, long a_head,
                                                                   const TW* __restrict__ wt, TO* __restrict__ out, long ldo,
                                                                   long o_head, int T, int K, int N,
-                                                                  const float* __restrict__ gate, long ld_gate, int gate_off,
+                                                                  const float* gate, long ld_gate, int gate_off,
                                                                   int tail, int rot, const int* __restrict__ pos,
                                                                   const float2* __restrict__ table,
                                                                   const int* __restrict__ row_req,
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(HL_THREADS) heads_linear_kernel(const float* _
 // asked for before the wait for the kernel ahead. The lanes' sums meet by a transposing butterfly that leaves lane l the sum
 // of (row l / 8, column l % 8): 31 shuffles for 32 sums, no shared memory, no barrier. Bound by latency: the weight of a head is
 // 32 KB (4 rows, 32 heads of 256 x 64: 13.5 us with two-byte loads of one k after the other, 4.4 now). row_list: the rows the
-// call is for (indices in a, out, gate and pos), or null: all T. What the kernel ahead wrote (a, the gate) has no __restrict__.
+// call is for (indices in a, out, gate and pos), or null: all T.
 constexpr int HV_ROWS = 4, HV_K = 8;
 struct HeadsVec {
   const float* a; long lda, a_head;
@@ -302,7 +302,7 @@ HB_EXPORT int hb_heads_linear(const float* a, long lda, long a_head, const void*
 // The rows of one request's tokens [0, n) of a cache plane with one head ([page][1][page_size][W]) copied, in the
 // order of their positions, into a contiguous buffer [n][W]: the input of a product over a request's whole context.
 template <typename TC>
-__global__ void __launch_bounds__(256) gather_rows_kernel(const TC* __restrict__ plane, const int* __restrict__ table,
+__global__ void __launch_bounds__(256) gather_rows_kernel(const TC* plane, const int* __restrict__ table,
                                                           TC* __restrict__ dst, int n, int W, int page_size) {
   hb_pdl_launch();
   hb_pdl_wait();

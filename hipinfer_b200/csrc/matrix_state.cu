@@ -325,9 +325,9 @@ __device__ __forceinline__ float ms_cap(float z, float cap) { return cap * tanhf
 // so a run of tokens acts on it as m -> max(m + F, M): a scan over the tokens, a warp's 32 by shuffles, then the warps' pairs.
 // a and b are made from the m values themselves, so that however m was rounded, they fit together. grid (heads, requests).
 template <typename TW>
-__global__ void __launch_bounds__(1024) ms_exp_gates_kernel(const float* __restrict__ zi, const float* __restrict__ zf, long ldz,
+__global__ void __launch_bounds__(1024) ms_exp_gates_kernel(const float* zi, const float* zf, long ldz,
                                                             const TW* __restrict__ bi, const TW* __restrict__ bf, float cap,
-                                                            float* __restrict__ m_state, const int* __restrict__ q_start,
+                                                            float* m_state, const int* __restrict__ q_start,
                                                             const int* __restrict__ q_len, const int* __restrict__ slot,
                                                             float* __restrict__ a, float* __restrict__ b, float* __restrict__ e, int H) {
   __shared__ float wF[32], wM[32], ms[1025];
@@ -395,8 +395,8 @@ HB_EXPORT int hb_ms_exp_gates(const float* zi, const float* zf, long ldz, const 
 // A block a row, a warp a group.
 
 template <typename TW>
-__global__ void __launch_bounds__(256) ms_delta_prepare_kernel(const float* __restrict__ q_rows, const float* __restrict__ k_rows, long ld,
-                                                               const float* __restrict__ za, const float* __restrict__ zb, long ldz,
+__global__ void __launch_bounds__(256) ms_delta_prepare_kernel(const float* q_rows, const float* k_rows, long ld,
+                                                               const float* za, const float* zb, long ldz,
                                                                const TW* __restrict__ a_log, const TW* __restrict__ dt_bias,
                                                                const int* __restrict__ row_req, const int* __restrict__ q_start,
                                                                float* __restrict__ scal, int H, int G, int N, float q_scale,
@@ -640,9 +640,9 @@ HB_EXPORT int hb_ms_delta_walk(const float* q, long ldq, const float* k, long ld
 // a (token, head).
 // ---------------------------------------------------------------------------------------------------------------------
 template <typename TW, typename TO>
-__global__ void __launch_bounds__(256) ms_finish_kernel(const float* __restrict__ y, const float* __restrict__ nq,
-                                                        const float* __restrict__ e, float den_eps, const TW* __restrict__ w,
-                                                        int w_shared, const float* __restrict__ gate, long ldg, int gate_silu,
+__global__ void __launch_bounds__(256) ms_finish_kernel(const float* y, const float* nq,
+                                                        const float* e, float den_eps, const TW* __restrict__ w,
+                                                        int w_shared, const float* gate, long ldg, int gate_silu,
                                                         TO* __restrict__ out, long ldo, long pairs, int H, int P, float eps) {
   hb_pdl_launch();
   hb_pdl_wait();
@@ -671,9 +671,9 @@ __global__ void __launch_bounds__(256) ms_finish_kernel(const float* __restrict_
 
 // The same with four values a lane: P / 4 lanes (a power of two up to 32) share a (token, head).
 template <typename TW, typename TO>
-__global__ void __launch_bounds__(256) ms_finish_vec_kernel(const float* __restrict__ y, const float* __restrict__ nq,
-                                                            const float* __restrict__ e, float den_eps, const TW* __restrict__ w,
-                                                            int w_shared, const float* __restrict__ gate, long ldg, int gate_silu,
+__global__ void __launch_bounds__(256) ms_finish_vec_kernel(const float* y, const float* nq,
+                                                            const float* e, float den_eps, const TW* __restrict__ w,
+                                                            int w_shared, const float* gate, long ldg, int gate_silu,
                                                             TO* __restrict__ out, long ldo, long pairs, int H, int P, float eps) {
   hb_pdl_launch();
   hb_pdl_wait();

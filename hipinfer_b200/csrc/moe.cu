@@ -62,7 +62,7 @@ __device__ __forceinline__ float mr_dot8(const TA* a, const TW* w, float acc) {
 // A warp a router row (and the shared expert's gate), the token's row read beside it; then warp 0 ranks the groups, marks the
 // experts of those that do not stay as taken (NaN), and picks the largest `top` times, ties to the lower index.
 template <typename TA, typename TW>
-__global__ void __launch_bounds__(MR_THREADS) moe_route_kernel(const TA* __restrict__ xn, long ldx, const TW* __restrict__ router,
+__global__ void __launch_bounds__(MR_THREADS) moe_route_kernel(const TA* xn, long ldx, const TW* __restrict__ router,
                                                                const TW* __restrict__ bias, int* __restrict__ expert,
                                                                float* __restrict__ weight, int W, int E, int top, int mode,
                                                                const TW* __restrict__ correction, int groups, int keep, float scale,
@@ -207,7 +207,7 @@ HB_EXPORT int hb_moe_route(const void* xn, int x_dt, long ldx, const void* route
 // A warp's dot product of a weight row with a 32-bit row in shared memory: lanes take groups of four columns (scalar
 // columns where K is no multiple of four), the lanes' sums are joined in a fixed order.
 template <typename TW>
-__device__ __forceinline__ float moe_warp_dot(const TW* __restrict__ w, const float* __restrict__ a, int K, int lane, bool vec) {
+__device__ __forceinline__ float moe_warp_dot(const TW* __restrict__ w, const float* a, int K, int lane, bool vec) {
   float acc = 0.f;
   if (vec) {
     for (int i = lane * 4; i < K; i += 128) {
@@ -231,9 +231,9 @@ constexpr int MG_THREADS = 256, MG_ROWS = 32;
 __device__ __forceinline__ int moe_gate_row(int j, int grp) { return j / grp * 2 * grp + j % grp; }
 
 template <typename TA, typename TW, typename TO>
-__global__ void __launch_bounds__(MG_THREADS) moe_gate_up_rows_kernel(const TA* __restrict__ xn, long ldx,
-                                                                      const TW* __restrict__ wgu, const int* __restrict__ expert,
-                                                                      const float* __restrict__ weight, TO* __restrict__ act,
+__global__ void __launch_bounds__(MG_THREADS) moe_gate_up_rows_kernel(const TA* xn, long ldx,
+                                                                      const TW* __restrict__ wgu, const int* expert,
+                                                                      const float* weight, TO* __restrict__ act,
                                                                       int W, int F, int top, int vec, int at_output, int E, int grp) {
   extern __shared__ __align__(16) float mg_row[];      // [W]
   hb_pdl_launch();
@@ -275,10 +275,10 @@ HB_EXPORT int hb_moe_gate_up_rows(const void* xn, int x_dt, long ldx, const void
 }
 
 template <typename TA, typename TW>
-__global__ void __launch_bounds__(MG_THREADS) moe_down_rows_kernel(const TA* __restrict__ act, const TW* __restrict__ wd,
-                                                                   const int* __restrict__ expert, float* __restrict__ y, long ldy,
-                                                                   int W, int F, int top, int vec, int E, const TA* __restrict__ xn,
-                                                                   long ldx, const float* __restrict__ identity_weight) {
+__global__ void __launch_bounds__(MG_THREADS) moe_down_rows_kernel(const TA* act, const TW* __restrict__ wd,
+                                                                   const int* expert, float* y, long ldy,
+                                                                   int W, int F, int top, int vec, int E, const TA* xn,
+                                                                   long ldx, const float* identity_weight) {
   extern __shared__ __align__(16) float md_act[];      // [top][F4], F4 = F rounded up to four
   hb_pdl_launch();
   hb_pdl_wait();
@@ -344,7 +344,7 @@ template <> struct MxVec4<__nv_bfloat16> { using type = uint2; };
 
 // One round: R rows (the first nr of them live) against the block's MX_TILE output features.
 template <typename TA, typename TW, int R>
-__device__ __forceinline__ void mx_round(const TA* __restrict__ a, long lda, const int* mx_row, int nr, const TW* __restrict__ we,
+__device__ __forceinline__ void mx_round(const TA* a, long lda, const int* mx_row, int nr, const TW* __restrict__ we,
                                          float* __restrict__ out, TA* rows, int g0, int n0, int Nout, int K, int KS, int vec) {
   using V4 = typename MxVec4<TA>::type;
   const int tid = threadIdx.x, lane = tid & 31;
@@ -414,8 +414,8 @@ __device__ __forceinline__ void mx_round(const TA* __restrict__ a, long lda, con
 }
 
 template <typename TA, typename TW>
-__global__ void __launch_bounds__(MX_THREADS) moe_grouped_kernel(const TA* __restrict__ a, long lda, const int* __restrict__ src,
-                                                                 int top, const TW* __restrict__ w, const int* __restrict__ offsets,
+__global__ void __launch_bounds__(MX_THREADS) moe_grouped_kernel(const TA* a, long lda, const int* src,
+                                                                 int top, const TW* __restrict__ w, const int* offsets,
                                                                  float* __restrict__ out, int Nout, int K, int KS, int vec) {
   extern __shared__ __align__(16) unsigned char mx_raw[];
   __shared__ int mx_row[MX_RB];
@@ -638,7 +638,7 @@ constexpr int MS_THREADS = 1024;
 
 // One block. Which sorted row a pair gets inside its expert's block depends on the order in which the threads arrive; a
 // row's result does not depend on where it lies.
-__global__ void __launch_bounds__(MS_THREADS) moe_sort_kernel(const int* __restrict__ expert, int* __restrict__ offsets,
+__global__ void __launch_bounds__(MS_THREADS) moe_sort_kernel(const int* expert, int* __restrict__ offsets,
                                                               int* __restrict__ pos, int* __restrict__ src, int pairs, int E) {
   extern __shared__ int ms_sm[];       // [E] counts, then cursors; [E] first sorted row of each expert
   int* count = ms_sm;
@@ -678,8 +678,8 @@ HB_EXPORT int hb_moe_sort(const int* expert, int* offsets, int* pos, int* src, i
 }
 
 template <typename TA>
-__global__ void __launch_bounds__(128) moe_gather_kernel(const TA* __restrict__ xn, long ldx, const int* __restrict__ src,
-                                                         TA* __restrict__ xs, int W, int top, const int* __restrict__ limit) {
+__global__ void __launch_bounds__(128) moe_gather_kernel(const TA* xn, long ldx, const int* src,
+                                                         TA* __restrict__ xs, int W, int top, const int* limit) {
   hb_pdl_launch();
   hb_pdl_wait();
   if (limit && blockIdx.x >= *limit) return;
@@ -698,9 +698,9 @@ HB_EXPORT int hb_moe_gather(const void* xn, int x_dt, long ldx, const int* src, 
 
 // gu [rows][g (F) | u (F)] 32-bit, sorted rows; the pair's score enters here
 template <typename TO>
-__global__ void __launch_bounds__(256) moe_act_kernel(const float* __restrict__ gu, const int* __restrict__ src,
-                                                      const float* __restrict__ weight, TO* __restrict__ act, long n, int F,
-                                                      int at_output, const int* __restrict__ limit, int grp) {
+__global__ void __launch_bounds__(256) moe_act_kernel(const float* gu, const int* src,
+                                                      const float* weight, TO* __restrict__ act, long n, int F,
+                                                      int at_output, const int* limit, int grp) {
   hb_pdl_launch();
   hb_pdl_wait();
   if (limit) n = (long)*limit * F;
@@ -717,9 +717,9 @@ __global__ void __launch_bounds__(256) moe_act_kernel(const float* __restrict__ 
 
 // Four columns a thread (F a multiple of four, aligned rows): the same values.
 template <typename TO>
-__global__ void __launch_bounds__(256) moe_act_vec_kernel(const float* __restrict__ gu, const int* __restrict__ src,
-                                                          const float* __restrict__ weight, TO* __restrict__ act, long n4, int F,
-                                                          int at_output, const int* __restrict__ limit, int grp) {
+__global__ void __launch_bounds__(256) moe_act_vec_kernel(const float* gu, const int* src,
+                                                          const float* weight, TO* __restrict__ act, long n4, int F,
+                                                          int at_output, const int* limit, int grp) {
   hb_pdl_launch();
   hb_pdl_wait();
   const int F4 = F >> 2;
@@ -757,10 +757,10 @@ HB_EXPORT int hb_moe_act(const float* gu, const int* src, const float* weight, v
 }
 
 template <typename TA>
-__global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restrict__ ys, const int* __restrict__ pos,
-                                                          float* __restrict__ y, long ldy, long n, int W, int top,
-                                                          const int* __restrict__ limit, const TA* __restrict__ xn, long ldx,
-                                                          const float* __restrict__ identity_weight) {
+__global__ void __launch_bounds__(256) moe_combine_kernel(const float* ys, const int* pos,
+                                                          float* y, long ldy, long n, int W, int top,
+                                                          const int* limit, const TA* xn, long ldx,
+                                                          const float* identity_weight) {
   hb_pdl_launch();
   hb_pdl_wait();
   const int lim = limit ? *limit : 0x7fffffff;
@@ -779,10 +779,10 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restric
 
 // Four columns a thread: the same sums.
 template <typename TA>
-__global__ void __launch_bounds__(256) moe_combine_vec_kernel(const float* __restrict__ ys, const int* __restrict__ pos,
-                                                              float* __restrict__ y, long ldy, long n4, int W4, int top,
-                                                              const int* __restrict__ limit, const TA* __restrict__ xn, long ldx,
-                                                              const float* __restrict__ identity_weight) {
+__global__ void __launch_bounds__(256) moe_combine_vec_kernel(const float* ys, const int* pos,
+                                                              float* y, long ldy, long n4, int W4, int top,
+                                                              const int* limit, const TA* xn, long ldx,
+                                                              const float* identity_weight) {
   hb_pdl_launch();
   hb_pdl_wait();
   const int lim = limit ? *limit : 0x7fffffff;

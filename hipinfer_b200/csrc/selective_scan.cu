@@ -317,7 +317,7 @@ HB_EXPORT int hb_selective_scan(const float* x, long ldx, const float* dt, long 
 
 // A 32-bit matrix as the sum of two bfloat16 matrices, hi = round(a) and lo = round(a - hi): two tensor-core products
 // with them, added in 32-bit, carry 16 bits of a's mantissa instead of 8 (the low-rank step sizes into their product).
-__global__ void __launch_bounds__(256) split_rounded_kernel(const float* __restrict__ a, long lda, __nv_bfloat16* __restrict__ hi,
+__global__ void __launch_bounds__(256) split_rounded_kernel(const float* a, long lda, __nv_bfloat16* __restrict__ hi,
                                                             __nv_bfloat16* __restrict__ lo, long n, int K) {
   hb_pdl_launch();
   hb_pdl_wait();
@@ -351,8 +351,8 @@ HB_EXPORT int hb_split_rounded(const float* a, long lda, void* hi, void* lo, int
 // with eps inside the root; everything 32-bit; one block a row, the row kept in shared memory between the passes.
 // ---------------------------------------------------------------------------------------------------------------------
 template <typename TW, typename TO>
-__global__ void __launch_bounds__(256) residual_norm_kernel(float* __restrict__ x, const float* __restrict__ y,
-                                                            const float* __restrict__ a, const float* __restrict__ b,
+__global__ void __launch_bounds__(256) residual_norm_kernel(float* x, const float* y,
+                                                            const float* a, const float* b,
                                                             const TW* __restrict__ wa, const TW* __restrict__ wb, float mix,
                                                             float pair_eps, float alpha, const float* __restrict__ w,
                                                             float eps, TO* __restrict__ xb, int W) {

@@ -23,9 +23,9 @@ constexpr int SC_THREADS = 128;
 // inputs before them in registers. Only the block of a request's first chunk reads the carried inputs, and it alone writes
 // the new ones, after it has read the old: nothing else in the launch touches them.
 template <typename TW, int TAPS>
-__global__ void __launch_bounds__(SC_THREADS) ssd_conv_kernel(const float* __restrict__ proj, long ld, int off,
+__global__ void __launch_bounds__(SC_THREADS) ssd_conv_kernel(const float* proj, long ld, int off,
                                                               const TW* __restrict__ w, const TW* __restrict__ bias,
-                                                              float* __restrict__ carried, const int* __restrict__ q_start,
+                                                              float* carried, const int* __restrict__ q_start,
                                                               const int* __restrict__ q_len, const int* __restrict__ slot,
                                                               float* __restrict__ out, int C, int K) {
   hb_pdl_launch();
@@ -409,7 +409,7 @@ HB_EXPORT int hb_ssd_scan(const float* xbc, long ldx, const float* dt, long lddt
 
 // One block a row: y silu(z), then every part of the row by its own root mean square, times the weight.
 template <typename TW, typename TO>
-__global__ void __launch_bounds__(256) ssd_gate_norm_kernel(const float* __restrict__ y, const float* __restrict__ z, long ldz,
+__global__ void __launch_bounds__(256) ssd_gate_norm_kernel(const float* y, const float* z, long ldz,
                                                             const TW* __restrict__ w, TO* __restrict__ out, int inner,
                                                             int parts, float eps) {
   __shared__ float sh[32];
