@@ -443,8 +443,9 @@ def gemm_plain(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: 
     M, K = a.shape
     N = w.shape[0]
     assert w.shape[1] == K and out.shape == (M, N), (a.shape, w.shape, out.shape)
+    ws = _simt_workspace(M, N, K, out.device)      # (held until the launch)
     _call("core", "hb_gemm_simt", a.data_ptr(), _dt(a), a.stride(0), w.data_ptr(), _dt(w), w.stride(0),
-          out.data_ptr(), _dt(out), out.stride(0), M, N, K, 1 if accumulate else 0, _ptr(_simt_workspace(M, N, K, out.device)), _stream())
+          out.data_ptr(), _dt(out), out.stride(0), M, N, K, 1 if accumulate else 0, _ptr(ws), _stream())
     return out
 
 
@@ -685,8 +686,9 @@ def linear_scaled_add(a: torch.Tensor, w: Weight, x: torch.Tensor, scale: torch.
         y = torch.empty(M, N, dtype=torch.float32, device=a.device)
         gemm_plain(a, w.t, y)
         return scale_add(x, y, scale)
+    ws = _simt_workspace(M, N, a.shape[1], x.device)      # (held until the launch)
     _call("core", "hb_gemm_simt_scaled", a.data_ptr(), _dt(a), a.stride(0), w.t.data_ptr(), _dt(w.t), w.t.stride(0),
-          x.data_ptr(), x.stride(0), M, N, a.shape[1], scale.data_ptr(), _ptr(_simt_workspace(M, N, a.shape[1], x.device)), _stream())
+          x.data_ptr(), x.stride(0), M, N, a.shape[1], scale.data_ptr(), _ptr(ws), _stream())
     return x
 
 
