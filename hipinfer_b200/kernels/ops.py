@@ -450,15 +450,21 @@ def gemm_plain(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: 
 
 
 def _simt_workspace(M, N, K, device):
-    """The partial sums of a plain product whose K is split over blocks (None: it is not)."""
+    """The partial sums of a plain product whose K is split over blocks. None: it is not, or no memory is left for them (the
+    unsplit kernel needs none and gives the same bits)."""
     if M <= 8:          # a few rows never need one (csrc/gemm_simt.cu: SR_ROWS); where their sizes refuse that kernel, unsplit
         return None
     lib = library.load("core")
     lib.hb_gemm_simt_workspace.restype = C.c_long
     n = lib.hb_gemm_simt_workspace(M, N, K)
-    if n:
-        library.launches[0] += 1     # the kernel that adds the slices
-    return torch.empty(n, dtype=torch.float32, device=device) if n else None
+    if not n:
+        return None
+    try:
+        ws = torch.empty(n, dtype=torch.float32, device=device)
+    except torch.OutOfMemoryError:
+        return None
+    library.launches[0] += 1     # the kernel that adds the slices
+    return ws
 
 
 def swiglu(gate_up: torch.Tensor, out: torch.Tensor, group: int) -> torch.Tensor:

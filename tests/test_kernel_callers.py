@@ -46,3 +46,16 @@ def test_a_plain_product_holds_its_workspace_until_it_is_launched(launches, whic
     """A buffer given back before the launch may be another thread's by then, or unmapped."""
     list(products())[which]()
     assert len(launches) == 1 and launches[0].buffers and launches[0].buffers[-1] in launches[0].args and launches[0].held[-1]
+
+
+@pytest.mark.parametrize("which", [0, 1])
+def test_a_plain_product_runs_unsplit_where_no_memory_is_left(launches, which, monkeypatch):
+    """The workspace is for speed alone: without one the kernel gives the same bits."""
+    def none_left(*size, **kw):
+        raise torch.OutOfMemoryError("CUDA out of memory")
+
+    run = list(products())[which]
+    counted = library.launches[0]
+    monkeypatch.setattr(torch, "empty", none_left)
+    run()
+    assert len(launches) == 1 and launches[0].args[-2] is None and library.launches[0] == counted
