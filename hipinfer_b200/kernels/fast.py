@@ -176,13 +176,13 @@ def gemm_stream(a, w, out, epi):
 
 
 class Slices:
-    """A small product a @ w.T left as the K slices it was computed in: fp32 [ksplit][rows][row_stride]
-    in the scratch that all small products share, so it has to be consumed (or finished) before
-    the next of them runs; `check()` raises if it was not."""
+    """A product a @ w.T left as the K slices it was computed in: fp32 [ksplit][rows][row_stride]. Those of a few rows lie in the
+    scratch that all small products share, so they have to be consumed (or finished) before the next of them runs; `check()`
+    raises if they were not. Those of a portion (gen None) lie in a buffer of their own, which the object holds."""
     __slots__ = ("ws", "ksplit", "slice_stride", "row_stride", "M", "N", "K", "gen")      # (slice_stride: rows of a slice x row_stride)
 
     def check(self):
-        if self.gen != _scratch_gen[0]:
+        if self.gen is not None and self.gen != _scratch_gen[0]:
             raise RuntimeError("a product left as slices was overwritten by a later product before it was consumed")
 
 
@@ -248,23 +248,21 @@ def linear_slices(a, w):
 
 
 def gemm_tc_slices(a, w):
-    """The CTA-pair kernel with K in slices that are left for the consumer (csrc/gemm_tc.cu); None where it would not split."""
+    """The CTA-pair kernel with K in slices that are left for the consumer (csrc/gemm_tc.cu); None where it would not split. The
+    slices' buffer is the call's own (prompts on two streams or threads of a device may run at the same time)."""
     M, K = a.shape
     N = w.shape[0]
     n = _fn("hb_gemm_tc_splits")(M, N, K)
     if not n:
         return None
     rows, ld = -(-M // 256) * 256, -(-N // 32) * 32
-    ws, _ = _stream_scratch(a.device, n * rows * ld, 0)
-    _scratch_gen[0] += 1
+    ws = torch.empty(n * rows * ld, dtype=torch.float32, device=a.device)
     _call("hb_gemm_tc_slices", a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), ws.data_ptr(), ld, ws.numel(), M, N, K, n,
           _status_ptr(), _stream())
     sl = Slices()
     sl.ws, sl.ksplit, sl.row_stride, sl.slice_stride = ws, n, ld, rows * ld
-    sl.M, sl.N, sl.K, sl.gen = M, N, K, _scratch_gen[0]
+    sl.M, sl.N, sl.K, sl.gen = M, N, K, None
     return sl
-
-
 
 
 def _gemm(a, w, out, epi):

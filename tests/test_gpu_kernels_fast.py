@@ -767,3 +767,23 @@ def test_products_of_few_tiles_in_slices(M, N, K):
     fast().finish_slices(fast().gemm_tc_slices(a, w), x, fast().EPI_ADD_F32)
     assert torch.equal(x, want)
     assert fast().gemm_tc_slices(rnd(2048, 512, seed=84), rnd(4096, 512, seed=85)) is None
+
+
+def test_slices_of_two_portions_at_the_same_time():
+    """Slices of portions lie in buffers of their own: two are left at once, with a product of a few rows (which uses the scratch that
+    small products share) in between, and each finishes as its own product."""
+    from hipinfer_b200.kernels import ops
+
+    a, w = rnd(130, 1024, seed=86), ops.Weight(rnd(512, 1024, seed=87, scale=0.05))
+    b, v = rnd(300, 2048, seed=88), ops.Weight(rnd(264, 2048, seed=89, scale=0.05))
+    one, two = (torch.zeros(m, n, device=DEV) for m, n in ((130, 512), (300, 264)))
+    first, second = ops.linear_deferred(a, w, one), ops.linear_deferred(b, v, two)
+    assert first is not None and second is not None
+    small = torch.empty(20, 512, device=DEV)
+    ops.linear(a[:20], w, small)
+    second.finish()
+    first.finish()
+    sync_check()
+    for got, x, y in ((one, a, w.t), (two, b, v.t), (small, a[:20], w.t)):
+        bound = x.shape[1] * 2.0 ** -23 * (x.double().abs() @ y.double().abs().T)
+        assert bool(((got.double() - x.double() @ y.double().T).abs() <= bound).all())
