@@ -314,7 +314,7 @@ static int delta_rule_launch_reg(const DeltaArgs& A, dim3 grid, cudaStream_t s) 
 template <typename TW, typename TO>
 static int delta_rule_launch(const DeltaArgs& A, int R, cudaStream_t s) {
   const dim3 grid(A.heads, R);
-  switch (A.D) {
+  if (!((uintptr_t)A.state & 7)) switch (A.D) {      // (the register kernels read the state in pairs)
     case 32: return delta_rule_launch_reg<TW, TO, 8>(A, grid, s);
     case 64: return delta_rule_launch_reg<TW, TO, 16>(A, grid, s);
     case 128: return delta_rule_launch_reg<TW, TO, 32>(A, grid, s);

@@ -350,7 +350,8 @@ HB_EXPORT int hb_gla(const float* proj, long ld, int q_off, int k_off, int v_off
   if (smem > 200 * 1024) HB_FAIL("hb_gla: heads of %d x %d do not fit shared memory", D, E);
   dim3 grid(H, n_requests);
   // two jobs a block: the fewest threads a channel pair (a power of two) that give 128 walkers or more with 8 to 32 key channels each
-  if (A.vec4) {
+  // (the walkers read the state in pairs)
+  if (A.vec4 && !((uintptr_t)state & 7)) {
     for (int c = 1; c <= 32; c *= 2) {
       const int dpt = D % c ? 0 : D / c, walkers = E / 2 * c;
       if ((dpt != 8 && dpt != 16 && dpt != 32) || walkers < 128 || walkers % 32 || walkers > (dpt == 32 ? 256 : 512)) continue;

@@ -170,6 +170,31 @@ def test_delta_rule_against_token_by_token(dtype, heads, D, force_any):
     assert torch.equal(out1, out)
 
 
+@pytest.mark.parametrize("D", [32, 64, 128])
+def test_delta_rule_with_a_state_on_an_odd_address(D):
+    """A state tensor that starts on no multiple of eight bytes: the register kernels read it in pairs and leave it to the kernel in
+    shared memory."""
+    from hipinfer_b200.kernels import ops
+
+    heads, T = 2, 5
+    HD = heads * D
+    proj, w_raw = rnd(T, 5 * HD, seed=1).to(DEV), rnd(T, HD, seed=2).to(DEV)
+    vec = [t.to(DEV) for t in (rnd(HD, seed=3), rnd(HD, seed=4), 1 + 0.2 * rnd(HD, seed=5))]
+    i32 = lambda v: torch.tensor([v], dtype=torch.int32, device=DEV)
+    batch = SimpleNamespace(n_requests=1, req_q_start=i32(0), req_q_len=i32(T), req_state_slot=i32(1))
+    state0, got = rnd(2, heads, D, D, seed=6).to(DEV), []
+    for offset, any_ in ((1, False), (0, True)):
+        room = torch.zeros(state0.numel() + 4, device=DEV)
+        state = room[offset:offset + state0.numel()].view_as(state0)
+        state.copy_(state0)
+        out = torch.empty(T, HD, device=DEV)
+        ops.delta_rule(proj, (0, HD, 2 * HD, 3 * HD, 4 * HD), w_raw, *vec, state, batch, out, heads, D, 0.6, 1e-6, 1e-5, force_any=any_)
+        got.append((out, state.clone(), room[:offset].clone(), room[offset + state0.numel():].clone()))
+    torch.cuda.synchronize()
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and torch.isfinite(got[0][0]).all()
+    assert not got[0][2].any() and not got[0][3].any()
+
+
 def test_delta_rule_register_and_shared_memory_kernels_agree():
     from hipinfer_b200.kernels import ops
 

@@ -310,6 +310,27 @@ def test_gated_linear_attention(dtype, H, D, E, tau):
     assert torch.equal(out2, out) and torch.equal(state2, state)
 
 
+def test_gated_linear_attention_with_a_state_on_an_odd_address():
+    """A state tensor that starts on no multiple of eight bytes: the kernel whose walkers read it in pairs leaves it to the other."""
+    from hipinfer_b200.kernels import ops
+
+    H, D, E, T = 2, 64, 64, 21
+    HD, HE = H * D, H * E
+    proj, z, ab, nw = rnd(T, 2 * HD + 2 * HE, seed=1), rnd(T, HD, seed=2), rnd(HD, seed=3), 1 + 0.2 * rnd(E, seed=4)
+    state0 = rnd(1, H, D, E, seed=5)
+    room = torch.zeros(state0.numel() + 4, device=DEV)
+    state = room[1:1 + state0.numel()].view_as(state0)
+    state.copy_(state0)
+    i32 = lambda v: torch.tensor([v], dtype=torch.int32, device=DEV)
+    batch = SimpleNamespace(n_requests=1, req_q_start=i32(0), req_q_len=i32(T), req_state_slot=i32(0))
+    out = torch.empty(T, HE, device=DEV)
+    ops.gla(proj.to(DEV), (0, HD, 2 * HD, 2 * HD + HE), z.to(DEV), ab.to(DEV), nw.to(DEV), state, batch, out, H, D, E, 16.0, 1e-5)
+    want, state_want = _gla_plain(proj, z, ab, nw, state0, [T], [0], H, D, E, 16.0, 1e-5)
+    close(out, want, torch.float32, "outputs")
+    close(state, state_want, torch.float32, "states")
+    assert float(room[0]) == 0.0 and not room[1 + state0.numel():].any()
+
+
 def test_a_decay_of_one_keeps_and_a_decay_of_zero_forgets():
     """With a large positive pre-activation the state keeps everything (o is the running sum of k v^T applied to q); with a
     large negative one only the current token is left."""
