@@ -5,7 +5,10 @@
 // One CTA of four warps per (tile of 64 ABSOLUTE positions, kv head and tile of 16 MT heads of the group, row); MT = 1 (up to 16
 // heads a tile) or 2 (up to 32). The CTAs of HS_SPLIT_TILES = 8 neighbouring tiles are one cluster: a decode step of few
 // requests has few tiles, and a CTA that walked four of them in a row kept 20 of 148 SMs busy for 36 us (4 rows of 1,200 keys, 32
-// heads, a latent of 256 + 32; 12 us now). Within a CTA the warps split the keys for the scores (16 keys each, all heads)
+// heads, a latent of 256 + 32; 14 us now). CTAs of a cluster that have no tile leave at once, and where no row of the call
+// has as many as eight tiles the cluster is smaller; while the call's CTAs are fewer than two an SM, some without a tile stay and share
+// the join. With all eight kept to the end many short rows paid for them: 64 rows of 40 keys, 32 heads over 8 kv heads of 64,
+// took 35 us, 10.5 before the tiles had CTAs of their own, 7.5 now; 64 rows of 600 keys 78, 62 and 60 us. Within a CTA the warps split the keys for the scores (16 keys each, all heads)
 // and the value columns for the sums; scores and probabilities pass through shared memory. The keys are read as soon as the
 // block runs, ahead of the wait for the kernel before it, where the whole tile is of earlier steps. Queries lie in shared memory
 // (any D that is a multiple of 16); the values may be the first E columns of the key rows (a latent that serves as both), in
@@ -35,7 +38,7 @@ struct HeadsArgs {
   const int* q_len; int row_limit;
   float* part;                          // [T][G][ZT][splits][16 MT][E + 4], T by the place in the list
   int G_ZT;                             // head tiles: G * ZT
-  int splits;
+  int splits, cs, join;                 // clusters of a row, their CTAs, and how many of those stay for the join where they have no tile
   const float* r1; const float* r2;     // [H] or null: r1 ln(1 + r2 (p - j)) is taken off the score
 };
 
@@ -71,14 +74,18 @@ __global__ void __launch_bounds__(HS_THREADS) attn_masked_heads_kernel(HeadsArgs
   __shared__ __align__(8) float mls[HS_SPLIT_TILES][MR][2];   // every CTA's maxima and weight sums, put here by that CTA
   hb_pdl_launch();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quad = lane >> 2, qi = lane & 3;
-  const int rank = blockIdx.x % HS_SPLIT_TILES, split = blockIdx.x / HS_SPLIT_TILES, ZT = A.G_ZT / A.G, g = blockIdx.y / ZT, z = blockIdx.y % ZT;
+  const int rank = blockIdx.x % A.cs, split = blockIdx.x / A.cs, ZT = A.G_ZT / A.G, g = blockIdx.y / ZT, z = blockIdx.y % ZT;
   const int tw = blockIdx.z, t = A.row_list ? A.row_list[tw] : tw, rq = A.row_req[t], p = A.pos[t];
   int lo = 0, keep = 0;
   if (A.mask == 1 && A.window > 0) { lo = max(0, p - A.window + 1); keep = min(A.keep_first, p + 1); }
   else if (A.mask == 2 && A.chunk > 0) lo = (p / A.chunk) * A.chunk;
   const int n_tiles = hs_tile_count(p, lo, keep);
   const int n_splits_row = (n_tiles + HS_SPLIT_TILES - 1) / HS_SPLIT_TILES;       // a matter of the row's position alone
-  if ((A.q_len && A.q_len[rq] >= A.row_limit) || split >= n_splits_row) {          // the same for the whole cluster
+  const int n_here = min(A.cs, n_tiles - split * HS_SPLIT_TILES);                 // (one cluster a row where cs is less than eight)
+  const int n_join = n_here > 0 ? max(n_here, A.join) : 0;
+  const bool has = rank < n_here;
+  // nothing for this CTA to do: it leaves (the cluster's barriers are of the CTAs that have not left, and nobody writes to it)
+  if ((A.q_len && A.q_len[rq] >= A.row_limit) || rank >= n_join) {
     if ((blockIdx.x | blockIdx.y | blockIdx.z) == 0) hb_pdl_wait();                // the grid never ends before the one ahead of it
     return;
   }
@@ -93,8 +100,6 @@ __global__ void __launch_bounds__(HS_THREADS) attn_masked_heads_kernel(HeadsArgs
   __nv_bfloat16* Ps = (__nv_bfloat16*)(Ss + MR * SP);        // [MR][PP]
   const int RS = E + 4;                 // a row's sums, then its maximum and weight sum; rows stay 16-byte aligned
   float* stage = (float*)hs_smem;       // [MR][RS] over queries and keys, when these are done with
-  const int n_here = min(HS_SPLIT_TILES, n_tiles - split * HS_SPLIT_TILES);
-  const bool has = rank < n_here;
   const int k0 = has ? hs_tile_at(split * HS_SPLIT_TILES + rank, lo, keep) * HK : 0;
   // where the tile's 64 keys lie, one thread a key
   if (tid < HK) {
@@ -192,8 +197,8 @@ __global__ void __launch_bounds__(HS_THREADS) attn_masked_heads_kernel(HeadsArgs
       const float l = hb_warp_sum(ea + eb);
       Ps[r * PP + lane] = __float2bfloat16_rn(ea);
       Ps[r * PP + 32 + lane] = __float2bfloat16_rn(eb);
-      // to every CTA of the cluster, the CTA itself included
-      if (lane < HS_SPLIT_TILES)
+      // to every CTA of the join, the CTA itself included
+      if (lane < n_join)
         asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(hb_mapa(&mls[rank][r][0], lane)), "f"(m), "f"(l) : "memory");
     }
     __syncthreads();
@@ -243,7 +248,7 @@ __global__ void __launch_bounds__(HS_THREADS) attn_masked_heads_kernel(HeadsArgs
   const int C4 = E / 4;
   const size_t slot = ((size_t)tw * A.G + g) * ZT + z;
   float* part = n_splits_row > 1 ? A.part + (slot * A.splits + split) * (size_t)MR * RS : nullptr;
-  for (int i = rank * HS_THREADS + tid; i < nh * C4; i += HS_SPLIT_TILES * HS_THREADS) {
+  for (int i = rank * HS_THREADS + tid; i < nh * C4; i += n_join * HS_THREADS) {
     const int r = i / C4, e = (i - r * C4) * 4;
     float4 v[HS_SPLIT_TILES];
 #pragma unroll
@@ -352,17 +357,19 @@ static size_t hs_smem_bytes(int MT, int D, int E, int alias) {
   const size_t stage = MR * (E + 4) * 4;
   return tiles > stage ? tiles : stage;
 }
-static int hs_splits(int mask, int window, int keep_first, int chunk, int max_pos) {
+// The most tiles a row up to max_pos can have.
+static int hs_most_tiles(int mask, int window, int keep_first, int chunk, int max_pos) {
   int worst = max_pos / HK + 1;
   if (mask == 1 && window > 0) {
     const int w = (window - 1 + HK - 1) / HK + 1 + (keep_first > 0 ? (keep_first - 1) / HK + 1 : 0);
     if (w < worst) worst = w;
   } else if (mask == 2 && chunk > 0) {
-    const int w = (chunk - 1 + HK - 1) / HK + 1;
+    const int w = chunk % HK == 0 ? chunk / HK : (chunk - 1 + HK - 1) / HK + 1;
     if (w < worst) worst = w;
   }
-  return (worst + HS_SPLIT_TILES - 1) / HS_SPLIT_TILES;
+  return worst < 1 ? 1 : worst;
 }
+static int hs_splits(int most_tiles) { return (most_tiles + HS_SPLIT_TILES - 1) / HS_SPLIT_TILES; }
 
 // units of 16 value columns a warp owns for these sizes; 0: not a size the kernel takes
 static int hs_units(int H, int G, int D, int E, int alias) {
@@ -380,7 +387,7 @@ HB_EXPORT int hb_attn_masked_heads_supported(int H, int G, int D, int E, int ali
 
 HB_EXPORT long hb_attn_masked_heads_workspace(int T, int H, int G, int E, int mask, int window, int keep_first, int chunk, int max_pos) {
   const int HG = H / G, MT = hs_mt(HG), ZT = (HG + 16 * MT - 1) / (16 * MT);
-  const int splits = hs_splits(mask, window, keep_first, chunk, max_pos);
+  const int splits = hs_splits(hs_most_tiles(mask, window, keep_first, chunk, max_pos));
   if (splits <= 1) return 0;
   return (long)T * G * ZT * splits * 16 * MT * (E + 4);
 }
@@ -409,19 +416,24 @@ HB_EXPORT int hb_attn_masked_heads(const void* q, long ldq, const void* kc, long
   A.MT = hs_mt(HG);
   const int ZT = (HG + 16 * A.MT - 1) / (16 * A.MT);
   A.G_ZT = G * ZT;
-  A.splits = hs_splits(mask, window, keep_first, chunk, max_pos);
-  if (A.splits < 1) A.splits = 1;
+  const int most = hs_most_tiles(mask, window, keep_first, chunk, max_pos);
+  A.splits = hs_splits(most);
+  // the join's CTAs: a power of two, two an SM at most over the whole call, no more than there are columns for
+  A.join = HS_SPLIT_TILES;
+  while (A.join > 1 && ((long)T * A.G_ZT * A.splits * A.join > 296 || A.join * HS_THREADS / 2 >= (HG < 16 * A.MT ? HG : 16 * A.MT) * (E / 4))) A.join /= 2;
+  A.cs = most > 4 ? HS_SPLIT_TILES : most > 2 ? 4 : most;
+  if (A.cs < A.join) A.cs = A.join;
   if (A.splits > 1 && (!part || n_part < (long)T * G * ZT * A.splits * 16 * A.MT * (E + 4)))
     HB_FAIL("hb_attn_masked_heads: rows of up to %d key tiles need a workspace", A.splits * HS_SPLIT_TILES);
   if ((long)ZT * G > 65535) HB_FAIL("hb_attn_masked_heads: the grid is too large");
   const size_t smem = hs_smem_bytes(A.MT, D, E, alias);
-  const dim3 grid(HS_SPLIT_TILES * A.splits, G * ZT, T);
+  const dim3 grid(A.cs * A.splits, G * ZT, T);
   cudaError_t e = cudaErrorInvalidValue;
 #define HS_RUN(EU, MT)                                                                                                            \
   do {                                                                                                                            \
     auto kern = o_dt == HB_BF16 ? attn_masked_heads_kernel<EU, MT, __nv_bfloat16> : attn_masked_heads_kernel<EU, MT, float>;      \
     e = smem + 8192 > 48 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : cudaSuccess; \
-    if (e == cudaSuccess) e = hb_launch_cluster(kern, grid, dim3(HS_THREADS), smem, s, dim3(HS_SPLIT_TILES, 1, 1), A);            \
+    if (e == cudaSuccess) e = hb_launch_cluster(kern, grid, dim3(HS_THREADS), smem, s, dim3(A.cs, 1, 1), A);            \
   } while (0)
   if (A.MT == 2) {
     if (eu == 1) HS_RUN(1, 2);

@@ -486,3 +486,33 @@ def test_heads_linear_of_all_and_of_listed_rows(wdt, H, K, N, tail, T):
     batch = SimpleNamespace(row_request=i32([0] * T), req_q_len=i32([T]), short_rows=lambda limit: (i32(pick), 0))
     ops.heads_linear(a.to(DEV), K + tail, w.to(DEV), some, N + tail, batch=batch, row_limit=16, **kw)
     assert torch.equal(some[pick], out[pick]) and bool((some[[t for t in range(T) if t not in pick]] == 5.0).all())
+
+
+@pytest.mark.parametrize("H,G,D,E", [(32, 1, 288, 256), (8, 2, 64, 64)])
+def test_single_rows_in_clusters_of_every_size(H, G, D, E):
+    """One, two, three to four and more tiles of 64 keys (clusters of 1, 2, 4 and 8 CTAs, CTAs without a tile that leave or stay for
+    the join, rows of two clusters): a row's bits depend neither on the call's longest row nor on how many rows it has."""
+    from hipinfer_b200.kernels import ops
+
+    dtype, ps, alias = torch.bfloat16, 16, G == 1
+    lens = [40, 64, 65, 128, 180, 256, 300, 512, 513, 700]
+    keys = [rnd(n, G, D, seed=10 + r) for r, n in enumerate(lens)]
+    values = [k[..., :E] if alias else rnd(n, G, E, seed=30 + r) for r, (k, n) in enumerate(zip(keys, lens))]
+    kc, vc, bt = _paged(keys, values, ps, dtype, seed=3, **(dict(alias=True) if alias else {}))
+    q = rnd(len(lens), H * D, seed=5).to(dtype).to(DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+
+    def run(rows, max_pos):
+        batch = SimpleNamespace(block_tables=[bt], row_request=i32(rows), positions=i32([lens[r] - 1 for r in rows]), max_pos=max_pos)
+        out = torch.empty(len(rows), H * E, dtype=torch.float32, device=DEV)
+        ops.attention_masked(q[rows].contiguous(), kc, kc if alias else vc, batch, 0, out, H, G, D, E, ps, D ** -0.5, "causal", 0, 0, 0)
+        return out
+
+    every = run(list(range(len(lens))), 2047)
+    for r, n in enumerate(lens):
+        want = _attend_plain(q[r].cpu().double().view(H, D), keys[r].to(dtype).double(), values[r].to(dtype).double(), n - 1, H, G, D ** -0.5,
+                             "causal", 0, 0, 0, None, None, False)
+        close(every[r], want, dtype, f"{n} keys")
+        assert torch.equal(run([r], n - 1)[0], every[r]), n                         # the smallest cluster that holds the row
+        many = run([r] * 200, n - 1)                                                # no CTA to spare for the join
+        assert torch.equal(many, every[r].expand_as(many)), n
