@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(HL_THREADS) heads_linear_kernel(const float* a
                                                                   const float* gate, long ld_gate, int gate_off,
                                                                   int tail, int rot, const int* __restrict__ pos,
                                                                   const float2* __restrict__ table,
-                                                                  const int* __restrict__ row_req,
+                                                                  const int* __restrict__ row_list, const int* __restrict__ row_req,
                                                                   const int* __restrict__ q_len, int row_limit, int pairing,
                                                                   int gate_per_head) {
   extern __shared__ float hl_a[];      // [HL_TM][K + tail], then [HL_KZ][HL_TM][HL_TN] partial sums
@@ -87,14 +87,15 @@ __global__ void __launch_bounds__(HL_THREADS) heads_linear_kernel(const float* a
   const int n = blockIdx.x * HL_TN + nl;
   const int KT_ = K + tail, rows = min(HL_TM, T - t0);
   float* red = hl_a + HL_TM * KT_;
+  auto row_of = [&](int r) { return row_list ? row_list[t0 + r] : t0 + r; };      // the row's place in a, out, gate and pos
   // rows of requests that bring row_limit rows or more belong to another path: a block all of whose rows do is idle
   unsigned skip = 0;
   if (q_len)
-    for (int r = 0; r < rows; r++) skip |= (q_len[row_req[t0 + r]] >= row_limit ? 1u : 0u) << r;
+    for (int r = 0; r < rows; r++) skip |= (q_len[row_req[row_of(r)]] >= row_limit ? 1u : 0u) << r;
   if (q_len && skip == (1u << rows) - 1u) return;
   for (int i = threadIdx.x; i < rows * KT_; i += HL_THREADS) {
     const int r = i / KT_, k = i - r * KT_;
-    hl_a[r * KT_ + k] = a[(size_t)(t0 + r) * lda + (size_t)h * a_head + k];
+    hl_a[r * KT_ + k] = a[(size_t)row_of(r) * lda + (size_t)h * a_head + k];
   }
   __syncthreads();
   float acc[HL_TM];
@@ -119,8 +120,8 @@ __global__ void __launch_bounds__(HL_THREADS) heads_linear_kernel(const float* a
       float o = 0.f;
 #pragma unroll
       for (int z = 0; z < HL_KZ; z++) o += red[(z * HL_TM + r) * HL_TN + nl];
-      if (gate) o *= 1.f / (1.f + expf(-gate[(size_t)(t0 + r) * ld_gate + gate_off + (gate_per_head ? (size_t)h : (size_t)h * N + n)]));
-      out[(size_t)(t0 + r) * ldo + (size_t)h * o_head + n] = hb_from_float<TO>(o);
+      if (gate) o *= 1.f / (1.f + expf(-gate[(size_t)row_of(r) * ld_gate + gate_off + (gate_per_head ? (size_t)h : (size_t)h * N + n)]));
+      out[(size_t)row_of(r) * ldo + (size_t)h * o_head + n] = hb_from_float<TO>(o);
     }
   } else if (n < N + tail && kz == 0) {
     const int j = n - N, half = rot >> 1;
@@ -131,11 +132,11 @@ __global__ void __launch_bounds__(HL_THREADS) heads_linear_kernel(const float* a
       if (j < rot) {
         const int i = pairing ? j >> 1 : (j < half ? j : j - half);
         const bool second = pairing ? (j & 1) : (j >= half);
-        const float2 c = table[(size_t)pos[t0 + r] * half + i];
+        const float2 c = table[(size_t)pos[row_of(r)] * half + i];
         const float u = src[pairing ? 2 * i : i], v = src[pairing ? 2 * i + 1 : i + half];
         y = second ? __fadd_rn(__fmul_rn(v, c.x), __fmul_rn(u, c.y)) : __fsub_rn(__fmul_rn(u, c.x), __fmul_rn(v, c.y));
       }
-      out[(size_t)(t0 + r) * ldo + (size_t)h * o_head + n] = hb_from_float<TO>(y);
+      out[(size_t)row_of(r) * ldo + (size_t)h * o_head + n] = hb_from_float<TO>(y);
     }
   }
 }
@@ -264,6 +265,17 @@ __global__ void __launch_bounds__(256) heads_linear_vec_kernel(HeadsVec A) {
   ((TO*)A.out)[(size_t)t * A.ldo + (size_t)h * A.o_head + n] = hb_from_float<TO>(y);
 }
 
+// Whether the rows are so few that latency bounds them. The kernel above pays 31 shuffles for 32 sums, whatever K is, and reads
+// a head's weight once for 4 rows; the one before it fills the SMs better when there are many. The line lies where the two took
+// the same time, in warps of the kernel above: up to K = 64 between 1,280 and 1,536 (32 heads of 64 x 64, 16 rows: 2.3 us against
+// 3.2; 24 rows 3.7 against 3.4), at K = 128 between 3,072 and 4,096 (16 heads of 128 x 512, 8 rows: 5.2 against 6.4; 16 rows 10.0
+// against 9.4), at K = 256 and 512 between 5,120 and 6,144 (32 heads of 256 x 64, 64 rows: 12.4 against 17.5; 128 rows 23.7
+// against 23.2, 2,048 rows 398 against 189).
+static bool hv_few(int T, int H, int K, int N) {
+  const long warps = (long)((T + HV_ROWS - 1) / HV_ROWS) * H * (N / 8);
+  return warps < 24l * (K < 64 ? 64 : K < 216 ? K : 216);
+}
+
 // a float32 [T][lda], head h's K (+ tail) inputs at column h * a_head; wt [H][K][N]; out [T][ldo], head h's N (+ tail)
 // outputs at column h * o_head.
 HB_EXPORT int hb_heads_linear(const float* a, long lda, long a_head, const void* wt, int w_dt, void* out, int o_dt, long ldo,
@@ -272,7 +284,7 @@ HB_EXPORT int hb_heads_linear(const float* a, long lda, long a_head, const void*
                               int pairing, int gate_per_head, const int* row_list, cudaStream_t s) {
   if (T <= 0 || H <= 0) return 0;
   if (tail && (!pos || !table || rot > tail || (rot & 1))) HB_FAIL("hb_heads_linear: a rotated tail needs positions and a table");
-  if (N % 8 == 0 && ((uintptr_t)wt & 15) == 0 && H <= 65535 && (T + HV_ROWS - 1) / HV_ROWS <= 65535) {     // (a row of 8 is 16 or 32 bytes)
+  if (N % 8 == 0 && ((uintptr_t)wt & 15) == 0 && H <= 65535 && hv_few(T, H, K, N)) {     // (a row of 8 is 16 or 32 bytes)
     const HeadsVec A{a, lda, a_head, wt, out, ldo, o_head, T, K, N, gate, ld_gate, gate_off, tail, rot, pos, (const float2*)table, row_list,
                      row_req, q_len, row_limit, pairing, gate_per_head};
     const dim3 grid((N + 63) / 64 + (tail ? 1 : 0), H, (T + HV_ROWS - 1) / HV_ROWS);
@@ -280,7 +292,6 @@ HB_EXPORT int hb_heads_linear(const float* a, long lda, long a_head, const void*
     HB_CHECK_LAUNCH("hb_heads_linear");
     return 0;
   }
-  if (row_list) HB_FAIL("hb_heads_linear: a list of rows wants outputs in multiples of 8 and a weight on a 16-byte boundary");
   const size_t smem = ((size_t)HL_TM * (K + tail) + (size_t)HL_KZ * HL_TM * HL_TN) * sizeof(float);
   if (smem > 96 * 1024) HB_FAIL("hb_heads_linear: K = %d is too wide", K);
   if ((T + HL_TM - 1) / HL_TM > 65535 || H > 65535) HB_FAIL("hb_heads_linear: the grid is too large");
@@ -290,7 +301,7 @@ HB_EXPORT int hb_heads_linear(const float* a, long lda, long a_head, const void*
     auto kern = heads_linear_kernel<TW, TO>;                                                                    \
     if (smem + 4096 > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
     hb_launch(kern, grid, dim3(HL_THREADS), smem, s, a, lda, a_head, (const TW*)wt, (TO*)out, ldo, o_head, T, K, N, gate,  \
-              ld_gate, gate_off, tail, rot, pos, (const float2*)table, row_req, q_len, row_limit, pairing,     \
+              ld_gate, gate_off, tail, rot, pos, (const float2*)table, row_list, row_req, q_len, row_limit, pairing,     \
               gate_per_head);                                                                                   \
   } while (0)
   HB_DISPATCH_2(w_dt, o_dt, "hb_heads_linear", HL_LAUNCH(TA, TB));

@@ -516,3 +516,35 @@ def test_single_rows_in_clusters_of_every_size(H, G, D, E):
         assert torch.equal(run([r], n - 1)[0], every[r]), n                         # the smallest cluster that holds the row
         many = run([r] * 200, n - 1)                                                # no CTA to spare for the join
         assert torch.equal(many, every[r].expand_as(many)), n
+
+
+@pytest.mark.parametrize("wdt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,K,N,tail,T,few", [(32, 64, 64, 0, 20, True), (32, 64, 64, 0, 24, False), (32, 64, 256, 32, 70, False), (8, 128, 96, 8, 124, True),
+                                              (8, 128, 96, 8, 128, False), (32, 256, 64, 0, 90, False), (4, 33, 12, 4, 50, False)])
+def test_heads_linear_of_few_and_of_many_rows(wdt, H, K, N, tail, T, few):
+    """Both sides of the line between the kernel of few rows and that of many (and outputs in no multiple of 8), all rows and a list of
+    them, against 64 bits. The bound: 32-bit sums of K products."""
+    from hipinfer_b200.kernels import ops
+
+    a, w = rnd(T, H * (K + tail), seed=51), rnd(H, K, N, seed=52, scale=0.1).to(wdt)
+    table = torch.stack([torch.cos(rnd(50, max(tail // 2, 1), seed=54)), torch.sin(rnd(50, max(tail // 2, 1), seed=54))], -1).contiguous()
+    pos = torch.arange(T, dtype=torch.int32) % 50
+    kw = dict(tail=tail, rot=tail, positions=pos.to(DEV), table=table.to(DEV)) if tail else {}
+    out = torch.empty(T, H * (N + tail), device=DEV)
+    ops.heads_linear(a.to(DEV), K + tail, w.to(DEV), out, N + tail, **kw)
+    ad, wd, got = a.double().view(T, H, K + tail), w.double(), out.double().cpu().view(T, H, N + tail)
+    bound = (K + 16) * 2.0 ** -24 * torch.einsum("thk,hkn->thn", ad[..., :K].abs(), wd.abs()) + 1e-12
+    assert bool(((got[..., :N] - torch.einsum("thk,hkn->thn", ad[..., :K], wd)).abs() <= bound).all())
+    if tail:
+        u, v = ad[..., K::2], ad[..., K + 1::2]
+        c, s = (table[pos.long()][:, None, :, i].double() for i in (0, 1))
+        torch.testing.assert_close(got[..., N:], torch.stack([u * c - v * s, v * c + u * s], -1).flatten(-2), rtol=1e-5, atol=1e-6)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    pick = list(range(T - 1, 1, -1))                    # nearly all of them, backwards: the same kernel
+    some = torch.full_like(out, 5.0)
+    batch = SimpleNamespace(row_request=i32([0] * T), req_q_len=i32([T]), short_rows=lambda limit: (i32(pick), 0))
+    ops.heads_linear(a.to(DEV), K + tail, w.to(DEV), some, N + tail, batch=batch, row_limit=16, **kw)
+    assert torch.equal(some[pick], out[pick]) and bool((some[:2] == 5.0).all())
+    one = torch.empty(1, H * (N + tail), device=DEV)    # a row by itself is the kernel of few rows where there is one for these sizes
+    ops.heads_linear(a[T - 1:].to(DEV), K + tail, w.to(DEV), one, N + tail, **(dict(kw, positions=pos[T - 1:].to(DEV)) if tail else {}))
+    assert torch.equal(one[0], out[T - 1]) == (few or N % 8 != 0)
