@@ -16,7 +16,7 @@
 // launch is the same for every batch of as many requests and replays from a CUDA graph.
 //
 //   delta_rule_kernel      four threads share two value channels, each with D / 4 key channels of them in registers; tokens
-//                          in chunks, what does not depend on the state a chunk at a time (D = 32, 64, 128).
+//                          in chunks, what does not depend on the state a chunk at a time (D = 32, 64, 128); two forms.
 //   delta_rule_any_kernel  any D: the state in shared memory, a thread per value channel.
 #include "common.cuh"
 
@@ -105,142 +105,160 @@ __global__ void delta_rule_any_kernel(DeltaArgs A) {
 }
 
 // A thread holds S[q * NR + i][j], i < NR, of two neighbouring value channels j in registers; the four threads q of a channel
-// pair (D = 4 NR) are neighbouring lanes, so the parts of u^T S meet by two shuffles and no thread waits for another warp while
-// the state walks. Two channels a thread halve the reads of the token's vectors, which (with a barrier a token before that)
-// bounded the walk: one read of 16 bytes serves 8 products instead of 4.
+// pair (D = 4 NR) are neighbouring lanes, so the parts of u^T S meet by shuffles (each lane fetches all four and adds them in the
+// order of q) and no thread waits for another warp while the state walks. Two channels a thread halve the reads of the token's
+// vectors, which (with a barrier a token before that) bounded the walk: one read of 16 bytes serves 8 products instead of 4.
 //
-// The tokens go by in chunks of DR_CH, and the block's warps have two jobs. The first D / 16 warps WALK the state through the
-// chunk at hand: per token 10 NR multiply-adds a thread and its share of the reads. DR_HELP further warps make, meanwhile, what does
-// not depend on the state for the chunk after it, a warp per token (the unit key, decay and removal rate: a warp sum and two
-// expf), and finish the chunk before it (the parts of the outputs added, head norm, gate). The raw values of the chunk after next
-// are then already on their way from global memory. One barrier a chunk. With one job after the other in the same warps the
-// walk stands still meanwhile (32 heads of 64, two requests, 2,048 tokens: 598 us, and 556 without the barrier a
-// token; 551 us with the helpers: the walk itself is what is left).
-constexpr int DR_CH = 16, DR_Q = 4, DR_HELP = 4;
+// The tokens go by in chunks of CH. What does not depend on the state is made for a chunk at once, a warp per token (the unit
+// key, decay and removal rate: a warp sum and two expf), the raw values of a later chunk on their way from global memory
+// meanwhile; the chunk's outputs are finished (their parts added, head norm, gate) a warp per token too.
+//
+// HELP: the first D / 16 warps only WALK, 10 NR multiply-adds a thread and its share of the reads a token, and DR_HELP further warps
+// prepare the next chunk and finish the one before beside them, one barrier a chunk: for few blocks, where the walk must not
+// stand still (32 heads of 64, two requests, 2,048 tokens: 598 us with a barrier a token, 556 without, 551 with the helpers: the walk
+// itself is what is left). It keeps two chunks of 16 in shared memory, two blocks an SM at D = 64. Without (HELP false) the same warps
+// do both in turn, for short chunks in an eighth of the shared memory, so that an SM holds more blocks: for many of them (64
+// requests of a token each, 32 heads of 64, took 35 us with the helpers, 16 without). Both do the same arithmetic in the same order.
+constexpr int DR_Q = 4, DR_HELP = 4;
 
-template <typename TW, typename TO, int NR>
-__global__ void __launch_bounds__(2 * DR_Q * NR + 32 * DR_HELP, 1) delta_rule_kernel(DeltaArgs A) {
-  constexpr int D = NR * DR_Q, WALKERS = D / 2 * DR_Q, TPW = DR_CH / DR_HELP, CPL = D / 32;
-  static_assert(WALKERS % 32 == 0 && TPW * DR_HELP == DR_CH && CPL >= 1 && NR % 4 == 0, "chunk, warps and head size must fit");
+template <int NR, bool HELP, int CH> struct DeltaCfg {
+  static constexpr int D = NR * DR_Q, WALKERS = D / 2 * DR_Q, THREADS = WALKERS + (HELP ? 32 * DR_HELP : 0);
+  static constexpr int NW = HELP ? DR_HELP : WALKERS / 32, TPW = CH / NW, CPL = D / 32;      // warps that prepare and finish, tokens of each
   // a vector lies in four parts of NR + 4: the lanes of a warp read four places at once, of banks of their own; the rows of the
   // output's parts are D + 8 apart for the same reason
-  constexpr int SEG = NR + 4, VS = DR_Q * SEG, OS = D + 8, VEC = DR_CH * VS, IN = 5 * VEC + DR_CH * D, OUT = DR_CH * DR_Q * OS;
-  extern __shared__ __align__(16) float dr_smem[];     // [2] inputs of a chunk (r, w, au, k, u [DR_CH][VS] each, v [DR_CH][D]), [2] outputs
+  static constexpr int SEG = NR + 4, VS = DR_Q * SEG, OS = D + 8, VEC = CH * VS, IN = 5 * VEC + CH * D, OUT = CH * DR_Q * OS;
+  static constexpr size_t SMEM = (size_t)(HELP ? 2 : 1) * (IN + OUT) * sizeof(float);
+  static_assert(WALKERS % 32 == 0 && TPW * NW == CH && CPL >= 1 && NR % 4 == 0, "chunk, warps and head size must fit");
+};
+
+template <typename TW, typename TO, int NR, bool HELP, int CH>
+__global__ void __launch_bounds__(DeltaCfg<NR, HELP, CH>::THREADS, HELP || NR > 16 ? 1 : 512 / (8 * NR)) delta_rule_kernel(DeltaArgs A) {
+  using C = DeltaCfg<NR, HELP, CH>;
+  constexpr int D = C::D, NW = C::NW, TPW = C::TPW, CPL = C::CPL, SEG = C::SEG, VS = C::VS, OS = C::OS, VEC = C::VEC, IN = C::IN, OUT = C::OUT;
+  // HELP: [2] inputs of a chunk (r, w, au, k, u [CH][VS] each, v [CH][D]), [2] outputs; else one of each
+  extern __shared__ __align__(16) float dr_smem[];
   hb_pdl_launch();
   hb_pdl_wait();
   const int h = blockIdx.x, req = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
-  const int t0 = A.q_start[req], n = A.q_len[req], chunks = (n + DR_CH - 1) / DR_CH;
+  const int t0 = A.q_start[req], n = A.q_len[req], chunks = (n + CH - 1) / CH;
   const int hc = h * D;
-  if (tid >= WALKERS) {                  // ---------------- the helpers
-    const int warp = (tid - WALKERS) >> 5;
-    const TW* wb = (const TW*)A.w_bias, *ab = (const TW*)A.a_bias, *nwt = (const TW*)A.norm_w;
-    // raw values of a chunk's tokens: a warp takes tokens warp, warp + DR_HELP, ..; a lane channels lane, lane + 32, ..
-    float pre[TPW][CPL][5];              // k, r, v, a_raw, w_raw
-    float gate[TPW][CPL];                // the gate's raw values of the chunk to be finished next
-    float cab[CPL], cwb[CPL], cnw[CPL];  // this lane's channels of the two biases and the norm weight
+  const bool helper = HELP && tid >= C::WALKERS;
+  auto inputs = [&](int c) { return dr_smem + (HELP ? (c & 1) * IN : 0); };
+  auto outputs = [&](int c) { return dr_smem + (HELP ? 2 * IN + (c & 1) * OUT : IN); };
+
+  // ---------------- what a warp does for its tokens of a chunk (HELP: the helpers alone): warp, warp + NW, ..
+  const int warp = HELP ? (tid - C::WALKERS) >> 5 : tid >> 5;
+  const TW* wb = (const TW*)A.w_bias, *ab = (const TW*)A.a_bias, *nwt = (const TW*)A.norm_w;
+  float pre[TPW][CPL][5];              // raw values: k, r, v, a_raw, w_raw of channels lane, lane + 32, ..
+  float gate[TPW][CPL];                // the gate's raw values of the chunk to be finished next
+  float cab[CPL], cwb[CPL], cnw[CPL];  // this lane's channels of the two biases and the norm weight
+  auto fetch_gate = [&](int base) {
+#pragma unroll
+    for (int x = 0; x < TPW; x++) {
+      const int tt = warp + x * NW;
+      if (base + tt < n) {
+        const float* row = A.proj + (size_t)(t0 + base + tt) * A.ld;
+#pragma unroll
+        for (int y = 0; y < CPL; y++) gate[x][y] = row[A.g_off + hc + lane + 32 * y];
+      }
+    }
+  };
+  auto fetch = [&](int base) {
+#pragma unroll
+    for (int x = 0; x < TPW; x++) {
+      const int tt = warp + x * NW;
+      if (base + tt < n) {
+        const float* row = A.proj + (size_t)(t0 + base + tt) * A.ld;
+        const float* wrow = A.w_raw + (size_t)(t0 + base + tt) * A.ldw;
+#pragma unroll
+        for (int y = 0; y < CPL; y++) {
+          const int c = hc + lane + 32 * y;
+          pre[x][y][0] = row[A.k_off + c];
+          pre[x][y][1] = row[A.r_off + c];
+          pre[x][y][2] = row[A.v_off + c];
+          pre[x][y][3] = row[A.a_off + c];
+          pre[x][y][4] = wrow[c];
+        }
+      }
+    }
+  };
+  auto prepare = [&](int c) {          // the fetched chunk's vectors into shared memory
+    float* vr = inputs(c), *vw = vr + VEC, *vau = vw + VEC, *vk = vau + VEC, *vu = vk + VEC, *vv = vu + VEC;
+#pragma unroll
+    for (int x = 0; x < TPW; x++) {
+      const int tt = warp + x * NW;
+      if (c * CH + tt < n) {                                 // (uniform over the warp)
+        float kk = 0.f;
+#pragma unroll
+        for (int y = 0; y < CPL; y++) kk = fmaf(pre[x][y][0], pre[x][y][0], kk);
+        kk = hb_warp_sum(kk);
+        const float inv = 1.f / sqrtf(kk + A.unit_eps);
+#pragma unroll
+        for (int y = 0; y < CPL; y++) {
+          const int cl = lane + 32 * y, at = tt * VS + cl / NR * SEG + cl % NR;
+          const float kj = pre[x][y][0], uj = kj * inv;
+          vk[at] = kj;
+          vu[at] = uj;
+          vr[at] = pre[x][y][1];
+          vv[tt * D + cl] = pre[x][y][2];
+          vau[at] = sigmoidf_(pre[x][y][3] + cab[y]) * uj;
+          vw[at] = expf(-A.decay_scale * sigmoidf_(pre[x][y][4] + cwb[y]));
+        }
+      }
+    }
+  };
+  auto finish = [&](int c) {           // a walked chunk's outputs: head norm, weight and gate
+    const float* vo = outputs(c);
+#pragma unroll
+    for (int x = 0; x < TPW; x++) {
+      const int tt = warp + x * NW;
+      if (c * CH + tt < n) {
+        float ov[CPL], oo = 0.f;
+#pragma unroll
+        for (int y = 0; y < CPL; y++) {
+          ov[y] = vo[tt * DR_Q * OS + lane + 32 * y];
+#pragma unroll
+          for (int qq = 1; qq < DR_Q; qq++) ov[y] += vo[(tt * DR_Q + qq) * OS + lane + 32 * y];
+          oo = fmaf(ov[y], ov[y], oo);
+        }
+        oo = hb_warp_sum(oo);
+        const float f = rsqrtf(oo / (float)D + A.eps);
+        const size_t t = (size_t)(t0 + c * CH + tt);
+#pragma unroll
+        for (int y = 0; y < CPL; y++) {
+          const int cc = hc + lane + 32 * y;
+          ((TO*)A.out)[t * A.heads * D + cc] = hb_from_float<TO>(ov[y] * f * cnw[y] * sigmoidf_(gate[x][y]));
+        }
+      }
+    }
+  };
+  if (!HELP || helper) {
+    fetch(0);
 #pragma unroll
     for (int y = 0; y < CPL; y++) {
       cab[y] = hb_to_float(ab[hc + lane + 32 * y]);
       cwb[y] = hb_to_float(wb[hc + lane + 32 * y]);
       cnw[y] = hb_to_float(nwt[hc + lane + 32 * y]);
     }
-    auto fetch_gate = [&](int base) {
-#pragma unroll
-      for (int x = 0; x < TPW; x++) {
-        const int tt = warp + x * DR_HELP;
-        if (base + tt < n) {
-          const float* row = A.proj + (size_t)(t0 + base + tt) * A.ld;
-#pragma unroll
-          for (int y = 0; y < CPL; y++) gate[x][y] = row[A.g_off + hc + lane + 32 * y];
-        }
-      }
-    };
-    auto fetch = [&](int base) {
-#pragma unroll
-      for (int x = 0; x < TPW; x++) {
-        const int tt = warp + x * DR_HELP;
-        if (base + tt < n) {
-          const float* row = A.proj + (size_t)(t0 + base + tt) * A.ld;
-          const float* wrow = A.w_raw + (size_t)(t0 + base + tt) * A.ldw;
-#pragma unroll
-          for (int y = 0; y < CPL; y++) {
-            const int c = hc + lane + 32 * y;
-            pre[x][y][0] = row[A.k_off + c];
-            pre[x][y][1] = row[A.r_off + c];
-            pre[x][y][2] = row[A.v_off + c];
-            pre[x][y][3] = row[A.a_off + c];
-            pre[x][y][4] = wrow[c];
-          }
-        }
-      }
-    };
-    auto prepare = [&](int c) {          // the fetched chunk's vectors into shared memory
-      float* vr = dr_smem + (c & 1) * IN, *vw = vr + VEC, *vau = vw + VEC, *vk = vau + VEC, *vu = vk + VEC, *vv = vu + VEC;
-#pragma unroll
-      for (int x = 0; x < TPW; x++) {
-        const int tt = warp + x * DR_HELP;
-        if (c * DR_CH + tt < n) {                            // (uniform over the warp)
-          float kk = 0.f;
-#pragma unroll
-          for (int y = 0; y < CPL; y++) kk = fmaf(pre[x][y][0], pre[x][y][0], kk);
-          kk = hb_warp_sum(kk);
-          const float inv = 1.f / sqrtf(kk + A.unit_eps);
-#pragma unroll
-          for (int y = 0; y < CPL; y++) {
-            const int cl = lane + 32 * y, at = tt * VS + cl / NR * SEG + cl % NR;
-            const float kj = pre[x][y][0], uj = kj * inv;
-            vk[at] = kj;
-            vu[at] = uj;
-            vr[at] = pre[x][y][1];
-            vv[tt * D + cl] = pre[x][y][2];
-            vau[at] = sigmoidf_(pre[x][y][3] + cab[y]) * uj;
-            vw[at] = expf(-A.decay_scale * sigmoidf_(pre[x][y][4] + cwb[y]));
-          }
-        }
-      }
-    };
-    auto finish = [&](int c) {           // a walked chunk's outputs: head norm, weight and gate
-      const float* vo = dr_smem + 2 * IN + (c & 1) * OUT;
-#pragma unroll
-      for (int x = 0; x < TPW; x++) {
-        const int tt = warp + x * DR_HELP;
-        if (c * DR_CH + tt < n) {
-          float ov[CPL], oo = 0.f;
-#pragma unroll
-          for (int y = 0; y < CPL; y++) {
-            ov[y] = vo[tt * DR_Q * OS + lane + 32 * y];
-#pragma unroll
-            for (int qq = 1; qq < DR_Q; qq++) ov[y] += vo[(tt * DR_Q + qq) * OS + lane + 32 * y];
-            oo = fmaf(ov[y], ov[y], oo);
-          }
-          oo = hb_warp_sum(oo);
-          const float f = rsqrtf(oo / (float)D + A.eps);
-          const size_t t = (size_t)(t0 + c * DR_CH + tt);
-#pragma unroll
-          for (int y = 0; y < CPL; y++) {
-            const int cc = hc + lane + 32 * y;
-            ((TO*)A.out)[t * A.heads * D + cc] = hb_from_float<TO>(ov[y] * f * cnw[y] * sigmoidf_(gate[x][y]));
-          }
-        }
-      }
-    };
-    fetch(0);
+  }
+  if (helper) {
     prepare(0);
-    fetch(DR_CH);
+    fetch(CH);
     __syncthreads();
     for (int c = 0; c < chunks; c++) {
       if (c > 0) finish(c - 1);
-      fetch_gate(c * DR_CH);
+      fetch_gate(c * CH);
       if (c + 1 < chunks) {
         prepare(c + 1);
-        fetch((c + 2) * DR_CH);
+        fetch((c + 2) * CH);
       }
       __syncthreads();
     }
     if (chunks > 0) finish(chunks - 1);
     return;
   }
-  // ---------------- the walkers
+
+  // ---------------- the walk
   const int q = lane & 3, j = (tid >> 2) * 2;
   float* Sg = A.state + ((size_t)A.slot[req] * A.heads + h) * D * D;
   float S[NR][2];
@@ -250,11 +268,17 @@ __global__ void __launch_bounds__(2 * DR_Q * NR + 32 * DR_HELP, 1) delta_rule_ke
     S[i][0] = v.x;
     S[i][1] = v.y;
   }
-  __syncthreads();
+  if (HELP) __syncthreads();
   for (int ch = 0; ch < chunks; ch++) {
-    const float* vr = dr_smem + (ch & 1) * IN, *vw = vr + VEC, *vau = vw + VEC, *vk = vau + VEC, *vu = vk + VEC, *vv = vu + VEC;
-    float* vo = dr_smem + 2 * IN + (ch & 1) * OUT;
-    const int m = min(DR_CH, n - ch * DR_CH);
+    if (!HELP) {
+      prepare(ch);
+      __syncthreads();
+      fetch_gate(ch * CH);                                   // both in flight during the walk
+      if (ch + 1 < chunks) fetch((ch + 1) * CH);
+    }
+    const float* vr = inputs(ch), *vw = vr + VEC, *vau = vw + VEC, *vk = vau + VEC, *vu = vk + VEC, *vv = vu + VEC;
+    float* vo = outputs(ch);
+    const int m = min(CH, n - ch * CH);
     for (int tt = 0; tt < m; tt++) {
       const int at = tt * VS + q * SEG;
       float4 u[NR / 4];
@@ -262,7 +286,7 @@ __global__ void __launch_bounds__(2 * DR_Q * NR + 32 * DR_HELP, 1) delta_rule_ke
       for (int i = 0; i < NR / 4; i++) u[i] = *(const float4*)(vu + at + 4 * i);
       const float2 v2 = *(const float2*)(vv + tt * D + j);
       const float vj[2] = {v2.x, v2.y};
-      float sa[2];
+      float part[2], sa[2];
 #pragma unroll
       for (int c = 0; c < 2; c++) {
         float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
@@ -271,12 +295,19 @@ __global__ void __launch_bounds__(2 * DR_Q * NR + 32 * DR_HELP, 1) delta_rule_ke
           s0 = fmaf(u[i].x, S[4 * i][c], s0); s1 = fmaf(u[i].y, S[4 * i + 1][c], s1);
           s2 = fmaf(u[i].z, S[4 * i + 2][c], s2); s3 = fmaf(u[i].w, S[4 * i + 3][c], s3);
         }
-        sa[c] = (s0 + s1) + (s2 + s3);
+        part[c] = (s0 + s1) + (s2 + s3);
       }
+      float all[2][DR_Q];
 #pragma unroll
-      for (int o = 1; o < DR_Q; o <<= 1)
+      for (int qq = 0; qq < DR_Q; qq++)
 #pragma unroll
-        for (int c = 0; c < 2; c++) sa[c] += __shfl_xor_sync(0xffffffffu, sa[c], o);
+        for (int c = 0; c < 2; c++) all[c][qq] = __shfl_sync(0xffffffffu, part[c], qq, DR_Q);
+#pragma unroll
+      for (int c = 0; c < 2; c++) {
+        sa[c] = all[c][0];
+#pragma unroll
+        for (int qq = 1; qq < DR_Q; qq++) sa[c] += all[c][qq];
+      }
       float o[2][4] = {};
 #pragma unroll
       for (int i = 0; i < NR / 4; i++) {
@@ -293,31 +324,51 @@ __global__ void __launch_bounds__(2 * DR_Q * NR + 32 * DR_HELP, 1) delta_rule_ke
       *(float2*)(vo + (tt * DR_Q + q) * OS + j) = make_float2((o[0][0] + o[0][1]) + (o[0][2] + o[0][3]), (o[1][0] + o[1][1]) + (o[1][2] + o[1][3]));
     }
     __syncthreads();
+    if (!HELP) finish(ch);
   }
 #pragma unroll
   for (int i = 0; i < NR; i++) *(float2*)(Sg + (q * NR + i) * D + j) = make_float2(S[i][0], S[i][1]);
 }
 
-template <typename TW, typename TO, int NR>
-static int delta_rule_launch_reg(const DeltaArgs& A, dim3 grid, cudaStream_t s) {
-  constexpr int D = NR * DR_Q;
-  const size_t smem = 2 * ((size_t)5 * DR_CH * DR_Q * (NR + 4) + DR_CH * D + (size_t)DR_CH * DR_Q * (D + 8)) * sizeof(float);
-  auto kern = delta_rule_kernel<TW, TO, NR>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+enum { DR_RULE = 0, DR_ANY = 1, DR_HELPERS = 2, DR_SHORT = 3 };
+// Which form a launch takes. Portions: with helpers while the blocks that an SM then holds (four, two, one for heads of 32, 64, 128)
+// are enough for one round; at 128 always, where both hold one and the helpers are 1 to 3 % ahead. 300 tokens of 32 heads, us with
+// helpers / without: of 64, 4 requests 122 / 236, 8 280 / 326, 12 420 / 338; of 32, 12 requests 210 / 245; of 128, 4 291 / 306.
+// Single tokens: without, but for the few block counts at which the wider block is ahead (32 heads of 64: 1 request 3.30 / 3.07, 4
+// 3.33 / 3.95, 8 5.66 / 4.80, 64 35.3 / 16.0; of 32, 8 requests 2.68 / 2.86, 64 14.0 / 6.1; of 128, 4 6.2 / 5.7).
+static int dr_form(int D, long blocks, bool single) {
+  if (single) return D <= 64 && blocks > 74 && blocks <= (D <= 32 ? 296 : 148) ? DR_HELPERS : DR_SHORT;
+  return D > 64 || blocks <= 148 * (D <= 32 ? 4 : 2) ? DR_HELPERS : DR_SHORT;
+}
+
+constexpr int dr_short(int NR) { return NR > 16 ? NR / 4 : 4; }      // tokens of a chunk without helpers: one a warp, at least four
+
+template <typename TW, typename TO, int NR, bool HELP, int CH>
+static int delta_rule_launch_form(const DeltaArgs& A, dim3 grid, cudaStream_t s) {
+  using C = DeltaCfg<NR, HELP, CH>;
+  auto kern = delta_rule_kernel<TW, TO, NR, HELP, CH>;
+  if (C::SMEM > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
     if (e != cudaSuccess) HB_FAIL("hb_delta_rule: %s", cudaGetErrorString(e));
   }
-  hb_launch(kern, grid, 2 * D + 32 * DR_HELP, smem, s, A);
+  hb_launch(kern, grid, C::THREADS, C::SMEM, s, A);
   return 0;
 }
 
+template <typename TW, typename TO, int NR>
+static int delta_rule_launch_reg(const DeltaArgs& A, dim3 grid, int rows, int form, cudaStream_t s) {
+  if (form == DR_RULE) form = dr_form(4 * NR, (long)grid.x * grid.y, rows == (int)grid.y);
+  if (form == DR_HELPERS) return delta_rule_launch_form<TW, TO, NR, true, 16>(A, grid, s);
+  return delta_rule_launch_form<TW, TO, NR, false, dr_short(NR)>(A, grid, s);
+}
+
 template <typename TW, typename TO>
-static int delta_rule_launch(const DeltaArgs& A, int R, cudaStream_t s) {
+static int delta_rule_launch(const DeltaArgs& A, int R, int rows, int form, cudaStream_t s) {
   const dim3 grid(A.heads, R);
   if (!((uintptr_t)A.state & 7)) switch (A.D) {      // (the register kernels read the state in pairs)
-    case 32: return delta_rule_launch_reg<TW, TO, 8>(A, grid, s);
-    case 64: return delta_rule_launch_reg<TW, TO, 16>(A, grid, s);
-    case 128: return delta_rule_launch_reg<TW, TO, 32>(A, grid, s);
+    case 32: return delta_rule_launch_reg<TW, TO, 8>(A, grid, rows, form, s);
+    case 64: return delta_rule_launch_reg<TW, TO, 16>(A, grid, rows, form, s);
+    case 128: return delta_rule_launch_reg<TW, TO, 32>(A, grid, rows, form, s);
     default: break;
   }
   const int threads = (A.D + 31) / 32 * 32;
@@ -332,12 +383,13 @@ static int delta_rule_launch(const DeltaArgs& A, int R, cudaStream_t s) {
   return 0;
 }
 
-// force_any: run the shared-memory kernel also where a register kernel exists (tests compare the two).
+// rows: the step's rows (as many as requests: every portion is a single token). form: 0 by the rule, or the form to run (tests compare
+// them): 1 the shared-memory kernel, 2 and 3 the register kernel with and without helpers.
 HB_EXPORT int hb_delta_rule(const float* proj, long ld, int r_off, int k_off, int v_off, int a_off, int g_off,
                             const float* w_raw, long ldw, const void* w_bias, const void* a_bias, const void* norm_w,
                             int w_dt, float* state, const int* q_start, const int* q_len, const int* slot, void* out,
                             int out_dt, int R, int heads, int D, float decay_scale, float unit_eps, float eps,
-                            int force_any, cudaStream_t s) {
+                            int rows, int form, cudaStream_t s) {
   if (R <= 0) return 0;
   if (heads <= 0 || D <= 0) HB_FAIL("hb_delta_rule: %d heads of %d", heads, D);
   if (R > 65535) HB_FAIL("hb_delta_rule: %d requests are beyond the grid limit", R);
@@ -345,7 +397,7 @@ HB_EXPORT int hb_delta_rule(const float* proj, long ld, int r_off, int k_off, in
               out, heads, D, decay_scale, unit_eps, eps};
   int r = -1;
   HB_DISPATCH_2(w_dt, out_dt, "hb_delta_rule", {
-    if (force_any) {
+    if (form == DR_ANY) {
       const int threads = (D + 31) / 32 * 32;
       const size_t smem = ((size_t)D * D + 5 * (size_t)D + 32) * sizeof(float);
       if (threads > 1024 || smem > 200 * 1024) HB_FAIL("hb_delta_rule: heads of %d are too wide for one block's shared memory", D);
@@ -357,7 +409,7 @@ HB_EXPORT int hb_delta_rule(const float* proj, long ld, int r_off, int k_off, in
       hb_launch(kern, dim3(heads, R), threads, smem, s, A);
       r = 0;
     } else {
-      r = delta_rule_launch<TA, TB>(A, R, s);
+      r = delta_rule_launch<TA, TB>(A, R, rows, form, s);
     }
   });
   if (r) return r;

@@ -96,7 +96,7 @@ _SIGS = {
     },
     "mixers": {
         "hb_delta_rule": [_p, _l, _i, _i, _i, _i, _i, _p, _l, _p, _p, _p, _i, _p, _p, _p, _p, _p, _i, _i, _i, _i, _f, _f, _f,
-                          _i, _p],
+                          _i, _i, _p],
         "hb_attn_window": [_p, _i, _p, _p, _i, _p, _i, _p, _p, _p, _l, _i, _p, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _f, _f,
                            _f, _i, _p, _i, _i, _p, _l, _p, _i, _p],
         "hb_attn_window_flash": [_p, _p, _p, _p, _i, _p, _p, _p, _p, _l, _i, _p, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _f,
@@ -315,10 +315,11 @@ def qkv_bias_store(qkv: torch.Tensor, bq, bk, bv, slot_map: Optional[torch.Tenso
 
 def delta_rule(proj: torch.Tensor, offsets, w_raw: torch.Tensor, w_bias, a_bias, norm_weight, state: torch.Tensor, batch,
                out: torch.Tensor, heads: int, dim: int, decay_scale: float, unit_eps: float, eps: float,
-               force_any: bool = False) -> torch.Tensor:
+               force_any: int = 0) -> torch.Tensor:
     """The generalized delta rule over the step's rows, request by request, from and into each request's state slot
     (csrc/delta_rule.cu). proj float32 [T, *] holds r, k, v, the removal rate's and the gate's pre-activations at the
-    column `offsets` (r, k, v, a, g); w_raw float32 [T, heads * dim] the decay's; state float32 [slots, heads, dim, dim]."""
+    column `offsets` (r, k, v, a, g); w_raw float32 [T, heads * dim] the decay's; state float32 [slots, heads, dim, dim].
+    force_any: 0 the kernel that the sizes call for, 1 the one with the state in shared memory, 2 and 3 a form of the register kernel."""
     _need_cuda(proj, w_raw, w_bias, a_bias, norm_weight, state, out)
     _rows_contiguous(proj, "delta_rule proj")
     _rows_contiguous(w_raw, "delta_rule w_raw")
@@ -329,7 +330,7 @@ def delta_rule(proj: torch.Tensor, offsets, w_raw: torch.Tensor, w_bias, a_bias,
     _call("mixers", "hb_delta_rule", proj.data_ptr(), proj.stride(0), r, k, v, a, g, w_raw.data_ptr(), w_raw.stride(0),
           w_bias.data_ptr(), a_bias.data_ptr(), norm_weight.data_ptr(), _dt(w_bias), state.data_ptr(),
           batch.req_q_start.data_ptr(), batch.req_q_len.data_ptr(), batch.req_state_slot.data_ptr(), out.data_ptr(),
-          _dt(out), batch.n_requests, heads, dim, float(decay_scale), float(unit_eps), float(eps), 1 if force_any else 0,
+          _dt(out), batch.n_requests, heads, dim, float(decay_scale), float(unit_eps), float(eps), proj.shape[0], int(force_any),
           _stream())
     return out
 

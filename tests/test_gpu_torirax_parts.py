@@ -195,6 +195,29 @@ def test_delta_rule_with_a_state_on_an_odd_address(D):
     assert not got[0][2].any() and not got[0][3].any()
 
 
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("lens", [[1], [1] * 5, [37, 1, 16], [3, 4, 5, 8, 9, 33]])
+def test_delta_rule_forms_give_the_same_bits(D, lens):
+    """The register kernel with helper warps and without (chunks of 16 and of 4 or 8 tokens, one or several chunks, single tokens), and
+    whichever of them the rule takes."""
+    from hipinfer_b200.kernels import ops
+
+    heads, T = 3, sum(lens)
+    HD = heads * D
+    proj, w_raw = rnd(T, 5 * HD, seed=1).to(DEV), rnd(T, HD, seed=2).to(DEV)
+    vec = [t.to(DEV) for t in (rnd(HD, seed=3), rnd(HD, seed=4), 1 + 0.2 * rnd(HD, seed=5))]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    batch = SimpleNamespace(n_requests=len(lens), req_q_start=i32([sum(lens[:r]) for r in range(len(lens))]), req_q_len=i32(lens),
+                            req_state_slot=i32(list(range(len(lens)))[::-1]))
+    state0, got = rnd(len(lens) + 1, heads, D, D, seed=6).to(DEV), []
+    for form in (0, 2, 3):
+        state, out = state0.clone(), torch.empty(T, HD, device=DEV)
+        ops.delta_rule(proj, (0, HD, 2 * HD, 3 * HD, 4 * HD), w_raw, *vec, state, batch, out, heads, D, 0.6, 1e-6, 1e-5, force_any=form)
+        got.append((out, state))
+    assert torch.isfinite(got[0][0]).all() and torch.equal(got[0][1][len(lens)], state0[len(lens)])
+    assert all(torch.equal(o, got[0][0]) and torch.equal(s, got[0][1]) for o, s in got[1:])
+
+
 def test_delta_rule_register_and_shared_memory_kernels_agree():
     from hipinfer_b200.kernels import ops
 
