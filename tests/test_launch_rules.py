@@ -22,7 +22,7 @@ CONSTANT = {
     "gemm_simt.cu": "W colscale",
     "gemm_stream_consumers.cu": "w pos slot_map table rows",
     "hyper_streams.cu": "rows a w b M a_next w_next bias",
-    "latent.cu": "wq wc pos slot_map table wt row_req q_len",
+    "latent.cu": "wq wc pos slot_map table wt row_list row_req q_len",
     "matrix_state.cu": "bi bf q_start q_len slot a_log dt_bias row_req w",
     "moe.cu": "router bias correction shared_gate w wgu wd we",
     "selective_scan.cu": "wa wb w",
