@@ -237,14 +237,25 @@ def rope_kv_slices(sl: Slices, positions, slot_map, table, q_out, k_cache, v_cac
     return q_out
 
 
-def linear_slices(a, w):
-    """a @ w.T as slices when it is computed in slices: a few bf16 rows, or more rows of a product whose tiles are too few for the
-    SMs; else None."""
+def slices_pay(M, N, K) -> bool:
+    """Whether a portion's product is better cut along K (csrc/gemm_tc.cu) than run whole on narrower tiles. What a cut saves grows with
+    K, what it costs (the partial sums out and in again) with the number of slices. Product and norm, us whole / in slices: K = 2,048
+    in four 16.2 / 13.0 (512 x 2,048), in three 17.4 / 15.4 (700 rows), in two 17.7 / 18.1 (1,000 rows); K = 3,072 in three 22.7 / 20.3
+    (512 x 3,072), in two 22.5 / 24.4 (700 rows); K = 4,096 in two 28.0 / 25.2; K = 1,024 in two 9.8 / 10.0, at 1,000 rows 11.1 / 13.7."""
+    n = _fn("hb_gemm_tc_splits")(M, N, K)
+    return n > 2 and K >= 2048 or n == 2 and K >= 4096
+
+
+def linear_slices(a, w, residual=False):
+    """a @ w.T as slices when it is computed in slices: a few bf16 rows, or (a product that is added to the residual, whose next norm
+    then adds the slices) more rows whose tiles are too few for the SMs; else None. The rotation is no such reader: q/k/v of 200 rows,
+    24 and 8 heads of 128 over 3,072, took 23.9 us with it in slices, 21.5 whole; of 512 rows, 16 and 4 heads over 2,048, 27.9
+    against 17.7."""
     if not _tc_ok(a, w.t):
         return None
-    if a.shape[0] > STREAM_MAX_ROWS:
-        return gemm_tc_slices(a, w.t)
-    return gemm_stream_slices(a, w.t)
+    if a.shape[0] <= STREAM_MAX_ROWS:
+        return gemm_stream_slices(a, w.t)
+    return gemm_tc_slices(a, w.t) if residual and slices_pay(a.shape[0], w.shape[0], a.shape[1]) else None
 
 
 def gemm_tc_slices(a, w):

@@ -781,10 +781,10 @@ class Pending:
 
 
 def linear_deferred(a: torch.Tensor, w: Weight, out: torch.Tensor, accumulate: bool = False) -> Optional[Pending]:
-    """out (+)= a @ w.T, with the last step (adding the K slices of a small product) left to the
-    consumer where that applies: then a Pending comes back and `out` is not yet written. None: out is done."""
+    """out (+)= a @ w.T, with the last step (adding the K slices of a product of a few rows, or of a portion's residual product
+    of few tiles) left to the consumer where that applies: then a Pending comes back and `out` is not yet written. None: out is done."""
     if out.dtype == torch.float32 and a.is_cuda:
-        sl = fast.linear_slices(a, w)
+        sl = fast.linear_slices(a, w, residual=accumulate)
         if sl is not None:
             return Pending(sl, out, accumulate)
     linear(a, w, out, accumulate)

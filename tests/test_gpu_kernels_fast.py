@@ -774,10 +774,10 @@ def test_slices_of_two_portions_at_the_same_time():
     small products share) in between, and each finishes as its own product."""
     from hipinfer_b200.kernels import ops
 
-    a, w = rnd(130, 1024, seed=86), ops.Weight(rnd(512, 1024, seed=87, scale=0.05))
+    a, w = rnd(130, 2048, seed=86), ops.Weight(rnd(512, 2048, seed=87, scale=0.05))
     b, v = rnd(300, 2048, seed=88), ops.Weight(rnd(264, 2048, seed=89, scale=0.05))
     one, two = (torch.zeros(m, n, device=DEV) for m, n in ((130, 512), (300, 264)))
-    first, second = ops.linear_deferred(a, w, one), ops.linear_deferred(b, v, two)
+    first, second = ops.linear_deferred(a, w, one, accumulate=True), ops.linear_deferred(b, v, two, accumulate=True)
     assert first is not None and second is not None
     small = torch.empty(20, 512, device=DEV)
     ops.linear(a[:20], w, small)

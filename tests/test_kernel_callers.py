@@ -5,7 +5,7 @@ import weakref
 import pytest
 import torch
 
-from hipinfer_b200.kernels import library, ops
+from hipinfer_b200.kernels import fast, library, ops
 
 
 @pytest.fixture
@@ -59,3 +59,16 @@ def test_a_plain_product_runs_unsplit_where_no_memory_is_left(launches, which, m
     monkeypatch.setattr(torch, "empty", none_left)
     run()
     assert len(launches) == 1 and launches[0].args[-2] is None and library.launches[0] == counted
+
+
+@pytest.mark.parametrize("M,N,K,n,cut", [(512, 2048, 2048, 4, True), (700, 2048, 2048, 3, True), (1000, 2048, 2048, 2, False), (128, 1024, 1024, 2, False),
+                                         (512, 3072, 3072, 3, True), (700, 3072, 3072, 2, False), (512, 4096, 4096, 2, True), (1000, 2048, 8192, 2, True),
+                                         (2048, 4096, 4096, 0, False), (64, 1024, 1024, 2, None), (300, 512, 1536, 3, False)])
+def test_products_of_portions_are_cut_along_k_where_that_pays(monkeypatch, M, N, K, n, cut):
+    """Both sides of the rule (n: the slices that fit the SM pairs); up to 64 rows the small products' kernel has them."""
+    monkeypatch.setattr(fast, "_tc_ok", lambda a, w: True)
+    monkeypatch.setattr(fast, "_fn", lambda name: {"hb_gemm_tc_splits": lambda *size: n}[name])
+    monkeypatch.setattr(fast, "gemm_tc_slices", lambda a, w: True)
+    monkeypatch.setattr(fast, "gemm_stream_slices", lambda a, w: None)
+    a, w = torch.empty(M, K, device="meta"), ops.Weight(torch.empty(N, K, device="meta"))
+    assert fast.linear_slices(a, w, residual=True) == (cut or None) and fast.linear_slices(a, w) is None
