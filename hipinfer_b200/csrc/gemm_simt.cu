@@ -193,15 +193,19 @@ __global__ void __launch_bounds__(256) simt_reduce_kernel(const float* ws, TC* C
 // columns; warp w of a block makes slice w by itself: it asks for its slice's next piece (16 columns x KC), waits for the oldest
 // and multiplies, with no barrier until the slices are added. Lane l makes column l & 15 of the rows (l >> 4), (l >> 4) + 2,
 // ...: a 16-byte read of W serves RP rows, whose chains are independent. The first pieces of W are asked for before the wait
-// for the kernel ahead. Bound by HBM; about 130 KB a SM are in flight.
-constexpr int SR_COLS = 16, SR_ROWS = 8, SR_RING = 5;
+// for the kernel ahead. RING: the pieces of a warp's ring, five where two blocks then fit an SM, else four (32-bit operands, from
+// five rows on, from four with more than four slices: with five pieces only one block fitted, and the blocks, dealt two an SM, ran
+// in two rounds). Bound by HBM up to four rows, by the reads of shared memory above: 16,384 x 2,048 at 1, 4 and 8 rows 24.4, 28.5 and
+// 41.6 us (8 rows with five pieces: 46.8), 4,096 x 14,336 45.4, 44.9 and 62.1 (4 and 8 rows with five pieces: 55.4 and 77.3).
+constexpr int SR_COLS = 16, SR_ROWS = 8;
 template <typename TA, typename TW, int KC> struct RowsPiece {
   static constexpr int PW = 16 / sizeof(TW), PA = 16 / sizeof(TA);        // elements of a 16-byte access
   // a column's piece is padded by 16 bytes: the 16-byte reads of eight columns meet no bank twice
   static constexpr int W_BYTES = SR_COLS * (KC + PW) * sizeof(TW);
   __host__ __device__ static constexpr int bytes(int M) { return W_BYTES + M * KC * (int)sizeof(TA); }
 };
-template <typename TA, typename TW, typename TC, int EPI, int RP, int KC>
+constexpr int SR_STATIC = 2 * SM_MAX_SLICES * SR_ROWS * SR_COLS * (int)sizeof(float), SR_MOST = 228 * 512 - 1024 - SR_STATIC;   // dynamic bytes of a block of two
+template <typename TA, typename TW, typename TC, int EPI, int RP, int KC, int RING>
 __global__ void __launch_bounds__(256, 2) simt_rows_kernel(const TA* A, long lda, const TW* __restrict__ W, long ldw, TC* C, long ldc,
                                                            int M, int N, int K, const TW* __restrict__ colscale, int depth) {
   using P = RowsPiece<TA, TW, KC>;
@@ -211,14 +215,14 @@ __global__ void __launch_bounds__(256, 2) simt_rows_kernel(const TA* A, long lda
   const int per_tile = depth / KC, tiles = (N + SR_COLS - 1) / SR_COLS, k_lo = warp * depth, k_hi = min(K, k_lo + depth);
   const int total = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x * per_tile;      // this block's pieces
   const int piece = P::bytes(M);
-  const uint8_t* ring = sr_smem + (size_t)warp * SR_RING * piece;
+  const uint8_t* ring = sr_smem + (size_t)warp * RING * piece;
   const uint32_t ring_s = hb_smem_u32(ring);
   // this lane's place in a piece: LW lanes a column, LA lanes a row of A
   constexpr int LW = KC / P::PW, LA = KC / P::PA;
   static_assert(LW <= 32 && LA <= 32, "a piece's row is at most a warp wide");
   int wi = 0, wt = blockIdx.x, wk = k_lo;              // the next piece of W to ask for: its count, tile and k
   auto load_w = [&]() {
-    const uint32_t dst = ring_s + (uint32_t)(wi % SR_RING) * piece + (uint32_t)((lane / LW) * (KC + P::PW) + lane % LW * P::PW) * sizeof(TW);
+    const uint32_t dst = ring_s + (uint32_t)(wi % RING) * piece + (uint32_t)((lane / LW) * (KC + P::PW) + lane % LW * P::PW) * sizeof(TW);
     const int k = wk + lane % LW * P::PW, n = wt * SR_COLS + lane / LW;
     const TW* src = W + (size_t)n * ldw + k;
     if (k < k_hi) {
@@ -232,7 +236,7 @@ __global__ void __launch_bounds__(256, 2) simt_rows_kernel(const TA* A, long lda
   };
   int ai = 0, ak = k_lo;
   auto load_a = [&]() {
-    const uint32_t dst = ring_s + (uint32_t)(ai % SR_RING) * piece + P::W_BYTES + (uint32_t)(lane % LA * P::PA) * sizeof(TA);
+    const uint32_t dst = ring_s + (uint32_t)(ai % RING) * piece + P::W_BYTES + (uint32_t)(lane % LA * P::PA) * sizeof(TA);
     const int k = ak + lane % LA * P::PA;
     if (k < k_hi)
       for (int m = lane / LA; m < M; m += 32 / LA) hb_cp_async16(dst + (uint32_t)(m * KC) * sizeof(TA), A + (size_t)m * lda + k);
@@ -240,11 +244,11 @@ __global__ void __launch_bounds__(256, 2) simt_rows_kernel(const TA* A, long lda
     ak += KC;
     if (ak == k_lo + depth) ak = k_lo;
   };
-  for (int i = 0; i < SR_RING - 1 && i < total; i++) load_w();
+  for (int i = 0; i < RING - 1 && i < total; i++) load_w();
   hb_pdl_wait();
   hb_pdl_launch();      // not earlier: blocks of kernels further on would hold room on the SMs ahead of those that can run
 #pragma unroll
-  for (int i = 0; i < SR_RING - 1; i++) {
+  for (int i = 0; i < RING - 1; i++) {
     if (i < total) load_a();
     hb_cp_async_commit();
   }
@@ -254,9 +258,9 @@ __global__ void __launch_bounds__(256, 2) simt_rows_kernel(const TA* A, long lda
   for (int r = 0; r < RP; r++) acc[r] = 0.f;
   int step = 0, tile = blockIdx.x, buf = 0;
   for (int i = 0; i < total; i++) {
-    hb_cp_async_wait<SR_RING - 2>();
+    hb_cp_async_wait<RING - 2>();
     __syncwarp();
-    const uint8_t* st = ring + (size_t)(i % SR_RING) * piece;
+    const uint8_t* st = ring + (size_t)(i % RING) * piece;
     const TW* wr = (const TW*)st + n * (KC + P::PW);
     const TA* ar = (const TA*)(st + P::W_BYTES);
     const int len = min(KC, k_hi - k_lo - step * KC);      // a multiple of 4, or none
@@ -334,22 +338,24 @@ static int simt_launch(const TA* A, long lda, const TW* W, long ldw, TC* C, long
   // 16-byte pieces of both operands' rows: a slice starts at a multiple of 64, so K alone decides about the last one
   if (M <= SR_ROWS && bytes16 && (K * sizeof(TA)) % 16 == 0 && (K * sizeof(TW)) % 16 == 0) {
     const int tiles = (N + SR_COLS - 1) / SR_COLS, most = 2 * simt_sms(), blocks = tiles < most ? tiles : most;
-    // a warp's ring holds five pieces, 64 deep with up to four slices, 32 deep with more: at most 100 KB a block
-#define HB_SIMT_ROWS(RP, KC)                                                                                                  \
+    // pieces 64 deep with up to four slices, 32 deep with more
+#define HB_SIMT_ROWS(RP, KC, RING)                                                                                            \
   do {                                                                                                                        \
-    auto kern = simt_rows_kernel<TA, TW, TC, EPI, RP, KC>;                                                                    \
-    const size_t smem = (size_t)slices * SR_RING * RowsPiece<TA, TW, KC>::bytes(M);                                           \
-    e = smem > 40 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) : cudaSuccess; \
+    auto kern = simt_rows_kernel<TA, TW, TC, EPI, RP, KC, RING>;                                                              \
+    static_assert((KC == 64 ? 4 : 8) * 4 * RowsPiece<float, float, KC>::bytes(8) <= SR_MOST, "two blocks an SM");              \
+    const size_t smem = (size_t)slices * RING * RowsPiece<TA, TW, KC>::bytes(M);                                              \
+    e = smem > 40 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SR_MOST) : cudaSuccess;    \
     if (e == cudaSuccess) e = hb_launch(kern, blocks, 32 * slices, smem, s, A, lda, W, ldw, C, ldc, M, N, K, colscale, depth); \
   } while (0)
     if (slices <= 4) {
-      if (M <= 2) HB_SIMT_ROWS(1, 64);
-      else if (M <= 4) HB_SIMT_ROWS(2, 64);
-      else HB_SIMT_ROWS(4, 64);
+      if (M <= 2) HB_SIMT_ROWS(1, 64, 5);
+      else if (M <= 4) HB_SIMT_ROWS(2, 64, 5);
+      else HB_SIMT_ROWS(4, 64, 4);
     } else {
-      if (M <= 2) HB_SIMT_ROWS(1, 32);
-      else if (M <= 4) HB_SIMT_ROWS(2, 32);
-      else HB_SIMT_ROWS(4, 32);
+      if (M <= 2) HB_SIMT_ROWS(1, 32, 5);
+      else if (slices * 5 * RowsPiece<TA, TW, 32>::bytes(M) <= SR_MOST && M <= 4) HB_SIMT_ROWS(2, 32, 5);
+      else if (M <= 4) HB_SIMT_ROWS(2, 32, 4);
+      else HB_SIMT_ROWS(4, 32, 4);
     }
 #undef HB_SIMT_ROWS
     if (e != cudaSuccess) HB_FAIL("hb_gemm_simt: %s", cudaGetErrorString(e));

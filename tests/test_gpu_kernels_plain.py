@@ -115,6 +115,20 @@ def test_gemm_plain_slices(adt, wdt, N, K):
     assert torch.equal(acc, want) and torch.equal(few, want[3:6])
 
 
+@pytest.mark.parametrize("adt,wdt", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32)])
+@pytest.mark.parametrize("N,K", [(100, 512), (5000, 2048), (300, 4104), (9500, 8192)])
+def test_gemm_plain_one_to_eight_rows(adt, wdt, N, K):
+    """The streaming kernel at every number of rows (rings of four and of five pieces, one to eight slices, one and several rounds of
+    column groups): a row's bits are those of the tile kernel."""
+    a, w = rnd(9, K, dtype=adt, seed=35), rnd(N, K, dtype=wdt, seed=36, scale=0.1)
+    full = torch.empty(9, N, device=DEV)
+    ops().gemm_plain(a, w, full)
+    for M in range(1, 9):
+        few = torch.full((M + 1, N), 7.0, device=DEV)
+        ops().gemm_plain(a[:M], w, few[:M])
+        assert torch.equal(few[:M], full[:M]) and bool((few[M] == 7.0).all()), M
+
+
 @pytest.mark.parametrize("idt", DT)
 @pytest.mark.parametrize("odt", DT)
 def test_swiglu(idt, odt):
