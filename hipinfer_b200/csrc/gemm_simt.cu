@@ -305,9 +305,6 @@ __global__ void __launch_bounds__(256, 2) simt_rows_kernel(const TA* A, long lda
   }
 }
 
-// Products of fewer tiles than this give their slices to blocks of their own: two tiles an SM fit at once, and a whole-K
-// block of the last, partly filled wave takes as long as the whole wave. 640 tiles on 296 places (301 x 16,384 x 2,048) took
-// 502 us in whole-K blocks and about 410 us split, the reduction of 79 MB of partial sums included.
 static int simt_sms() {
   static int n[64] = {};
   int dev = 0;
@@ -315,9 +312,14 @@ static int simt_sms() {
   if (!n[dev] && cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n[dev] = 148;
   return n[dev];
 }
+// Whether slices get blocks of their own: while the tiles are at most three rounds of two an SM, since a whole-K block of the last,
+// partly filled round takes as long as the whole round. us whole / split: 640 tiles (301 x 16,384 x 2,048) 500 / 455, 768 (1,531 x 4,096 x
+// 14,336) 4,114 / 3,475, but 1,024 of four slices (512 x 16,384 x 2,048) 699 / 713. Beyond, eight slices still gain some 5 % (2,048 x
+// 4,096 x 14,336: 4,841 / 4,628), for 268 MB of partial sums; up to the line they are at most 233 MB. Two slices only where
+// the tiles are more than the SMs: 64 x 4,096 x 1,024 took 60 / 77, 301 x 4,096 x 1,024 105 / 84.
 static bool simt_splits(int M, int N, int slices) {
   const long tiles = (long)((M + SM_TM - 1) / SM_TM) * ((N + SM_TN - 1) / SM_TN);
-  return slices > 1 && tiles < 10l * simt_sms();
+  return slices > 1 && tiles <= 6l * simt_sms() && (slices > 2 || tiles > simt_sms());
 }
 
 // Floats of workspace that a product of more than SR_ROWS rows can use (0: none; without one it runs unsplit, same bits).

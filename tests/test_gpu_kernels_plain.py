@@ -129,6 +129,24 @@ def test_gemm_plain_one_to_eight_rows(adt, wdt, N, K):
         assert torch.equal(few[:M], full[:M]) and bool((few[M] == 7.0).all()), M
 
 
+@pytest.mark.parametrize("M,N,K,slices", [(70, 12000, 1024, 2), (64, 4096, 1024, 0), (64, 113000, 1100, 3), (64, 114000, 1100, 0), (9, 300, 4096, 8), (70, 300, 512, 0)])
+def test_gemm_plain_where_slices_have_blocks_of_their_own(M, N, K, slices):
+    """Both sides of the rule (tiles of 64 x 128 against the SMs, two slices and more); split or not, the bits are the same."""
+    from hipinfer_b200.kernels import library
+
+    lib = library.load("core")
+    lib.hb_gemm_simt_workspace.restype = ctypes.c_long
+    assert lib.hb_gemm_simt_workspace(M, N, K) == slices * M * N
+    a, w = rnd(M, K, dtype=torch.float32, seed=37), rnd(N, K, dtype=torch.float32, seed=38, scale=0.1)
+    out, whole = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    ops().gemm_plain(a, w, out)
+    assert lib.hb_gemm_simt(*[ctypes.c_void_p(a.data_ptr()), 0, ctypes.c_long(K), ctypes.c_void_p(w.data_ptr()), 0, ctypes.c_long(K),
+                              ctypes.c_void_p(whole.data_ptr()), 0, ctypes.c_long(N), M, N, K, 0, None, ctypes.c_void_p(library.current_stream())]) == 0
+    assert torch.equal(out, whole)
+    bound = (max(512, -(-K // 8)) + 72) * 2.0 ** -24 * (a[:4].double().abs() @ w.double().abs().T)
+    assert bool(((out[:4].double() - a[:4].double() @ w.double().T).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("idt", DT)
 @pytest.mark.parametrize("odt", DT)
 def test_swiglu(idt, odt):
