@@ -14,7 +14,22 @@ from typing import Optional
 
 import torch
 
-from . import fast, library
+from . import library
+
+
+class _AtFirstUse:
+    """The module of the fast kernels, imported when one of them is first chosen, for it reads its switch (HIPINFER_B200_PLAIN) at its
+    import; from then on `fast` is that module."""
+
+    def __getattr__(self, name):
+        global fast
+        from . import fast as module
+
+        fast = module
+        return getattr(module, name)
+
+
+fast = _AtFirstUse()
 
 _DT = {torch.float32: 0, torch.bfloat16: 1}
 _p, _i, _l, _f = C.c_void_p, C.c_int, C.c_long, C.c_float

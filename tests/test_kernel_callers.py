@@ -72,3 +72,16 @@ def test_products_of_portions_are_cut_along_k_where_that_pays(monkeypatch, M, N,
     monkeypatch.setattr(fast, "gemm_stream_slices", lambda a, w: None)
     a, w = torch.empty(M, K, device="meta"), ops.Weight(torch.empty(N, K, device="meta"))
     assert fast.linear_slices(a, w, residual=True) == (cut or None) and fast.linear_slices(a, w) is None
+
+
+def test_the_plain_kernels_may_be_asked_for_after_the_import():
+    """HIPINFER_B200_PLAIN is read when a kernel is first chosen, not when the package is imported."""
+    import os
+    import subprocess
+    import sys
+
+    code = ("import os, hipinfer_b200, hipinfer_b200.engine\nfrom hipinfer_b200.kernels import ops\n"
+            "os.environ['HIPINFER_B200_PLAIN'] = '1'\nassert not ops.fast_kernels_on()\n"
+            "from hipinfer_b200.kernels import fast\nassert fast.PLAIN_ONLY and ops.fast is fast")
+    env = {k: v for k, v in os.environ.items() if k != "HIPINFER_B200_PLAIN"}
+    subprocess.run([sys.executable, "-c", code], check=True, env=env, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
