@@ -284,6 +284,8 @@ HB_EXPORT int hb_heads_linear(const float* a, long lda, long a_head, const void*
                               int pairing, int gate_per_head, const int* row_list, cudaStream_t s) {
   if (T <= 0 || H <= 0) return 0;
   if (tail && (!pos || !table || rot > tail || (rot & 1))) HB_FAIL("hb_heads_linear: a rotated tail needs positions and a table");
+  const size_t smem = ((size_t)HL_TM * (K + tail) + (size_t)HL_KZ * HL_TM * HL_TN) * sizeof(float);
+  if (smem > 96 * 1024) HB_FAIL("hb_heads_linear: K = %d is too wide", K);      // (whichever kernel: the rule below goes by the rows)
   if (N % 8 == 0 && ((uintptr_t)wt & 15) == 0 && H <= 65535 && hv_few(T, H, K, N)) {     // (a row of 8 is 16 or 32 bytes)
     const HeadsVec A{a, lda, a_head, wt, out, ldo, o_head, T, K, N, gate, ld_gate, gate_off, tail, rot, pos, (const float2*)table, row_list,
                      row_req, q_len, row_limit, pairing, gate_per_head};
@@ -292,8 +294,6 @@ HB_EXPORT int hb_heads_linear(const float* a, long lda, long a_head, const void*
     HB_CHECK_LAUNCH("hb_heads_linear");
     return 0;
   }
-  const size_t smem = ((size_t)HL_TM * (K + tail) + (size_t)HL_KZ * HL_TM * HL_TN) * sizeof(float);
-  if (smem > 96 * 1024) HB_FAIL("hb_heads_linear: K = %d is too wide", K);
   if ((T + HL_TM - 1) / HL_TM > 65535 || H > 65535) HB_FAIL("hb_heads_linear: the grid is too large");
   dim3 grid((N + tail + HL_TN - 1) / HL_TN, H, (T + HL_TM - 1) / HL_TM);
 #define HL_LAUNCH(TW, TO)                                                                                       \

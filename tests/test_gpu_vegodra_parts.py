@@ -548,3 +548,22 @@ def test_heads_linear_of_few_and_of_many_rows(wdt, H, K, N, tail, T, few):
     one = torch.empty(1, H * (N + tail), device=DEV)    # a row by itself is the kernel of few rows where there is one for these sizes
     ops.heads_linear(a[T - 1:].to(DEV), K + tail, w.to(DEV), one, N + tail, **(dict(kw, positions=pos[T - 1:].to(DEV)) if tail else {}))
     assert torch.equal(one[0], out[T - 1]) == (few or N % 8 != 0)
+
+
+@pytest.mark.parametrize("T", [1, 2000])
+def test_heads_linear_refuses_what_one_of_its_kernels_cannot_hold(T):
+    from hipinfer_b200.kernels import ops
+
+    H, K, N = 1, 2976, 8
+    a, w, out = torch.zeros(T, H * K, device=DEV), torch.zeros(H, K, N, device=DEV), torch.empty(T, H * N, device=DEV)
+    with pytest.raises(ops.KernelError, match="too wide"):
+        ops.heads_linear(a, K, w, out, N)
+    ops.heads_linear(a[:, :2944].contiguous(), 2944, w[:, :2944].contiguous(), out, N)
+    assert not out.any()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,D,E,tau", [(2, 32, 64, 8.0), (2, 64, 32, 4.0), (2, 32, 72, 2.0), (1, 128, 64, 8.0)])
+def test_gated_linear_attention_in_its_other_forms(dtype, H, D, E, tau):
+    """Eight key channels a walking thread, sixteen of wide keys, and aligned sizes that the kernel with helpers does not take."""
+    test_gated_linear_attention(dtype, H, D, E, tau)
