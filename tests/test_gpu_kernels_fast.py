@@ -787,3 +787,55 @@ def test_slices_of_two_portions_at_the_same_time():
     for got, x, y in ((one, a, w.t), (two, b, v.t), (small, a[:20], w.t)):
         bound = x.shape[1] * 2.0 ** -23 * (x.double().abs() @ y.double().abs().T)
         assert bool(((got.double() - x.double() @ y.double().T).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("M,H,K,n", [(65, 300, 1024, 2), (130, 776, 2048, 4), (300, 1044, 2560, 5), (300, 520, 4096, 8), (700, 2048, 2048, 3)])
+def test_slices_of_portions_added_by_the_norm(M, H, K, n):
+    """Slices of M rounded up to 256 rows of H rounded up to 32 columns, two to eight of them (four loads of a thread in flight, and
+    sixteen): x as finish() makes it, bit for bit; the norm equal to the plain norm of that x up to the order of its sum of squares
+    and the rounding to bfloat16; gathered rows, where x stays."""
+    from hipinfer_b200.kernels import ops
+
+    a, w = rnd(M, K, seed=41), ops.Weight(rnd(H, K, seed=42, scale=0.05))
+    x0 = rnd(M, H, seed=43, scale=2.0, dtype=torch.float32)
+    nw = (1 + rnd(H, seed=44, dtype=torch.float32) * 0.1).to(torch.bfloat16)
+    cut = lambda x: ops.Pending(fast().gemm_tc_slices(a, w.t), x, True)
+    x_ref = x0.clone()
+    pend = cut(x_ref)
+    assert pend.slices.ksplit == n and torch.equal(x_ref, x0)
+    pend.finish()
+    bound = K * 2.0 ** -23 * (a.double().abs() @ w.t.double().abs().T) + 2.0 ** -22 * x0.double().abs()
+    assert bool(((x_ref.double() - x0.double() - a.double() @ w.t.double().T).abs() <= bound).all())
+    y_ref = ops.rmsnorm(x_ref, nw, 1e-5, torch.empty(M, H, dtype=torch.bfloat16, device=DEV))
+    x = x0.clone()
+    y = ops.rmsnorm(x, nw, 1e-5, torch.full((M, H), 3.0, dtype=torch.bfloat16, device=DEV), pending=cut(x))
+    sync_check()
+    assert torch.equal(x, x_ref)
+    ulp = float(((y.float() - y_ref.float()).abs() / y_ref.float().abs().clamp_min(1e-3)).max())
+    assert ulp <= 2.0 ** -7 and float((y != y_ref).float().mean()) < 0.01
+    rows = torch.tensor([M - 1, 0, M - 1], dtype=torch.int32, device=DEV)
+    x = x0.clone()
+    y2 = ops.rmsnorm(x, nw, 1e-5, torch.empty(3, H, dtype=torch.bfloat16, device=DEV), rows=rows, pending=cut(x))
+    assert torch.equal(y2, y[[M - 1, 0, M - 1]]) and torch.equal(x, x0)
+
+
+@pytest.mark.parametrize("M,Hq,Hkv,D,K", [(65, 3, 1, 72, 1024), (300, 4, 2, 128, 4096)])
+def test_slices_of_portions_added_by_the_rotation(M, Hq, Hkv, D, K):
+    """The same layout read by the rotation: q, k and v as from the finished product, bit for bit."""
+    from hipinfer_b200.kernels import ops
+    from hipinfer_b200.parts.rotary import rope_inv_freq
+
+    ps, N = 16, (Hq + 2 * Hkv) * D
+    xn, w = rnd(M, K, seed=51), ops.Weight(rnd(N, K, seed=53, scale=0.05))
+    table = ops.rope_table(rope_inv_freq(D, 500000.0).to(DEV), 512)
+    pos = torch.arange(M, dtype=torch.int32, device=DEV)
+    fill = lambda: torch.full((-(-M // ps) + 1, Hkv, ps, D), 9.0, dtype=torch.bfloat16, device=DEV)
+    qkv, out = torch.empty(M, N, device=DEV), []
+    for finished in (True, False):
+        pend, q, kc, vc = ops.Pending(fast().gemm_tc_slices(xn, w.t), qkv, False), torch.empty(M, Hq * D, dtype=torch.bfloat16, device=DEV), fill(), fill()
+        if finished:
+            pend.finish()
+        ops.rope_kv_write(qkv, pos, pos, table, q, kc, vc, Hq, Hkv, D, D, ps, pending=None if finished else pend)
+        out.append((q, kc, vc))
+    sync_check()
+    assert all(torch.equal(x, y) for x, y in zip(*out))

@@ -392,3 +392,41 @@ def test_single_rows_on_warp_mmas(H, G, D, E, window, keep):
         plant.append((8, keep - 1))
     got, want = _attend(torch.bfloat16, H, G, D, E, 2, 1000, rows, window, keep, 16, plant=plant, seed=H + D)
     close(got, want, torch.bfloat16)
+
+
+@pytest.mark.parametrize("D,E", [(32, 64), (64, 128)])
+@pytest.mark.parametrize("window,keep", [(100, 3), (0, 0), (40, 70)])
+def test_window_rows_beside_a_portion_and_keys_read_ahead(D, E, window, keep):
+    """Short portions beside one for the flash kernel go to the row kernel as a list, with the requests' earlier lengths known (tiles of
+    earlier keys are read before the kernel ahead has ended: earlier lengths of none, of whole tiles of 64 keys, and one less and
+    more): the bits of the row kernel over all rows. A list that is the step's own is in test_step_batch.py."""
+    from hipinfer_b200.kernels import ops
+
+    H, G, ps = 8, 2, 16
+    ctx, new = [130, 64, 0, 127, 128, 129, 5], [20, 1, 2, 3, 1, 1, 15]
+    lens = [c + n for c, n in zip(ctx, new)]
+    planes = [_paged(rnd(n, G, 2 * D, seed=10 + r).to(torch.bfloat16), rnd(n, G, E, seed=30 + r).to(torch.bfloat16), G, ps, r)
+              for r, n in enumerate(lens)]
+    kc, vc = (torch.cat([p[i] for p in planes]).to(DEV) for i in (0, 1))
+    bt, first = torch.full((len(lens), max(p[2].numel() for p in planes)), -1, dtype=torch.int32), 0
+    for r, p in enumerate(planes):
+        bt[r, :p[2].numel()] = p[2] + first
+        first += p[0].shape[0]
+    rows = [(r, p) for r in range(len(lens)) for p in range(ctx[r], lens[r])]
+    T = len(rows)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    short = [t for t, (r, _) in enumerate(rows) if new[r] < 16]
+    common = dict(block_tables=[bt.to(DEV)], row_request=i32([r for r, _ in rows]), positions=i32([p for _, p in rows]), max_pos=max(lens) - 1,
+                  n_requests=len(lens), max_q_len=max(new), h_q_len=new, req_q_start=i32([sum(new[:r]) for r in range(len(new))]), req_q_len=i32(new))
+    q, gate = rnd(T, H * 2 * D, seed=5).to(torch.bfloat16).to(DEV), rnd(T, 4 + H * E, seed=6).to(DEV)
+    args = (H, G, D, E, 2, ps, window, keep, D ** -0.5, 0.6, 0.7, 1e-5, True, gate, 4)
+    every, beside = (torch.empty(T, H * E, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    # (force_rows keeps the flash kernel out; a first kept token keeps the TMA decode kernel out of both calls)
+    ops.attention_window(q, kc, vc, SimpleNamespace(**common), 0, every, *args, force_rows=True)
+    listed = SimpleNamespace(**common, req_ctx_len=i32(ctx), short_rows=lambda limit: (i32(short), max(rows[t][1] for t in short)))
+    ops.attention_window(q, kc, vc, listed, 0, beside, *args)
+    torch.cuda.synchronize()
+    if keep or E != 2 * D:
+        assert torch.equal(beside[short], every[short])
+    err = (beside.float() - every.float()).abs().max() / every.float().abs().max()
+    assert torch.isfinite(beside.float()).all() and float(err) < 2e-2      # another kernel: probabilities and results rounded to bf16
