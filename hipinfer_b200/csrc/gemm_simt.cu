@@ -73,7 +73,7 @@ template <typename TA, typename TW, typename TC, int EPI, bool WHOLE, bool VEC>
 __global__ void __launch_bounds__(128, 2) simt_tile_kernel(const TA* A, long lda, const TW* __restrict__ W, long ldw,
                                                            TC* C, long ldc, int M, int N, int K,
                                                            const TW* __restrict__ colscale, float* ws, int depth) {
-  // rows of 64 + 4 and 128 + 4: a float4 read of one k by a warp meets no bank twice
+  // rows of 64 + 4 and 128 + 4: a float4 read of one k by a warp meets no bank twice (the transposing stores below do: two passes each)
   __shared__ __align__(16) float As[2][SM_TK][SM_TM + 4], Ws[2][SM_TK][SM_TN + 4];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int m0 = blockIdx.y * SM_TM, n0 = blockIdx.x * SM_TN;

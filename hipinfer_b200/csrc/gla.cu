@@ -187,7 +187,8 @@ __global__ void __launch_bounds__(GlaThreads<DPT>::MAX, 1) gla_kernel(GlaArgs A)
 // neighbouring value channels each, DPT key channels of them, and do nothing but walk; GL_HELP further threads bring the rows of
 // the chunk after next, make scaled query and decay of the next one (a log1p and two exponentials a channel and token) and
 // finish the chunk before (norm, gate, rounding), one barrier a chunk. Rows lie in three buffers: walked and then finished, prepared,
-// on their way. The arithmetic and its order are the kernel's above. In one job after the other this work stood between the chunks of
+// on their way. The arithmetic is the kernel's above, and its order too where a
+// channel is shared by as many threads (heads of 64 x 64; at 128 x 128 four share it here, two there: the last bits of o differ). In one job after the other this work stood between the chunks of
 // the walk: 32 heads of 64 x 64, two requests, 2,048 tokens: 752 us, 467 with the helpers.
 constexpr int GL_HELP = 128;
 template <int DPT, typename TW, typename TO>
