@@ -68,8 +68,8 @@ HB_EXPORT int hb_latent_prepare(const float* proj, long ld, int cq_off, int c_of
 constexpr int HL_TM = 8, HL_THREADS = 128, HL_TN = 32, HL_KZ = HL_THREADS / HL_TN;
 
 // A block owns HL_TM rows, one head and HL_TN output columns; its threads are HL_TN columns x HL_KZ interleaved slices of
-// k, summed in a fixed order (slice 0 .. HL_KZ - 1) through shared memory: few rows still fill the machine, and a
-// thread's loads of the weight are independent of one another.
+// k, which meet in shared memory: few rows still fill the machine, and a thread's loads of the weight are independent of one
+// another. The sums are those of heads_linear_vec_kernel, bit for bit: a row's result does not depend on how many rows there are.
 template <typename TW, typename TO>
 __global__ void __launch_bounds__(HL_THREADS) heads_linear_kernel(const float* a, long lda, long a_head,
                                                                   const TW* __restrict__ wt, TO* __restrict__ out, long ldo,
@@ -98,28 +98,43 @@ __global__ void __launch_bounds__(HL_THREADS) heads_linear_kernel(const float* a
     hl_a[r * KT_ + k] = a[(size_t)row_of(r) * lda + (size_t)h * a_head + k];
   }
   __syncthreads();
-  float acc[HL_TM];
+  // partial sums as the lanes of heads_linear_vec_kernel make them: chain l of a row has the k = l, l + 32, ..; chain kz + 4 u is acc[.][u]
+  float acc[HL_TM][8];
 #pragma unroll
-  for (int r = 0; r < HL_TM; r++) acc[r] = 0.f;
+  for (int r = 0; r < HL_TM; r++)
+#pragma unroll
+    for (int u = 0; u < 8; u++) acc[r][u] = 0.f;
   if (n < N) {
     const TW* w = wt + (size_t)h * K * N + n;
-#pragma unroll 4
-    for (int k = kz; k < K; k += HL_KZ) {
-      const float wv = hb_to_float(w[(size_t)k * N]);
+    int k = kz;
+    for (; k + 28 < K; k += 32) {
+      float wv[8];
 #pragma unroll
-      for (int r = 0; r < HL_TM; r++) acc[r] = fmaf(hl_a[r * KT_ + k], wv, acc[r]);
+      for (int u = 0; u < 8; u++) wv[u] = hb_to_float(w[(size_t)(k + 4 * u) * N]);
+#pragma unroll
+      for (int u = 0; u < 8; u++)
+#pragma unroll
+        for (int r = 0; r < HL_TM; r++) acc[r][u] = fmaf(hl_a[r * KT_ + k + 4 * u], wv[u], acc[r][u]);
     }
-  }
 #pragma unroll
-  for (int r = 0; r < HL_TM; r++) red[(kz * HL_TM + r) * HL_TN + nl] = acc[r];
+    for (int u = 0; u < 8; u++)
+      if (k + 4 * u < K) {
+        const float wv = hb_to_float(w[(size_t)(k + 4 * u) * N]);
+#pragma unroll
+        for (int r = 0; r < HL_TM; r++) acc[r][u] = fmaf(hl_a[r * KT_ + k + 4 * u], wv, acc[r][u]);
+      }
+  }
+  // .. and added as the lanes' butterfly adds them: chains 16 apart, then 8, 4, 2 and 1 (the last two between the threads)
+#pragma unroll
+  for (int r = 0; r < HL_TM; r++)
+    red[(kz * HL_TM + r) * HL_TN + nl] = ((acc[r][0] + acc[r][4]) + (acc[r][2] + acc[r][6])) + ((acc[r][1] + acc[r][5]) + (acc[r][3] + acc[r][7]));
   __syncthreads();
   if (n < N) {
     // thread (nl, kz) finishes rows kz, kz + HL_KZ, ...
     for (int r = kz; r < rows; r += HL_KZ) {
       if (skip >> r & 1) continue;
-      float o = 0.f;
-#pragma unroll
-      for (int z = 0; z < HL_KZ; z++) o += red[(z * HL_TM + r) * HL_TN + nl];
+      const float* z = red + r * HL_TN + nl;
+      float o = (z[0] + z[2 * HL_TM * HL_TN]) + (z[HL_TM * HL_TN] + z[3 * HL_TM * HL_TN]);
       if (gate) o *= 1.f / (1.f + expf(-gate[(size_t)row_of(r) * ld_gate + gate_off + (gate_per_head ? (size_t)h : (size_t)h * N + n)]));
       out[(size_t)row_of(r) * ldo + (size_t)h * o_head + n] = hb_from_float<TO>(o);
     }
@@ -271,6 +286,7 @@ __global__ void __launch_bounds__(256) heads_linear_vec_kernel(HeadsVec A) {
 // 3.2; 24 rows 3.7 against 3.4), at K = 128 between 3,072 and 4,096 (16 heads of 128 x 512, 8 rows: 5.2 against 6.4; 16 rows 10.0
 // against 9.4), at K = 256 and 512 between 5,120 and 6,144 (32 heads of 256 x 64, 64 rows: 12.4 against 17.5; 128 rows 23.7
 // against 23.2, 2,048 rows 398 against 189).
+static_assert(HL_KZ == 4, "the order of the sums");
 static bool hv_few(int T, int H, int K, int N) {
   const long warps = (long)((T + HV_ROWS - 1) / HV_ROWS) * H * (N / 8);
   return warps < 24l * (K < 64 ? 64 : K < 216 ? K : 216);
