@@ -148,12 +148,18 @@ __device__ __forceinline__ void rope_head_store(float* x1, float* x2, int head, 
 
 // 32 accumulator columns (chunk c of the tile at column n0) of 32 rows, one row a lane, through this warp's two
 // 4 KB boxes of swizzled shared memory and out by a TMA tensor store (or reduce). PER chunks fill one box of
-// 128-byte rows: 1 (fp32), 2 (bf16), 4 (SwiGLU: 16 outputs each). row0: the first of the warp's 32 rows in C.
+// 128-byte rows: 1 (fp32), 2 (bf16), 4 (SwiGLU: 16 outputs each). row0: the first of the warp's 32 rows in C. sent: the boxes this
+// warp has sent so far, over all its tiles (the last tile of a row may have an odd number of them).
+// A box of bf16 that C's last row cuts is slow to store (gate/up of 1,531 rows, 16,384 x 2,048: 105 us with such boxes, 80 with
+// those rows stored directly; 1,536 rows 80): ts_whole says whether a warp's rows go this way. Boxes of fp32 showed no such cost.
+template <int EPI> __device__ __forceinline__ bool ts_whole(int row0, int M) {
+  return EPI == EPI_F32 || EPI == EPI_ADD_F32 || row0 + 32 <= M;
+}
 template <int EPI>
-__device__ __forceinline__ void ts_chunk(const float* v, int c, int n0, int N, int row0, uint8_t* boxes, int lane,
+__device__ __forceinline__ void ts_chunk(const float* v, int c, int n0, int N, int row0, uint8_t* boxes, uint32_t& sent, int lane,
                                          const CUtensorMap* map_c) {
   constexpr int PER = EPI_IS_GLU(EPI) ? 4 : EPI_IS_BF16(EPI) ? 2 : 1;
-  uint8_t* box = boxes + ((c / PER) & 1) * 4096;
+  uint8_t* box = boxes + (sent & 1) * 4096;
   if (c % PER == 0) {
     if (lane == 0) hb_tma_store_wait_read<1>();   // the store that last read this box is done with it
     __syncwarp();
@@ -195,6 +201,7 @@ __device__ __forceinline__ void ts_chunk(const float* v, int c, int n0, int N, i
       else hb_tma_store_2d(map_c, box, x, row0);
       hb_tma_store_commit();
     }
+    sent++;
   }
 }
 
@@ -242,20 +249,28 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
   __syncthreads();
   hb_tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  hb_pdl_wait();   // barriers and tensor memory were set up while the kernel ahead was still running
+  if (warp != 4) hb_pdl_wait();   // barriers and tensor memory were set up while the kernel ahead was still running
 
   if (warp == 4) {
     if (lane == 0) {  // ---------------- TMA producer
-      uint32_t it = 0;
+      uint32_t it = 0, early = 0;
       bool ok = true;
+      // the first weight tiles do not depend on the kernel ahead (every CTA has a tile)
+      for (; early < STAGES && early < num_kb; early++) {
+        hb_mbar_expect_tx(&full[early], S::STAGE_BYTES);
+        hb_tma_load_2d(smem + early * S::STAGE_BYTES + S::A_BYTES, &map_w, &full[early], early * BK, (blockIdx.x / m_tiles) * BN);
+      }
+      hb_pdl_wait();
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * BN;
         for (int kb = 0; kb < num_kb; kb++, it++) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          if (!hb_mbar_wait(&empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
-          hb_mbar_expect_tx(&full[s], S::STAGE_BYTES);
+          if (it >= early) {
+            if (!hb_mbar_wait(&empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
+            hb_mbar_expect_tx(&full[s], S::STAGE_BYTES);
+            hb_tma_load_2d(smem + s * S::STAGE_BYTES + S::A_BYTES, &map_w, &full[s], kb * BK, n0);
+          }
           hb_tma_load_2d(smem + s * S::STAGE_BYTES, &map_a, &full[s], kb * BK, m0);
-          hb_tma_load_2d(smem + s * S::STAGE_BYTES + S::A_BYTES, &map_w, &full[s], kb * BK, n0);
         }
       }
     }
@@ -283,7 +298,7 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
       }
     }
   } else {  // ---------------- epilogue warps 0..3
-    uint32_t tile_i = 0;
+    uint32_t tile_i = 0, sent = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, tile_i++) {
       const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * BN;
       const uint32_t buf = tile_i & 1, aph = (tile_i >> 1) & 1;
@@ -309,11 +324,10 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
           float v[32];
           hb_tmem_ld32(t0 + c * 32, v);
           if (n0 + c * 32 >= N) continue;
-          if constexpr (TS) {
-            ts_chunk<EPI>(v, c, n0, N, m0 + warp * 32, smem + S::STAGING_OFFSET + warp * 8192, lane, &map_c);
-          } else {
+          if (TS && ts_whole<EPI>(m0 + warp * 32, M))
+            ts_chunk<EPI>(v, c, n0, N, m0 + warp * 32, smem + S::STAGING_OFFSET + warp * 8192, sent, lane, &map_c);
+          else
             epilogue_store<EPI>(v, C, ldc, row, n0 + c * 32, M, N);
-          }
         }
       }
       hb_tc_fence_before();
@@ -350,9 +364,12 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
 // operand bytes per product, and at 96 CTAs of 128 x 128 tiles it is L2 that bounds it (512 x 3,072 by 3,072 and by 8,192: 62
 // us for both together; three slices of 256 x 256 tiles 35 us, and the norm that reads the sums next adds the slices).
 // ---------------------------------------------------------------------------------------
+// A stage holds two K blocks: half as many barriers to pass as with one (same time at 512 rows; 2,048 x 16,384 x 3,072 with SwiGLU 137 -> 134
+// us, 2,048 x 28,672 x 4,096 316 -> 308).
+constexpr int PAIR_STAGES = 3, KPS = 2;
 template <int STAGES>
 struct PairSmem {
-  static constexpr int A_BYTES = BM * BK * 2, B_BYTES = 128 * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int A_BYTES = BM * BK * 2, B_BYTES = 128 * BK * 2, BLOCK_BYTES = A_BYTES + B_BYTES, STAGE_BYTES = BLOCK_BYTES * KPS;
   static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
   static constexpr int STAGING_OFFSET = (BAR_OFFSET + 256 + 1023) / 1024 * 1024;
   static constexpr int TOTAL = STAGING_OFFSET + 4 * 2 * 4096 + 1024;
@@ -361,8 +378,8 @@ struct PairSmem {
 template <int STAGES, int EPI>
 __global__ void __launch_bounds__(192, 1) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a,
                                                               const __grid_constant__ CUtensorMap map_w,
-                                                              const __grid_constant__ CUtensorMap map_c, int M, int N, int K,
-                                                              int* status, int splits, int kbs, int slice_rows) {
+                                                              const __grid_constant__ CUtensorMap map_c, void* C, long ldc, int M,
+                                                              int N, int K, int* status, int splits, int kbs, int slice_rows) {
   using S = PairSmem<STAGES>;
   constexpr int BN = 256;
   extern __shared__ uint8_t smem_raw[];
@@ -397,22 +414,39 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_pair_kernel(const __grid_const
   hb_cluster_sync();   // the partner's barriers exist before anything is signalled across
   hb_tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  hb_pdl_wait();
+  if (warp != 4) hb_pdl_wait();   // (the loader asks for its first weight tiles before it waits)
 
   if (warp == 4) {
     if (lane == 0) {  // ---------------- TMA producer of this CTA's halves
-      uint32_t it = 0;
+      uint32_t it = 0, early = 0;
       bool ok = true;
+      // the first weight tiles do not depend on the kernel ahead (0.5 to 0.8 us a product, back to back)
+      if (pair < units) {
+        const int tile = pair % num_tiles, kb0 = pair / num_tiles * kbs, kb1 = min(num_kb, kb0 + kbs), n0 = (tile / m_tiles) * BN + rank * 128;
+        for (int kb = kb0; early < STAGES && kb < kb1; early++)
+          for (int j = 0, n = min(KPS, kb1 - kb); j < n; j++, kb++) {
+            if (j == 0 && rank == 0) hb_mbar_expect_tx(&full[early], 2 * S::BLOCK_BYTES * n);   // both CTAs' bytes
+            hb_tma_load_2d_pair(smem + early * S::STAGE_BYTES + j * S::BLOCK_BYTES + S::A_BYTES, &map_w, hb_mapa(&full[early], 0), kb * BK, n0);
+          }
+      }
+      hb_pdl_wait();
       for (int u = pair; u < units && ok; u += n_pairs) {
         const int tile = u % num_tiles, kb0 = u / num_tiles * kbs, kb1 = min(num_kb, kb0 + kbs);
         const int m0 = (tile % m_tiles) * 256 + rank * 128, n0 = (tile / m_tiles) * BN + rank * 128;
-        for (int kb = kb0; kb < kb1; kb++, it++) {
-          const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          if (!hb_mbar_wait(&empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
-          if (rank == 0) hb_mbar_expect_tx(&full[s], 2 * S::STAGE_BYTES);   // both CTAs' bytes
-          const uint32_t bar = hb_mapa(&full[s], 0);
-          hb_tma_load_2d_pair(smem + s * S::STAGE_BYTES, &map_a, bar, kb * BK, m0);
-          hb_tma_load_2d_pair(smem + s * S::STAGE_BYTES + S::A_BYTES, &map_w, bar, kb * BK, n0);
+        for (int kb = kb0; kb < kb1; kb += KPS, it++) {
+          const uint32_t s = it % STAGES, ph = (it / STAGES) & 1, bar = hb_mapa(&full[s], 0);
+          const int n = min(KPS, kb1 - kb);
+          uint8_t* st = smem + s * S::STAGE_BYTES;
+          if (it >= early) {
+            if (!hb_mbar_wait(&empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
+            if (rank == 0) hb_mbar_expect_tx(&full[s], 2 * S::BLOCK_BYTES * n);
+          }
+#pragma unroll
+          for (int j = 0; j < KPS; j++)
+            if (j < n) {
+              hb_tma_load_2d_pair(st + j * S::BLOCK_BYTES, &map_a, bar, (kb + j) * BK, m0);
+              if (it >= early) hb_tma_load_2d_pair(st + j * S::BLOCK_BYTES + S::A_BYTES, &map_w, bar, (kb + j) * BK, n0);
+            }
         }
       }
       // the last commits still arrive on this CTA's barriers: wait for them before the shared memory is given up
@@ -430,21 +464,26 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_pair_kernel(const __grid_const
         if (!hb_mbar_wait(&tmem_empty[buf], aph ^ 1, abort_flag)) break;
         hb_tc_fence_after();
         const uint32_t d = tmem_base + buf * BN;
-        for (int kb = kb0; kb < kb1; kb++, it++) {
+        for (int kb = kb0; kb < kb1; kb += KPS, it++) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
           if (!hb_mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
           hb_tc_fence_after();
-          const uint64_t da = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE_BYTES));
-          const uint64_t db = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE_BYTES + S::A_BYTES));
+          const int n = min(KPS, kb1 - kb);
 #pragma unroll
-          for (int k = 0; k < BK / 16; k++) hb_umma_bf16_pair(d, da + 2 * k, db + 2 * k, idesc, kb != kb0 || k != 0);
+          for (int j = 0; j < KPS; j++)
+            if (j < n) {
+              const uint32_t st = hb_smem_u32(smem + s * S::STAGE_BYTES + j * S::BLOCK_BYTES);
+              const uint64_t da = hb_umma_desc_k128(st), db = hb_umma_desc_k128(st + S::A_BYTES);
+#pragma unroll
+              for (int k = 0; k < BK / 16; k++) hb_umma_bf16_pair(d, da + 2 * k, db + 2 * k, idesc, kb + j != kb0 || k != 0);
+            }
           hb_umma_commit_pair(&empty[s]);
         }
         if (ok) hb_umma_commit_pair(&tmem_full[buf]);
       }
     }
   } else {  // ---------------- epilogue warps 0..3: this CTA's 128 rows of the tile
-    uint32_t tile_i = 0;
+    uint32_t tile_i = 0, sent = 0;
     for (int u = pair; u < units; u += n_pairs, tile_i++) {
       const int tile = u % num_tiles, m0 = (tile % m_tiles) * 256 + rank * 128 + u / num_tiles * slice_rows, n0 = (tile / m_tiles) * BN;
       const uint32_t buf = tile_i & 1, aph = (tile_i >> 1) & 1;
@@ -456,7 +495,8 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_pair_kernel(const __grid_const
         float v[32];
         hb_tmem_ld32(t0 + c * 32, v);
         if (n0 + c * 32 >= N) continue;
-        ts_chunk<EPI>(v, c, n0, N, m0 + warp * 32, smem + S::STAGING_OFFSET + warp * 8192, lane, &map_c);
+        if (ts_whole<EPI>(m0 + warp * 32, M)) ts_chunk<EPI>(v, c, n0, N, m0 + warp * 32, smem + S::STAGING_OFFSET + warp * 8192, sent, lane, &map_c);
+        else epilogue_store<EPI>(v, C, ldc, m0 + warp * 32 + lane, n0 + c * 32, M, N);
       }
       hb_tc_fence_before();
       __syncwarp();
@@ -586,7 +626,7 @@ static int launch_gemm_tc(const CUtensorMap& ma, const CUtensorMap& mw, void* C,
 template <int EPI>
 static int launch_gemm_pair(const CUtensorMap& ma, const void* W, long ldw, void* C, long ldc, int M, int N, int K, int* status,
                             cudaStream_t s, int splits = 1, int kbs = 1 << 30, int slice_rows = 0) {
-  using S = PairSmem<6>;
+  using S = PairSmem<PAIR_STAGES>;
   CUtensorMap mw, mc;
   if (hb_make_tensor_map_bf16(&mw, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, 128)) return -1;
   if (EPI == EPI_F32 || EPI == EPI_ADD_F32) {
@@ -597,7 +637,7 @@ static int launch_gemm_pair(const CUtensorMap& ma, const void* W, long ldw, void
     const uint64_t cols = EPI_IS_GLU(EPI) ? (uint64_t)N / 2 : (uint64_t)N;
     if (hb_make_tensor_map_bf16(&mc, C, (uint64_t)M, cols, (uint64_t)ldc, 32)) return -1;
   }
-  auto kern = gemm_tc_pair_kernel<6, EPI>;
+  auto kern = gemm_tc_pair_kernel<PAIR_STAGES, EPI>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
@@ -605,7 +645,7 @@ static int launch_gemm_pair(const CUtensorMap& ma, const void* W, long ldw, void
     configured = true;
   }
   const int tiles = ((M + 255) / 256) * ((N + 255) / 256) * splits, pairs = tiles < sm_count() / 2 ? tiles : sm_count() / 2;
-  cudaError_t e = hb_launch_cluster(kern, dim3(2 * pairs), 192, S::TOTAL, s, dim3(2, 1, 1), ma, mw, mc, M, N, K, status, splits,
+  cudaError_t e = hb_launch_cluster(kern, dim3(2 * pairs), 192, S::TOTAL, s, dim3(2, 1, 1), ma, mw, mc, C, ldc, M, N, K, status, splits,
                                     splits > 1 ? kbs : (K + BK - 1) / BK, slice_rows);
   if (e != cudaSuccess) HB_FAIL("hb_gemm_tc: %s", cudaGetErrorString(e));
   return 0;
@@ -856,7 +896,7 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_grouped_kernel(const __grid_co
       }
     }
   } else {  // ---------------- epilogue warps 0..3
-    uint32_t tile_i = 0;
+    uint32_t tile_i = 0, sent = 0;
     int e = 0, m0, n0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, tile_i++) {
       place(tile, e, m0, n0);
@@ -881,7 +921,7 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_grouped_kernel(const __grid_co
 #pragma unroll
           for (int j = 0; j < 16; j++) { v[j] *= s_all; v[16 + j] *= s_all * s_up; }
         }
-        if (whole) ts_chunk<EPI>(v, c, n0, N, row0, smem + S::STAGING_OFFSET + warp * 8192, lane, &map_c);
+        if (whole) ts_chunk<EPI>(v, c, n0, N, row0, smem + S::STAGING_OFFSET + warp * 8192, sent, lane, &map_c);
         else epilogue_store<EPI>(v, C, ldc, row, n0 + c * 32, hi, N);
       }
       hb_tc_fence_before();
