@@ -1,29 +1,39 @@
 // Causal flash attention of prompt portions on the 5th-generation tensor cores (head_dim 64 or 128).
 //
-// One CTA = 128 consecutive query rows of one request and one query head; it walks the
-// request's keys in tiles of 128 ABSOLUTE positions. Six warps:
-//   warp 4 (one thread)  TMA: the Q tile once, then per tile the K pages and the V pages, each
-//                        page one box of the cache's tensor map (128-byte swizzle, no multicast);
-//   warp 5 (one thread)  tcgen05.mma: S = Q K^T into tensor memory, and, once the softmax
-//                        warps have written P, O_tile = P V (V is read as an MN-major operand
-//                        straight from its [key][d] page layout);
-//   warps 0-3            softmax: a thread owns one query ROW: it reads its row of S from
-//                        tensor memory (no shuffles for max or sum), masks on absolute positions,
-//                        exponentiates in the exp2 domain in fp32, writes P as bf16 into shared
-//                        memory in the swizzled K-major layout the tensor core reads. The output
-//                        row stays in tensor memory over all the tiles (the products accumulate);
-//                        it is in units of 2^m, where m follows the row's maximum lazily: only a
-//                        maximum that exceeds m by more than 8 raises it, and only then is the row
-//                        read, rescaled and written back.
-// K and V are double-buffered in shared memory, S and P single. A CTA takes 256 columns of tensor
-// memory (S 128, O head_dim), 113 KB of shared memory at head_dim 64 and 114 registers a thread (a
-// row of S is read in two halves of 64, the first one twice: once for the maximum, once for the
-// exponentials), so that TWO CTAs share an SM: while the softmax of one keeps the
-// special-function unit busy, the other stores P or waits for the
-// tensor core. Because tiles are cut at absolute
-// positions and a row's running max and sum are its own, a row's result does not depend on how
-// the prompt was cut or on what else is in the batch. Replaces flash_prefill_mma_kernel of the
-// reference (src/kernels.cuh:1335-1482). Every wait is bounded.
+// Persistent CTAs walk items: 128 consecutive query rows of one request and one query head, over the request's keys in tiles of 128
+// ABSOLUTE positions. Every CTA lists the step's (request, query tile) pairs by falling work and takes items in turn; requests of
+// few rows cost nothing (a grid over all requests and query tiles spent 130 us on CTAs that only left, beside 60 decoding rows). Roles:
+//   softmax warps        a thread owns one query ROW: it reads its row of S from tensor memory (no shuffles for max or sum),
+//                        masks on absolute positions, exponentiates in the exp2 domain in fp32, and writes P as bf16 into shared
+//                        memory in the swizzled K-major layout the tensor core reads. The output row stays in tensor memory over all
+//                        the tiles (the products accumulate); it is in units of 2^m, where m follows the row's maximum
+//                        lazily: only a maximum that exceeds m by more than 8 raises it, and only then is the row read, rescaled and
+//                        written back;
+//   a warp each for Q and K, and for V:  TMA through a ring of their own; a page is one box of the cache's tensor map (128-byte
+//                        swizzle, no multicast), a lane holds its number, asked for a tile ahead;
+//   MMA warps            tcgen05.mma: S = Q K^T into tensor memory one tile ahead, and, once P is written, O += P V (V is read as
+//                        an MN-major operand straight from its [key][d] page layout).
+// Because tiles are cut at absolute positions and a row's running max and sum are its own, a row's result does not depend on how the
+// prompt was cut or on what else is in the batch. Replaces flash_prefill_mma_kernel of the reference (src/kernels.cuh:1335-1482).
+// Every wait is bounded.
+//
+// head_dim 128 (flash_prefill_tc_kernel): a CTA an SM, and an item's tiles go to TWO chains by the parity of their absolute number: each
+// chain has a softmax warpgroup, an MMA warp, scores, probabilities, running maximum, sum and output accumulator of its own, and the
+// two are joined at the item's end. The softmax of one chain runs while the other waits for the tensor cores, and an item takes half
+// as long where there are fewer items than SMs. Both warpgroups read both accumulators, each half of the columns, and write
+// (O_even 2^(m_even - m) + O_odd 2^(m_odd - m)) / l. (One MMA warp for both chains was the bound: it stands in the queue while
+// an MMA of 64 to 80 cycles runs, and its waits came on top, 2,300 cycles a tile.)
+// head_dim 64 (flash_prefill_tc64_kernel): items are short beside their ends, so two CTAs of one chain share an SM, each within
+// 113 KB of shared memory, 256 columns of tensor memory and 128 registers (a row of S is read in two halves of 64, the first one twice:
+// once for the maximum, once for the exponentials).
+//
+// What bounds it: the softmax warps, some 2,500 cycles a tile of a chain alone, 1,024 of them exponentials (16 a cycle an SM, so two chains
+// cannot fall below 1,024 cycles a tile; the MMAs take 900 to 1,250). Measured against its forerunner (a CTA per query tile of a grid over
+// all requests, one chain, MMAs issued behind "lane == 0", page numbers loaded when they were needed), us: 32 heads over 8 of 128, 2,048
+// rows 74.7 -> 51.2, behind 2,048 more 182 -> 113 (910 TFLOP/s); 24 heads of 128, 512 rows behind 1,536 34.9 -> 22.9; 32 heads over 8 of
+// 64, 2,048 rows 40.7 -> 39.6, four portions of 512 23.9 -> 20.4, 1,988 rows beside 60 decoding requests 173 -> 39.7. At head_dim 64 the
+// two-chain form was slower (45 us at 2,048 rows: an item of 8.5 tiles spends a third of its time at its ends), and so was one that
+// joined the chains later, behind the next item's first tile (49 us).
 //
 // EX: a distance bias, r1 ln(1 + r2 (i - j)) off the score of query i and key j (r1, r2 >= 0, a number per head), and a
 // sink, exp(sink) in the denominator (a number per head). The bias grows with the distance, so the unbiased maximum of a
@@ -34,6 +44,8 @@
 
 constexpr int FT_BM = 128, FT_BN = 128;
 constexpr int FT_TILE = 128 * 64 * 2;  // one [128][64] bf16 tile: 16 KB; a [128][head_dim] operand is head_dim / 64 of them, 64 columns each
+constexpr int FT_THREADS = 384;        // 168 registers each: a row of S is 128 of them
+constexpr int FT_MAX_ENTRIES = 640, FT_MAX_ENTRIES64 = 200;    // (request, query tile) pairs of one launch; the launcher cuts larger steps
 
 // MN-major operand with the 128-byte swizzle: 64 contiguous elements of the MN dimension per row,
 // eight K rows per 1,024-byte group (stride SBO); further MN atoms would lie LBO apart (one here).
@@ -44,287 +56,684 @@ __device__ __forceinline__ uint64_t ft_desc_mn128(uint32_t smem_addr) {
 // kind::f16 instruction descriptor as hb_umma_idesc_bf16, with B read MN-major.
 __host__ __device__ constexpr uint32_t ft_idesc_b_mn(int M, int N) { return hb_umma_idesc_bf16(M, N) | (1u << 16); }
 
+__device__ __forceinline__ uint64_t ft_pack2(uint32_t lo, uint32_t hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+  return r;
+}
+__device__ __forceinline__ void ft_unpack2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t ft_fma2(uint64_t a, uint64_t b, uint64_t c) {   // two fmaf, each rounded by itself
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t ft_add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 
+// 32 columns of this thread's lane, not waited for (see hb_tmem_ld64_nowait), and back.
+__device__ __forceinline__ void ft_ld32(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]) : "r"(taddr));
+}
+__device__ __forceinline__ void ft_ld32_fence(uint32_t* r) { asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31]) :: "memory"); }
+__device__ __forceinline__ void ft_st32(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
+}
+
+// head_dim 128: Q, P of both chains, rings of two K and two V tiles, and the list of the items.
 struct FtBars {
-  uint64_t q_full, k_full[2], k_free[2], v_full[2], v_free[2], s_full, s_free, o_full, p_full, p_free;
+  uint64_t q_full, q_free, k_full[2], k_free[2], v_full[2], v_free[2], s_full[2], s_free[2], p_full[2], pv_done[2];
+  uint32_t entries[FT_MAX_ENTRIES];  // request << 16 | query tile, by falling work
+  int n_entries;
   uint32_t tmem_slot;
   int abort_flag;
 };
+constexpr int FT_SMEM = 14 * FT_TILE + (int)sizeof(FtBars);
+// head_dim 64: Q, P, rings of two K and two V tiles.
+struct FtBars64 {
+  uint64_t q_full, q_free, k_full[2], k_free[2], v_full[2], v_free[2], s_full, s_free, p_full, pv_done;
+  uint32_t entries[FT_MAX_ENTRIES64];
+  int n_entries;
+  uint32_t tmem_slot;
+  int abort_flag;
+};
+constexpr int FT_SMEM64 = 7 * FT_TILE + (int)sizeof(FtBars64);
+static_assert(FT_SMEM <= 227 * 1024 && 2 * (FT_SMEM64 + 1024) <= 228 * 1024, "shared memory of one block and of two");
 
-// Buffers that alternate tile by tile: index i & 1, phase (i >> 1) & 1.
-#define FT_B(i) ((i) & 1)
-#define FT_PH(i) (((i) >> 1) & 1)
+// Item k of this CTA: CTAs take the items in turn, back and forth (the items come by falling work).
+__device__ __forceinline__ int ft_item(int k) { return k * (int)gridDim.x + ((k & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x); }
 
-// head_dim 128: operands of two 64-column tiles each, the output tile 128 columns wide (192 KB of
-// shared memory: one CTA per SM).
-template <int FT_D, bool EX>
-__global__ void __launch_bounds__(FT_D == 64 ? 256 : 192, FT_D == 64 ? 2 : 1) flash_prefill_tc_kernel(
+// (first row, rows, position of the first row, request) of a (request, query tile) pair.
+__device__ __forceinline__ int4 ft_entry(uint32_t e, const int* q_start, const int* q_len, const int* ctx_len) {
+  const int r = e >> 16, row = (int)(e & 0xffffu) * FT_BM;
+  return make_int4(q_start[r] + row, min(FT_BM, q_len[r] - row), ctx_len[r] + row, r);
+}
+// Key tiles of an item: the first and how many.
+struct FtSpan { int kt_lo, n, lo, p_last; };
+__device__ __forceinline__ FtSpan ft_span(const int4& e, int window) {
+  FtSpan s;
+  s.p_last = e.z + e.y - 1;
+  s.lo = window > 0 ? max(0, e.z - window + 1) : 0;
+  s.kt_lo = s.lo / FT_BN;
+  s.n = s.p_last / FT_BN - s.kt_lo + 1;
+  return s;
+}
+
+// One warp: the (request, query tile) pairs of this launch and their key tiles, unordered.
+__device__ __forceinline__ void ft_list(uint2* raw, int* n_entries, int most, const int* q_len, const int* ctx_len, int window, int min_rows,
+                                        int req0, int reqs, int qt0, int qts) {
+  const int lane = threadIdx.x & 31;
+  int n = 0;
+  for (int base = 0; base < reqs; base += 32) {
+    const int r = req0 + base + lane;
+    int len = base + lane < reqs ? q_len[r] : 0;
+    if (len < min_rows) len = 0;
+    const int tiles = max(0, min((len + FT_BM - 1) / FT_BM - qt0, qts));
+    int at = tiles;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, at, o);
+      if (lane >= o) at += v;
+    }
+    const int total = __shfl_sync(0xffffffffu, at, 31);
+    at += n - tiles;
+    if (tiles) {
+      const int ctx = ctx_len[r];
+      for (int t = 0; t < tiles && at + t < most; t++) {
+        const int row = (qt0 + t) * FT_BM;
+        raw[at + t] = make_uint2((uint32_t)r << 16 | (uint32_t)(qt0 + t), ft_span(make_int4(0, min(FT_BM, len - row), ctx + row, r), window).n);
+      }
+    }
+    n += total;
+  }
+  if (lane == 0) *n_entries = min(n, most);
+}
+// All threads: the pairs by falling work; a pair's place is the number of pairs with more key tiles to walk.
+__device__ __forceinline__ void ft_sort(const uint2* raw, uint32_t* entries, int n_entries) {
+  for (int i = threadIdx.x; i < n_entries; i += blockDim.x) {
+    const uint2 e = raw[i];
+    int place = 0;
+    for (int j = 0; j < n_entries; j++) {
+      const uint32_t w = raw[j].y;
+      place += w > e.y || (w == e.y && j < i);
+    }
+    entries[place] = e.x;
+  }
+}
+// The loader of K or V: a warp brings the tiles of an item, page by page, through a ring of two; lane l holds page l of the tile.
+template <int FT_D>
+__device__ __forceinline__ bool ft_bring(const FtSpan& sp, const int* table, int page_size, int Hkv, int h, const CUtensorMap* map, uint8_t* ring,
+                                         uint64_t* full, uint64_t* free, uint32_t& it, volatile int* abort_flag) {
+  constexpr int NH = FT_D / 64, OPND = NH * FT_TILE;
+  const int lane = threadIdx.x & 31, last = sp.p_last / page_size;       // the item's last page
+  // the page of this lane in tile t, asked for one tile ahead
+  auto page = [&](int t) {
+    const int pg = max((sp.kt_lo + t) * FT_BN, sp.lo) / page_size + lane;
+    return lane < FT_BN / page_size && pg <= last ? table[pg] : 0;
+  };
+  int next = page(0);
+  for (int t = 0; t < sp.n; t++, it++) {
+    const uint32_t s = it & 1, ph = (it >> 1) & 1;
+    const int k_base = (sp.kt_lo + t) * FT_BN;
+    const int first_page = max(k_base, sp.lo) / page_size, np = min((k_base + FT_BN - 1) / page_size, last) - first_page + 1;
+    const int row = (next * Hkv + h) * page_size;
+    next = t + 1 < sp.n ? page(t + 1) : 0;
+    if (!__all_sync(0xffffffffu, hb_mbar_wait(&free[s], ph ^ 1, abort_flag))) return false;
+    uint8_t* dst = ring + s * OPND + (first_page * page_size - k_base) * 128;   // rows of 128 bytes in each 64-column tile
+    if (hb_elect()) hb_mbar_expect_tx(&full[s], (uint32_t)np * page_size * FT_D * 2);
+    __syncwarp();
+    for (int p = 0; p < np; p++, dst += page_size * 128) {
+      const int from = __shfl_sync(0xffffffffu, row, p);
+      if (hb_elect()) {
+#pragma unroll
+        for (int hf = 0; hf < NH; hf++) hb_tma_load_2d(dst + hf * FT_TILE, map, &full[s], hf * 64, from);
+      }
+    }
+  }
+  return true;
+}
+// The exponentials of two scores, rounded to bf16 for P and added to the row's sums.
+template <bool EX>
+__device__ __forceinline__ uint32_t ft_prob(uint32_t s0, uint32_t s1, uint64_t scale2, uint64_t sub2, float r1, float r2, float dist, uint64_t& sum2) {
+  float e0, e1;
+  ft_unpack2(ft_fma2(ft_pack2(s0, s1), scale2, sub2), e0, e1);
+  if (EX) {   // (a key behind the row is masked: any finite bias will do)
+    e0 = fmaf(-r1, __log2f(fmaxf(fmaf(r2, dist, 1.f), 1.f)), e0);
+    e1 = fmaf(-r1, __log2f(fmaxf(fmaf(r2, dist - 1.f, 1.f), 1.f)), e1);
+  }
+  const float p0 = hb_exp2(e0), p1 = hb_exp2(e1);
+  sum2 = ft_add2(sum2, ft_pack2(__float_as_uint(p0), __float_as_uint(p1)));
+  return hb_pack_bf16(p0, p1);
+}
+// m_run follows the row's maximum lazily: it is raised (and the row of O rescaled) only when a tile's maximum exceeds it by
+// more than FT_SLACK, so P <= 2^FT_SLACK; the sum l_run is in the same units, and O / l_run is exact whichever maxima were used.
+constexpr float FT_SLACK = 8.f;
+
+template <bool EX>
+__global__ void __launch_bounds__(FT_THREADS, 1) flash_prefill_tc_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, const int* __restrict__ bt, int bt_stride, const int* __restrict__ q_start,
     const int* __restrict__ q_len, const int* __restrict__ ctx_len, __nv_bfloat16* __restrict__ out, int Hq, int Hkv,
     int page_size, int window, float scale_log2, int min_rows, int* status, const float* __restrict__ r1p,
-    const float* __restrict__ r2p, const float* __restrict__ sink) {
-  // the 128-byte swizzle wants the tiles on 1 KB boundaries; with no room for slack (two CTAs an SM) the
-  // dynamic shared memory itself has to start on one, which is checked below
+    const float* __restrict__ r2p, const float* __restrict__ sink, int req0, int reqs, int qt0, int qts) {
+  constexpr int FT_D = 128, NH = FT_D / 64, OPND = NH * FT_TILE;
+  // the 128-byte swizzle wants the tiles on 1 KB boundaries, and there is no room for slack: checked below
   extern __shared__ __align__(1024) uint8_t smem[];
-  constexpr int NH = FT_D / 64, OPND = NH * FT_TILE;   // 64-column tiles and bytes of a [128][head_dim] operand
-  uint8_t* sQ = smem;                  // [128][head_dim]
-  uint8_t* sK = sQ + OPND;             // two stages of [128 keys][head_dim]
-  uint8_t* sV = sK + 2 * OPND;         // two stages of [128 keys][head_dim]
-  uint8_t* sP = sV + 2 * OPND;         // two K blocks of [128 rows][64 keys]
-  FtBars* bar = (FtBars*)(sP + 2 * FT_TILE);
+  uint8_t* sQ = smem;                      // [128][head_dim]
+  uint8_t* sP = sQ + OPND;                 // per chain two K blocks of [128 rows][64 keys]
+  uint8_t* sK = sP + 4 * FT_TILE;          // two stages of [128 keys][head_dim]
+  uint8_t* sV = sK + 2 * OPND;             // and two more
+  FtBars* bar = (FtBars*)(sV + 2 * OPND);
   volatile int* abort_flag = &bar->abort_flag;
 
-  // the last query tiles of a portion have the most keys to walk: they are started first
-  // blocks start in the order of blockIdx.x, then y: all heads' heaviest query tile first, then the next one
-  // (longest work first: with the query tile fastest, the last head's heaviest tile would start last and run alone)
-  const int req = blockIdx.z, hq = blockIdx.x, qt = gridDim.y - 1 - blockIdx.y;
   // the step's own metadata (lengths, tables) was copied before the step's first kernel began; everything else
   // that an earlier kernel wrote is read after hb_pdl_wait() below
   hb_pdl_launch();
-  const int n_rows = q_len[req];
-  if (n_rows < min_rows || qt * FT_BM >= n_rows) {
-    if ((blockIdx.x | blockIdx.y | blockIdx.z) == 0) hb_pdl_wait();   // the grid never ends before the one ahead of it
-    return;
-  }
   if (hb_smem_u32(smem) & 1023) {   // never seen; the tiles would not be where the tensor core expects them
     if (threadIdx.x == 0) atomicExch(status, 1);
+    hb_pdl_wait();
     return;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = hq / (Hq / Hkv);
-  const int row0 = q_start[req] + qt * FT_BM, rows_here = min(FT_BM, n_rows - qt * FT_BM);
-  const int p_first = ctx_len[req] + qt * FT_BM, p_last = p_first + rows_here - 1;
-  const int lo = window > 0 ? max(0, p_first - window + 1) : 0;
-  const int kt_lo = lo / FT_BN, kt_hi = p_last / FT_BN, n_tiles = kt_hi - kt_lo + 1;
-  const int* table = bt + (size_t)req * bt_stride;
-
-  if (threadIdx.x == 0) {
-    hb_mbar_init(&bar->q_full, 1);
+  if (warp == 0) ft_list((uint2*)sP, &bar->n_entries, FT_MAX_ENTRIES, q_len, ctx_len, window, min_rows, req0, reqs, qt0, qts);
+  if (threadIdx.x == 32) {
+    hb_mbar_init(&bar->q_full, 1); hb_mbar_init(&bar->q_free, 2);
     for (int b = 0; b < 2; b++) {
       hb_mbar_init(&bar->k_full[b], 1); hb_mbar_init(&bar->k_free[b], 1);
       hb_mbar_init(&bar->v_full[b], 1); hb_mbar_init(&bar->v_free[b], 1);
     }
-    hb_mbar_init(&bar->o_full, 1);
-    hb_mbar_init(&bar->p_full, 128); hb_mbar_init(&bar->p_free, 1);
-    hb_mbar_init(&bar->s_full, 1); hb_mbar_init(&bar->s_free, 128);
+    for (int c = 0; c < 2; c++) {
+      hb_mbar_init(&bar->s_full[c], 1); hb_mbar_init(&bar->s_free[c], 4);
+      hb_mbar_init(&bar->p_full[c], 4); hb_mbar_init(&bar->pv_done[c], 1);
+    }
     bar->abort_flag = 0;
     hb_fence_barrier_init();
   }
-  // masked keys of a last, ragged tile are never loaded: what the tensor core reads in their place
-  // must be finite (P is exactly 0 there, and 0 * NaN would poison the row)
-  for (int i = threadIdx.x; i < 4 * OPND / 16; i += 192) ((uint4*)sK)[i] = make_uint4(0, 0, 0, 0);
-  if (warp == 5) {
-    hb_tmem_alloc(&bar->tmem_slot, 256);
+  if (warp == 8 && lane == 0) { hb_tma_prefetch_desc(&map_q); hb_tma_prefetch_desc(&map_k); hb_tma_prefetch_desc(&map_v); }
+  __syncthreads();
+  const int n_entries = bar->n_entries, n_items = n_entries * Hq;
+  if ((int)blockIdx.x >= n_items) {   // the grid is made for the most items there can be
+    hb_pdl_wait();
+    return;
+  }
+  ft_sort((const uint2*)sP, bar->entries, n_entries);
+  // masked keys of a last, ragged tile are never loaded: what the tensor core reads in their place must be finite (P is exactly 0
+  // there, and 0 * NaN would poison the row). Later tiles leave finite values behind.
+  for (int i = threadIdx.x; i < 4 * OPND / 16; i += FT_THREADS) ((uint4*)sK)[i] = make_uint4(0, 0, 0, 0);
+  if (warp == 10) {
+    hb_tmem_alloc(&bar->tmem_slot, 512);
     hb_tmem_relinquish();
   }
-  if (warp == 4 && lane == 0) { hb_tma_prefetch_desc(&map_q); hb_tma_prefetch_desc(&map_k); hb_tma_prefetch_desc(&map_v); }
   hb_fence_proxy_async();
   hb_tc_fence_before();
   __syncthreads();
   hb_tc_fence_after();
-  const uint32_t tmem_s = bar->tmem_slot, tmem_o = tmem_s + FT_BN;  // S: 128 columns, O: head_dim columns
+  const uint32_t tmem = bar->tmem_slot;   // S of chain c: 128 columns at c * 128; O of chain c: head_dim columns at 256 + c * 128
   hb_pdl_wait();   // barriers, shared and tensor memory were set up while the kernel ahead was still running
 
-  if (warp == 4) {  // ---------------- TMA: lane l brings page l of the tile (the page ids come in one load)
-    if (lane == 0) {
-      hb_mbar_expect_tx(&bar->q_full, OPND);
+  // an item's numbers are fetched while the one before it is worked on
+  auto entry = [&](int k) { const int u = ft_item(k); return ft_entry(bar->entries[u < n_items ? u / Hq : 0], q_start, q_len, ctx_len); };
+
+  if (warp == 8 || warp == 9) {  // ---------------- TMA: lane l brings page l of a tile
+    const bool is_k = warp == 8;
+    const CUtensorMap* map = is_k ? &map_k : &map_v;
+    uint64_t *full = is_k ? bar->k_full : bar->v_full, *free = is_k ? bar->k_free : bar->v_free;
+    uint8_t* ring = is_k ? sK : sV;
+    uint32_t it = 0;
+    bool ok = true;
+    int4 ahead = entry(0);
+    for (int k = 0, u; (u = ft_item(k)) < n_items && ok; k++) {
+      const int4 e = ahead;
+      ahead = entry(k + 1);
+      const int hq = u % Hq, h = hq / (Hq / Hkv);
+      const FtSpan sp = ft_span(e, window);
+      if (is_k) {
+        if (!__all_sync(0xffffffffu, hb_mbar_wait(&bar->q_free, (k & 1) ^ 1, abort_flag))) break;
+        if (hb_elect()) {
+          hb_mbar_expect_tx(&bar->q_full, OPND);
 #pragma unroll
-      for (int hf = 0; hf < NH; hf++) hb_tma_load_2d(sQ + hf * FT_TILE, &map_q, &bar->q_full, hq * FT_D + hf * 64, row0);
-    }
-    for (int i = 0; i < n_tiles; i++) {
-      const int k_base = (kt_lo + i) * FT_BN, b = FT_B(i);
-      const int first_page = max(k_base, lo) / page_size, last_page = min(k_base + FT_BN - 1, p_last) / page_size;
-      const int np = last_page - first_page + 1;
-      const uint32_t bytes = (uint32_t)np * page_size * FT_D * 2;
-      const int pg = first_page + lane;
-      const int row = lane < np ? (table[pg] * Hkv + h) * page_size : 0;
-      const int off = b * OPND + (pg * page_size - k_base) * 128;   // rows of 128 bytes in each 64-column tile
-      int ok = 1;
-      if (lane == 0) {
-        ok = hb_mbar_wait(&bar->k_free[b], FT_PH(i) ^ 1, abort_flag);
-        if (ok) hb_mbar_expect_tx(&bar->k_full[b], bytes);
-      }
-      if (!__shfl_sync(0xffffffffu, ok, 0)) break;
-      if (lane < np) {
-#pragma unroll
-        for (int hf = 0; hf < NH; hf++) hb_tma_load_2d(sK + off + hf * FT_TILE, &map_k, &bar->k_full[b], hf * 64, row);
-      }
-      if (lane == 0) {
-        ok = hb_mbar_wait(&bar->v_free[b], FT_PH(i) ^ 1, abort_flag);
-        if (ok) hb_mbar_expect_tx(&bar->v_full[b], bytes);
-      }
-      if (!__shfl_sync(0xffffffffu, ok, 0)) break;
-      if (lane < np) {
-#pragma unroll
-        for (int hf = 0; hf < NH; hf++) hb_tma_load_2d(sV + off + hf * FT_TILE, &map_v, &bar->v_full[b], hf * 64, row);
-      }
-    }
-  } else if (warp == 5) {
-    if (lane == 0) {  // ---------------- tensor cores: S_i is issued before O_{i-1}, so it overlaps the softmax of tile i - 1
-      constexpr uint32_t idesc_s = hb_umma_idesc_bf16(FT_BM, FT_BN), idesc_o = ft_idesc_b_mn(FT_BM, FT_D);
-      bool ok = hb_mbar_wait(&bar->q_full, 0, abort_flag);
-      for (int i = 0; i <= n_tiles && ok; i++) {
-        if (i < n_tiles) {
-          const int b = FT_B(i);
-          if (!hb_mbar_wait(&bar->k_full[b], FT_PH(i), abort_flag) || !hb_mbar_wait(&bar->s_free, (i & 1) ^ 1, abort_flag)) break;
-          hb_tc_fence_after();
-#pragma unroll
-          for (int k = 0; k < FT_D / 16; k++) {   // 16 columns a step: four steps in each 64-column tile
-            const uint64_t dq = hb_umma_desc_k128(hb_smem_u32(sQ + (k >> 2) * FT_TILE)) + 2 * (k & 3);
-            const uint64_t dk = hb_umma_desc_k128(hb_smem_u32(sK + b * OPND + (k >> 2) * FT_TILE)) + 2 * (k & 3);
-            hb_umma_bf16(tmem_s, dq, dk, idesc_s, k != 0);
-          }
-          hb_umma_commit(&bar->s_full);
-          hb_umma_commit(&bar->k_free[b]);
+          for (int hf = 0; hf < NH; hf++) hb_tma_load_2d(sQ + hf * FT_TILE, &map_q, &bar->q_full, hq * FT_D + hf * 64, e.x);
         }
-        if (i > 0) {
-          const int j = i - 1, b = FT_B(j);
-          if (!hb_mbar_wait(&bar->p_full, j & 1, abort_flag) || !hb_mbar_wait(&bar->v_full[b], FT_PH(j), abort_flag)) break;
+        __syncwarp();
+      }
+      ok = ft_bring<FT_D>(sp, bt + (size_t)e.w * bt_stride, page_size, Hkv, h, map, ring, full, free, it, abort_flag);
+    }
+  } else if (warp >= 10) {  // ---------------- tensor cores, chain c
+    constexpr uint32_t idesc_s = hb_umma_idesc_bf16(FT_BM, FT_BN), idesc_o = ft_idesc_b_mn(FT_BM, FT_D);
+    const int c = warp - 10;
+    uint32_t base = 0, ns = 0, np = 0;      // tiles of the items before; the chain's scores and products so far
+    bool ok = true;
+    int4 ahead = entry(0);
+    for (int k = 0; ft_item(k) < n_items && ok; k++) {
+      const FtSpan sp = ft_span(ahead, window);
+      ahead = entry(k + 1);
+      ok = __all_sync(0xffffffffu, hb_mbar_wait(&bar->q_full, k & 1, abort_flag));
+      const int i0 = (sp.kt_lo ^ c) & 1;
+      if (i0 >= sp.n && lane == 0) hb_mbar_arrive(&bar->q_free);      // one tile, the other chain's
+      for (int i = i0; i < sp.n + 2 && ok; i += 2) {
+        if (i < sp.n) {         // S of tile i
+          const uint32_t it = base + i, s = it & 1, ph = (it >> 1) & 1;
+          ok = hb_mbar_wait(&bar->k_full[s], ph, abort_flag) && hb_mbar_wait(&bar->s_free[c], (ns & 1) ^ 1, abort_flag);
+          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+          ns++;
           hb_tc_fence_after();
+          if (hb_elect()) {
 #pragma unroll
-          for (int k = 0; k < FT_BN / 16; k++) {
-            const uint64_t dp = hb_umma_desc_k128(hb_smem_u32(sP + (k >> 2) * FT_TILE)) + 2 * (k & 3);
-            const uint64_t dv = ft_desc_mn128(hb_smem_u32(sV + b * OPND + k * 16 * 128));   // 16 keys on; the second 64 columns lie FT_TILE further (the descriptor's leading offset)
-            hb_umma_bf16(tmem_o, dp, dv, idesc_o, j != 0 || k != 0);   // O stays in tensor memory over all the tiles
+            for (int kk = 0; kk < FT_D / 16; kk++) {   // 16 columns a step: four steps in each 64-column tile
+              const uint64_t dq = hb_umma_desc_k128(hb_smem_u32(sQ + (kk >> 2) * FT_TILE)) + 2 * (kk & 3);
+              const uint64_t dk = hb_umma_desc_k128(hb_smem_u32(sK + s * OPND + (kk >> 2) * FT_TILE)) + 2 * (kk & 3);
+              hb_umma_bf16(tmem + c * FT_BN, dq, dk, idesc_s, kk != 0);
+            }
+            hb_umma_commit(&bar->s_full[c]);
+            hb_umma_commit(&bar->k_free[s]);
+            if (i + 2 >= sp.n) hb_umma_commit(&bar->q_free);
           }
-          hb_umma_commit(&bar->o_full);
-          hb_umma_commit(&bar->v_free[b]);
-          hb_umma_commit(&bar->p_free);
+          __syncwarp();
+        }
+        if (i >= i0 + 2) {      // O of tile i - 2
+          const uint32_t it = base + i - 2, s = it & 1, ph = (it >> 1) & 1;
+          ok = hb_mbar_wait(&bar->v_full[s], ph, abort_flag) && hb_mbar_wait(&bar->p_full[c], np & 1, abort_flag);
+          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+          np++;
+          hb_tc_fence_after();
+          if (hb_elect()) {
+#pragma unroll
+            for (int kk = 0; kk < FT_BN / 16; kk++) {
+              const uint64_t dp = hb_umma_desc_k128(hb_smem_u32(sP + (2 * c + (kk >> 2)) * FT_TILE)) + 2 * (kk & 3);
+              const uint64_t dv = ft_desc_mn128(hb_smem_u32(sV + s * OPND + kk * 16 * 128));   // 16 keys on; the second 64 columns lie FT_TILE further (the descriptor's leading offset)
+              hb_umma_bf16(tmem + 256 + c * 128, dp, dv, idesc_o, i > i0 + 2 || kk != 0);      // O stays in tensor memory over the chain's tiles
+            }
+            hb_umma_commit(&bar->v_free[s]);
+            hb_umma_commit(&bar->pv_done[c]);
+          }
+          __syncwarp();
         }
       }
+      base += sp.n;
     }
-  } else {  // ---------------- softmax: thread = query row
-    const int r = warp * 32 + lane;
-    const int qp = p_first + min(r, rows_here - 1);  // rows past the portion's end are computed, never stored
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
-    // The output row accumulates in tensor memory over all the tiles, in units of 2^m_run. m_run follows the
-    // row's maximum lazily: it is raised (and the row of O rescaled, which has to wait for the product of the
-    // tile before) only when a tile's maximum exceeds it by more than FT_SLACK, so P <= 2^FT_SLACK; the sum
-    // l_run is in the same units, and O / l_run is exact whichever maxima were used.
-    constexpr float FT_SLACK = 8.f;
-    float m_run = -INFINITY, l_run = 0.f;
-    const float r1 = EX && r1p ? r1p[hq] : 0.f, r2 = EX && r1p ? r2p[hq] : 0.f;
-    bool ok = true;   // every wait's outcome is made uniform over the warp: the tensor-memory accesses below are warp-wide
-    for (int i = 0; i < n_tiles && ok; i++) {
-      const int k_base = (kt_lo + i) * FT_BN;
-      const bool need_mask = k_base + FT_BN - 1 > p_first || (window > 0 && k_base < p_last - window + 1);
-      if (!__all_sync(0xffffffffu, hb_mbar_wait(&bar->s_full, i & 1, abort_flag))) { ok = false; break; }
-      hb_tc_fence_after();
-      // the row of S in two halves of 64 keys, the first one read twice (once for the maximum, once for the
-      // exponentials): 128 registers a thread is all that lets a new CTA start beside one that is still
-      // running (see the launch bounds). A softmax warp is alone on its scheduler: four independent chains
-      // for the maximum and for the sum, and the mask only where one is needed
-      uint32_t sr[64];
-      const int hi_j = qp - k_base, lo_j = window > 0 ? qp - window - k_base : -1;  // key j of the tile is visible iff lo_j < j <= hi_j
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  } else {  // ---------------- softmax: chain c, thread = query row
+    const int c = warp >> 2, r = threadIdx.x & 127;
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t tmem_s = tmem + c * FT_BN + lane_base, tmem_o = tmem + 256 + lane_base;
+    uint32_t cnt = 0;      // this chain's tiles so far, over all items
+    bool ok = true;        // every wait's outcome is made uniform over the warp: the tensor-memory accesses below are warp-wide
+    int4 ahead = entry(0);
+    for (int k = 0, u; (u = ft_item(k)) < n_items; k++) {     // (a warp that gave up still meets the others at the item's two barriers)
+      const int4 e = ahead;
+      ahead = entry(k + 1);
+      const int hq = u % Hq;
+      const FtSpan sp = ft_span(e, window);
+      const int qp = e.z + min(r, e.y - 1);      // rows past the portion's end are computed, never stored
+      const float r1 = EX && r1p ? r1p[hq] : 0.f, r2 = EX && r1p ? r2p[hq] : 0.f;
+      float m_run = -INFINITY, l_run = 0.f;
+      const int i0 = (sp.kt_lo ^ c) & 1;         // the chain's first tile
+      for (int i = i0; i < sp.n && ok; i += 2, cnt++) {
+        const int k_base = (sp.kt_lo + i) * FT_BN;
+        const bool need_mask = k_base + FT_BN - 1 > e.z || (window > 0 && k_base < sp.p_last - window + 1);
+        if (!__all_sync(0xffffffffu, hb_mbar_wait(&bar->s_full[c], cnt & 1, abort_flag))) { ok = false; break; }
+        hb_tc_fence_after();
+        uint32_t sr[128];
 #pragma unroll
-      for (int hh = 0; hh < 2; hh++) {
-        hb_tmem_ld64_nowait(tmem_s + lane_base + hh * 64, sr);
+        for (int q = 0; q < 4; q++) ft_ld32(tmem_s + 32 * q, sr + 32 * q);
         hb_tmem_ld_wait();
-        hb_tmem_ld_fence64(sr);
+#pragma unroll
+        for (int q = 0; q < 4; q++) ft_ld32_fence(sr + 32 * q);
+        hb_tc_fence_before();
+        __syncwarp();
+        if (lane == 0) hb_mbar_arrive(&bar->s_free[c]);   // the scores of the chain's next tile may overwrite S
         if (need_mask) {
+          const int hi_j = qp - k_base, lo_j = window > 0 ? qp - window - k_base : -1;  // key j of the tile is visible iff lo_j < j <= hi_j
 #pragma unroll
-          for (int j = 0; j < 64; j++) {
-            const float v = (j + hh * 64 <= hi_j && j + hh * 64 > lo_j) ? __uint_as_float(sr[j]) : -INFINITY;
-            sr[j] = __float_as_uint(v);
-            mx4[j & 3] = fmaxf(mx4[j & 3], v);
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 64; j++) mx4[j & 3] = fmaxf(mx4[j & 3], __uint_as_float(sr[j]));
+          for (int j = 0; j < 128; j++)
+            if (!(j <= hi_j && j > lo_j)) sr[j] = __float_as_uint(-INFINITY);
         }
-      }
-      float m_tile = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
-      const float dist0 = (float)(qp - k_base);                     // of the tile's first key
-      if (EX) m_tile -= r1 * __log2f(fmaf(r2, fmaxf(dist0 - (FT_BN - 1), 0.f), 1.f));
-      const bool grow = m_tile > m_run + FT_SLACK;   // also the first tile with a visible key: m_run is -inf
-      float corr = 1.f;
-      if (grow) {
-        corr = hb_exp2(m_run - m_tile);   // 0 while nothing has been summed
-        m_run = m_tile;
-      }
-      const float sub = m_run == -INFINITY ? 0.f : m_run;
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-      // the exponentials: keys 64-127 are still in the registers (masked), keys 0-63 are read again
+        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int hh = 1; hh >= 0; hh--) {
-        if (hh == 0) {
-          hb_tmem_ld64_nowait(tmem_s + lane_base, sr);
-          hb_tmem_ld_wait();
-          hb_tmem_ld_fence64(sr);
-          hb_tc_fence_before();
-          hb_mbar_arrive(&bar->s_free);  // the last read of S: the scores of the next tile may overwrite it
-          if (need_mask) {
-#pragma unroll
-            for (int j = 0; j < 64; j++)
-              if (!(j <= hi_j && j > lo_j)) sr[j] = __float_as_uint(-INFINITY);
-          }
+        for (int j = 0; j < 128; j += 2) mx[(j >> 1) & 3] = fmaxf(fmaxf(mx[(j >> 1) & 3], __uint_as_float(sr[j])), __uint_as_float(sr[j + 1]));
+        float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2;
+        const float dist0 = (float)(qp - k_base);                     // of the tile's first key
+        if (EX) m_tile -= r1 * __log2f(fmaf(r2, fmaxf(dist0 - (FT_BN - 1), 0.f), 1.f));
+        const bool grow = m_tile > m_run + FT_SLACK;   // also the first tile with a visible key: m_run is -inf
+        float corr = 1.f;
+        if (grow) {
+          corr = hb_exp2(m_run - m_tile);   // 0 while nothing has been summed
+          m_run = m_tile;
         }
+        const float sub = m_run == -INFINITY ? 0.f : m_run;
+        const uint64_t scale2 = ft_pack2(__float_as_uint(scale_log2), __float_as_uint(scale_log2)), sub2 = ft_pack2(__float_as_uint(-sub), __float_as_uint(-sub));
+        uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
-        for (int j = 0; j < 64; j += 2) {  // masked scores are -inf: 2^-inf = 0
-          float e0 = fmaf(__uint_as_float(sr[j]), scale_log2, -sub), e1 = fmaf(__uint_as_float(sr[j + 1]), scale_log2, -sub);
-          if (EX) {   // (a key behind the row is masked: any finite bias will do)
-            e0 = fmaf(-r1, __log2f(fmaxf(fmaf(r2, dist0 - (float)(j + hh * 64), 1.f), 1.f)), e0);
-            e1 = fmaf(-r1, __log2f(fmaxf(fmaf(r2, dist0 - (float)(j + 1 + hh * 64), 1.f), 1.f)), e1);
-          }
-          const float p0 = hb_exp2(e0), p1 = hb_exp2(e1);
-          sum4[(j >> 1) & 3] += p0 + p1;
-          sr[j >> 1] = hb_pack_bf16(p0, p1);
-        }
-        if (hh == 1) {
-          if (!__all_sync(0xffffffffu, hb_mbar_wait(&bar->p_free, (i & 1) ^ 1, abort_flag))) { ok = false; break; }
-        }
-        // 64 keys = eight 16-byte chunks of this row in K block hh of P
+        for (int j = 0; j < 128; j += 2)   // masked scores are -inf: 2^-inf = 0
+          sr[j >> 1] = ft_prob<EX>(sr[j], sr[j + 1], scale2, sub2, r1, r2, dist0 - (float)j, sum2[(j >> 1) & 3]);
+        float s0, s1;
+        ft_unpack2(ft_add2(ft_add2(sum2[0], sum2[1]), ft_add2(sum2[2], sum2[3])), s0, s1);
+        l_run = l_run * corr + (s0 + s1);
+        // the chain's product before this one has read its P and written its O
+        if (cnt > 0 && !__all_sync(0xffffffffu, hb_mbar_wait(&bar->pv_done[c], (cnt - 1) & 1, abort_flag))) { ok = false; break; }
+        // the row: eight 16-byte chunks in each of the two K blocks of P
 #pragma unroll
-        for (int cc = 0; cc < 8; cc++) {
-          const uint32_t dst = hb_smem_u32(sP + hh * FT_TILE) + r * 128 + ((cc ^ (r & 7)) << 4);
+        for (int cc = 0; cc < 16; cc++) {
+          const uint32_t dst = hb_smem_u32(sP + (2 * c + (cc >> 3)) * FT_TILE) + r * 128 + (((cc & 7) ^ (r & 7)) << 4);
           asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(sr[4 * cc]), "r"(sr[4 * cc + 1]),
                        "r"(sr[4 * cc + 2]), "r"(sr[4 * cc + 3]) : "memory");
         }
-      }
-      if (!ok) break;
-      l_run = l_run * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
-      // a raised maximum: the rows of O so far, which the product of the tile before has to have finished writing
-      // (it is the only one that can still be running: the scores of this tile were committed after the one before it)
-      if (i > 0 && __any_sync(0xffffffffu, grow)) {
-        if (!__all_sync(0xffffffffu, hb_mbar_wait(&bar->o_full, (i - 1) & 1, abort_flag))) { ok = false; break; }
-        hb_tc_fence_after();
+        if (i > i0 && __any_sync(0xffffffffu, grow)) {   // a raised maximum: the chain's rows of O so far
+          hb_tc_fence_after();
 #pragma unroll
-        for (int hf = 0; hf < NH; hf++) {
-          hb_tmem_ld64_nowait(tmem_o + hf * 64 + lane_base, sr);
+          for (int q = 0; q < FT_D / 32; q++) {
+            uint32_t o[32];
+            ft_ld32(tmem_o + c * 128 + q * 32, o);
+            hb_tmem_ld_wait();
+            ft_ld32_fence(o);
+#pragma unroll
+            for (int d = 0; d < 32; d++) o[d] = __float_as_uint(__uint_as_float(o[d]) * corr);
+            ft_st32(tmem_o + c * 128 + q * 32, o);
+          }
+          hb_tmem_st_wait();
+        }
+        hb_tc_fence_before();
+        hb_fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) hb_mbar_arrive(&bar->p_full[c]);
+      }
+      // ---- the two chains joined
+      if (ok && i0 < sp.n) ok = __all_sync(0xffffffffu, hb_mbar_wait(&bar->pv_done[c], (cnt - 1) & 1, abort_flag));
+      float2* ml = (float2*)(sP + 2 * c * FT_TILE);      // where P lay: the chain's products are done
+      ml[r] = make_float2(m_run, l_run);
+      hb_tc_fence_before();
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      hb_tc_fence_after();
+      if (ok) {
+        const float2 a = ((const float2*)sP)[r], b = ((const float2*)(sP + 2 * FT_TILE))[r];
+        const float m = fmaxf(a.x, b.x);
+        const float fa = hb_exp2(a.x - m), fb = hb_exp2(b.x - m);   // a chain without a visible key: 2^-inf = 0
+        float l = a.y * fa + b.y * fb;
+        if (EX && sink) l += hb_exp2(fmaf(sink[hq], 1.4426950408889634f, -m));
+        const float inv = 1.f / l, ga = fa * inv, gb = fb * inv;
+        const bool both = sp.n > 1, even = !(sp.kt_lo & 1);         // (with one tile, the other chain's accumulator is not of this item)
+        constexpr int HC = FT_D / 2;                                 // this warpgroup's columns: c * HC ..
+        __nv_bfloat16* dst = out + ((size_t)(e.x + r) * Hq + hq) * FT_D + c * HC;
+#pragma unroll
+        for (int q = 0; q < HC; q += 32) {
+          float v[32], w[32];
+          hb_tmem_ld32(tmem_o + (both || even ? 0 : 128) + c * HC + q, v);
+          if (both) {
+            hb_tmem_ld32(tmem_o + 128 + c * HC + q, w);
+#pragma unroll
+            for (int d = 0; d < 32; d++) v[d] = fmaf(w[d], gb, v[d] * ga);
+          } else {
+            const float g = even ? ga : gb;
+#pragma unroll
+            for (int d = 0; d < 32; d++) v[d] *= g;
+          }
+          if (r < e.y) {
+#pragma unroll
+            for (int d = 0; d < 32; d += 8)
+              *(uint4*)(dst + q + d) = make_uint4(hb_pack_bf16(v[d], v[d + 1]), hb_pack_bf16(v[d + 2], v[d + 3]),
+                                                  hb_pack_bf16(v[d + 4], v[d + 5]), hb_pack_bf16(v[d + 6], v[d + 7]));
+          }
+        }
+      }
+      hb_tc_fence_before();
+      asm volatile("bar.sync 2, 256;" ::: "memory");   // both accumulators and the chains' numbers may be overwritten
+      hb_tc_fence_after();
+    }
+  }
+
+  hb_tc_fence_before();
+  __syncthreads();
+  if (*abort_flag) {
+    if (threadIdx.x == 0) atomicExch(status, 1);
+    __nanosleep(100000);
+  }
+  if (warp == 10) {
+    __syncwarp();
+    hb_tmem_dealloc(tmem, 512);
+  }
+}
+
+// ---------------------------------------------------------------------------------------
+// head_dim 64: one chain, two CTAs an SM.
+// ---------------------------------------------------------------------------------------
+template <bool EX>
+__global__ void __launch_bounds__(256, 2) flash_prefill_tc64_kernel(
+    const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+    const __grid_constant__ CUtensorMap map_v, const int* __restrict__ bt, int bt_stride, const int* __restrict__ q_start,
+    const int* __restrict__ q_len, const int* __restrict__ ctx_len, __nv_bfloat16* __restrict__ out, int Hq, int Hkv,
+    int page_size, int window, float scale_log2, int min_rows, int* status, const float* __restrict__ r1p,
+    const float* __restrict__ r2p, const float* __restrict__ sink, int req0, int reqs, int qt0, int qts) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* sQ = smem;                 // [128][64]
+  uint8_t* sP = sQ + FT_TILE;         // two K blocks of [128 rows][64 keys]
+  uint8_t* sK = sP + 2 * FT_TILE;     // two stages of [128 keys][64]
+  uint8_t* sV = sK + 2 * FT_TILE;     // and two more
+  FtBars64* bar = (FtBars64*)(sV + 2 * FT_TILE);
+  volatile int* abort_flag = &bar->abort_flag;
+
+  hb_pdl_launch();
+  if (hb_smem_u32(smem) & 1023) {   // as above
+    if (threadIdx.x == 0) atomicExch(status, 1);
+    hb_pdl_wait();
+    return;
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == 0) ft_list((uint2*)sP, &bar->n_entries, FT_MAX_ENTRIES64, q_len, ctx_len, window, min_rows, req0, reqs, qt0, qts);
+  if (threadIdx.x == 32) {
+    hb_mbar_init(&bar->q_full, 1); hb_mbar_init(&bar->q_free, 1);
+    for (int b = 0; b < 2; b++) {
+      hb_mbar_init(&bar->k_full[b], 1); hb_mbar_init(&bar->k_free[b], 1);
+      hb_mbar_init(&bar->v_full[b], 1); hb_mbar_init(&bar->v_free[b], 1);
+    }
+    hb_mbar_init(&bar->s_full, 1); hb_mbar_init(&bar->s_free, 4);
+    hb_mbar_init(&bar->p_full, 4); hb_mbar_init(&bar->pv_done, 1);
+    bar->abort_flag = 0;
+    hb_fence_barrier_init();
+  }
+  if (warp == 4 && lane == 0) { hb_tma_prefetch_desc(&map_q); hb_tma_prefetch_desc(&map_k); hb_tma_prefetch_desc(&map_v); }
+  __syncthreads();
+  const int n_entries = bar->n_entries, n_items = n_entries * Hq;
+  if ((int)blockIdx.x >= n_items) {
+    hb_pdl_wait();
+    return;
+  }
+  ft_sort((const uint2*)sP, bar->entries, n_entries);
+  for (int i = threadIdx.x; i < 2 * FT_TILE / 16; i += 256) ((uint4*)sV)[i] = make_uint4(0, 0, 0, 0);   // what P's zeros meet must be finite, as above
+  if (warp == 6) {
+    hb_tmem_alloc(&bar->tmem_slot, 256);
+    hb_tmem_relinquish();
+  }
+  hb_fence_proxy_async();
+  hb_tc_fence_before();
+  __syncthreads();
+  hb_tc_fence_after();
+  const uint32_t tmem_s = bar->tmem_slot, tmem_o = tmem_s + FT_BN;  // S: 128 columns, O: 64 columns
+  hb_pdl_wait();
+
+  auto entry = [&](int k) { const int u = ft_item(k); return ft_entry(bar->entries[u < n_items ? u / Hq : 0], q_start, q_len, ctx_len); };
+  if (warp == 4 || warp == 5) {  // ---------------- TMA
+    const bool is_k = warp == 4;
+    uint32_t it = 0;
+    bool ok = true;
+    int4 ahead = entry(0);
+    for (int k = 0, u; (u = ft_item(k)) < n_items && ok; k++) {
+      const int4 e = ahead;
+      ahead = entry(k + 1);
+      const int hq = u % Hq, h = hq / (Hq / Hkv);
+      if (is_k) {
+        if (!__all_sync(0xffffffffu, hb_mbar_wait(&bar->q_free, (k & 1) ^ 1, abort_flag))) break;
+        if (hb_elect()) {
+          hb_mbar_expect_tx(&bar->q_full, FT_TILE);
+          hb_tma_load_2d(sQ, &map_q, &bar->q_full, hq * 64, e.x);
+        }
+        __syncwarp();
+      }
+      ok = ft_bring<64>(ft_span(e, window), bt + (size_t)e.w * bt_stride, page_size, Hkv, h, is_k ? &map_k : &map_v, is_k ? sK : sV,
+                        is_k ? bar->k_full : bar->v_full, is_k ? bar->k_free : bar->v_free, it, abort_flag);
+    }
+  } else if (warp == 6) {  // ---------------- tensor cores: S_i is issued before O_{i-1}, so it overlaps the softmax of tile i - 1
+    constexpr uint32_t idesc_s = hb_umma_idesc_bf16(FT_BM, FT_BN), idesc_o = ft_idesc_b_mn(FT_BM, 64);
+    uint32_t base = 0;      // tiles of the items before
+    bool ok = true;
+    int4 ahead = entry(0);
+    for (int k = 0; ft_item(k) < n_items && ok; k++) {
+      const int n = ft_span(ahead, window).n;
+      ahead = entry(k + 1);
+      ok = __all_sync(0xffffffffu, hb_mbar_wait(&bar->q_full, k & 1, abort_flag));
+      for (int i = 0; i <= n && ok; i++) {
+        if (i < n) {
+          const uint32_t it = base + i, s = it & 1, ph = (it >> 1) & 1;
+          ok = hb_mbar_wait(&bar->k_full[s], ph, abort_flag) && hb_mbar_wait(&bar->s_free, (it & 1) ^ 1, abort_flag);
+          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+          hb_tc_fence_after();
+          if (hb_elect()) {
+            const uint64_t dq = hb_umma_desc_k128(hb_smem_u32(sQ)), dk = hb_umma_desc_k128(hb_smem_u32(sK + s * FT_TILE));
+#pragma unroll
+            for (int kk = 0; kk < 4; kk++) hb_umma_bf16(tmem_s, dq + 2 * kk, dk + 2 * kk, idesc_s, kk != 0);
+            hb_umma_commit(&bar->s_full);
+            hb_umma_commit(&bar->k_free[s]);
+            if (i == n - 1) hb_umma_commit(&bar->q_free);
+          }
+          __syncwarp();
+        }
+        if (i > 0) {
+          const uint32_t it = base + i - 1, s = it & 1, ph = (it >> 1) & 1;
+          ok = hb_mbar_wait(&bar->v_full[s], ph, abort_flag) && hb_mbar_wait(&bar->p_full, it & 1, abort_flag);
+          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+          hb_tc_fence_after();
+          if (hb_elect()) {
+#pragma unroll
+            for (int kk = 0; kk < FT_BN / 16; kk++) {
+              const uint64_t dp = hb_umma_desc_k128(hb_smem_u32(sP + (kk >> 2) * FT_TILE)) + 2 * (kk & 3);
+              const uint64_t dv = ft_desc_mn128(hb_smem_u32(sV + s * FT_TILE + kk * 16 * 128));   // 16 keys on
+              hb_umma_bf16(tmem_o, dp, dv, idesc_o, i > 1 || kk != 0);
+            }
+            hb_umma_commit(&bar->v_free[s]);
+            hb_umma_commit(&bar->pv_done);
+          }
+          __syncwarp();
+        }
+      }
+      base += n;
+    }
+  } else if (warp < 4) {  // ---------------- softmax: thread = query row
+    const int r = threadIdx.x;
+    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
+    uint32_t cnt = 0;      // tiles so far, over all items
+    bool ok = true;        // every wait's outcome is made uniform over the warp
+    int4 ahead = entry(0);
+    for (int k = 0, u; (u = ft_item(k)) < n_items && ok; k++) {
+      const int4 e = ahead;
+      ahead = entry(k + 1);
+      const int hq = u % Hq;
+      const FtSpan sp = ft_span(e, window);
+      const int qp = e.z + min(r, e.y - 1);      // rows past the portion's end are computed, never stored
+      const float r1 = EX && r1p ? r1p[hq] : 0.f, r2 = EX && r1p ? r2p[hq] : 0.f;
+      float m_run = -INFINITY, l_run = 0.f;
+      for (int i = 0; i < sp.n && ok; i++, cnt++) {
+        const int k_base = (sp.kt_lo + i) * FT_BN;
+        const bool need_mask = k_base + FT_BN - 1 > e.z || (window > 0 && k_base < sp.p_last - window + 1);
+        const int hi_j = qp - k_base, lo_j = window > 0 ? qp - window - k_base : -1;  // key j of the tile is visible iff lo_j < j <= hi_j
+        if (!__all_sync(0xffffffffu, hb_mbar_wait(&bar->s_full, cnt & 1, abort_flag))) { ok = false; break; }
+        hb_tc_fence_after();
+        uint32_t sr[64];
+        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int hh = 0; hh < 2; hh++) {
+          hb_tmem_ld64_nowait(tmem_s + lane_base + hh * 64, sr);
+          hb_tmem_ld_wait();
+          hb_tmem_ld_fence64(sr);
+          if (need_mask) {
+#pragma unroll
+            for (int j = 0; j < 64; j++)
+              if (!(j + hh * 64 <= hi_j && j + hh * 64 > lo_j)) sr[j] = __float_as_uint(-INFINITY);
+          }
+#pragma unroll
+          for (int j = 0; j < 64; j += 2) mx[(j >> 1) & 3] = fmaxf(fmaxf(mx[(j >> 1) & 3], __uint_as_float(sr[j])), __uint_as_float(sr[j + 1]));
+        }
+        float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2;
+        const float dist0 = (float)(qp - k_base);                     // of the tile's first key
+        if (EX) m_tile -= r1 * __log2f(fmaf(r2, fmaxf(dist0 - (FT_BN - 1), 0.f), 1.f));
+        const bool grow = m_tile > m_run + FT_SLACK;   // also the first tile with a visible key: m_run is -inf
+        float corr = 1.f;
+        if (grow) {
+          corr = hb_exp2(m_run - m_tile);   // 0 while nothing has been summed
+          m_run = m_tile;
+        }
+        const float sub = m_run == -INFINITY ? 0.f : m_run;
+        const uint64_t scale2 = ft_pack2(__float_as_uint(scale_log2), __float_as_uint(scale_log2)), sub2 = ft_pack2(__float_as_uint(-sub), __float_as_uint(-sub));
+        uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};
+        // the exponentials: keys 64-127 are still in the registers (masked), keys 0-63 are read again
+#pragma unroll
+        for (int hh = 1; hh >= 0; hh--) {
+          if (hh == 0) {
+            hb_tmem_ld64_nowait(tmem_s + lane_base, sr);
+            hb_tmem_ld_wait();
+            hb_tmem_ld_fence64(sr);
+            hb_tc_fence_before();
+            __syncwarp();
+            if (lane == 0) hb_mbar_arrive(&bar->s_free);  // the last read of S: the scores of the next tile may overwrite it
+            if (need_mask) {
+#pragma unroll
+              for (int j = 0; j < 64; j++)
+                if (!(j <= hi_j && j > lo_j)) sr[j] = __float_as_uint(-INFINITY);
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < 64; j += 2)  // masked scores are -inf: 2^-inf = 0
+            sr[j >> 1] = ft_prob<EX>(sr[j], sr[j + 1], scale2, sub2, r1, r2, dist0 - (float)(j + hh * 64), sum2[(j >> 1) & 3]);
+          // the product of the tile before has read its P and written its O
+          if (hh == 1 && cnt > 0 && !__all_sync(0xffffffffu, hb_mbar_wait(&bar->pv_done, (cnt - 1) & 1, abort_flag))) { ok = false; break; }
+          // 64 keys = eight 16-byte chunks of this row in K block hh of P
+#pragma unroll
+          for (int cc = 0; cc < 8; cc++) {
+            const uint32_t dst = hb_smem_u32(sP + hh * FT_TILE) + r * 128 + ((cc ^ (r & 7)) << 4);
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(sr[4 * cc]), "r"(sr[4 * cc + 1]),
+                         "r"(sr[4 * cc + 2]), "r"(sr[4 * cc + 3]) : "memory");
+          }
+        }
+        if (!ok) break;
+        float s0, s1;
+        ft_unpack2(ft_add2(ft_add2(sum2[0], sum2[1]), ft_add2(sum2[2], sum2[3])), s0, s1);
+        l_run = l_run * corr + (s0 + s1);
+        if (i > 0 && __any_sync(0xffffffffu, grow)) {   // a raised maximum: the row of O so far
+          hb_tc_fence_after();
+          hb_tmem_ld64_nowait(tmem_o + lane_base, sr);
           hb_tmem_ld_wait();
           hb_tmem_ld_fence64(sr);
 #pragma unroll
           for (int d = 0; d < 64; d++) sr[d] = __float_as_uint(__uint_as_float(sr[d]) * corr);
-          hb_tmem_st64(tmem_o + hf * 64 + lane_base, sr);
+          hb_tmem_st64(tmem_o + lane_base, sr);
+          hb_tmem_st_wait();
         }
-        hb_tmem_st_wait();
+        hb_tc_fence_before();
+        hb_fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) hb_mbar_arrive(&bar->p_full);
       }
-      hb_tc_fence_before();
-      hb_fence_proxy_async();
-      hb_mbar_arrive(&bar->p_full);
-    }
-    if (ok && __all_sync(0xffffffffu, hb_mbar_wait(&bar->o_full, (n_tiles - 1) & 1, abort_flag))) {
-      hb_tc_fence_after();
-      if (EX && sink) l_run += hb_exp2(fmaf(sink[hq], 1.4426950408889634f, -m_run));
-      const float inv = 1.f / l_run;
-      __nv_bfloat16* dst = out + ((size_t)(row0 + r) * Hq + hq) * FT_D;
-#pragma unroll
-      for (int hf = 0; hf < NH; hf++) {
-        uint32_t orr[64];
-        hb_tmem_ld64_nowait(tmem_o + hf * 64 + lane_base, orr);
+      // the item's end: the next one's first product comes behind the arrivals of these warps, so O is theirs until then
+      if (ok) ok = __all_sync(0xffffffffu, hb_mbar_wait(&bar->pv_done, (cnt - 1) & 1, abort_flag));
+      if (ok) {
+        hb_tc_fence_after();
+        if (EX && sink) l_run += hb_exp2(fmaf(sink[hq], 1.4426950408889634f, -m_run));
+        const float inv = 1.f / l_run;
+        uint32_t o[64];
+        hb_tmem_ld64_nowait(tmem_o + lane_base, o);
         hb_tmem_ld_wait();
-        hb_tmem_ld_fence64(orr);
-        if (r < rows_here) {
+        hb_tmem_ld_fence64(o);
+        hb_tc_fence_before();
+        if (r < e.y) {
+          __nv_bfloat16* dst = out + ((size_t)(e.x + r) * Hq + hq) * 64;
 #pragma unroll
           for (int d = 0; d < 64; d += 8) {
             uint4 w;
-            w.x = hb_pack_bf16(__uint_as_float(orr[d]) * inv, __uint_as_float(orr[d + 1]) * inv);
-            w.y = hb_pack_bf16(__uint_as_float(orr[d + 2]) * inv, __uint_as_float(orr[d + 3]) * inv);
-            w.z = hb_pack_bf16(__uint_as_float(orr[d + 4]) * inv, __uint_as_float(orr[d + 5]) * inv);
-            w.w = hb_pack_bf16(__uint_as_float(orr[d + 6]) * inv, __uint_as_float(orr[d + 7]) * inv);
-            *(uint4*)(dst + hf * 64 + d) = w;
+            w.x = hb_pack_bf16(__uint_as_float(o[d]) * inv, __uint_as_float(o[d + 1]) * inv);
+            w.y = hb_pack_bf16(__uint_as_float(o[d + 2]) * inv, __uint_as_float(o[d + 3]) * inv);
+            w.z = hb_pack_bf16(__uint_as_float(o[d + 4]) * inv, __uint_as_float(o[d + 5]) * inv);
+            w.w = hb_pack_bf16(__uint_as_float(o[d + 6]) * inv, __uint_as_float(o[d + 7]) * inv);
+            *(uint4*)(dst + d) = w;
           }
         }
       }
@@ -337,7 +746,7 @@ __global__ void __launch_bounds__(FT_D == 64 ? 256 : 192, FT_D == 64 ? 2 : 1) fl
     if (threadIdx.x == 0) atomicExch(status, 1);
     __nanosleep(100000);
   }
-  if (warp == 5) {
+  if (warp == 6) {
     __syncwarp();
     hb_tmem_dealloc(tmem_s, 256);
   }
@@ -345,6 +754,14 @@ __global__ void __launch_bounds__(FT_D == 64 ? 256 : 192, FT_D == 64 ? 2 : 1) fl
 
 HB_EXPORT int hb_flash_prefill_tc_supported(int Hq, int Hkv, int D, int page_size) {
   return Hkv > 0 && Hq % Hkv == 0 && (D == 64 || D == 128) && page_size >= 8 && page_size <= FT_BN && (page_size & (page_size - 1)) == 0;
+}
+
+static int ft_sms() {
+  static int n[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  if (!n[dev] && cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n[dev] = 148;
+  return n[dev];
 }
 
 // q, out [T, Hq, D] bf16; caches [num_pages, Hkv, page_size, D] bf16 (D 64 or 128); per request q_start, q_len,
@@ -367,26 +784,38 @@ HB_EXPORT int hb_flash_prefill_tc(const void* q, const void* kc, const void* vc,
   const uint64_t rows = (uint64_t)num_pages * Hkv * page_size;
   if (hb_make_tensor_map_bf16(&mk, kc, rows, (uint64_t)D, (uint64_t)D, (uint32_t)page_size)) return -1;
   if (hb_make_tensor_map_bf16(&mv, vc, rows, (uint64_t)D, (uint64_t)D, (uint32_t)page_size)) return -1;
-  dim3 grid(Hq, (max_q_len + FT_BM - 1) / FT_BM, R);
   const float sl2 = scale * 1.4426950408889634f;
-  cudaError_t e;
-  // head_dim 64: 113 KB, two CTAs an SM; head_dim 128: Q, 2 K, 2 V of 32 KB each and P: 192 KB
-  const size_t smem = (D == 64 ? 7 : 12) * (size_t)FT_TILE + sizeof(FtBars);
-#define FT_LAUNCH(DD, EX)                                                                                                       \
+  cudaError_t e = cudaSuccess;
+  // (request, query tile) pairs: portions of T rows in all have at most T / 128 tiles and one more each, and there are at most T / min_rows
+  // portions. A step of more pairs than the list holds is cut into launches of some requests, or of some requests and query tiles.
+  const int tiles = (max_q_len + FT_BM - 1) / FT_BM, most = D == 64 ? FT_MAX_ENTRIES64 : FT_MAX_ENTRIES;
+  const long full = T / FT_BM, portions = min_rows > 1 && T / min_rows < R ? T / min_rows : R, bound = full + portions;
+  int req_step = R, qt_step = tiles;
+  if (bound > most && (long)R * tiles > most) {
+    if (full <= most / 2) req_step = most - (int)full;
+    else { req_step = 32; qt_step = most / 32; }
+  }
+#define FT_LAUNCH(KERN, THREADS, SMEM)                                                                                           \
   do {                                                                                                                          \
     static bool configured = false;                                                                                             \
     if (!configured) {                                                                                                          \
-      e = cudaFuncSetAttribute(flash_prefill_tc_kernel<DD, EX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);        \
+      e = cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);                                        \
       if (e != cudaSuccess) HB_FAIL("hb_flash_prefill_tc: %s", cudaGetErrorString(e));                                          \
       configured = true;                                                                                                        \
     }                                                                                                                           \
-    e = hb_launch(flash_prefill_tc_kernel<DD, EX>, grid, 192, smem, st, mq, mk, mv, bt, bt_stride, q_start, q_len, ctx_len,     \
-                  (__nv_bfloat16*)out, Hq, Hkv, page_size, window, sl2, min_rows, status, r1, r2, sink);                        \
+    e = hb_launch(KERN, grid, THREADS, SMEM, st, mq, mk, mv, bt, bt_stride, q_start, q_len, ctx_len, (__nv_bfloat16*)out, Hq,   \
+                  Hkv, page_size, window, sl2, min_rows, status, r1, r2, sink, req0, reqs, qt0, qts);                           \
   } while (0)
-  if (D == 64 && !ex) FT_LAUNCH(64, false);
-  else if (D == 64) FT_LAUNCH(64, true);
-  else if (!ex) FT_LAUNCH(128, false);
-  else FT_LAUNCH(128, true);
+  for (int req0 = 0; req0 < R && e == cudaSuccess; req0 += req_step)
+    for (int qt0 = 0; qt0 < tiles && e == cudaSuccess; qt0 += qt_step) {
+      const int reqs = R - req0 < req_step ? R - req0 : req_step, qts = tiles - qt0 < qt_step ? tiles - qt0 : qt_step;
+      const long items = ((long)reqs * qts < bound ? (long)reqs * qts : bound) * Hq, ctas = (D == 64 ? 2 : 1) * ft_sms();
+      const int grid = (int)(items < ctas ? (items > 0 ? items : 1) : ctas);
+      if (D == 64 && !ex) FT_LAUNCH(flash_prefill_tc64_kernel<false>, 256, FT_SMEM64);
+      else if (D == 64) FT_LAUNCH(flash_prefill_tc64_kernel<true>, 256, FT_SMEM64);
+      else if (!ex) FT_LAUNCH(flash_prefill_tc_kernel<false>, FT_THREADS, FT_SMEM);
+      else FT_LAUNCH(flash_prefill_tc_kernel<true>, FT_THREADS, FT_SMEM);
+    }
 #undef FT_LAUNCH
   if (e != cudaSuccess) HB_FAIL("hb_flash_prefill_tc: %s", cudaGetErrorString(e));
   HB_CHECK_LAUNCH("hb_flash_prefill_tc");

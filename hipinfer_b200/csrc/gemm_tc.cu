@@ -252,49 +252,57 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
   if (warp != 4) hb_pdl_wait();   // barriers and tensor memory were set up while the kernel ahead was still running
 
   if (warp == 4) {
-    if (lane == 0) {  // ---------------- TMA producer
+    {  // ---------------- TMA producer
       uint32_t it = 0, early = 0;
       bool ok = true;
       // the first weight tiles do not depend on the kernel ahead (every CTA has a tile)
-      for (; early < STAGES && early < num_kb; early++) {
-        hb_mbar_expect_tx(&full[early], S::STAGE_BYTES);
-        hb_tma_load_2d(smem + early * S::STAGE_BYTES + S::A_BYTES, &map_w, &full[early], early * BK, (blockIdx.x / m_tiles) * BN);
-      }
+      for (; early < STAGES && early < num_kb; early++)
+        if (hb_elect()) {
+          hb_mbar_expect_tx(&full[early], S::STAGE_BYTES);
+          hb_tma_load_2d(smem + early * S::STAGE_BYTES + S::A_BYTES, &map_w, &full[early], early * BK, (blockIdx.x / m_tiles) * BN);
+        }
+      __syncwarp();
       hb_pdl_wait();
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * BN;
         for (int kb = 0; kb < num_kb; kb++, it++) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          if (it >= early) {
-            if (!hb_mbar_wait(&empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
-            hb_mbar_expect_tx(&full[s], S::STAGE_BYTES);
-            hb_tma_load_2d(smem + s * S::STAGE_BYTES + S::A_BYTES, &map_w, &full[s], kb * BK, n0);
+          if (it >= early && !__all_sync(0xffffffffu, hb_mbar_wait(&empty[s], ph ^ 1, abort_flag))) { ok = false; break; }
+          if (hb_elect()) {
+            if (it >= early) {
+              hb_mbar_expect_tx(&full[s], S::STAGE_BYTES);
+              hb_tma_load_2d(smem + s * S::STAGE_BYTES + S::A_BYTES, &map_w, &full[s], kb * BK, n0);
+            }
+            hb_tma_load_2d(smem + s * S::STAGE_BYTES, &map_a, &full[s], kb * BK, m0);
           }
-          hb_tma_load_2d(smem + s * S::STAGE_BYTES, &map_a, &full[s], kb * BK, m0);
+          __syncwarp();
         }
       }
     }
   } else if (warp == 5) {
-    if (lane == 0) {  // ---------------- MMA issuer
+    {  // ---------------- MMA issuer
       constexpr uint32_t idesc = hb_umma_idesc_bf16(BM, BN);
       uint32_t it = 0, tile_i = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, tile_i++) {
         const uint32_t buf = tile_i & 1, aph = (tile_i >> 1) & 1;
-        if (!hb_mbar_wait(&tmem_empty[buf], aph ^ 1, abort_flag)) break;
+        if (!__all_sync(0xffffffffu, hb_mbar_wait(&tmem_empty[buf], aph ^ 1, abort_flag))) break;
         hb_tc_fence_after();
         const uint32_t d = tmem_base + buf * BN;
         for (int kb = 0; kb < num_kb; kb++, it++) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          if (!hb_mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, hb_mbar_wait(&full[s], ph, abort_flag))) { ok = false; break; }
           hb_tc_fence_after();
           const uint64_t da = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE_BYTES));
           const uint64_t db = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE_BYTES + S::A_BYTES));
+          if (hb_elect()) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; k++) hb_umma_bf16(d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-          hb_umma_commit(&empty[s]);
+            for (int k = 0; k < BK / 16; k++) hb_umma_bf16(d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+            hb_umma_commit(&empty[s]);
+            if (kb == num_kb - 1) hb_umma_commit(&tmem_full[buf]);
+          }
+          __syncwarp();
         }
-        if (ok) hb_umma_commit(&tmem_full[buf]);
       }
     }
   } else {  // ---------------- epilogue warps 0..3
@@ -417,17 +425,20 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_pair_kernel(const __grid_const
   if (warp != 4) hb_pdl_wait();   // (the loader asks for its first weight tiles before it waits)
 
   if (warp == 4) {
-    if (lane == 0) {  // ---------------- TMA producer of this CTA's halves
+    {  // ---------------- TMA producer of this CTA's halves
       uint32_t it = 0, early = 0;
       bool ok = true;
       // the first weight tiles do not depend on the kernel ahead (0.5 to 0.8 us a product, back to back)
       if (pair < units) {
         const int tile = pair % num_tiles, kb0 = pair / num_tiles * kbs, kb1 = min(num_kb, kb0 + kbs), n0 = (tile / m_tiles) * BN + rank * 128;
-        for (int kb = kb0; early < STAGES && kb < kb1; early++)
-          for (int j = 0, n = min(KPS, kb1 - kb); j < n; j++, kb++) {
-            if (j == 0 && rank == 0) hb_mbar_expect_tx(&full[early], 2 * S::BLOCK_BYTES * n);   // both CTAs' bytes
-            hb_tma_load_2d_pair(smem + early * S::STAGE_BYTES + j * S::BLOCK_BYTES + S::A_BYTES, &map_w, hb_mapa(&full[early], 0), kb * BK, n0);
+        for (int kb = kb0; early < STAGES && kb < kb1; early++, kb += KPS)
+          if (hb_elect()) {
+            const int n = min(KPS, kb1 - kb);
+            if (rank == 0) hb_mbar_expect_tx(&full[early], 2 * S::BLOCK_BYTES * n);   // both CTAs' bytes
+            for (int j = 0; j < n; j++)
+              hb_tma_load_2d_pair(smem + early * S::STAGE_BYTES + j * S::BLOCK_BYTES + S::A_BYTES, &map_w, hb_mapa(&full[early], 0), (kb + j) * BK, n0);
           }
+        __syncwarp();
       }
       hb_pdl_wait();
       for (int u = pair; u < units && ok; u += n_pairs) {
@@ -437,16 +448,17 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_pair_kernel(const __grid_const
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1, bar = hb_mapa(&full[s], 0);
           const int n = min(KPS, kb1 - kb);
           uint8_t* st = smem + s * S::STAGE_BYTES;
-          if (it >= early) {
-            if (!hb_mbar_wait(&empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
-            if (rank == 0) hb_mbar_expect_tx(&full[s], 2 * S::BLOCK_BYTES * n);
-          }
+          if (it >= early && !__all_sync(0xffffffffu, hb_mbar_wait(&empty[s], ph ^ 1, abort_flag))) { ok = false; break; }
+          if (hb_elect()) {
+            if (it >= early && rank == 0) hb_mbar_expect_tx(&full[s], 2 * S::BLOCK_BYTES * n);
 #pragma unroll
-          for (int j = 0; j < KPS; j++)
-            if (j < n) {
-              hb_tma_load_2d_pair(st + j * S::BLOCK_BYTES, &map_a, bar, (kb + j) * BK, m0);
-              if (it >= early) hb_tma_load_2d_pair(st + j * S::BLOCK_BYTES + S::A_BYTES, &map_w, bar, (kb + j) * BK, n0);
-            }
+            for (int j = 0; j < KPS; j++)
+              if (j < n) {
+                hb_tma_load_2d_pair(st + j * S::BLOCK_BYTES, &map_a, bar, (kb + j) * BK, m0);
+                if (it >= early) hb_tma_load_2d_pair(st + j * S::BLOCK_BYTES + S::A_BYTES, &map_w, bar, (kb + j) * BK, n0);
+              }
+          }
+          __syncwarp();
         }
       }
       // the last commits still arrive on this CTA's barriers: wait for them before the shared memory is given up
@@ -454,32 +466,35 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_pair_kernel(const __grid_const
         ok = hb_mbar_wait(&empty[j % STAGES], (j / STAGES) & 1, abort_flag);
     }
   } else if (warp == 5) {
-    if (lane == 0 && rank == 0) {  // ---------------- MMA issuer of the pair
+    if (rank == 0) {  // ---------------- MMA issuer of the pair
       constexpr uint32_t idesc = hb_umma_idesc_bf16(256, BN);
       uint32_t it = 0, tile_i = 0;
       bool ok = true;
       for (int u = pair; u < units && ok; u += n_pairs, tile_i++) {
         const int kb0 = u / num_tiles * kbs, kb1 = min(num_kb, kb0 + kbs);
         const uint32_t buf = tile_i & 1, aph = (tile_i >> 1) & 1;
-        if (!hb_mbar_wait(&tmem_empty[buf], aph ^ 1, abort_flag)) break;
+        if (!__all_sync(0xffffffffu, hb_mbar_wait(&tmem_empty[buf], aph ^ 1, abort_flag))) break;
         hb_tc_fence_after();
         const uint32_t d = tmem_base + buf * BN;
         for (int kb = kb0; kb < kb1; kb += KPS, it++) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          if (!hb_mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, hb_mbar_wait(&full[s], ph, abort_flag))) { ok = false; break; }
           hb_tc_fence_after();
           const int n = min(KPS, kb1 - kb);
+          if (hb_elect()) {
 #pragma unroll
-          for (int j = 0; j < KPS; j++)
-            if (j < n) {
-              const uint32_t st = hb_smem_u32(smem + s * S::STAGE_BYTES + j * S::BLOCK_BYTES);
-              const uint64_t da = hb_umma_desc_k128(st), db = hb_umma_desc_k128(st + S::A_BYTES);
+            for (int j = 0; j < KPS; j++)
+              if (j < n) {
+                const uint32_t st = hb_smem_u32(smem + s * S::STAGE_BYTES + j * S::BLOCK_BYTES);
+                const uint64_t da = hb_umma_desc_k128(st), db = hb_umma_desc_k128(st + S::A_BYTES);
 #pragma unroll
-              for (int k = 0; k < BK / 16; k++) hb_umma_bf16_pair(d, da + 2 * k, db + 2 * k, idesc, kb + j != kb0 || k != 0);
-            }
-          hb_umma_commit_pair(&empty[s]);
+                for (int k = 0; k < BK / 16; k++) hb_umma_bf16_pair(d, da + 2 * k, db + 2 * k, idesc, kb + j != kb0 || k != 0);
+              }
+            hb_umma_commit_pair(&empty[s]);
+            if (kb + KPS >= kb1) hb_umma_commit_pair(&tmem_full[buf]);
+          }
+          __syncwarp();
         }
-        if (ok) hb_umma_commit_pair(&tmem_full[buf]);
       }
     }
   } else {  // ---------------- epilogue warps 0..3: this CTA's 128 rows of the tile
@@ -857,7 +872,7 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_grouped_kernel(const __grid_co
   };
 
   if (warp == 4) {
-    if (lane == 0) {  // ---------------- TMA producer
+    {  // ---------------- TMA producer
       uint32_t it = 0;
       int e = 0, m0, n0;
       bool ok = true;
@@ -865,34 +880,40 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_grouped_kernel(const __grid_co
         place(tile, e, m0, n0);
         for (int kb = 0; kb < num_kb; kb++, it++) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          if (!hb_mbar_wait(&empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
-          hb_mbar_expect_tx(&full[s], S::STAGE_BYTES);
-          hb_tma_load_2d(smem + s * S::STAGE_BYTES, &map_a, &full[s], kb * BK, m0);
-          hb_tma_load_2d(smem + s * S::STAGE_BYTES + S::A_BYTES, &map_w, &full[s], kb * BK, e * N + n0);
+          if (!__all_sync(0xffffffffu, hb_mbar_wait(&empty[s], ph ^ 1, abort_flag))) { ok = false; break; }
+          if (hb_elect()) {
+            hb_mbar_expect_tx(&full[s], S::STAGE_BYTES);
+            hb_tma_load_2d(smem + s * S::STAGE_BYTES, &map_a, &full[s], kb * BK, m0);
+            hb_tma_load_2d(smem + s * S::STAGE_BYTES + S::A_BYTES, &map_w, &full[s], kb * BK, e * N + n0);
+          }
+          __syncwarp();
         }
       }
     }
   } else if (warp == 5) {
-    if (lane == 0) {  // ---------------- MMA issuer
+    {  // ---------------- MMA issuer
       constexpr uint32_t idesc = hb_umma_idesc_bf16(BM, BN);
       uint32_t it = 0, tile_i = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, tile_i++) {
         const uint32_t buf = tile_i & 1, aph = (tile_i >> 1) & 1;
-        if (!hb_mbar_wait(&tmem_empty[buf], aph ^ 1, abort_flag)) break;
+        if (!__all_sync(0xffffffffu, hb_mbar_wait(&tmem_empty[buf], aph ^ 1, abort_flag))) break;
         hb_tc_fence_after();
         const uint32_t d = tmem_base + buf * BN;
         for (int kb = 0; kb < num_kb; kb++, it++) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          if (!hb_mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, hb_mbar_wait(&full[s], ph, abort_flag))) { ok = false; break; }
           hb_tc_fence_after();
           const uint64_t da = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE_BYTES));
           const uint64_t db = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE_BYTES + S::A_BYTES));
+          if (hb_elect()) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; k++) hb_umma_bf16(d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-          hb_umma_commit(&empty[s]);
+            for (int k = 0; k < BK / 16; k++) hb_umma_bf16(d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+            hb_umma_commit(&empty[s]);
+            if (kb == num_kb - 1) hb_umma_commit(&tmem_full[buf]);
+          }
+          __syncwarp();
         }
-        if (ok) hb_umma_commit(&tmem_full[buf]);
       }
     }
   } else {  // ---------------- epilogue warps 0..3

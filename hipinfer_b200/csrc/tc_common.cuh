@@ -48,6 +48,21 @@ __device__ __forceinline__ bool hb_mbar_wait(uint64_t* bar, uint32_t parity, vol
   return false;
 }
 
+// One lane of a converged warp. What only one thread may issue (tcgen05.mma, its commit, TMA copies) stands in a branch on this inside
+// code that the WHOLE warp runs: the compiler then knows that a single lane is active, which it cannot know behind "lane == 0" (an MMA
+// of the attention kernels took 130 cycles to issue there, 65 here: the MMA's own time).
+__device__ __forceinline__ bool hb_elect() {
+  uint32_t p;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(p));
+  return p != 0;
+}
+
 // ---------------------------------------------------------------- TMA (tile mode, no multicast)
 __device__ __forceinline__ void hb_tma_prefetch_desc(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)m) : "memory");

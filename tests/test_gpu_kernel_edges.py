@@ -1,0 +1,148 @@
+"""Edges of the prompt kernels: rows and columns that cut a box or leave a tile an odd number of them, and attention items in the
+forms the persistent kernels walk (one key tile of either parity, many short requests beside a portion, more items than one
+list holds)."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def fast():
+    from hipinfer_b200.kernels import fast as f
+    return f
+
+
+def rnd(*shape, seed=0, scale=1.0):
+    g = torch.Generator().manual_seed(seed)
+    return (torch.randn(*shape, generator=g) * scale).to(torch.bfloat16).to(DEV)
+
+
+def i32(v):
+    return torch.tensor(v, dtype=torch.int32, device=DEV)
+
+
+# rows around a warp's 32 and a tile's 128; K of one, an odd number and many blocks of 64; more column tiles than CTAs with one box in the last
+@pytest.mark.parametrize("M,N,K", [(65, 64, 64), (159, 320, 192), (287, 544, 520), (300, 4128, 64), (1531, 288, 320)])
+@pytest.mark.parametrize("tile_n", [128, 256, 512])
+def test_rows_that_cut_a_box(M, N, K, tile_n):
+    f = fast()
+    a, w = rnd(M, K, seed=1), rnd(N, K, seed=2, scale=0.1)
+    ref = a.double() @ w.double().T
+    tol = 2e-5 * max(1.0, float(ref.abs().max())) * math.sqrt(K)       # 32-bit sums of K products
+    for epi in (f.EPI_F32, f.EPI_BF16):
+        out = torch.full((M + 1, N), 7.0, dtype=torch.float32 if epi == f.EPI_F32 else torch.bfloat16, device=DEV)
+        f.gemm_tc(a, w, out[:M], epi, tile_n)
+        torch.cuda.synchronize()
+        f.check_status()
+        rounding = 0.0 if epi == f.EPI_F32 else 2.0 ** -8              # and one rounding to bfloat16
+        assert bool(((out[:M].double() - ref).abs() <= tol + rounding * ref.abs()).all())
+        assert bool((out[M] == 7.0).all()), "wrote past the last row"
+    act = torch.full((M + 1, N // 2), 7.0, dtype=torch.bfloat16, device=DEV)
+    f.gemm_tc(a, w, act[:M], f.EPI_SWIGLU_BF16, tile_n)
+    torch.cuda.synchronize()
+    f.check_status()
+    gu = ref.view(M, N // 32, 2, 16)
+    want = (torch.nn.functional.silu(gu[:, :, 0]) * gu[:, :, 1]).reshape(M, N // 2)
+    scale = (1.0 + gu.abs()).amax(2).reshape(M, N // 2)                # an error of the sums times the other factor, and the rounding
+    assert bool(((act[:M].double() - want).abs() <= 3 * tol * scale + 2.0 ** -8 * want.abs()).all())
+    assert bool((act[M] == 7.0).all()), "wrote past the last row"
+
+
+def test_last_column_of_one_box_over_many_tiles():
+    """Two tiles in a row of the same CTA pair whose last column has a single box each: each box leaves before the next fills its place."""
+    f = fast()
+    M, N, K = 256 * 150, 288, 64
+    a, w = rnd(M, K, seed=3), rnd(N, K, seed=4, scale=0.1)
+    out = torch.empty(M, N, dtype=torch.float32, device=DEV)
+    f.gemm_tc(a, w, out, f.EPI_F32, 512)
+    torch.cuda.synchronize()
+    f.check_status()
+    ref = a.float() @ w.float().T
+    assert float((out - ref).abs().max()) < 1e-4 * max(1.0, float(ref.abs().max()))
+
+
+def attention_case(Hq, Hkv, D, ps, ctx, rows, window, seed):
+    """Paged caches with shuffled pages, and the plain result in 64 bits of every request."""
+    lens = [c + n for c, n in zip(ctx, rows)]
+    pages = [-(-n // ps) for n in lens]
+    order = torch.randperm(sum(pages), generator=torch.Generator().manual_seed(seed)).tolist()
+    bt = torch.zeros(len(rows), max(pages), dtype=torch.int32)
+    at = 0
+    for r, n in enumerate(pages):
+        bt[r, :n] = torch.tensor(order[at:at + n], dtype=torch.int32)
+        at += n
+    kc, vc = rnd(at, Hkv, ps, D, seed=seed + 1), rnd(at, Hkv, ps, D, seed=seed + 2)
+    T = sum(rows)
+    q = rnd(T, Hq * D, seed=seed + 3)
+    want = torch.full((T, Hq, D), 7.0, dtype=torch.float64, device=DEV)
+    s = 0
+    for r, n in enumerate(rows):
+        if n >= 16:
+            idx = bt[r, :pages[r]].long().to(DEV)
+            k, v = (c[idx].transpose(1, 2).reshape(-1, Hkv, D)[:lens[r]].double().repeat_interleave(Hq // Hkv, 1) for c in (kc, vc))
+            sc = torch.einsum("thd,shd->hts", q[s:s + n].view(n, Hq, D).double(), k) / math.sqrt(D)
+            i, j = torch.arange(ctx[r], lens[r], device=DEV)[:, None], torch.arange(lens[r], device=DEV)[None]
+            seen = (j <= i) & (j > i - window if window else j >= 0)
+            want[s:s + n] = torch.einsum("hts,shd->thd", torch.softmax(sc.masked_fill(~seen, -math.inf), -1), v)
+        s += n
+    return q, kc, vc, bt.to(DEV), T, want
+
+
+# windows that leave one key tile, of an even and of an odd number; short requests (left alone) between portions; portions of one row more
+# than a tile; a long context
+@pytest.mark.parametrize("D,Hq,Hkv", [(64, 4, 2), (128, 3, 1)])
+@pytest.mark.parametrize("ctx,rows,window", [
+    ([130, 260, 0], [20, 16, 17], 3),
+    ([300] * 40 + [0] + [77] * 20, [1] * 40 + [700] + [1] * 20, 0),
+    ([0, 127, 128, 129, 1000], [129, 128, 16, 257, 40], 0),
+    ([900, 0, 5], [300, 33, 1], 200),
+])
+@pytest.mark.parametrize("ps", [8, 16, 128])
+def test_attention_items(D, Hq, Hkv, ctx, rows, window, ps):
+    q, kc, vc, bt, T, want = attention_case(Hq, Hkv, D, ps, ctx, rows, window, 11)
+    out = torch.full((T, Hq * D), 7.0, dtype=torch.bfloat16, device=DEV)
+    starts = [sum(rows[:i]) for i in range(len(rows))]
+    fast().flash_prefill_tc(q, kc, vc, bt, i32(starts), i32(rows), i32(ctx), out, max(rows), Hq, Hkv, D, ps, window, 1 / math.sqrt(D), 16)
+    torch.cuda.synchronize()
+    fast().check_status()
+    # P and the result are rounded to bfloat16: 2^-9 of values of about 3, and of the result
+    torch.testing.assert_close(out.double().view(T, Hq, D), want, rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("requests,rows,long", [(700, 16, 0), (40, 16, 16000)])      # more requests, and more query tiles, than one list holds
+def test_attention_of_more_items_than_a_list(D, requests, rows, long):
+    q_len = [rows] * requests + ([long] if long else [])
+    ctx = [3] * requests + ([0] if long else [])
+    Hq = Hkv = 1
+    f = fast()
+    q, kc, vc, bt, T, want = attention_case(Hq, Hkv, D, 16, ctx, q_len if not long else q_len[:-1] + [16], 0, 21)
+    if long:        # the long portion's rows read their own short prefix: a window of one key
+        q_len[-1] = long
+        T = sum(q_len)
+        q = torch.cat([q[:-16], rnd(long, D, seed=31)])
+        pages = -(-long // 16)
+        kc = torch.cat([kc, rnd(pages, 1, 16, D, seed=32)])
+        vc = torch.cat([vc, rnd(pages, 1, 16, D, seed=33)])
+        wide = torch.zeros(len(q_len), pages, dtype=torch.int32, device=DEV)
+        wide[:, :bt.shape[1]] = bt
+        wide[-1] = torch.arange(kc.shape[0] - pages, kc.shape[0], device=DEV)
+        bt = wide
+        for window in (1,):
+            out = torch.zeros(T, D, dtype=torch.bfloat16, device=DEV)
+            f.flash_prefill_tc(q, kc, vc, bt, i32([sum(q_len[:i]) for i in range(len(q_len))]), i32(q_len), i32(ctx), out, long, 1, 1, D, 16,
+                               window, 1 / math.sqrt(D), 16)
+            torch.cuda.synchronize()
+            f.check_status()
+            own = vc[bt[-1].long()].transpose(1, 2).reshape(-1, D)[:long]
+            assert torch.equal(out[-long:], own)              # a row that sees its own key alone is that key's value
+        return
+    out = torch.zeros(T, D, dtype=torch.bfloat16, device=DEV)
+    f.flash_prefill_tc(q, kc, vc, bt, i32([sum(q_len[:i]) for i in range(len(q_len))]), i32(q_len), i32(ctx), out, max(q_len), 1, 1, D, 16, 0,
+                       1 / math.sqrt(D), 16)
+    torch.cuda.synchronize()
+    f.check_status()
+    torch.testing.assert_close(out.double().view(T, 1, D), want, rtol=2e-2, atol=2e-2)
