@@ -40,6 +40,8 @@ _SIGS = {
     "hb_gemm_tc_rope_kv": [_p, _l, _p, _l, _i, _i, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _p, _p],
     "hb_attn_decode_supported": [_i, _i, _i],
     "hb_wait_selftest": [_p, _i, _p, _p],
+    "hb_gemm_split": [_p, _l, _p, _l, _p, _l, _i, _i, _i, _i, _p, _l, _p, _p],
+    "hb_gemm_split_workspace": [_i, _i, _i, _p],
     "hb_rows_norm_qkv_rope": [_p, _l, _p, _f, _p, _l, _i, _i, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _p, _p],
     "hb_rows_add": [_p, _l, _p, _l, _p, _l, _i, _i, _i, _p, _p, _l, _p, _i, _p, _p],
     "hb_rows_scaled_qkv_rope": [_p, _l, _p, _i, _f, _p, _l, _i, _i, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _p, _p],
@@ -276,13 +278,52 @@ def gemm_tc_slices(a, w):
     return sl
 
 
+# The 32-bit product on the tensor cores: from 9 rows on (up to 8 the plain kernel streams the weights once, at the memory's rate) and where it was
+# measured faster, us plain / here: 9 rows x 256 x 256 16 / 9, x 256 x 1,024 58 / 16; 600 x 256 x 256 17 / 13.5. Smaller ones stay plain.
+SPLIT_MIN_ROWS, SPLIT_MIN_WEIGHTS, SPLIT_MIN_K = 9, 1 << 16, 256
+
+
+def gemm_split(a, w, out, accumulate=False):
+    """out (+)= a @ w.T for 32-bit operands as sums of three bfloat16 numbers on the tensor cores (csrc/gemm_split.cu)."""
+    M, K = a.shape
+    N = w.shape[0]
+    key = ("split", M, N, K)
+    if key not in _plans:
+        f, n = _fn("hb_gemm_split_workspace"), C.c_int()
+        f.restype = C.c_long
+        _plans[key] = (f(M, N, K, C.byref(n)), n.value)
+    size, launches = _plans[key]
+    ws = torch.empty(size, dtype=torch.uint8, device=a.device)
+    library.launches[0] += launches
+    _call("hb_gemm_split", a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), M, N, K, 1 if accumulate else 0,
+          ws.data_ptr(), size, _status_ptr(), _stream())
+    return out
+
+
 def _gemm(a, w, out, epi):
     if a.shape[0] <= STREAM_MAX_ROWS:
         return gemm_stream(a, w, out, epi)
     return gemm_tc(a, w, out, epi)
 
 
+def linear32(a, w, out, accumulate) -> bool:
+    """The 32-bit product of more than a few rows on the tensor cores; False where its kernel does not take it, or no memory is left
+    for its workspace."""
+    if (PLAIN_ONLY or not SPLIT_MIN_ROWS <= a.shape[0] or a.dtype != torch.float32 or w.dtype != torch.float32 or out.dtype != torch.float32
+            or w.shape[0] * w.shape[1] < SPLIT_MIN_WEIGHTS or w.shape[1] < SPLIT_MIN_K
+            or (a.shape[1] | w.shape[0] | a.stride(0) | w.stride(0) | out.stride(0)) & 3
+            or (a.data_ptr() | w.data_ptr() | out.data_ptr()) & 15 or not (a.stride(1) == w.stride(1) == out.stride(1) == 1)):
+        return False
+    try:
+        gemm_split(a, w, out, accumulate)
+    except torch.OutOfMemoryError:
+        return False
+    return True
+
+
 def linear(a, w, out, accumulate) -> bool:
+    if a.dtype == torch.float32:
+        return linear32(a, w.t, out, accumulate)
     if not _tc_ok(a, w.t):
         return False
     if out.dtype == torch.float32:

@@ -668,8 +668,8 @@ class Weight:
 
 
 def linear(a: torch.Tensor, w: Weight, out: torch.Tensor, accumulate: bool = False) -> torch.Tensor:
-    """out (+)= a @ w.T. bfloat16 operands go to the tensor-core kernels when those take the
-    sizes; everything else to the plain 32-bit kernel."""
+    """out (+)= a @ w.T. bfloat16 operands, and 32-bit ones of more than a few rows, go to the tensor-core kernels when
+    those take the sizes; everything else to the plain 32-bit kernel."""
     if fast.linear(a, w, out, accumulate):
         return out
     return gemm_plain(a, w.t, out, accumulate)
@@ -719,7 +719,7 @@ def linear_swiglu(a: torch.Tensor, w_gate_up: Weight, act_out: torch.Tensor, gro
     if fast.linear_swiglu(a, w_gate_up, act_out, group):
         return act_out
     gu = torch.empty(a.shape[0], w_gate_up.shape[0], dtype=torch.float32, device=a.device)
-    gemm_plain(a, w_gate_up.t, gu)
+    linear(a, w_gate_up, gu)
     return swiglu(gu, act_out, group)
 
 

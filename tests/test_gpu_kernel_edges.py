@@ -146,3 +146,67 @@ def test_attention_of_more_items_than_a_list(D, requests, rows, long):
     torch.cuda.synchronize()
     f.check_status()
     torch.testing.assert_close(out.double().view(T, 1, D), want, rtol=2e-2, atol=2e-2)
+
+
+# rows around tiles of 16 and 160; N and K off the tiles of 128 and 64, with slices (few tiles, K of 1,024 and more) and without
+@pytest.mark.parametrize("M", [9, 16, 17, 160, 161, 330])
+@pytest.mark.parametrize("N,K", [(260, 260), (128, 4100), (20004, 320), (2048, 1024)])
+def test_products_of_split_32_bit_operands(M, N, K):
+    """Against 64 bits, stored and added. The bound: an MMA's sum is off by at most a unit in its last place, 2^-23 of the terms' magnitudes,
+    24 of them a block of 64 k; the blocks' and the slices' sums are rounded to nearest."""
+    from hipinfer_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(M + N)
+    a = (torch.randn(M, K, generator=g) * torch.exp(3 * torch.randn(M, 1, generator=g))).to(DEV)
+    w = (torch.randn(N, K, generator=g) * 0.1).to(DEV)
+    ref = a.double() @ w.double().T
+    bound = (32 + K / 64) * 2.0 ** -23 * (a.double().abs() @ w.double().abs().T)
+    out = torch.full((M + 1, N), 7.0, device=DEV)
+    assert fast().linear32(a, w, out[:M], False)
+    torch.cuda.synchronize()
+    fast().check_status()
+    assert bool(((out[:M].double() - ref).abs() <= bound).all()) and bool((out[M] == 7.0).all())
+    plain = torch.empty(M, N, device=DEV)
+    ops.gemm_plain(a, w, plain)
+    assert float((out[:M] - ref).norm()) <= float((plain - ref).norm())          # no less exact than the FFMA chains
+    acc = torch.randn(M, N, generator=g).to(DEV)
+    want = acc + out[:M]
+    assert fast().linear32(a, w, acc, True)
+    assert torch.equal(acc, want)
+
+
+@pytest.mark.parametrize("M,N,K", [(70, 260, 1028), (200, 20000, 512), (33, 1024, 4096)])
+def test_split_operands_that_are_no_sum_of_three(M, N, K):
+    """Infinities, NaN, numbers that round to an infinite bfloat16, and rows below the range of their remainders: where FFMA gives an infinity
+    or NaN so does this, and the rest is as exact."""
+    from hipinfer_b200.kernels import ops
+
+    a, w = torch.randn(M, K, generator=torch.Generator().manual_seed(1)).to(DEV), torch.randn(N, K, generator=torch.Generator().manual_seed(2)).to(DEV) * 0.1
+    a[3, 5], a[7, 9], a[20, 100] = math.inf, math.nan, 3.4e38
+    w[11, 3], w[130, 200] = -math.inf, 3.39e38
+    a[9] *= 1e-30
+    a[12] *= 1e-36
+    w[77] *= 1e-33
+    a[11], w[40] = 0, 0
+    plain, out = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    ops.gemm_plain(a, w, plain)
+    assert fast().linear32(a, w, out, False)
+    torch.cuda.synchronize()
+    fast().check_status()
+    assert torch.equal(torch.isinf(plain), torch.isinf(out)) and torch.equal(torch.isnan(plain), torch.isnan(out))
+    fine = torch.isfinite(plain)
+    size = a.double().abs() @ w.double().abs().T
+    # both within their bounds of the sum, and of a few units of the smallest number
+    assert bool(((plain.double() - out.double()).abs() <= (K + 96) * 2.0 ** -23 * size + 2.0 ** -140)[fine].all())
+
+
+def test_split_products_that_stay_plain():
+    """Forms the kernel does not take: few rows, K or rows off four, a view that starts off 16 bytes, other types."""
+    f = fast()
+    t = lambda *s: torch.zeros(*s, device=DEV)
+    assert not f.linear32(t(8, 512), t(512, 512), t(8, 512), False)
+    assert not f.linear32(t(16, 510), t(512, 510), t(16, 512), False)
+    assert not f.linear32(t(16, 512), t(511, 512), t(16, 511), False)
+    assert not f.linear32(t(16, 516)[:, 1:513], t(512, 512), t(16, 512), False)
+    assert not f.linear32(t(16, 512), t(512, 512).bfloat16(), t(16, 512), False)
+    assert not f.linear32(t(16, 512), t(64, 512), t(16, 64), False)
