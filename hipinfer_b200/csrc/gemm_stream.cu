@@ -92,41 +92,46 @@ __global__ void __launch_bounds__(192) gemm_stream_kernel(const __grid_constant_
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 4) {
-    if (lane == 0) {
-      // the weights do not depend on the kernel before this one: the first stages' weight tiles
-      // are requested before the wait, the activations after it
-      const int pre = num_kb < S::STAGES ? num_kb : S::STAGES;
+    // the weights do not depend on the kernel before this one: the first stages' weight tiles
+    // are requested before the wait, the activations after it
+    const int pre = num_kb < S::STAGES ? num_kb : S::STAGES;
+    if (hb_elect())
       for (int kb = 0; kb < pre; kb++) {
         hb_mbar_expect_tx(&full[kb], S::STAGE);
         hb_tma_load_2d(smem + kb * S::STAGE, &map_w, &full[kb], k_begin + kb * ST_BK, n0);
       }
-      hb_pdl_wait();
-      HB_TL_MARK_T(0, 1, 128);
+    __syncwarp();
+    hb_pdl_wait();
+    HB_TL_MARK_T(0, 1, 128);
+    if (hb_elect())
       for (int kb = 0; kb < pre; kb++)
         hb_tma_load_2d(smem + kb * S::STAGE + ST_W_BYTES, &map_x, &full[kb], k_begin + kb * ST_BK, 0);
-      for (int kb = pre; kb < num_kb; kb++) {
-        const uint32_t s = kb % S::STAGES, ph = (kb / S::STAGES) & 1;
-        if (!hb_mbar_wait(&empty[s], ph ^ 1, abort_flag)) break;
+    __syncwarp();
+    for (int kb = pre; kb < num_kb; kb++) {
+      const uint32_t s = kb % S::STAGES, ph = (kb / S::STAGES) & 1;
+      if (!__all_sync(0xffffffffu, hb_mbar_wait(&empty[s], ph ^ 1, abort_flag))) break;
+      if (hb_elect()) {
         hb_mbar_expect_tx(&full[s], S::STAGE);
         hb_tma_load_2d(smem + s * S::STAGE, &map_w, &full[s], k_begin + kb * ST_BK, n0);
         hb_tma_load_2d(smem + s * S::STAGE + ST_W_BYTES, &map_x, &full[s], k_begin + kb * ST_BK, 0);
       }
+      __syncwarp();
     }
   } else if (warp == 5) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = hb_umma_idesc_bf16(ST_ROWS, NT);
-      bool ok = true;
-      for (int kb = 0; kb < num_kb; kb++) {
-        const uint32_t s = kb % S::STAGES, ph = (kb / S::STAGES) & 1;
-        if (!hb_mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
-        hb_tc_fence_after();
+    constexpr uint32_t idesc = hb_umma_idesc_bf16(ST_ROWS, NT);
+    for (int kb = 0; kb < num_kb; kb++) {
+      const uint32_t s = kb % S::STAGES, ph = (kb / S::STAGES) & 1;
+      if (!__all_sync(0xffffffffu, hb_mbar_wait(&full[s], ph, abort_flag))) break;
+      hb_tc_fence_after();
+      if (hb_elect()) {
         const uint64_t dw = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE));
         const uint64_t dx = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE + ST_W_BYTES));
 #pragma unroll
         for (int k = 0; k < ST_BK / 16; k++) hb_umma_bf16(tmem_base, dw + 2 * k, dx + 2 * k, idesc, (kb | k) != 0);
         hb_umma_commit(&empty[s]);
+        if (kb == num_kb - 1) hb_umma_commit(done);
       }
-      if (ok) hb_umma_commit(done);
+      __syncwarp();
     }
   } else {
     // epilogue warps: lane = output column n0 + 32 * warp + lane, v[m] = token m
@@ -259,45 +264,55 @@ __global__ void __launch_bounds__(192, 1) gemm_stream_persist_kernel(const __gri
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 4) {
-    if (lane == 0) {  // ---------------- TMA producer; the ring's first weight tiles do not wait for the kernel ahead
+    {  // ---------------- TMA producer; the ring's first weight tiles do not wait for the kernel ahead
       const int pre = total < S::STAGES ? total : S::STAGES;
-      for (int it = 0; it < pre; it++) {
-        hb_mbar_expect_tx(&full[it], S::STAGE);
-        hb_tma_load_2d(smem + it * S::STAGE, &map_w, &full[it], it % num_kb * ST_BK, (int)(blockIdx.x + it / num_kb * gridDim.x) * ST_ROWS);
-      }
+      if (hb_elect())
+        for (int it = 0; it < pre; it++) {
+          hb_mbar_expect_tx(&full[it], S::STAGE);
+          hb_tma_load_2d(smem + it * S::STAGE, &map_w, &full[it], it % num_kb * ST_BK, (int)(blockIdx.x + it / num_kb * gridDim.x) * ST_ROWS);
+        }
+      __syncwarp();
       hb_pdl_wait();
-      for (int it = 0; it < pre; it++)
-        hb_tma_load_2d(smem + it * S::STAGE + ST_W_BYTES, &map_x, &full[it], it % num_kb * ST_BK, 0);
+      if (hb_elect())
+        for (int it = 0; it < pre; it++)
+          hb_tma_load_2d(smem + it * S::STAGE + ST_W_BYTES, &map_x, &full[it], it % num_kb * ST_BK, 0);
+      __syncwarp();
       int kb = pre % num_kb, nb = blockIdx.x + pre / num_kb * gridDim.x;
       for (int it = pre; it < total; it++) {
         const uint32_t s = it % S::STAGES, ph = (it / S::STAGES) & 1;
-        if (!hb_mbar_wait(&empty[s], ph ^ 1, abort_flag)) break;
-        hb_mbar_expect_tx(&full[s], S::STAGE);
-        hb_tma_load_2d(smem + s * S::STAGE, &map_w, &full[s], kb * ST_BK, nb * ST_ROWS);
-        hb_tma_load_2d(smem + s * S::STAGE + ST_W_BYTES, &map_x, &full[s], kb * ST_BK, 0);
+        if (!__all_sync(0xffffffffu, hb_mbar_wait(&empty[s], ph ^ 1, abort_flag))) break;
+        if (hb_elect()) {
+          hb_mbar_expect_tx(&full[s], S::STAGE);
+          hb_tma_load_2d(smem + s * S::STAGE, &map_w, &full[s], kb * ST_BK, nb * ST_ROWS);
+          hb_tma_load_2d(smem + s * S::STAGE + ST_W_BYTES, &map_x, &full[s], kb * ST_BK, 0);
+        }
+        __syncwarp();
         if (++kb == num_kb) { kb = 0; nb += gridDim.x; }
       }
     }
   } else if (warp == 5) {
-    if (lane == 0) {  // ---------------- MMA issuer
+    {  // ---------------- MMA issuer
       constexpr uint32_t idesc = hb_umma_idesc_bf16(ST_ROWS, NT);
       uint32_t it = 0;
       bool ok = true;
       for (int i = 0; i < mine && ok; i++) {
         const uint32_t buf = i & 1, aph = (i >> 1) & 1;
-        if (!hb_mbar_wait(&tmem_empty[buf], aph ^ 1, abort_flag)) break;
+        if (!__all_sync(0xffffffffu, hb_mbar_wait(&tmem_empty[buf], aph ^ 1, abort_flag))) break;
         hb_tc_fence_after();
         for (int kb = 0; kb < num_kb; kb++, it++) {
           const uint32_t s = it % S::STAGES, ph = (it / S::STAGES) & 1;
-          if (!hb_mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, hb_mbar_wait(&full[s], ph, abort_flag))) { ok = false; break; }
           hb_tc_fence_after();
-          const uint64_t dw = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE));
-          const uint64_t dx = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE + ST_W_BYTES));
+          if (hb_elect()) {
+            const uint64_t dw = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE));
+            const uint64_t dx = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE + ST_W_BYTES));
 #pragma unroll
-          for (int k = 0; k < ST_BK / 16; k++) hb_umma_bf16(tmem_base + buf * NT, dw + 2 * k, dx + 2 * k, idesc, (kb | k) != 0);
-          hb_umma_commit(&empty[s]);
+            for (int k = 0; k < ST_BK / 16; k++) hb_umma_bf16(tmem_base + buf * NT, dw + 2 * k, dx + 2 * k, idesc, (kb | k) != 0);
+            hb_umma_commit(&empty[s]);
+            if (kb == num_kb - 1) hb_umma_commit(&tmem_full[buf]);
+          }
+          __syncwarp();
         }
-        if (ok) hb_umma_commit(&tmem_full[buf]);
       }
     }
   } else {  // ---------------- epilogue warps: lane = output column, v[m] = token m
