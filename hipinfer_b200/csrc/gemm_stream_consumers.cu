@@ -37,8 +37,10 @@ __device__ __forceinline__ float4 slices_sum4(const float* p, int ksplit, long s
 // output head) x itself is left as it is: two entries may name the same row.
 // SLM: the slices whose loads are in flight together: with four a thread needs half the registers and two blocks lie on an SM, which a
 // portion's hundreds of rows want (512 rows of 3,072 from three slices: 14.0 us with sixteen, 10.7 with four).
-template <int NV, int SLM>
-__global__ void __launch_bounds__(512) add_rmsnorm_slices_kernel(float* x, long ldx, const float* ws,
+// TPB: 512 threads for a few rows (their latency counts); 256 for a portion's rows of up to four slices, so that three to four rows lie on an SM and
+// 512 of them are one round (512 rows of 3,072 from three slices: 7.3 us with 512 threads, 5.3 with 256).
+template <int NV, int SLM, int TPB>
+__global__ void __launch_bounds__(TPB) add_rmsnorm_slices_kernel(float* x, long ldx, const float* ws,
                                                                  int ksplit, long slice_stride, long row_stride,
                                                                  const __nv_bfloat16* __restrict__ w,
                                                                  __nv_bfloat16* __restrict__ y, const int* __restrict__ rows,
@@ -51,7 +53,7 @@ __global__ void __launch_bounds__(512) add_rmsnorm_slices_kernel(float* x, long 
   float4 ww[NV];
 #pragma unroll
   for (int i = 0; i < NV; i++) {   // the norm's weight does not depend on the kernel ahead
-    const int c = threadIdx.x + i * 512;
+    const int c = threadIdx.x + i * TPB;
     ww[i] = c < nvec ? hb_load4(w + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   hb_pdl_wait();
@@ -63,7 +65,7 @@ __global__ void __launch_bounds__(512) add_rmsnorm_slices_kernel(float* x, long 
   float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; i++) {
-    const int c = threadIdx.x + i * 512;
+    const int c = threadIdx.x + i * TPB;
     v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (c < nvec) {
       const float4 o = hb_load4(xr + 4 * c), a = slices_sum4<SLM>(pr + 4 * c, ksplit, slice_stride);
@@ -74,7 +76,7 @@ __global__ void __launch_bounds__(512) add_rmsnorm_slices_kernel(float* x, long 
   }
 #pragma unroll
   for (int i = 0; i < NV; i++) {   // behind all loads: for all the compiler knows x and the slices overlap
-    const int c = threadIdx.x + i * 512;
+    const int c = threadIdx.x + i * TPB;
     if (c < nvec && !rows) hb_store4(xr + 4 * c, v[i]);
   }
   HB_TL_MARK(tl, 2);
@@ -82,7 +84,7 @@ __global__ void __launch_bounds__(512) add_rmsnorm_slices_kernel(float* x, long 
   __nv_bfloat16* yr = y + (size_t)blockIdx.x * H;
 #pragma unroll
   for (int i = 0; i < NV; i++) {
-    const int c = threadIdx.x + i * 512;
+    const int c = threadIdx.x + i * TPB;
     if (c < nvec)
       hb_store4(yr + 4 * c, make_float4(ww[i].x * (v[i].x * inv), ww[i].y * (v[i].y * inv), ww[i].z * (v[i].z * inv),
                                         ww[i].w * (v[i].w * inv)));
@@ -100,12 +102,17 @@ HB_EXPORT int hb_add_rmsnorm_slices(float* x, long ldx, const float* ws, int ksp
   if (ksplit < 1) HB_FAIL("hb_add_rmsnorm_slices: %d slices", ksplit);
   const __nv_bfloat16* ww = (const __nv_bfloat16*)w;
   __nv_bfloat16* yy = (__nv_bfloat16*)y;
-#define HB_NS(NV)                                                                                                                   \
-  (ksplit <= 4 ? hb_launch(add_rmsnorm_slices_kernel<NV, 4>, M, 512, 0, s, x, ldx, ws, ksplit, slice_stride, row_stride, ww, yy, rows, H, eps) \
-               : hb_launch(add_rmsnorm_slices_kernel<NV, SL_MAX>, M, 512, 0, s, x, ldx, ws, ksplit, slice_stride, row_stride, ww, yy, rows, H, eps))
-  if (H <= 2048) HB_NS(1);
-  else if (H <= 4096) HB_NS(2);
-  else HB_NS(4);
+#define HB_NS(NV, SLM, TPB) hb_launch(add_rmsnorm_slices_kernel<NV, SLM, TPB>, M, TPB, 0, s, x, ldx, ws, ksplit, slice_stride, row_stride, ww, yy, rows, H, eps)
+  // (by the slices and the width alone: a row's bits do not depend on how many rows there are)
+  if (ksplit <= 4 && H <= 4096) {
+    if (H <= 1024) HB_NS(1, 4, 256);
+    else if (H <= 2048) HB_NS(2, 4, 256);
+    else if (H <= 3072) HB_NS(3, 4, 256);
+    else HB_NS(4, 4, 256);
+  } else if (ksplit <= 4) HB_NS(4, 4, 512);
+  else if (H <= 2048) HB_NS(1, SL_MAX, 512);
+  else if (H <= 4096) HB_NS(2, SL_MAX, 512);
+  else HB_NS(4, SL_MAX, 512);
 #undef HB_NS
   HB_CHECK_LAUNCH("hb_add_rmsnorm_slices");
   return 0;
