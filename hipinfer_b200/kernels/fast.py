@@ -287,14 +287,11 @@ def gemm_split(a, w, out, accumulate=False):
     """out (+)= a @ w.T for 32-bit operands as sums of three bfloat16 numbers on the tensor cores (csrc/gemm_split.cu)."""
     M, K = a.shape
     N = w.shape[0]
-    key = ("split", M, N, K)
-    if key not in _plans:
-        f, n = _fn("hb_gemm_split_workspace"), C.c_int()
-        f.restype = C.c_long
-        _plans[key] = (f(M, N, K, C.byref(n)), n.value)
-    size, launches = _plans[key]
+    f, launches = _fn("hb_gemm_split_workspace"), C.c_int()
+    f.restype = C.c_long
+    size = f(M, N, K, C.byref(launches))
     ws = torch.empty(size, dtype=torch.uint8, device=a.device)
-    library.launches[0] += launches
+    library.launches[0] += launches.value
     _call("hb_gemm_split", a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), M, N, K, 1 if accumulate else 0,
           ws.data_ptr(), size, _status_ptr(), _stream())
     return out
