@@ -335,7 +335,11 @@ __global__ void __launch_bounds__(FT_THREADS, 1) flash_prefill_tc_kernel(
         }
         if (i >= i0 + 2) {      // O of tile i - 2
           const uint32_t it = base + i - 2, s = it & 1, ph = (it >> 1) & 1;
-          ok = hb_mbar_wait(&bar->v_full[s], ph, abort_flag) && hb_mbar_wait(&bar->p_full[c], np & 1, abort_flag);
+          // P first. Across items a stage's tile before this one can be the OTHER chain's, and the wait for V could then return on the phase
+          // before that tile's (the same parity). Behind P every tile of the items before has been read (the softmax warps joined
+          // them), and of this item's the stage's last one was this chain's own. (K needs no such order: this item's Q came when both
+          // chains had read all K of the item before.)
+          ok = hb_mbar_wait(&bar->p_full[c], np & 1, abort_flag) && hb_mbar_wait(&bar->v_full[s], ph, abort_flag);
           if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
           np++;
           hb_tc_fence_after();

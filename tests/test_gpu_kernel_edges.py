@@ -112,6 +112,42 @@ def test_attention_items(D, Hq, Hkv, ctx, rows, window, ps):
     torch.testing.assert_close(out.double().view(T, Hq, D), want, rtol=2e-2, atol=2e-2)
 
 
+def items_behind_one_another(D, tiles):
+    """(heads, contexts) of requests of one query tile, 100 rows: for each (key tiles, first key tile) so many items that every CTA walks one
+    of them. The list goes by falling work and keeps the order of equals, so a CTA meets them in the order of `tiles`."""
+    heads = 16
+    ctas = torch.cuda.get_device_properties(0).multi_processor_count * (2 if D == 64 else 1)
+    return heads, [128 * (first + n - 1) + 20 for n, first in tiles for _ in range(-(-ctas // heads))]
+
+
+# key tiles of the items that a CTA walks one behind the other, and the first of them: an item of an odd number hands its chains' stages over
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("tiles,window", [
+    ([(5, 0), (3, 0), (3, 0), (2, 0), (1, 0)], 0),
+    ([(4, 0), (3, 0), (1, 0)], 0),
+    ([(3, 1), (3, 2), (3, 1), (3, 0), (1, 0)], 200),
+])
+def test_items_of_several_key_tiles_behind_one_another(D, tiles, window):
+    """Against 64 bits, and a request's bits are the same as by itself, every time."""
+    f = fast()
+    Hq, ctx = items_behind_one_another(D, tiles)
+    rows, Hkv, ps = [100] * len(ctx), 4, 16
+    q, kc, vc, bt, T, want = attention_case(Hq, Hkv, D, ps, ctx, rows, window, 41)
+    starts = [sum(rows[:i]) for i in range(len(rows))]
+    meta = (i32(starts), i32(rows), i32(ctx))
+    call = lambda q, bt, meta, out: f.flash_prefill_tc(q, kc, vc, bt, *meta, out, max(rows), Hq, Hkv, D, ps, window, 1 / math.sqrt(D), 16)
+    alone = torch.empty(T, Hq * D, dtype=torch.bfloat16, device=DEV)
+    for r, (s, n, c) in enumerate(zip(starts, rows, ctx)):
+        call(q[s:s + n], bt[r:r + 1], (i32([0]), i32([n]), i32([c])), alone[s:s + n])
+    torch.testing.assert_close(alone.double().view(T, Hq, D), want, rtol=2e-2, atol=2e-2)      # as above
+    for _ in range(10):
+        out = torch.zeros(T, Hq * D, dtype=torch.bfloat16, device=DEV)
+        call(q, bt, meta, out)
+        torch.cuda.synchronize()
+        f.check_status()
+        assert torch.equal(out, alone)
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("requests,rows,long", [(700, 16, 0), (40, 16, 16000)])      # more requests, and more query tiles, than one list holds
 def test_attention_of_more_items_than_a_list(D, requests, rows, long):
