@@ -163,31 +163,33 @@ __device__ __forceinline__ void ft_sort(const uint2* raw, uint32_t* entries, int
     entries[place] = e.x;
   }
 }
-// The loader of K or V: a warp brings the tiles of an item, page by page, through a ring of two; lane l holds page l of the tile.
+// The loader of K or V: a warp brings the tiles of an item, page by page, through a ring of two; lane l holds the page of a tile's place l. The
+// places behind the item's last page, and ahead of a window's first, have none. `fill` (V): they get boxes beyond the cache, which
+// arrive as zeros, since P is 0 there and 0 times what an earlier item left (another request's, perhaps an infinity or NaN) need not be 0. K
+// leaves them as they are: their scores are masked, whatever they are.
 template <int FT_D>
-__device__ __forceinline__ bool ft_bring(const FtSpan& sp, const int* table, int page_size, int Hkv, int h, const CUtensorMap* map, uint8_t* ring,
+__device__ __forceinline__ bool ft_bring(const FtSpan& sp, const int* table, int page_size, int Hkv, int h, bool fill, const CUtensorMap* map, uint8_t* ring,
                                          uint64_t* full, uint64_t* free, uint32_t& it, volatile int* abort_flag) {
   constexpr int NH = FT_D / 64, OPND = NH * FT_TILE;
-  const int lane = threadIdx.x & 31, last = sp.p_last / page_size;       // the item's last page
-  // the page of this lane in tile t, asked for one tile ahead
+  const int lane = threadIdx.x & 31, places = FT_BN / page_size, first = sp.lo / page_size, last = sp.p_last / page_size;
+  // the page of this lane's place in tile t, asked for one tile ahead
   auto page = [&](int t) {
-    const int pg = max((sp.kt_lo + t) * FT_BN, sp.lo) / page_size + lane;
-    return lane < FT_BN / page_size && pg <= last ? table[pg] : 0;
+    const int pg = (sp.kt_lo + t) * places + lane;
+    return lane < places && pg >= first && pg <= last ? table[pg] : -1;
   };
   int next = page(0);
   for (int t = 0; t < sp.n; t++, it++) {
     const uint32_t s = it & 1, ph = (it >> 1) & 1;
-    const int k_base = (sp.kt_lo + t) * FT_BN;
-    const int first_page = max(k_base, sp.lo) / page_size, np = min((k_base + FT_BN - 1) / page_size, last) - first_page + 1;
-    const int row = (next * Hkv + h) * page_size;
+    const uint32_t boxes = __ballot_sync(0xffffffffu, lane < places && (fill || next >= 0));
+    const int row = next >= 0 ? (next * Hkv + h) * page_size : -page_size;
     next = t + 1 < sp.n ? page(t + 1) : 0;
     if (!__all_sync(0xffffffffu, hb_mbar_wait(&free[s], ph ^ 1, abort_flag))) return false;
-    uint8_t* dst = ring + s * OPND + (first_page * page_size - k_base) * 128;   // rows of 128 bytes in each 64-column tile
-    if (hb_elect()) hb_mbar_expect_tx(&full[s], (uint32_t)np * page_size * FT_D * 2);
+    if (hb_elect()) hb_mbar_expect_tx(&full[s], (uint32_t)__popc(boxes) * page_size * FT_D * 2);
     __syncwarp();
-    for (int p = 0; p < np; p++, dst += page_size * 128) {
-      const int from = __shfl_sync(0xffffffffu, row, p);
+    for (uint32_t left = boxes; left; left &= left - 1) {
+      const int p = __ffs(left) - 1, from = __shfl_sync(0xffffffffu, row, p);
       if (hb_elect()) {
+        uint8_t* dst = ring + s * OPND + p * page_size * 128;            // rows of 128 bytes in each 64-column tile
 #pragma unroll
         for (int hf = 0; hf < NH; hf++) hb_tma_load_2d(dst + hf * FT_TILE, map, &full[s], hf * 64, from);
       }
@@ -260,14 +262,10 @@ __global__ void __launch_bounds__(FT_THREADS, 1) flash_prefill_tc_kernel(
     return;
   }
   ft_sort((const uint2*)sP, bar->entries, n_entries);
-  // masked keys of a last, ragged tile are never loaded: what the tensor core reads in their place must be finite (P is exactly 0
-  // there, and 0 * NaN would poison the row). Later tiles leave finite values behind.
-  for (int i = threadIdx.x; i < 4 * OPND / 16; i += FT_THREADS) ((uint4*)sK)[i] = make_uint4(0, 0, 0, 0);
   if (warp == 10) {
     hb_tmem_alloc(&bar->tmem_slot, 512);
     hb_tmem_relinquish();
   }
-  hb_fence_proxy_async();
   hb_tc_fence_before();
   __syncthreads();
   hb_tc_fence_after();
@@ -299,7 +297,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) flash_prefill_tc_kernel(
         }
         __syncwarp();
       }
-      ok = ft_bring<FT_D>(sp, bt + (size_t)e.w * bt_stride, page_size, Hkv, h, map, ring, full, free, it, abort_flag);
+      ok = ft_bring<FT_D>(sp, bt + (size_t)e.w * bt_stride, page_size, Hkv, h, !is_k, map, ring, full, free, it, abort_flag);
     }
   } else if (warp >= 10) {  // ---------------- tensor cores, chain c
     constexpr uint32_t idesc_s = hb_umma_idesc_bf16(FT_BM, FT_BN), idesc_o = ft_idesc_b_mn(FT_BM, FT_D);
@@ -544,12 +542,10 @@ __global__ void __launch_bounds__(256, 2) flash_prefill_tc64_kernel(
     return;
   }
   ft_sort((const uint2*)sP, bar->entries, n_entries);
-  for (int i = threadIdx.x; i < 2 * FT_TILE / 16; i += 256) ((uint4*)sV)[i] = make_uint4(0, 0, 0, 0);   // what P's zeros meet must be finite, as above
   if (warp == 6) {
     hb_tmem_alloc(&bar->tmem_slot, 256);
     hb_tmem_relinquish();
   }
-  hb_fence_proxy_async();
   hb_tc_fence_before();
   __syncthreads();
   hb_tc_fence_after();
@@ -574,7 +570,7 @@ __global__ void __launch_bounds__(256, 2) flash_prefill_tc64_kernel(
         }
         __syncwarp();
       }
-      ok = ft_bring<64>(ft_span(e, window), bt + (size_t)e.w * bt_stride, page_size, Hkv, h, is_k ? &map_k : &map_v, is_k ? sK : sV,
+      ok = ft_bring<64>(ft_span(e, window), bt + (size_t)e.w * bt_stride, page_size, Hkv, h, !is_k, is_k ? &map_k : &map_v, is_k ? sK : sV,
                         is_k ? bar->k_full : bar->v_full, is_k ? bar->k_free : bar->v_free, it, abort_flag);
     }
   } else if (warp == 6) {  // ---------------- tensor cores: S_i is issued before O_{i-1}, so it overlaps the softmax of tile i - 1

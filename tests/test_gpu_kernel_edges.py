@@ -148,6 +148,35 @@ def test_items_of_several_key_tiles_behind_one_another(D, tiles, window):
         assert torch.equal(out, alone)
 
 
+# items whose last tile has pages that are not loaded (and, with a window, whose first one has), behind items of requests with infinities and NaN
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("ps", [8, 16, 64])
+@pytest.mark.parametrize("tiles,window", [
+    ([(3, 0), (3, 0), (2, 0), (1, 0)], 0),
+    ([(3, 1), (3, 2), (3, 1), (1, 0)], 200),
+])
+def test_items_leave_nothing_to_other_requests(D, ps, tiles, window):
+    """Keys and values that are not finite in every second request's cache: the other requests' rows keep every bit."""
+    f = fast()
+    Hq, ctx = items_behind_one_another(D, tiles)
+    n, Hkv = 25, 4                                        # rows to position 44 of the last tile
+    q, kc, vc, bt, T, _ = attention_case(Hq, Hkv, D, ps, ctx, [n] * len(ctx), window, 51)
+    meta = (i32([n * r for r in range(len(ctx))]), i32([n] * len(ctx)), i32(ctx))
+    outs = []
+    for bad in (False, True):
+        if bad:
+            for r in range(0, len(ctx), 2):
+                pages = bt[r, :-(-(ctx[r] + n) // ps)].long()
+                kc[pages], vc[pages] = (math.nan, math.inf) if r % 4 else (-math.inf, math.nan)
+        out = torch.zeros(T, Hq * D, dtype=torch.bfloat16, device=DEV)
+        f.flash_prefill_tc(q, kc, vc, bt, *meta, out, n, Hq, Hkv, D, ps, window, 1 / math.sqrt(D), 16)
+        torch.cuda.synchronize()
+        f.check_status()
+        outs.append(out.view(len(ctx), n, -1))
+    assert bool(torch.isfinite(outs[0].float()).all()) and bool(torch.isnan(outs[1][::2].float()).all())
+    assert torch.equal(outs[0][1::2], outs[1][1::2])
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("requests,rows,long", [(700, 16, 0), (40, 16, 16000)])      # more requests, and more query tiles, than one list holds
 def test_attention_of_more_items_than_a_list(D, requests, rows, long):
