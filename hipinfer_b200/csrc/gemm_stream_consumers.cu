@@ -32,20 +32,21 @@ __device__ __forceinline__ float4 slices_sum4(const float* p, int ksplit, long s
   return acc;
 }
 
-// One block of 512 threads per row; the row stays in registers between the sum of squares and
-// the scaling (H a multiple of 4, at most 512 * 4 * NV). With `rows` (a gather of some rows, as before the
-// output head) x itself is left as it is: two entries may name the same row.
+// One block per row; the row stays in registers between the sum of squares and the scaling (H a multiple of 4, at most
+// TPB * 4 * NV). With `rows` (a gather of some rows, as before the output head) x itself is left as it is: two entries may name the same row.
 // SLM: the slices whose loads are in flight together: with four a thread needs half the registers and two blocks lie on an SM, which a
 // portion's hundreds of rows want (512 rows of 3,072 from three slices: 14.0 us with sixteen, 10.7 with four).
-// TPB: 512 threads for a few rows (their latency counts); 256 for a portion's rows of up to four slices, so that three to four rows lie on an SM and
-// 512 of them are one round (512 rows of 3,072 from three slices: 7.3 us with 512 threads, 5.3 with 256).
+// TPB: 512 threads, or 256 that each stand for two of the 512 and keep a sum of squares for each, so that all sums have the same order
+// and a row the same bits. Up to two rows an SM 512 threads are faster (us, 512 / 256 threads, three slices: 9 rows of 3,072 2.4 / 2.7, 128 2.5 /
+// 3.3, 256 rows of 2,048 2.6 / 2.9), above that 256, since more rows lie on an SM (512 rows of 3,072 6.9 / 5.3, 700 rows of 2,048 5.1 / 4.6). At
+// 2,048 < H <= 3,072, where 512 threads leave half of them idle in their second pass, the line is at one row an SM (149 rows 3.4 / 3.2).
 template <int NV, int SLM, int TPB>
 __global__ void __launch_bounds__(TPB) add_rmsnorm_slices_kernel(float* x, long ldx, const float* ws,
                                                                  int ksplit, long slice_stride, long row_stride,
                                                                  const __nv_bfloat16* __restrict__ w,
                                                                  __nv_bfloat16* __restrict__ y, const int* __restrict__ rows,
                                                                  int H, float eps) {
-  __shared__ float sh[32];
+  __shared__ float sh[16];
   hb_pdl_launch();
   const int tl = rows ? 2 : ksplit <= 8 ? 0 : 1;
   HB_TL_MARK(tl, 0);
@@ -61,8 +62,9 @@ __global__ void __launch_bounds__(TPB) add_rmsnorm_slices_kernel(float* x, long 
   const size_t r = rows ? (size_t)rows[blockIdx.x] : (size_t)blockIdx.x;
   float* xr = x + r * ldx;
   const float* pr = ws + r * row_stride;
+  constexpr int OF = 512 / TPB, WARPS = TPB / 32;       // the threads of 512 that this one stands for
   float4 v[NV];
-  float ss = 0.f;
+  float ss[OF] = {};
 #pragma unroll
   for (int i = 0; i < NV; i++) {
     const int c = threadIdx.x + i * TPB;
@@ -71,8 +73,9 @@ __global__ void __launch_bounds__(TPB) add_rmsnorm_slices_kernel(float* x, long 
       const float4 o = hb_load4(xr + 4 * c), a = slices_sum4<SLM>(pr + 4 * c, ksplit, slice_stride);
       v[i] = make_float4(o.x + a.x, o.y + a.y, o.z + a.z, o.w + a.w);
     }
-    ss = fmaf(v[i].x, v[i].x, ss); ss = fmaf(v[i].y, v[i].y, ss);
-    ss = fmaf(v[i].z, v[i].z, ss); ss = fmaf(v[i].w, v[i].w, ss);
+    float& q = ss[i % OF];
+    q = fmaf(v[i].x, v[i].x, q); q = fmaf(v[i].y, v[i].y, q);
+    q = fmaf(v[i].z, v[i].z, q); q = fmaf(v[i].w, v[i].w, q);
   }
 #pragma unroll
   for (int i = 0; i < NV; i++) {   // behind all loads: for all the compiler knows x and the slices overlap
@@ -80,7 +83,16 @@ __global__ void __launch_bounds__(TPB) add_rmsnorm_slices_kernel(float* x, long 
     if (c < nvec && !rows) hb_store4(xr + 4 * c, v[i]);
   }
   HB_TL_MARK(tl, 2);
-  const float inv = rsqrtf(hb_block_sum(ss, sh) / (float)H + eps);
+#pragma unroll
+  for (int o = 0; o < OF; o++) {
+    ss[o] = hb_warp_sum(ss[o]);
+    if ((threadIdx.x & 31) == 0) sh[o * WARPS + (threadIdx.x >> 5)] = ss[o];
+  }
+  __syncthreads();
+  float sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < 16; i++) sum += sh[i];
+  const float inv = rsqrtf(sum / (float)H + eps);
   __nv_bfloat16* yr = y + (size_t)blockIdx.x * H;
 #pragma unroll
   for (int i = 0; i < NV; i++) {
@@ -103,14 +115,17 @@ HB_EXPORT int hb_add_rmsnorm_slices(float* x, long ldx, const float* ws, int ksp
   const __nv_bfloat16* ww = (const __nv_bfloat16*)w;
   __nv_bfloat16* yy = (__nv_bfloat16*)y;
 #define HB_NS(NV, SLM, TPB) hb_launch(add_rmsnorm_slices_kernel<NV, SLM, TPB>, M, TPB, 0, s, x, ldx, ws, ksplit, slice_stride, row_stride, ww, yy, rows, H, eps)
-  // (by the slices and the width alone: a row's bits do not depend on how many rows there are)
-  if (ksplit <= 4 && H <= 4096) {
+  const int few = H > 2048 && H <= 3072 ? 148 : 2 * 148;   // (148 SMs)
+  if (ksplit <= 4 && H <= 4096 && M > few) {
     if (H <= 1024) HB_NS(1, 4, 256);
     else if (H <= 2048) HB_NS(2, 4, 256);
     else if (H <= 3072) HB_NS(3, 4, 256);
     else HB_NS(4, 4, 256);
-  } else if (ksplit <= 4) HB_NS(4, 4, 512);
-  else if (H <= 2048) HB_NS(1, SL_MAX, 512);
+  } else if (ksplit <= 4) {
+    if (H <= 2048) HB_NS(1, 4, 512);
+    else if (H <= 4096) HB_NS(2, 4, 512);
+    else HB_NS(4, 4, 512);
+  } else if (H <= 2048) HB_NS(1, SL_MAX, 512);
   else if (H <= 4096) HB_NS(2, SL_MAX, 512);
   else HB_NS(4, SL_MAX, 512);
 #undef HB_NS

@@ -275,3 +275,32 @@ def test_split_products_that_stay_plain():
     assert not f.linear32(t(16, 516)[:, 1:513], t(512, 512), t(16, 512), False)
     assert not f.linear32(t(16, 512), t(512, 512).bfloat16(), t(16, 512), False)
     assert not f.linear32(t(16, 512), t(64, 512), t(16, 64), False)
+
+
+# widths at and off the steps of the kernel's forms; rows at the lines where it changes from 512 threads a row to 256
+@pytest.mark.parametrize("H", [8, 1000, 1024, 2048, 2052, 3072, 4096])
+@pytest.mark.parametrize("slices", [1, 3, 4])
+def test_norm_of_slices_has_the_same_bits_in_every_form(H, slices):
+    """A row's sum and norm do not depend on how many rows there are, nor on whether slices of zeros follow (more than four take another form)."""
+    f = fast()
+    rows = 300
+    g = torch.Generator().manual_seed(H + slices)
+    x0, part = torch.randn(rows, H, generator=g).to(DEV), torch.randn(slices, rows, H, generator=g).to(DEV)
+    w = rnd(H, seed=61)
+
+    def norm(m, count):
+        sl = f.Slices()
+        sl.ws = torch.cat([part[:, :m], torch.zeros(count - slices, m, H, device=DEV)]).contiguous()
+        sl.ksplit, sl.row_stride, sl.slice_stride, sl.M, sl.N, sl.K, sl.gen = count, H, m * H, m, H, 0, None
+        x, y = x0[:m].clone(), torch.empty(m, H, dtype=torch.bfloat16, device=DEV)
+        f.add_rmsnorm_slices(x, sl, w, 1e-5, y)
+        torch.cuda.synchronize()
+        return x, y
+
+    x, y = norm(rows, 6)
+    total = x0.double() + part.double().sum(0)
+    want = total * torch.rsqrt(total.square().mean(1, keepdim=True) + 1e-5) * w.double()
+    torch.testing.assert_close(y.double(), want, rtol=2.0 ** -8, atol=1e-5)       # one rounding to bfloat16 of 32-bit sums
+    for m in (1, 9, 148, 149, 296, 297, 300):
+        a, b = norm(m, slices)
+        assert torch.equal(a, x[:m]) and torch.equal(b, y[:m]), m
