@@ -197,16 +197,23 @@ __device__ __forceinline__ bool ft_bring(const FtSpan& sp, const int* table, int
   }
   return true;
 }
-// The exponentials of two scores, rounded to bf16 for P and added to the row's sums.
+// The exponentials of two scores.
 template <bool EX>
-__device__ __forceinline__ uint32_t ft_prob(uint32_t s0, uint32_t s1, uint64_t scale2, uint64_t sub2, float r1, float r2, float dist, uint64_t& sum2) {
+__device__ __forceinline__ void ft_exp(uint32_t s0, uint32_t s1, uint64_t scale2, uint64_t sub2, float r1, float r2, float dist, float& p0, float& p1) {
   float e0, e1;
   ft_unpack2(ft_fma2(ft_pack2(s0, s1), scale2, sub2), e0, e1);
   if (EX) {   // (a key behind the row is masked: any finite bias will do)
     e0 = fmaf(-r1, __log2f(fmaxf(fmaf(r2, dist, 1.f), 1.f)), e0);
     e1 = fmaf(-r1, __log2f(fmaxf(fmaf(r2, dist - 1.f, 1.f), 1.f)), e1);
   }
-  const float p0 = hb_exp2(e0), p1 = hb_exp2(e1);
+  p0 = hb_exp2(e0);
+  p1 = hb_exp2(e1);
+}
+// And rounded to bf16 for P, and added to the row's sums.
+template <bool EX>
+__device__ __forceinline__ uint32_t ft_prob(uint32_t s0, uint32_t s1, uint64_t scale2, uint64_t sub2, float r1, float r2, float dist, uint64_t& sum2) {
+  float p0, p1;
+  ft_exp<EX>(s0, s1, scale2, sub2, r1, r2, dist, p0, p1);
   sum2 = ft_add2(sum2, ft_pack2(__float_as_uint(p0), __float_as_uint(p1)));
   return hb_pack_bf16(p0, p1);
 }
@@ -664,7 +671,7 @@ __global__ void __launch_bounds__(256, 2) flash_prefill_tc64_kernel(
         }
         const float sub = m_run == -INFINITY ? 0.f : m_run;
         const uint64_t scale2 = ft_pack2(__float_as_uint(scale_log2), __float_as_uint(scale_log2)), sub2 = ft_pack2(__float_as_uint(-sub), __float_as_uint(-sub));
-        uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};
+        uint64_t sum2[2] = {0ull, 0ull};   // four sums of pairs
         // the exponentials: keys 64-127 are still in the registers (masked), keys 0-63 are read again
 #pragma unroll
         for (int hh = 1; hh >= 0; hh--) {
@@ -682,8 +689,14 @@ __global__ void __launch_bounds__(256, 2) flash_prefill_tc64_kernel(
             }
           }
 #pragma unroll
-          for (int j = 0; j < 64; j += 2)  // masked scores are -inf: 2^-inf = 0
-            sr[j >> 1] = ft_prob<EX>(sr[j], sr[j + 1], scale2, sub2, r1, r2, dist0 - (float)(j + hh * 64), sum2[(j >> 1) & 3]);
+          for (int j = 0; j < 64; j += 4) {  // masked scores are -inf: 2^-inf = 0
+            float p0, p1, p2, p3;
+            ft_exp<EX>(sr[j], sr[j + 1], scale2, sub2, r1, r2, dist0 - (float)(j + hh * 64), p0, p1);
+            ft_exp<EX>(sr[j + 2], sr[j + 3], scale2, sub2, r1, r2, dist0 - (float)(j + 2 + hh * 64), p2, p3);
+            sum2[(j >> 2) & 1] = ft_add2(sum2[(j >> 2) & 1], ft_pack2(__float_as_uint(p0 + p1), __float_as_uint(p2 + p3)));
+            sr[j >> 1] = hb_pack_bf16(p0, p1);
+            sr[(j >> 1) + 1] = hb_pack_bf16(p2, p3);
+          }
           // the product of the tile before has read its P and written its O
           if (hh == 1 && cnt > 0 && !__all_sync(0xffffffffu, hb_mbar_wait(&bar->pv_done, (cnt - 1) & 1, abort_flag))) { ok = false; break; }
           // 64 keys = eight 16-byte chunks of this row in K block hh of P
@@ -695,9 +708,10 @@ __global__ void __launch_bounds__(256, 2) flash_prefill_tc64_kernel(
           }
         }
         if (!ok) break;
-        float s0, s1;
-        ft_unpack2(ft_add2(ft_add2(sum2[0], sum2[1]), ft_add2(sum2[2], sum2[3])), s0, s1);
-        l_run = l_run * corr + (s0 + s1);
+        float s0, s1, s2, s3;
+        ft_unpack2(sum2[0], s0, s1);
+        ft_unpack2(sum2[1], s2, s3);
+        l_run = l_run * corr + ((s0 + s1) + (s2 + s3));
         if (i > 0 && __any_sync(0xffffffffu, grow)) {   // a raised maximum: the row of O so far
           hb_tc_fence_after();
           hb_tmem_ld64_nowait(tmem_o + lane_base, sr);
