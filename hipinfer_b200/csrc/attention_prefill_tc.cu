@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) flash_prefill_tc_kernel(
       hb_tc_fence_after();
       if (ok) {
         const float2 a = ((const float2*)sP)[r], b = ((const float2*)(sP + 2 * FT_TILE))[r];
-        const float m = fmaxf(a.x, b.x);
+        const float top = fmaxf(a.x, b.x), m = top == -INFINITY ? 0.f : top;   // (no score above -inf: with a sink the row is 0)
         const float fa = hb_exp2(a.x - m), fb = hb_exp2(b.x - m);   // a chain without a visible key: 2^-inf = 0
         float l = a.y * fa + b.y * fb;
         if (EX && sink) l += hb_exp2(fmaf(sink[hq], 1.4426950408889634f, -m));

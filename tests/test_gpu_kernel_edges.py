@@ -178,6 +178,22 @@ def test_items_leave_nothing_to_other_requests(D, ps, tiles, window):
 
 
 @pytest.mark.parametrize("D", [64, 128])
+def test_a_row_whose_scores_are_all_minus_infinity(D):
+    """With a sink the denominator is the sink's alone: the row is 0, as far as its values are finite."""
+    f = fast()
+    Hq, Hkv, ps, n = 2, 1, 16, 200
+    q, kc, vc, bt, T, _ = attention_case(Hq, Hkv, D, ps, [0], [n], 0, 71)
+    q.view(n, Hq, D)[:, :, 0], q.view(n, Hq, D)[0, :, 0] = 0, 1e30         # the first row, which sees the first key alone, scores it -1e60
+    kc[bt[0, 0].long(), :, 0, 0] = -1e30
+    sink = torch.tensor([0.5, -3.0], device=DEV)
+    out = torch.full((T, Hq * D), 7.0, dtype=torch.bfloat16, device=DEV)
+    f.flash_prefill_tc(q, kc, vc, bt, i32([0]), i32([n]), i32([0]), out, n, Hq, Hkv, D, ps, 0, 1 / math.sqrt(D), 16, sink=sink)
+    torch.cuda.synchronize()
+    f.check_status()
+    assert bool((out[0] == 0).all()) and bool(torch.isfinite(out.float()).all())
+
+
+@pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("requests,rows,long", [(700, 16, 0), (40, 16, 16000)])      # more requests, and more query tiles, than one list holds
 def test_attention_of_more_items_than_a_list(D, requests, rows, long):
     q_len = [rows] * requests + ([long] if long else [])
