@@ -45,7 +45,10 @@
 constexpr int FT_BM = 128, FT_BN = 128;
 constexpr int FT_TILE = 128 * 64 * 2;  // one [128][64] bf16 tile: 16 KB; a [128][head_dim] operand is head_dim / 64 of them, 64 columns each
 constexpr int FT_THREADS = 384;        // 168 registers each: a row of S is 128 of them
-constexpr int FT_MAX_ENTRIES = 640, FT_MAX_ENTRIES64 = 200;    // (request, query tile) pairs of one launch; the launcher cuts larger steps
+// A launch lists up to FT_MAX_PAIRS (request, query tile) pairs, in the place of P, and a CTA keeps the pairs of its own items, FT_OWN at most; the
+// launcher cuts steps of more. (When every CTA kept all pairs, 200 of them at head_dim 64, one request of 32,768 rows was 43 launches and took
+// 10.8 ms, now 6.7; 16,000 rows beside 300 single rows 3.1 ms, now 1.6.)
+constexpr int FT_MAX_PAIRS = 4096, FT_OWN = 640, FT_OWN64 = 200;
 
 // MN-major operand with the 128-byte swizzle: 64 contiguous elements of the MN dimension per row,
 // eight K rows per 1,024-byte group (stride SBO); further MN atoms would lie LBO apart (one here).
@@ -86,7 +89,7 @@ __device__ __forceinline__ void ft_st32(uint32_t taddr, const uint32_t* r) {
 // head_dim 128: Q, P of both chains, rings of two K and two V tiles, and the list of the items.
 struct FtBars {
   uint64_t q_full, q_free, k_full[2], k_free[2], v_full[2], v_free[2], s_full[2], s_free[2], p_full[2], pv_done[2];
-  uint32_t entries[FT_MAX_ENTRIES];  // request << 16 | query tile, by falling work
+  uint32_t own[FT_OWN];              // request << 16 | query tile of this CTA's items, in their order
   int n_entries;
   uint32_t tmem_slot;
   int abort_flag;
@@ -95,13 +98,14 @@ constexpr int FT_SMEM = 14 * FT_TILE + (int)sizeof(FtBars);
 // head_dim 64: Q, P, rings of two K and two V tiles.
 struct FtBars64 {
   uint64_t q_full, q_free, k_full[2], k_free[2], v_full[2], v_free[2], s_full, s_free, p_full, pv_done;
-  uint32_t entries[FT_MAX_ENTRIES64];
+  uint32_t own[FT_OWN64];
   int n_entries;
   uint32_t tmem_slot;
   int abort_flag;
 };
 constexpr int FT_SMEM64 = 7 * FT_TILE + (int)sizeof(FtBars64);
 static_assert(FT_SMEM <= 227 * 1024 && 2 * (FT_SMEM64 + 1024) <= 228 * 1024, "shared memory of one block and of two");
+static_assert(FT_MAX_PAIRS * sizeof(uint2) <= 2 * FT_TILE, "the unordered pairs lie where P will");
 
 // Item k of this CTA: CTAs take the items in turn, back and forth (the items come by falling work).
 __device__ __forceinline__ int ft_item(int k) { return k * (int)gridDim.x + ((k & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x); }
@@ -151,8 +155,9 @@ __device__ __forceinline__ void ft_list(uint2* raw, int* n_entries, int most, co
   }
   if (lane == 0) *n_entries = min(n, most);
 }
-// All threads: the pairs by falling work; a pair's place is the number of pairs with more key tiles to walk.
-__device__ __forceinline__ void ft_sort(const uint2* raw, uint32_t* entries, int n_entries) {
+// All threads: the pairs by falling work; a pair's place is the number of pairs with more key tiles to walk, its items are Hq in a row from place *
+// Hq on, and those of them that are this CTA's are kept (at most one in gridDim.x items).
+__device__ __forceinline__ void ft_sort(const uint2* raw, uint32_t* own, int n_entries, int Hq) {
   for (int i = threadIdx.x; i < n_entries; i += blockDim.x) {
     const uint2 e = raw[i];
     int place = 0;
@@ -160,7 +165,11 @@ __device__ __forceinline__ void ft_sort(const uint2* raw, uint32_t* entries, int
       const uint32_t w = raw[j].y;
       place += w > e.y || (w == e.y && j < i);
     }
-    entries[place] = e.x;
+    const int u0 = place * Hq, u1 = u0 + Hq;
+    for (int k = u0 / (int)gridDim.x; k * (int)gridDim.x < u1; k++) {
+      const int u = ft_item(k);
+      if (u >= u0 && u < u1) own[k] = e.x;
+    }
   }
 }
 // The loader of K or V: a warp brings the tiles of an item, page by page, through a ring of two; lane l holds the page of a tile's place l. The
@@ -227,7 +236,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) flash_prefill_tc_kernel(
     const __grid_constant__ CUtensorMap map_v, const int* __restrict__ bt, int bt_stride, const int* __restrict__ q_start,
     const int* __restrict__ q_len, const int* __restrict__ ctx_len, __nv_bfloat16* __restrict__ out, int Hq, int Hkv,
     int page_size, int window, float scale_log2, int min_rows, int* status, const float* __restrict__ r1p,
-    const float* __restrict__ r2p, const float* __restrict__ sink, int req0, int reqs, int qt0, int qts) {
+    const float* __restrict__ r2p, const float* __restrict__ sink, int req0, int reqs, int qt0, int qts, int most) {
   constexpr int FT_D = 128, NH = FT_D / 64, OPND = NH * FT_TILE;
   // the 128-byte swizzle wants the tiles on 1 KB boundaries, and there is no room for slack: checked below
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -247,7 +256,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) flash_prefill_tc_kernel(
     return;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == 0) ft_list((uint2*)sP, &bar->n_entries, FT_MAX_ENTRIES, q_len, ctx_len, window, min_rows, req0, reqs, qt0, qts);
+  if (warp == 0) ft_list((uint2*)sP, &bar->n_entries, most, q_len, ctx_len, window, min_rows, req0, reqs, qt0, qts);
   if (threadIdx.x == 32) {
     hb_mbar_init(&bar->q_full, 1); hb_mbar_init(&bar->q_free, 2);
     for (int b = 0; b < 2; b++) {
@@ -268,7 +277,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) flash_prefill_tc_kernel(
     hb_pdl_wait();
     return;
   }
-  ft_sort((const uint2*)sP, bar->entries, n_entries);
+  ft_sort((const uint2*)sP, bar->own, n_entries, Hq);
   if (warp == 10) {
     hb_tmem_alloc(&bar->tmem_slot, 512);
     hb_tmem_relinquish();
@@ -280,7 +289,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) flash_prefill_tc_kernel(
   hb_pdl_wait();   // barriers, shared and tensor memory were set up while the kernel ahead was still running
 
   // an item's numbers are fetched while the one before it is worked on
-  auto entry = [&](int k) { const int u = ft_item(k); return ft_entry(bar->entries[u < n_items ? u / Hq : 0], q_start, q_len, ctx_len); };
+  auto entry = [&](int k) { const int u = ft_item(k); return ft_entry(bar->own[u < n_items ? k : 0], q_start, q_len, ctx_len); };
 
   if (warp == 8 || warp == 9) {  // ---------------- TMA: lane l brings page l of a tile
     const bool is_k = warp == 8;
@@ -513,7 +522,7 @@ __global__ void __launch_bounds__(256, 2) flash_prefill_tc64_kernel(
     const __grid_constant__ CUtensorMap map_v, const int* __restrict__ bt, int bt_stride, const int* __restrict__ q_start,
     const int* __restrict__ q_len, const int* __restrict__ ctx_len, __nv_bfloat16* __restrict__ out, int Hq, int Hkv,
     int page_size, int window, float scale_log2, int min_rows, int* status, const float* __restrict__ r1p,
-    const float* __restrict__ r2p, const float* __restrict__ sink, int req0, int reqs, int qt0, int qts) {
+    const float* __restrict__ r2p, const float* __restrict__ sink, int req0, int reqs, int qt0, int qts, int most) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sQ = smem;                 // [128][64]
   uint8_t* sP = sQ + FT_TILE;         // two K blocks of [128 rows][64 keys]
@@ -529,7 +538,7 @@ __global__ void __launch_bounds__(256, 2) flash_prefill_tc64_kernel(
     return;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == 0) ft_list((uint2*)sP, &bar->n_entries, FT_MAX_ENTRIES64, q_len, ctx_len, window, min_rows, req0, reqs, qt0, qts);
+  if (warp == 0) ft_list((uint2*)sP, &bar->n_entries, most, q_len, ctx_len, window, min_rows, req0, reqs, qt0, qts);
   if (threadIdx.x == 32) {
     hb_mbar_init(&bar->q_full, 1); hb_mbar_init(&bar->q_free, 1);
     for (int b = 0; b < 2; b++) {
@@ -548,7 +557,7 @@ __global__ void __launch_bounds__(256, 2) flash_prefill_tc64_kernel(
     hb_pdl_wait();
     return;
   }
-  ft_sort((const uint2*)sP, bar->entries, n_entries);
+  ft_sort((const uint2*)sP, bar->own, n_entries, Hq);
   if (warp == 6) {
     hb_tmem_alloc(&bar->tmem_slot, 256);
     hb_tmem_relinquish();
@@ -559,7 +568,7 @@ __global__ void __launch_bounds__(256, 2) flash_prefill_tc64_kernel(
   const uint32_t tmem_s = bar->tmem_slot, tmem_o = tmem_s + FT_BN;  // S: 128 columns, O: 64 columns
   hb_pdl_wait();
 
-  auto entry = [&](int k) { const int u = ft_item(k); return ft_entry(bar->entries[u < n_items ? u / Hq : 0], q_start, q_len, ctx_len); };
+  auto entry = [&](int k) { const int u = ft_item(k); return ft_entry(bar->own[u < n_items ? k : 0], q_start, q_len, ctx_len); };
   if (warp == 4 || warp == 5) {  // ---------------- TMA
     const bool is_k = warp == 4;
     uint32_t it = 0;
@@ -778,6 +787,37 @@ static int ft_sms() {
   return n[dev];
 }
 
+// How a step is cut into launches. Portions of T rows in all have at most T / 128 (request, query tile) pairs and one more each, and there are at
+// most T / min_rows portions; a launch takes `most` pairs (as many as a CTA has places for its share of the items). A step that may have more is cut
+// into launches of req_step requests, or of req_step requests and qt_step query tiles.
+struct FtCut { int req_step, qt_step, tiles, most, ctas; long bound; };
+static FtCut ft_cut(int T, int R, int max_q_len, int Hq, int D, int min_rows) {
+  FtCut c;
+  c.tiles = (max_q_len + FT_BM - 1) / FT_BM;
+  c.ctas = (D == 64 ? 2 : 1) * ft_sms();
+  const long share = (long)(D == 64 ? FT_OWN64 : FT_OWN) * c.ctas / Hq;
+  c.most = share < FT_MAX_PAIRS ? (int)share : FT_MAX_PAIRS;
+  const long full = T / FT_BM, portions = min_rows > 1 && T / min_rows < R ? T / min_rows : R;
+  c.bound = full + portions;
+  c.req_step = R;
+  c.qt_step = c.tiles;
+  if (c.most > 0 && c.bound > c.most && (long)R * c.tiles > c.most) {
+    if (full <= c.most / 2) c.req_step = c.most - (int)full;
+    else {
+      c.req_step = R < 32 ? R : 32;
+      if (c.req_step > c.most) c.req_step = c.most;
+      c.qt_step = c.most / c.req_step;
+    }
+  }
+  return c;
+}
+// The launches that a step of these sizes is.
+HB_EXPORT int hb_flash_prefill_tc_launches(int T, int R, int max_q_len, int Hq, int D, int min_rows) {
+  if (R <= 0 || max_q_len <= 0 || T <= 0) return 0;
+  const FtCut c = ft_cut(T, R, max_q_len, Hq, D, min_rows);
+  return ((R + c.req_step - 1) / c.req_step) * ((c.tiles + c.qt_step - 1) / c.qt_step);
+}
+
 // q, out [T, Hq, D] bf16; caches [num_pages, Hkv, page_size, D] bf16 (D 64 or 128); per request q_start, q_len,
 // ctx_len and a block table row, as hb_flash_prefill. Requests with fewer than min_rows rows are
 // skipped. `status` is set to 1 if a bounded wait ran out.
@@ -800,15 +840,8 @@ HB_EXPORT int hb_flash_prefill_tc(const void* q, const void* kc, const void* vc,
   if (hb_make_tensor_map_bf16(&mv, vc, rows, (uint64_t)D, (uint64_t)D, (uint32_t)page_size)) return -1;
   const float sl2 = scale * 1.4426950408889634f;
   cudaError_t e = cudaSuccess;
-  // (request, query tile) pairs: portions of T rows in all have at most T / 128 tiles and one more each, and there are at most T / min_rows
-  // portions. A step of more pairs than the list holds is cut into launches of some requests, or of some requests and query tiles.
-  const int tiles = (max_q_len + FT_BM - 1) / FT_BM, most = D == 64 ? FT_MAX_ENTRIES64 : FT_MAX_ENTRIES;
-  const long full = T / FT_BM, portions = min_rows > 1 && T / min_rows < R ? T / min_rows : R, bound = full + portions;
-  int req_step = R, qt_step = tiles;
-  if (bound > most && (long)R * tiles > most) {
-    if (full <= most / 2) req_step = most - (int)full;
-    else { req_step = 32; qt_step = most / 32; }
-  }
+  const FtCut c = ft_cut(T, R, max_q_len, Hq, D, min_rows);
+  if (c.most < 1) HB_FAIL("hb_flash_prefill_tc: %d heads are beyond the list of items", Hq);
 #define FT_LAUNCH(KERN, THREADS, SMEM)                                                                                           \
   do {                                                                                                                          \
     static bool configured = false;                                                                                             \
@@ -818,13 +851,15 @@ HB_EXPORT int hb_flash_prefill_tc(const void* q, const void* kc, const void* vc,
       configured = true;                                                                                                        \
     }                                                                                                                           \
     e = hb_launch(KERN, grid, THREADS, SMEM, st, mq, mk, mv, bt, bt_stride, q_start, q_len, ctx_len, (__nv_bfloat16*)out, Hq,   \
-                  Hkv, page_size, window, sl2, min_rows, status, r1, r2, sink, req0, reqs, qt0, qts);                           \
+                  Hkv, page_size, window, sl2, min_rows, status, r1, r2, sink, req0, reqs, qt0, qts, most);         \
   } while (0)
-  for (int req0 = 0; req0 < R && e == cudaSuccess; req0 += req_step)
-    for (int qt0 = 0; qt0 < tiles && e == cudaSuccess; qt0 += qt_step) {
-      const int reqs = R - req0 < req_step ? R - req0 : req_step, qts = tiles - qt0 < qt_step ? tiles - qt0 : qt_step;
-      const long items = ((long)reqs * qts < bound ? (long)reqs * qts : bound) * Hq, ctas = (D == 64 ? 2 : 1) * ft_sms();
-      const int grid = (int)(items < ctas ? (items > 0 ? items : 1) : ctas);
+  for (int req0 = 0; req0 < R && e == cudaSuccess; req0 += c.req_step)
+    for (int qt0 = 0; qt0 < c.tiles && e == cudaSuccess; qt0 += c.qt_step) {
+      const int reqs = R - req0 < c.req_step ? R - req0 : c.req_step, qts = c.tiles - qt0 < c.qt_step ? c.tiles - qt0 : c.qt_step;
+      const long items = ((long)reqs * qts < c.bound ? (long)reqs * qts : c.bound) * Hq;
+      const int grid = (int)(items < c.ctas ? (items > 0 ? items : 1) : c.ctas);
+      const long share = (long)(D == 64 ? FT_OWN64 : FT_OWN) * grid / Hq;      // (of a smaller grid: whatever the lengths say, a CTA's items have places)
+      const int most = share < c.most ? (int)share : c.most;
       if (D == 64 && !ex) FT_LAUNCH(flash_prefill_tc64_kernel<false>, 256, FT_SMEM64);
       else if (D == 64) FT_LAUNCH(flash_prefill_tc64_kernel<true>, 256, FT_SMEM64);
       else if (!ex) FT_LAUNCH(flash_prefill_tc_kernel<false>, FT_THREADS, FT_SMEM);

@@ -32,6 +32,7 @@ _SIGS = {
     "hb_flash_prefill_supported": [_i, _i, _i],
     "hb_flash_prefill_tc": [_p, _p, _p, _l, _p, _i, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _p, _p, _p, _p, _p],
     "hb_flash_prefill_tc_supported": [_i, _i, _i, _i],
+    "hb_flash_prefill_tc_launches": [_i, _i, _i, _i, _i, _i],
     "hb_attn_diff_decode": [_p, _p, _p, _l, _p, _i, _p, _p, _p, _l, _i, _p, _p, _p, _i, _i, _i, _i, _i, _i, _f, _f, _f, _f, _i, _p, _i, _p, _p, _p],
     "hb_attn_diff_decode_supported": [_i, _i, _i, _i],
     "hb_attn_diff_decode_splits": [_i, _i, _i],

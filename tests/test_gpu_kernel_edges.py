@@ -320,3 +320,31 @@ def test_norm_of_slices_has_the_same_bits_in_every_form(H, slices):
     for m in (1, 9, 148, 149, 296, 297, 300):
         a, b = norm(m, slices)
         assert torch.equal(a, x[:m]) and torch.equal(b, y[:m]), m
+
+
+def test_launches_of_large_attention_steps():
+    """One request, some long ones, and a portion beside hundreds of single rows are one launch; sizes beyond a list are a few."""
+    launches = fast()._fn("hb_flash_prefill_tc_launches")
+    for D in (64, 128):
+        assert launches(32768, 1, 32768, 32, D, 16) == 1
+        assert launches(131072, 3, 131072, 32, D, 16) == 1
+        assert launches(32768 + 300, 301, 32768, 32, D, 16) == 1
+        assert launches(1 << 20, 1, 1 << 20, 32, D, 16) <= 5
+        assert launches(1 << 20, 8, 1 << 20, 32, D, 16) <= 40
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("requests,tokens,heads", [(850, 16, 128), (4300, 16, 1), (3, 32000, 128)])
+def test_attention_of_more_pairs_than_a_launch_takes(D, requests, tokens, heads):
+    """Cut by requests, and by query tiles. Each row sees its own key alone (a window of one), so it is that key's value."""
+    f = fast()
+    T, ps = requests * tokens, 16
+    assert f._fn("hb_flash_prefill_tc_launches")(T, requests, tokens, heads, D, 16) > 1
+    q, kc, vc = torch.ones(T, heads * D, dtype=torch.bfloat16, device=DEV), rnd(T // ps, 1, ps, D, seed=82), rnd(T // ps, 1, ps, D, seed=83)
+    bt = torch.arange(T // ps, dtype=torch.int32, device=DEV).view(requests, -1)
+    out = torch.zeros(T, heads * D, dtype=torch.bfloat16, device=DEV)
+    f.flash_prefill_tc(q, kc, vc, bt, i32(list(range(0, T, tokens))), i32([tokens] * requests), i32([0] * requests), out, tokens, heads, 1, D, ps, 1,
+                       1 / math.sqrt(D), 16)
+    torch.cuda.synchronize()
+    f.check_status()
+    assert bool((out.view(T, heads, D) == vc.transpose(1, 2).reshape(T, 1, D)).all())
