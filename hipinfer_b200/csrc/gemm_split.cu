@@ -302,24 +302,21 @@ __global__ void __launch_bounds__(256) split_reduce_kernel(const float* ws, floa
 }
 
 // ---------------------------------------------------------------------------------------
-static int gs_sms() {
-  static int n[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (!n[dev] && cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n[dev] = 148;
-  return n[dev];
-}
-// The tile's rows of A (a multiple of 16), the K blocks of a slice and the slices: as many as fit one round of SMs, 512 deep or deeper.
+// The K blocks of a slice and the slices, by N and K alone, so that a row's bits do not depend on how many rows there are: 512 k deep or deeper, one
+// row of tiles at most a round of 148 SMs, and of those the number whose rounds take least for one row of tiles and for two together. (With the slices chosen for the rows there
+// are, three rows of tiles or more would be up to 30 % faster where they are few, us: 400 rows x 2,048 x 2,048 28 / 39, x 2,048 x 8,192 88 / 107, 2,048
+// rows x 2,048 x 2,048 110 / 128. One rule for one row of tiles alone takes 301 rows x 3,072 x 2,048 from 28 to 41, 9 rows from 19 to 15.)
+// nt: the tile's rows of A, a multiple of 16; an output's bits do not depend on it.
 static void gs_plan(int M, int N, int K, int* nt, int* kbs, int* splits) {
   const int tiles = (M + GS_NT - 1) / GS_NT, num_kb = (K + GS_BK - 1) / GS_BK;
   *nt = ((M + tiles - 1) / tiles + 15) / 16 * 16;
-  const long ctas = (long)((N + GS_WR - 1) / GS_WR) * ((M + *nt - 1) / *nt);
-  long n = gs_sms() / ctas;
-  if (n > K / 512) n = K / 512;
-  if (n > GS_MAX_SPLITS) n = GS_MAX_SPLITS;
-  if (n < 1 || (N & 3)) n = 1;
-  *kbs = (int)((num_kb + n - 1) / n);
-  *splits = (num_kb + *kbs - 1) / *kbs;
+  const long cols = (N + GS_WR - 1) / GS_WR;
+  long least = -1;
+  for (int n = 1; n <= GS_MAX_SPLITS && (n == 1 || (n * cols <= 148 && n <= K / 512 && !(N & 3))); n++) {
+    const int blocks = (num_kb + n - 1) / n, slices = (num_kb + blocks - 1) / blocks;
+    const long time = blocks * ((cols * slices + 147) / 148 + (2 * cols * slices + 147) / 148);
+    if (least < 0 || time < least) { least = time; *kbs = blocks; *splits = slices; }
+  }
 }
 static size_t gs_planes(int M, int K) { return (size_t)3 * M * ((K + GS_BK - 1) / GS_BK * GS_BK) * 2; }
 static size_t gs_flags(int M) { return ((size_t)M * 4 + 15) / 16 * 16; }

@@ -256,6 +256,24 @@ def test_products_of_split_32_bit_operands(M, N, K):
     assert torch.equal(acc, want)
 
 
+@pytest.mark.parametrize("N,K", [(2048, 8192), (3072, 2048), (260, 1028), (4096, 4096), (20004, 1024)])
+def test_split_products_give_a_row_the_same_bits_whatever_the_rows(N, K):
+    """From nine rows on: tiles of other widths, more tiles than SMs, flagged rows and weights among them."""
+    f = fast()
+    g = torch.Generator().manual_seed(N)
+    a, w = torch.randn(700, K, generator=g).to(DEV), (torch.randn(N, K, generator=g) * 0.1).to(DEV)
+    a[5, 600], a[8] = 3.4e38, a[8] * 1e-35
+    w[30, 100], w[200] = math.inf, w[200] * 1e-35
+    whole = torch.empty(700, N, device=DEV)
+    assert f.linear32(a, w, whole, False)
+    for M in (9, 16, 40, 160, 161, 301, 400):
+        for start in (0, 700 - M):
+            out = torch.empty(M, N, device=DEV)
+            assert f.linear32(a[start:start + M], w, out, False)
+            assert torch.equal(out.view(torch.int32), whole[start:start + M].view(torch.int32)), (M, start)
+    f.check_status()
+
+
 @pytest.mark.parametrize("M,N,K", [(70, 260, 1028), (200, 20000, 512), (33, 1024, 4096)])
 def test_split_operands_that_are_no_sum_of_three(M, N, K):
     """Infinities, NaN, numbers that round to an infinite bfloat16, and rows below the range of their remainders: where FFMA gives an infinity
