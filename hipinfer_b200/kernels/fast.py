@@ -307,7 +307,9 @@ def _gemm(a, w, out, epi):
 def linear32(a, w, out, accumulate) -> bool:
     """The 32-bit product of more than a few rows on the tensor cores; False where its kernel does not take it, or no memory is left
     for its workspace."""
-    if (PLAIN_ONLY or not SPLIT_MIN_ROWS <= a.shape[0] or a.dtype != torch.float32 or w.dtype != torch.float32 or out.dtype != torch.float32
+    if (PLAIN_ONLY or not a.is_cuda or not w.is_cuda or not out.is_cuda or a.dim() != 2 or w.shape[1] != a.shape[1]
+            or out.shape != (a.shape[0], w.shape[0])       # (what the plain kernel refuses is its to refuse)
+            or not SPLIT_MIN_ROWS <= a.shape[0] or a.dtype != torch.float32 or w.dtype != torch.float32 or out.dtype != torch.float32
             or w.shape[0] * w.shape[1] < SPLIT_MIN_WEIGHTS or w.shape[1] < SPLIT_MIN_K
             or (a.shape[1] | w.shape[0] | a.stride(0) | w.stride(0) | out.stride(0)) & 3
             or (a.data_ptr() | w.data_ptr() | out.data_ptr()) & 15 or not (a.stride(1) == w.stride(1) == out.stride(1) == 1)):
