@@ -150,11 +150,10 @@ __device__ __forceinline__ void rope_head_store(float* x1, float* x2, int head, 
 // 4 KB boxes of swizzled shared memory and out by a TMA tensor store (or reduce). PER chunks fill one box of
 // 128-byte rows: 1 (fp32), 2 (bf16), 4 (SwiGLU: 16 outputs each). row0: the first of the warp's 32 rows in C. sent: the boxes this
 // warp has sent so far, over all its tiles (the last tile of a row may have an odd number of them).
-// A box of bf16 that C's last row cuts is slow to store (gate/up of 1,531 rows, 16,384 x 2,048: 105 us with such boxes, 80 with
-// those rows stored directly; 1,536 rows 80): ts_whole says whether a warp's rows go this way. Boxes of fp32 showed no such cost.
-template <int EPI> __device__ __forceinline__ bool ts_whole(int row0, int M) {
-  return EPI == EPI_F32 || EPI == EPI_ADD_F32 || row0 + 32 <= M;
-}
+// A box of gated outputs that C's last row cuts is slow to store (gate/up of 1,531 rows, 16,384 x 2,048: 105 us with such boxes, 80 with
+// those rows stored directly; 1,536 rows 80): ts_whole says whether a warp's rows go this way. Boxes of 32-bit and of plain bf16 outputs showed no such
+// cost, and with both ways in its epilogue the bf16 product was slower at every size (1,531 x 3,072 x 2,048 16.2 us without, 19.2 with).
+template <int EPI> __device__ __forceinline__ bool ts_whole(int row0, int M) { return !EPI_IS_GLU(EPI) || row0 + 32 <= M; }
 template <int EPI>
 __device__ __forceinline__ void ts_chunk(const float* v, int c, int n0, int N, int row0, uint8_t* boxes, uint32_t& sent, int lane,
                                          const CUtensorMap* map_c) {
