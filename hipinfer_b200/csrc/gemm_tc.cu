@@ -366,12 +366,9 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_kernel(const __grid_constant__
 // operand bytes per product, and at 96 CTAs of 128 x 128 tiles it is L2 that bounds it (512 x 3,072 by 3,072 and by 8,192: 62
 // us for both together; three slices of 256 x 256 tiles 35 us, and the norm that reads the sums next adds the slices).
 // ---------------------------------------------------------------------------------------
-// A stage holds two K blocks: half as many barriers to pass as with one (same time at 512 rows; 2,048 x 16,384 x 3,072 with SwiGLU 137 -> 134
-// us, 2,048 x 28,672 x 4,096 316 -> 308).
-constexpr int PAIR_STAGES = 3, KPS = 2;
 template <int STAGES>
 struct PairSmem {
-  static constexpr int A_BYTES = BM * BK * 2, B_BYTES = 128 * BK * 2, BLOCK_BYTES = A_BYTES + B_BYTES, STAGE_BYTES = BLOCK_BYTES * KPS;
+  static constexpr int A_BYTES = BM * BK * 2, B_BYTES = 128 * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
   static constexpr int STAGING_OFFSET = (BAR_OFFSET + 256 + 1023) / 1024 * 1024;
   static constexpr int TOTAL = STAGING_OFFSET + 4 * 2 * 4096 + 1024;
@@ -416,43 +413,21 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_pair_kernel(const __grid_const
   hb_cluster_sync();   // the partner's barriers exist before anything is signalled across
   hb_tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (warp != 4) hb_pdl_wait();   // (the loader asks for its first weight tiles before it waits)
+  hb_pdl_wait();
 
   if (warp == 4) {
-    {  // ---------------- TMA producer of this CTA's halves
-      uint32_t it = 0, early = 0;
+    if (hb_elect()) {  // ---------------- TMA producer of this CTA's halves
+      uint32_t it = 0;
       bool ok = true;
-      // the first weight tiles do not depend on the kernel ahead (0.5 to 0.8 us a product, back to back)
-      if (pair < units) {
-        const int tile = pair % num_tiles, kb0 = pair / num_tiles * kbs, kb1 = min(num_kb, kb0 + kbs), n0 = (tile / m_tiles) * BN + rank * 128;
-        for (int kb = kb0; early < STAGES && kb < kb1; early++, kb += KPS)
-          if (hb_elect()) {
-            const int n = min(KPS, kb1 - kb);
-            if (rank == 0) hb_mbar_expect_tx(&full[early], 2 * S::BLOCK_BYTES * n);   // both CTAs' bytes
-            for (int j = 0; j < n; j++)
-              hb_tma_load_2d_pair(smem + early * S::STAGE_BYTES + j * S::BLOCK_BYTES + S::A_BYTES, &map_w, hb_mapa(&full[early], 0), (kb + j) * BK, n0);
-          }
-        __syncwarp();
-      }
-      hb_pdl_wait();
       for (int u = pair; u < units && ok; u += n_pairs) {
         const int tile = u % num_tiles, kb0 = u / num_tiles * kbs, kb1 = min(num_kb, kb0 + kbs);
         const int m0 = (tile % m_tiles) * 256 + rank * 128, n0 = (tile / m_tiles) * BN + rank * 128;
-        for (int kb = kb0; kb < kb1; kb += KPS, it++) {
+        for (int kb = kb0; kb < kb1; kb++, it++) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1, bar = hb_mapa(&full[s], 0);
-          const int n = min(KPS, kb1 - kb);
-          uint8_t* st = smem + s * S::STAGE_BYTES;
-          if (it >= early && !__all_sync(0xffffffffu, hb_mbar_wait(&empty[s], ph ^ 1, abort_flag))) { ok = false; break; }
-          if (hb_elect()) {
-            if (it >= early && rank == 0) hb_mbar_expect_tx(&full[s], 2 * S::BLOCK_BYTES * n);
-#pragma unroll
-            for (int j = 0; j < KPS; j++)
-              if (j < n) {
-                hb_tma_load_2d_pair(st + j * S::BLOCK_BYTES, &map_a, bar, (kb + j) * BK, m0);
-                if (it >= early) hb_tma_load_2d_pair(st + j * S::BLOCK_BYTES + S::A_BYTES, &map_w, bar, (kb + j) * BK, n0);
-              }
-          }
-          __syncwarp();
+          if (!hb_mbar_wait(&empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
+          if (rank == 0) hb_mbar_expect_tx(&full[s], 2 * S::STAGE_BYTES);   // both CTAs' bytes
+          hb_tma_load_2d_pair(smem + s * S::STAGE_BYTES, &map_a, bar, kb * BK, m0);
+          hb_tma_load_2d_pair(smem + s * S::STAGE_BYTES + S::A_BYTES, &map_w, bar, kb * BK, n0);
         }
       }
       // the last commits still arrive on this CTA's barriers: wait for them before the shared memory is given up
@@ -460,35 +435,27 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_pair_kernel(const __grid_const
         ok = hb_mbar_wait(&empty[j % STAGES], (j / STAGES) & 1, abort_flag);
     }
   } else if (warp == 5) {
-    if (rank == 0) {  // ---------------- MMA issuer of the pair
+    if (rank == 0 && hb_elect()) {  // ---------------- MMA issuer of the pair
       constexpr uint32_t idesc = hb_umma_idesc_bf16(256, BN);
       uint32_t it = 0, tile_i = 0;
       bool ok = true;
       for (int u = pair; u < units && ok; u += n_pairs, tile_i++) {
         const int kb0 = u / num_tiles * kbs, kb1 = min(num_kb, kb0 + kbs);
         const uint32_t buf = tile_i & 1, aph = (tile_i >> 1) & 1;
-        if (!__all_sync(0xffffffffu, hb_mbar_wait(&tmem_empty[buf], aph ^ 1, abort_flag))) break;
+        if (!hb_mbar_wait(&tmem_empty[buf], aph ^ 1, abort_flag)) break;
         hb_tc_fence_after();
         const uint32_t d = tmem_base + buf * BN;
-        for (int kb = kb0; kb < kb1; kb += KPS, it++) {
+        for (int kb = kb0; kb < kb1; kb++, it++) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          if (!__all_sync(0xffffffffu, hb_mbar_wait(&full[s], ph, abort_flag))) { ok = false; break; }
+          if (!hb_mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
           hb_tc_fence_after();
-          const int n = min(KPS, kb1 - kb);
-          if (hb_elect()) {
+          const uint64_t da = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE_BYTES));
+          const uint64_t db = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE_BYTES + S::A_BYTES));
 #pragma unroll
-            for (int j = 0; j < KPS; j++)
-              if (j < n) {
-                const uint32_t st = hb_smem_u32(smem + s * S::STAGE_BYTES + j * S::BLOCK_BYTES);
-                const uint64_t da = hb_umma_desc_k128(st), db = hb_umma_desc_k128(st + S::A_BYTES);
-#pragma unroll
-                for (int k = 0; k < BK / 16; k++) hb_umma_bf16_pair(d, da + 2 * k, db + 2 * k, idesc, kb + j != kb0 || k != 0);
-              }
-            hb_umma_commit_pair(&empty[s]);
-            if (kb + KPS >= kb1) hb_umma_commit_pair(&tmem_full[buf]);
-          }
-          __syncwarp();
+          for (int k = 0; k < BK / 16; k++) hb_umma_bf16_pair(d, da + 2 * k, db + 2 * k, idesc, kb != kb0 || k != 0);
+          hb_umma_commit_pair(&empty[s]);
         }
+        if (ok) hb_umma_commit_pair(&tmem_full[buf]);
       }
     }
   } else {  // ---------------- epilogue warps 0..3: this CTA's 128 rows of the tile
@@ -635,7 +602,7 @@ static int launch_gemm_tc(const CUtensorMap& ma, const CUtensorMap& mw, void* C,
 template <int EPI>
 static int launch_gemm_pair(const CUtensorMap& ma, const void* W, long ldw, void* C, long ldc, int M, int N, int K, int* status,
                             cudaStream_t s, int splits = 1, int kbs = 1 << 30, int slice_rows = 0) {
-  using S = PairSmem<PAIR_STAGES>;
+  using S = PairSmem<6>;
   CUtensorMap mw, mc;
   if (hb_make_tensor_map_bf16(&mw, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, 128)) return -1;
   if (EPI == EPI_F32 || EPI == EPI_ADD_F32) {
@@ -646,7 +613,7 @@ static int launch_gemm_pair(const CUtensorMap& ma, const void* W, long ldw, void
     const uint64_t cols = EPI_IS_GLU(EPI) ? (uint64_t)N / 2 : (uint64_t)N;
     if (hb_make_tensor_map_bf16(&mc, C, (uint64_t)M, cols, (uint64_t)ldc, 32)) return -1;
   }
-  auto kern = gemm_tc_pair_kernel<PAIR_STAGES, EPI>;
+  auto kern = gemm_tc_pair_kernel<6, EPI>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
