@@ -107,31 +107,29 @@ __global__ void __launch_bounds__(192) gemm_stream_kernel(const __grid_constant_
       for (int kb = 0; kb < pre; kb++)
         hb_tma_load_2d(smem + kb * S::STAGE + ST_W_BYTES, &map_x, &full[kb], k_begin + kb * ST_BK, 0);
     __syncwarp();
-    for (int kb = pre; kb < num_kb; kb++) {
-      const uint32_t s = kb % S::STAGES, ph = (kb / S::STAGES) & 1;
-      if (!__all_sync(0xffffffffu, hb_mbar_wait(&empty[s], ph ^ 1, abort_flag))) break;
-      if (hb_elect()) {
+    if (hb_elect())
+      for (int kb = pre; kb < num_kb; kb++) {
+        const uint32_t s = kb % S::STAGES, ph = (kb / S::STAGES) & 1;
+        if (!hb_mbar_wait(&empty[s], ph ^ 1, abort_flag)) break;
         hb_mbar_expect_tx(&full[s], S::STAGE);
         hb_tma_load_2d(smem + s * S::STAGE, &map_w, &full[s], k_begin + kb * ST_BK, n0);
         hb_tma_load_2d(smem + s * S::STAGE + ST_W_BYTES, &map_x, &full[s], k_begin + kb * ST_BK, 0);
       }
-      __syncwarp();
-    }
   } else if (warp == 5) {
-    constexpr uint32_t idesc = hb_umma_idesc_bf16(ST_ROWS, NT);
-    for (int kb = 0; kb < num_kb; kb++) {
-      const uint32_t s = kb % S::STAGES, ph = (kb / S::STAGES) & 1;
-      if (!__all_sync(0xffffffffu, hb_mbar_wait(&full[s], ph, abort_flag))) break;
-      hb_tc_fence_after();
-      if (hb_elect()) {
+    if (hb_elect()) {
+      constexpr uint32_t idesc = hb_umma_idesc_bf16(ST_ROWS, NT);
+      bool ok = true;
+      for (int kb = 0; kb < num_kb; kb++) {
+        const uint32_t s = kb % S::STAGES, ph = (kb / S::STAGES) & 1;
+        if (!hb_mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
+        hb_tc_fence_after();
         const uint64_t dw = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE));
         const uint64_t dx = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE + ST_W_BYTES));
 #pragma unroll
         for (int k = 0; k < ST_BK / 16; k++) hb_umma_bf16(tmem_base, dw + 2 * k, dx + 2 * k, idesc, (kb | k) != 0);
         hb_umma_commit(&empty[s]);
-        if (kb == num_kb - 1) hb_umma_commit(done);
       }
-      __syncwarp();
+      if (ok) hb_umma_commit(done);
     }
   } else {
     // epilogue warps: lane = output column n0 + 32 * warp + lane, v[m] = token m
@@ -278,41 +276,36 @@ __global__ void __launch_bounds__(192, 1) gemm_stream_persist_kernel(const __gri
           hb_tma_load_2d(smem + it * S::STAGE + ST_W_BYTES, &map_x, &full[it], it % num_kb * ST_BK, 0);
       __syncwarp();
       int kb = pre % num_kb, nb = blockIdx.x + pre / num_kb * gridDim.x;
-      for (int it = pre; it < total; it++) {
-        const uint32_t s = it % S::STAGES, ph = (it / S::STAGES) & 1;
-        if (!__all_sync(0xffffffffu, hb_mbar_wait(&empty[s], ph ^ 1, abort_flag))) break;
-        if (hb_elect()) {
+      if (hb_elect())
+        for (int it = pre; it < total; it++) {
+          const uint32_t s = it % S::STAGES, ph = (it / S::STAGES) & 1;
+          if (!hb_mbar_wait(&empty[s], ph ^ 1, abort_flag)) break;
           hb_mbar_expect_tx(&full[s], S::STAGE);
           hb_tma_load_2d(smem + s * S::STAGE, &map_w, &full[s], kb * ST_BK, nb * ST_ROWS);
           hb_tma_load_2d(smem + s * S::STAGE + ST_W_BYTES, &map_x, &full[s], kb * ST_BK, 0);
+          if (++kb == num_kb) { kb = 0; nb += gridDim.x; }
         }
-        __syncwarp();
-        if (++kb == num_kb) { kb = 0; nb += gridDim.x; }
-      }
     }
   } else if (warp == 5) {
-    {  // ---------------- MMA issuer
+    if (hb_elect()) {  // ---------------- MMA issuer
       constexpr uint32_t idesc = hb_umma_idesc_bf16(ST_ROWS, NT);
       uint32_t it = 0;
       bool ok = true;
       for (int i = 0; i < mine && ok; i++) {
         const uint32_t buf = i & 1, aph = (i >> 1) & 1;
-        if (!__all_sync(0xffffffffu, hb_mbar_wait(&tmem_empty[buf], aph ^ 1, abort_flag))) break;
+        if (!hb_mbar_wait(&tmem_empty[buf], aph ^ 1, abort_flag)) break;
         hb_tc_fence_after();
         for (int kb = 0; kb < num_kb; kb++, it++) {
           const uint32_t s = it % S::STAGES, ph = (it / S::STAGES) & 1;
-          if (!__all_sync(0xffffffffu, hb_mbar_wait(&full[s], ph, abort_flag))) { ok = false; break; }
+          if (!hb_mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
           hb_tc_fence_after();
-          if (hb_elect()) {
-            const uint64_t dw = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE));
-            const uint64_t dx = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE + ST_W_BYTES));
+          const uint64_t dw = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE));
+          const uint64_t dx = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE + ST_W_BYTES));
 #pragma unroll
-            for (int k = 0; k < ST_BK / 16; k++) hb_umma_bf16(tmem_base + buf * NT, dw + 2 * k, dx + 2 * k, idesc, (kb | k) != 0);
-            hb_umma_commit(&empty[s]);
-            if (kb == num_kb - 1) hb_umma_commit(&tmem_full[buf]);
-          }
-          __syncwarp();
+          for (int k = 0; k < ST_BK / 16; k++) hb_umma_bf16(tmem_base + buf * NT, dw + 2 * k, dx + 2 * k, idesc, (kb | k) != 0);
+          hb_umma_commit(&empty[s]);
         }
+        if (ok) hb_umma_commit(&tmem_full[buf]);
       }
     }
   } else {  // ---------------- epilogue warps: lane = output column, v[m] = token m

@@ -833,7 +833,7 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_grouped_kernel(const __grid_co
   };
 
   if (warp == 4) {
-    {  // ---------------- TMA producer
+    if (hb_elect()) {  // ---------------- TMA producer
       uint32_t it = 0;
       int e = 0, m0, n0;
       bool ok = true;
@@ -841,40 +841,34 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_grouped_kernel(const __grid_co
         place(tile, e, m0, n0);
         for (int kb = 0; kb < num_kb; kb++, it++) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          if (!__all_sync(0xffffffffu, hb_mbar_wait(&empty[s], ph ^ 1, abort_flag))) { ok = false; break; }
-          if (hb_elect()) {
-            hb_mbar_expect_tx(&full[s], S::STAGE_BYTES);
-            hb_tma_load_2d(smem + s * S::STAGE_BYTES, &map_a, &full[s], kb * BK, m0);
-            hb_tma_load_2d(smem + s * S::STAGE_BYTES + S::A_BYTES, &map_w, &full[s], kb * BK, e * N + n0);
-          }
-          __syncwarp();
+          if (!hb_mbar_wait(&empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
+          hb_mbar_expect_tx(&full[s], S::STAGE_BYTES);
+          hb_tma_load_2d(smem + s * S::STAGE_BYTES, &map_a, &full[s], kb * BK, m0);
+          hb_tma_load_2d(smem + s * S::STAGE_BYTES + S::A_BYTES, &map_w, &full[s], kb * BK, e * N + n0);
         }
       }
     }
   } else if (warp == 5) {
-    {  // ---------------- MMA issuer
+    if (hb_elect()) {  // ---------------- MMA issuer
       constexpr uint32_t idesc = hb_umma_idesc_bf16(BM, BN);
       uint32_t it = 0, tile_i = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, tile_i++) {
         const uint32_t buf = tile_i & 1, aph = (tile_i >> 1) & 1;
-        if (!__all_sync(0xffffffffu, hb_mbar_wait(&tmem_empty[buf], aph ^ 1, abort_flag))) break;
+        if (!hb_mbar_wait(&tmem_empty[buf], aph ^ 1, abort_flag)) break;
         hb_tc_fence_after();
         const uint32_t d = tmem_base + buf * BN;
         for (int kb = 0; kb < num_kb; kb++, it++) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          if (!__all_sync(0xffffffffu, hb_mbar_wait(&full[s], ph, abort_flag))) { ok = false; break; }
+          if (!hb_mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
           hb_tc_fence_after();
           const uint64_t da = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE_BYTES));
           const uint64_t db = hb_umma_desc_k128(hb_smem_u32(smem + s * S::STAGE_BYTES + S::A_BYTES));
-          if (hb_elect()) {
 #pragma unroll
-            for (int k = 0; k < BK / 16; k++) hb_umma_bf16(d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-            hb_umma_commit(&empty[s]);
-            if (kb == num_kb - 1) hb_umma_commit(&tmem_full[buf]);
-          }
-          __syncwarp();
+          for (int k = 0; k < BK / 16; k++) hb_umma_bf16(d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+          hb_umma_commit(&empty[s]);
         }
+        if (ok) hb_umma_commit(&tmem_full[buf]);
       }
     }
   } else {  // ---------------- epilogue warps 0..3
