@@ -126,32 +126,39 @@ __device__ __forceinline__ FtSpan ft_span(const int4& e, int window) {
   return s;
 }
 
-// One warp: the (request, query tile) pairs of this launch and their key tiles, unordered.
+// One warp: the (request, query tile) pairs of this launch and their key tiles, unordered. The numbers of 128 requests are asked for together: one
+// trip to memory after another, a step of 64 requests took 0.7 us longer (portions of 16 rows, 4 heads of 64: 9.0 us, now 8.3; a block per query tile 7.6).
 __device__ __forceinline__ void ft_list(uint2* raw, int* n_entries, int most, const int* q_len, const int* ctx_len, int window, int min_rows,
                                         int req0, int reqs, int qt0, int qts) {
   const int lane = threadIdx.x & 31;
   int n = 0;
-  for (int base = 0; base < reqs; base += 32) {
-    const int r = req0 + base + lane;
-    int len = base + lane < reqs ? q_len[r] : 0;
-    if (len < min_rows) len = 0;
-    const int tiles = max(0, min((len + FT_BM - 1) / FT_BM - qt0, qts));
-    int at = tiles;
+  for (int base = 0; base < reqs; base += 128) {
+    int q_lens[4], ctxs[4];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, at, o);
-      if (lane >= o) at += v;
+    for (int j = 0; j < 4; j++) {
+      const int i = base + 32 * j + lane;
+      q_lens[j] = i < reqs ? q_len[req0 + i] : 0;
+      ctxs[j] = i < reqs ? ctx_len[req0 + i] : 0;
     }
-    const int total = __shfl_sync(0xffffffffu, at, 31);
-    at += n - tiles;
-    if (tiles) {
-      const int ctx = ctx_len[r];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      if (base + 32 * j >= reqs) break;
+      const int r = req0 + base + 32 * j + lane, len = q_lens[j] < min_rows ? 0 : q_lens[j], ctx = ctxs[j];
+      const int tiles = max(0, min((len + FT_BM - 1) / FT_BM - qt0, qts));
+      int at = tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += v;
+      }
+      const int total = __shfl_sync(0xffffffffu, at, 31);
+      at += n - tiles;
       for (int t = 0; t < tiles && at + t < most; t++) {
         const int row = (qt0 + t) * FT_BM;
         raw[at + t] = make_uint2((uint32_t)r << 16 | (uint32_t)(qt0 + t), ft_span(make_int4(0, min(FT_BM, len - row), ctx + row, r), window).n);
       }
+      n += total;
     }
-    n += total;
   }
   if (lane == 0) *n_entries = min(n, most);
 }
@@ -195,13 +202,20 @@ __device__ __forceinline__ bool ft_bring(const FtSpan& sp, const int* table, int
     if (!__all_sync(0xffffffffu, hb_mbar_wait(&free[s], ph ^ 1, abort_flag))) return false;
     if (hb_elect()) hb_mbar_expect_tx(&full[s], (uint32_t)__popc(boxes) * page_size * FT_D * 2);
     __syncwarp();
-    for (uint32_t left = boxes; left; left &= left - 1) {
-      const int p = __ffs(left) - 1, from = __shfl_sync(0xffffffffu, row, p);
-      if (hb_elect()) {
-        uint8_t* dst = ring + s * OPND + p * page_size * 128;            // rows of 128 bytes in each 64-column tile
+    for (int p = 0; p < places; p += 4) {       // four boxes an election (pages of 8 one by one: 2,048 rows behind 2,048 106 us, now 102)
+      int from[4];
 #pragma unroll
-        for (int hf = 0; hf < NH; hf++) hb_tma_load_2d(dst + hf * FT_TILE, map, &full[s], hf * 64, from);
+      for (int j = 0; j < 4; j++) from[j] = __shfl_sync(0xffffffffu, row, p + j);
+      if (hb_elect()) {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          if (boxes >> (p + j) & 1) {
+            uint8_t* dst = ring + s * OPND + (p + j) * page_size * 128;            // rows of 128 bytes in each 64-column tile
+#pragma unroll
+            for (int hf = 0; hf < NH; hf++) hb_tma_load_2d(dst + hf * FT_TILE, map, &full[s], hf * 64, from[j]);
+          }
       }
+      __syncwarp();
     }
   }
   return true;
