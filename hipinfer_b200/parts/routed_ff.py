@@ -27,7 +27,8 @@ bfloat16 all of it runs on the device alone (csrc/moe.cu, gemm_tc.cu), so that i
 have few rows each, warp-MMA kernels stream their weights (gate/up product with its activation, then the down product); where they
 have more, two tcgen05 kernels do the same over tiles of 128 rows. In 32-bit (and at sizes those kernels do not take) a few rows
 run one by one, single rows of a larger step on any-size kernels, and in a step with prompt portions each expert's block of rows
-goes to the ordinary products, for which the host reads the experts' row counts once a layer.
+goes to the ordinary products (in 32-bit to the plain one, which gives a row the same bits however many there are), for which the host
+reads the experts' row counts once a layer.
 
 params: hidden_size, experts, top, expert_size, score (default "sigmoid"), weight_at (default "input"), router_bias
 (default False), groups (count, keep) (default none), identity (default 0), weight_scale (default 1), shared_size (default none), shared_gate (default
@@ -207,17 +208,19 @@ class RoutedFF(Part):
             ops.moe_combine(ys, pos, x, top, limit, rows_in, idw)
             return None
         bounds = offsets.tolist()                      # the one read by the host: how many rows each expert has
+        # 32-bit rows by the plain product: `linear` would choose a kernel by how many rows the expert has, and with them of other requests
+        product = (lambda a, w, out: ops.gemm_plain(a, w.t, out)) if xs.dtype == torch.float32 else ops.linear
         gu = torch.empty(T * top, 2 * F, dtype=torch.float32, device=xn.device)
         for e in range(self.experts):
             lo, hi = bounds[e], bounds[e + 1]
             if hi > lo:
-                ops.linear(xs[lo:hi], self.w_gu_e[e], gu[lo:hi])
+                product(xs[lo:hi], self.w_gu_e[e], gu[lo:hi])
         ops.moe_act(gu, src, score, act, self.at_output, limit, self.group)
         planes.record(batch, "activation", act)
         for e in range(self.experts):
             lo, hi = bounds[e], bounds[e + 1]
             if hi > lo:
-                ops.linear(act[lo:hi], self.w_down_e[e], ys[lo:hi])
+                product(act[lo:hi], self.w_down_e[e], ys[lo:hi])
         ops.moe_combine(ys, pos, x, top, limit, rows_in, idw)
         return None
 

@@ -273,6 +273,18 @@ def test_routed_feed_forward_row_by_row_grouped_and_sorted(dtype, W, F, E, top, 
         close(y - 0.25, want, dtype, what)
 
 
+def test_routed_rows_in_32_bit_have_the_same_bits_whatever_rows_are_beside_them():
+    """Portions: an expert has few rows of the one request alone (eight on average) and many beside the other's."""
+    part, _ = _routed(torch.float32, 256, 256, 16, 2)
+    h = (rnd(264, 256, seed=51) * 1.5).to(DEV)
+    outs = []
+    for T in (64, 264):
+        y = torch.zeros(T, 256, dtype=torch.float32, device=DEV)
+        part.forward(h[:T].contiguous(), y, SimpleNamespace(max_q_len=T, dump=None))
+        outs.append(y[:64])
+    assert torch.equal(outs[0], outs[1])
+
+
 def test_router_ties_go_to_the_lower_index():
     from hipinfer_b200.kernels import ops
 
