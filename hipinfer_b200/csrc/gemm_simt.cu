@@ -1,10 +1,10 @@
 // The plain matrix product C[M,N] = A[M,K] W[N,K]^T in true 32-bit arithmetic (FFMA chains, no tensor cores), W row-major
-// with K contiguous as the reference stores weights (src/api.cu:81-83). It is the 32-bit engine's product and serves whatever
-// the tensor-core kernels do not take.
+// with K contiguous as the reference stores weights (src/api.cu:81-83). It is the 32-bit engine's product of up to eight rows (more rows
+// go to gemm_split.cu where that takes their sizes) and serves whatever the tensor-core kernels do not take.
 //
 // K is cut into slices by a rule on K alone (slice_plan): at most eight, 512 deep or more. An output is the sum of its
 // slices' FFMA chains, each running its k in order from zero, added lowest slice first. Every kernel below adds in that
-// order, so a row's result is the same bits whatever M is and whichever kernel ran, and the chains are no longer than K / 8.
+// order, so a row's result is the same bits whatever M is and whichever kernel of this file ran, and the chains are no longer than K / 8.
 //
 // Three ways through the same sum:
 //   simt_rows_kernel   up to 8 rows (a decode step: W is read once, the floor is its bytes).

@@ -7,7 +7,7 @@
 // nearest. The error against 64 bits is smaller than that of gemm_simt.cu, whose FFMA chains are 512 and longer:
 // 512 x 2,048 x 8,192 1.7e-7 against 5.8e-7 (2-norm), 301 x 16,384 x 2,048 1.3e-7 against 4.1e-7.
 //
-// The weights are the MMA's 128-row side and the rows of A its N side (up to 160, so that 301 rows are two tiles of 160). A's three planes
+// The weights are the MMA's 128-row side and the rows of A its N side (up to 160: what two stages leave in 227 KB of shared memory). A's three planes
 // are written by a small kernel ahead (split_rows_kernel) and come by TMA; W is read as it is, 32 bits, and split on its way into
 // shared memory. A CTA makes one tile of 128 weights x NT rows, over all of K or a slice of it (few tiles: the slices' sums go to
 // a workspace and are added lowest first). Warps:
@@ -15,13 +15,15 @@
 //          on their way, the running sums of the stage before: a thread owns one weight row (TMEM lane) and half of the tile's columns
 //   8      TMA of A's planes;  9  tcgen05.mma, 24 a stage
 // Where the sum of three does not hold, the row is flagged and its outputs are FFMA chains in the order of gemm_simt.cu: numbers that are
-// not finite, or round to no finite bf16 (they would turn into NaN where FFMA gives an infinity), and rows without a number of 2^-100 or
-// more (the tensor cores do not see all of their remainders, which lie below the normal range).
+// not finite, or round to no finite bf16 (they would turn into NaN where FFMA gives an infinity), and rows whose numbers are all below
+// 2^-100 (the tensor cores do not see all of their remainders, which lie below the normal range). In a row that has a number of 2^-100 or more the
+// small ones lose those remainders: some 2^-120 of an error for each, beside a row of at least 2^-100. It shows only where all the large numbers meet zeros.
 //
-// What bounds it: the MMAs, 24 of 93 cycles a stage at N = 160, in 1.73 rounds of tiles for a gate/up of 301 rows (120 us; 67 us would be
-// six products at the measured bf16 rate); from some 64 rows down the workers (some 1,100 cycles a stage for the split of 128 x 64 weights and
-// the running sums). us, gemm_simt.cu / here, with the kernels ahead and behind: 301 rows x 16,384 x 2,048 458 / 121, x 2,048 x 8,192
-// 253 / 81, x 3,072 x 2,048 109 / 31; 64 rows x 16,384 x 2,048 111 / 55; 9 rows x 16,384 x 2,048 103 / 51, x 256 x 256 16 / 9.
+// What bounds it: a gate/up of 301 rows (119 us) is 256 tiles on 148 SMs, two rounds of 32 stages. The MMAs of a stage, 24 of 93 cycles at N = 160, are
+// 74 us of that (73 us would be six products at the measured burst rate of 1,666 TFLOP/s, 89 at the sustained one); the rest is what a stage's
+// workers, copies and MMAs wait for one another. From some 64 rows down the workers bound it (some 1,100 cycles a stage for the split of 128 x 64 weights and
+// the running sums). us, gemm_simt.cu / here, with the kernels ahead and behind: 301 rows x 16,384 x 2,048 455 / 119, x 2,048 x 8,192
+// 250 / 80, x 3,072 x 2,048 107 / 29; 64 rows x 16,384 x 2,048 109 / 55; 9 rows x 16,384 x 2,048 101 / 52, x 3,072 x 2,048 43 / 19, x 256 x 256 16 / 8.4.
 // Tried: sums in warps of their own (120 us more for the gate/up: four warps cannot split W as fast), the weights' lines asked into L2
 // five stages ahead (5 % slower).
 #include "tc_common.cuh"

@@ -1,4 +1,5 @@
-"""Dispatch to the tensor-core kernels of the `fast` library (bfloat16 operands). Each function
+"""Dispatch to the tensor-core kernels of the `fast` library (bfloat16 operands; 32-bit ones from nine rows on, as sums of
+three bfloat16 numbers). Each function
 returns False when its kernel does not take the element types or sizes; the caller then uses
 the plain kernel. Set HIPINFER_B200_PLAIN=1 to force the plain kernels everywhere.
 
