@@ -17,23 +17,23 @@
 // prompt was cut or on what else is in the batch. Replaces flash_prefill_mma_kernel of the reference (src/kernels.cuh:1335-1482).
 // Every wait is bounded.
 //
-// head_dim 128 (flash_prefill_tc_kernel): a CTA an SM, and an item's tiles go to TWO chains by the parity of their absolute number: each
-// chain has a softmax warpgroup, an MMA warp, scores, probabilities, running maximum, sum and output accumulator of its own, and the
-// two are joined at the item's end. The softmax of one chain runs while the other waits for the tensor cores, and an item takes half
-// as long where there are fewer items than SMs. Both warpgroups read both accumulators, each half of the columns, and write
-// (O_even 2^(m_even - m) + O_odd 2^(m_odd - m)) / l. (One MMA warp for both chains was the bound: it stands in the queue while
-// an MMA of 64 to 80 cycles runs, and its waits came on top, 2,300 cycles a tile.)
-// head_dim 64 (flash_prefill_tc64_kernel): items are short beside their ends, so two CTAs of one chain share an SM, each within
+// head_dim 128 (flash_prefill_tc_kernel): a CTA an SM, with TWO softmax warpgroups that take the tiles in turn, so that one's exponentials run while the
+// other reads scores, stores P or waits. A row's maximum goes from tile to tile through shared memory as soon as it is known, its sum when the tile is
+// done, and there is one output accumulator an item, whose products are issued in the tiles' order: all sums have the order of one warpgroup that
+// walks all tiles, and the same bits (a head of 64 padded with zeros gives what the kernel for 64 gives). Accumulators alternate item by item, so the
+// next item's products need not wait until the last one is written, each warpgroup half of its columns. Scores and products have an MMA warp each.
+// head_dim 64 (flash_prefill_tc64_kernel): items are short beside their ends, so two CTAs of one softmax warpgroup share an SM, each within
 // 113 KB of shared memory, 256 columns of tensor memory and 128 registers (a row of S is read in two halves of 64, the first one twice:
 // once for the maximum, once for the exponentials).
 //
-// What bounds it: the softmax warps, some 2,500 cycles a tile of a chain alone, 1,024 of them exponentials (16 a cycle an SM, so two chains
+// What bounds it: the softmax warps, some 2,500 cycles a tile of a warpgroup alone, 1,024 of them exponentials (16 a cycle an SM, so two
 // cannot fall below 1,024 cycles a tile; the MMAs take 900 to 1,250). Measured against its forerunner (a CTA per query tile of a grid over
-// all requests, one chain, MMAs issued behind "lane == 0", page numbers loaded when they were needed), us: 32 heads over 8 of 128, 2,048
-// rows 74.7 -> 51.2, behind 2,048 more 182 -> 113 (910 TFLOP/s); 24 heads of 128, 512 rows behind 1,536 34.9 -> 22.9; 32 heads over 8 of
-// 64, 2,048 rows 40.7 -> 39.6, four portions of 512 23.9 -> 20.4, 1,988 rows beside 60 decoding requests 173 -> 39.7. At head_dim 64 the
-// two-chain form was slower (45 us at 2,048 rows: an item of 8.5 tiles spends a third of its time at its ends), and so was one that
-// joined the chains later, behind the next item's first tile (49 us).
+// all requests, one warpgroup, MMAs issued behind "lane == 0", page numbers loaded when they were needed), us: 32 heads over 8 of 128, 2,048
+// rows 74.7 -> 52, behind 2,048 more 182 -> 115 (900 TFLOP/s); 24 heads of 128, 512 rows behind 1,536 34.9 -> 24.4, with bias and sink 58 -> 40; 32 heads over 8 of
+// 64, 2,048 rows 40.7 -> 40.0, four portions of 512 23.9 -> 20.4, 1,988 rows beside 60 decoding requests 173 -> 39.7. With two chains of their own (a
+// maximum, sum and accumulator for the even tiles and for the odd ones, joined at the item's end) the 128 kernel was 1 to 8 % faster (behind 2,048 113 us,
+// 512 behind 1,536 22.6), but every result differed in its last bits from one chain's. At head_dim 64 that form was slower (45 us at 2,048 rows: an item of 8.5 tiles
+// spends a third of its time at its ends), and so was one that joined the chains later, behind the next item's first tile (49 us).
 //
 // EX: a distance bias, r1 ln(1 + r2 (i - j)) off the score of query i and key j (r1, r2 >= 0, a number per head), and a
 // sink, exp(sink) in the denominator (a number per head). The bias grows with the distance, so the unbiased maximum of a
@@ -48,7 +48,7 @@ constexpr int FT_THREADS = 384;        // 168 registers each: a row of S is 128 
 // A launch lists up to FT_MAX_PAIRS (request, query tile) pairs, in the place of P, and a CTA keeps the pairs of its own items, FT_OWN at most; the
 // launcher cuts steps of more. (When every CTA kept all pairs, 200 of them at head_dim 64, one request of 32,768 rows was 43 launches and took
 // 10.8 ms, now 6.7; 16,000 rows beside 300 single rows 3.1 ms, now 1.6.)
-constexpr int FT_MAX_PAIRS = 4096, FT_OWN = 640, FT_OWN64 = 200;
+constexpr int FT_MAX_PAIRS = 4096, FT_OWN = 420, FT_OWN64 = 200;
 
 // MN-major operand with the 128-byte swizzle: 64 contiguous elements of the MN dimension per row,
 // eight K rows per 1,024-byte group (stride SBO); further MN atoms would lie LBO apart (one here).
@@ -86,9 +86,11 @@ __device__ __forceinline__ void ft_st32(uint32_t taddr, const uint32_t* r) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
 }
 
-// head_dim 128: Q, P of both chains, rings of two K and two V tiles, and the list of the items.
+// head_dim 128: Q, P of both warpgroups, rings of two K and two V tiles, and the list of the items.
 struct FtBars {
-  uint64_t q_full, q_free, k_full[2], k_free[2], v_full[2], v_free[2], s_full[2], s_free[2], p_full[2], pv_done[2];
+  uint64_t q_full, q_free, k_full[2], k_free[2], v_full[2], v_free[2], s_full[2], s_free[2], p_full[2], pv_done[2], o_free[2];
+  uint64_t m_full[2][4], l_full[2][4];   // a warp's rows have their maximum, and their sum, behind its tile
+  float m[128], l[128];                  // a row's running maximum and sum, handed from tile to tile
   uint32_t own[FT_OWN];              // request << 16 | query tile of this CTA's items, in their order
   int n_entries;
   uint32_t tmem_slot;
@@ -232,14 +234,6 @@ __device__ __forceinline__ void ft_exp(uint32_t s0, uint32_t s1, uint64_t scale2
   p0 = hb_exp2(e0);
   p1 = hb_exp2(e1);
 }
-// And rounded to bf16 for P, and added to the row's sums.
-template <bool EX>
-__device__ __forceinline__ uint32_t ft_prob(uint32_t s0, uint32_t s1, uint64_t scale2, uint64_t sub2, float r1, float r2, float dist, uint64_t& sum2) {
-  float p0, p1;
-  ft_exp<EX>(s0, s1, scale2, sub2, r1, r2, dist, p0, p1);
-  sum2 = ft_add2(sum2, ft_pack2(__float_as_uint(p0), __float_as_uint(p1)));
-  return hb_pack_bf16(p0, p1);
-}
 // m_run follows the row's maximum lazily: it is raised (and the row of O rescaled) only when a tile's maximum exceeds it by
 // more than FT_SLACK, so P <= 2^FT_SLACK; the sum l_run is in the same units, and O / l_run is exact whichever maxima were used.
 constexpr float FT_SLACK = 8.f;
@@ -255,7 +249,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) flash_prefill_tc_kernel(
   // the 128-byte swizzle wants the tiles on 1 KB boundaries, and there is no room for slack: checked below
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sQ = smem;                      // [128][head_dim]
-  uint8_t* sP = sQ + OPND;                 // per chain two K blocks of [128 rows][64 keys]
+  uint8_t* sP = sQ + OPND;                 // per warpgroup two K blocks of [128 rows][64 keys]
   uint8_t* sK = sP + 4 * FT_TILE;          // two stages of [128 keys][head_dim]
   uint8_t* sV = sK + 2 * OPND;             // and two more
   FtBars* bar = (FtBars*)(sV + 2 * OPND);
@@ -272,7 +266,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) flash_prefill_tc_kernel(
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0) ft_list((uint2*)sP, &bar->n_entries, most, q_len, ctx_len, window, min_rows, req0, reqs, qt0, qts);
   if (threadIdx.x == 32) {
-    hb_mbar_init(&bar->q_full, 1); hb_mbar_init(&bar->q_free, 2);
+    hb_mbar_init(&bar->q_full, 1); hb_mbar_init(&bar->q_free, 1);
     for (int b = 0; b < 2; b++) {
       hb_mbar_init(&bar->k_full[b], 1); hb_mbar_init(&bar->k_free[b], 1);
       hb_mbar_init(&bar->v_full[b], 1); hb_mbar_init(&bar->v_free[b], 1);
@@ -280,6 +274,8 @@ __global__ void __launch_bounds__(FT_THREADS, 1) flash_prefill_tc_kernel(
     for (int c = 0; c < 2; c++) {
       hb_mbar_init(&bar->s_full[c], 1); hb_mbar_init(&bar->s_free[c], 4);
       hb_mbar_init(&bar->p_full[c], 4); hb_mbar_init(&bar->pv_done[c], 1);
+      hb_mbar_init(&bar->o_free[c], 8);
+      for (int w = 0; w < 4; w++) { hb_mbar_init(&bar->m_full[c][w], 1); hb_mbar_init(&bar->l_full[c][w], 1); }
     }
     bar->abort_flag = 0;
     hb_fence_barrier_init();
@@ -299,12 +295,14 @@ __global__ void __launch_bounds__(FT_THREADS, 1) flash_prefill_tc_kernel(
   hb_tc_fence_before();
   __syncthreads();
   hb_tc_fence_after();
-  const uint32_t tmem = bar->tmem_slot;   // S of chain c: 128 columns at c * 128; O of chain c: head_dim columns at 256 + c * 128
+  const uint32_t tmem = bar->tmem_slot;   // S of warpgroup c: 128 columns at c * 128; O of the CTA's item k: head_dim columns at 256 + (k & 1) * 128
   hb_pdl_wait();   // barriers, shared and tensor memory were set up while the kernel ahead was still running
 
   // an item's numbers are fetched while the one before it is worked on
   auto entry = [&](int k) { const int u = ft_item(k); return ft_entry(bar->own[u < n_items ? k : 0], q_start, q_len, ctx_len); };
 
+  // The CTA's tiles are numbered through all its items: tile t has warpgroup, S, P and ring stages t & 1, and is their use t >> 1. A barrier is
+  // waited for use after use by one warp, or behind another's word that the use before is over, so a parity can only mean the use that is wanted.
   if (warp == 8 || warp == 9) {  // ---------------- TMA: lane l brings page l of a tile
     const bool is_k = warp == 8;
     const CUtensorMap* map = is_k ? &map_k : &map_v;
@@ -329,140 +327,186 @@ __global__ void __launch_bounds__(FT_THREADS, 1) flash_prefill_tc_kernel(
       }
       ok = ft_bring<FT_D>(sp, bt + (size_t)e.w * bt_stride, page_size, Hkv, h, !is_k, map, ring, full, free, it, abort_flag);
     }
-  } else if (warp >= 10) {  // ---------------- tensor cores, chain c
-    constexpr uint32_t idesc_s = hb_umma_idesc_bf16(FT_BM, FT_BN), idesc_o = ft_idesc_b_mn(FT_BM, FT_D);
-    const int c = warp - 10;
-    uint32_t base = 0, ns = 0, np = 0;      // tiles of the items before; the chain's scores and products so far
-    bool ok = true;
-    int4 ahead = entry(0);
-    for (int k = 0; ft_item(k) < n_items && ok; k++) {
-      const FtSpan sp = ft_span(ahead, window);
-      ahead = entry(k + 1);
-      ok = __all_sync(0xffffffffu, hb_mbar_wait(&bar->q_full, k & 1, abort_flag));
-      const int i0 = (sp.kt_lo ^ c) & 1;
-      if (i0 >= sp.n && lane == 0) hb_mbar_arrive(&bar->q_free);      // one tile, the other chain's
-      for (int i = i0; i < sp.n + 2 && ok; i += 2) {
-        if (i < sp.n) {         // S of tile i
-          const uint32_t it = base + i, s = it & 1, ph = (it >> 1) & 1;
-          ok = hb_mbar_wait(&bar->k_full[s], ph, abort_flag) && hb_mbar_wait(&bar->s_free[c], (ns & 1) ^ 1, abort_flag);
-          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
-          ns++;
+  } else if (warp == 10) {  // ---------------- tensor cores: S = Q K^T of every tile
+    if (hb_elect()) {
+      constexpr uint32_t idesc = hb_umma_idesc_bf16(FT_BM, FT_BN);
+      uint32_t t = 0;
+      bool ok = true;
+      int4 ahead = entry(0);
+      for (int k = 0; ft_item(k) < n_items && ok; k++) {
+        const int n = ft_span(ahead, window).n;
+        ahead = entry(k + 1);
+        ok = hb_mbar_wait(&bar->q_full, k & 1, abort_flag);
+        for (int i = 0; i < n && ok; i++, t++) {
+          const uint32_t c = t & 1, ph = (t >> 1) & 1;
+          ok = hb_mbar_wait(&bar->k_full[c], ph, abort_flag) && hb_mbar_wait(&bar->s_free[c], ph ^ 1, abort_flag);
+          if (!ok) break;
           hb_tc_fence_after();
-          if (hb_elect()) {
 #pragma unroll
-            for (int kk = 0; kk < FT_D / 16; kk++) {   // 16 columns a step: four steps in each 64-column tile
-              const uint64_t dq = hb_umma_desc_k128(hb_smem_u32(sQ + (kk >> 2) * FT_TILE)) + 2 * (kk & 3);
-              const uint64_t dk = hb_umma_desc_k128(hb_smem_u32(sK + s * OPND + (kk >> 2) * FT_TILE)) + 2 * (kk & 3);
-              hb_umma_bf16(tmem + c * FT_BN, dq, dk, idesc_s, kk != 0);
-            }
-            hb_umma_commit(&bar->s_full[c]);
-            hb_umma_commit(&bar->k_free[s]);
-            if (i + 2 >= sp.n) hb_umma_commit(&bar->q_free);
+          for (int kk = 0; kk < FT_D / 16; kk++) {   // 16 columns a step: four steps in each 64-column tile
+            const uint64_t dq = hb_umma_desc_k128(hb_smem_u32(sQ + (kk >> 2) * FT_TILE)) + 2 * (kk & 3);
+            const uint64_t dk = hb_umma_desc_k128(hb_smem_u32(sK + c * OPND + (kk >> 2) * FT_TILE)) + 2 * (kk & 3);
+            hb_umma_bf16(tmem + c * FT_BN, dq, dk, idesc, kk != 0);
           }
-          __syncwarp();
-        }
-        if (i >= i0 + 2) {      // O of tile i - 2
-          const uint32_t it = base + i - 2, s = it & 1, ph = (it >> 1) & 1;
-          // P first. Across items a stage's tile before this one can be the OTHER chain's, and the wait for V could then return on the phase
-          // before that tile's (the same parity). Behind P every tile of the items before has been read (the softmax warps joined
-          // them), and of this item's the stage's last one was this chain's own. (K needs no such order: this item's Q came when both
-          // chains had read all K of the item before.)
-          ok = hb_mbar_wait(&bar->p_full[c], np & 1, abort_flag) && hb_mbar_wait(&bar->v_full[s], ph, abort_flag);
-          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
-          np++;
-          hb_tc_fence_after();
-          if (hb_elect()) {
-#pragma unroll
-            for (int kk = 0; kk < FT_BN / 16; kk++) {
-              const uint64_t dp = hb_umma_desc_k128(hb_smem_u32(sP + (2 * c + (kk >> 2)) * FT_TILE)) + 2 * (kk & 3);
-              const uint64_t dv = ft_desc_mn128(hb_smem_u32(sV + s * OPND + kk * 16 * 128));   // 16 keys on; the second 64 columns lie FT_TILE further (the descriptor's leading offset)
-              hb_umma_bf16(tmem + 256 + c * 128, dp, dv, idesc_o, i > i0 + 2 || kk != 0);      // O stays in tensor memory over the chain's tiles
-            }
-            hb_umma_commit(&bar->v_free[s]);
-            hb_umma_commit(&bar->pv_done[c]);
-          }
-          __syncwarp();
+          hb_umma_commit(&bar->s_full[c]);
+          hb_umma_commit(&bar->k_free[c]);
+          if (i == n - 1) hb_umma_commit(&bar->q_free);
         }
       }
-      base += sp.n;
     }
-  } else {  // ---------------- softmax: chain c, thread = query row
-    const int c = warp >> 2, r = threadIdx.x & 127;
-    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t tmem_s = tmem + c * FT_BN + lane_base, tmem_o = tmem + 256 + lane_base;
-    uint32_t cnt = 0;      // this chain's tiles so far, over all items
+  } else if (warp == 11) {  // ---------------- tensor cores: O += P V, tile after tile
+    if (hb_elect()) {
+      constexpr uint32_t idesc = ft_idesc_b_mn(FT_BM, FT_D);
+      uint32_t t = 0;
+      bool ok = true;
+      int4 ahead = entry(0);
+      for (int k = 0; ft_item(k) < n_items && ok; k++) {
+        const int n = ft_span(ahead, window).n;
+        ahead = entry(k + 1);
+        ok = hb_mbar_wait(&bar->o_free[k & 1], ((k >> 1) & 1) ^ 1, abort_flag);     // the item before the last one is written
+        for (int i = 0; i < n && ok; i++, t++) {
+          const uint32_t c = t & 1, ph = (t >> 1) & 1;
+          ok = hb_mbar_wait(&bar->v_full[c], ph, abort_flag) && hb_mbar_wait(&bar->p_full[c], ph, abort_flag);
+          if (!ok) break;
+          hb_tc_fence_after();
+#pragma unroll
+          for (int kk = 0; kk < FT_BN / 16; kk++) {
+            const uint64_t dp = hb_umma_desc_k128(hb_smem_u32(sP + (2 * c + (kk >> 2)) * FT_TILE)) + 2 * (kk & 3);
+            const uint64_t dv = ft_desc_mn128(hb_smem_u32(sV + c * OPND + kk * 16 * 128));   // 16 keys on; the second 64 columns lie FT_TILE further (the descriptor's leading offset)
+            hb_umma_bf16(tmem + 256 + (k & 1) * 128, dp, dv, idesc, i > 0 || kk != 0);      // O stays in tensor memory over the item's tiles
+          }
+          hb_umma_commit(&bar->v_free[c]);
+          hb_umma_commit(&bar->pv_done[c]);
+        }
+      }
+    }
+  } else {  // ---------------- softmax: warpgroup c has every second tile; thread = query row
+    const int c = warp >> 2, w = warp & 3, r = threadIdx.x & 127;
+    const uint32_t lane_base = (uint32_t)(w * 32) << 16, tmem_s = tmem + c * FT_BN + lane_base;
+    uint32_t t0 = 0;       // the item's first tile
     bool ok = true;        // every wait's outcome is made uniform over the warp: the tensor-memory accesses below are warp-wide
+    auto wait = [&](uint64_t* b, uint32_t parity) { ok = __all_sync(0xffffffffu, hb_mbar_wait(b, parity, abort_flag)); return ok; };
     int4 ahead = entry(0);
-    for (int k = 0, u; (u = ft_item(k)) < n_items; k++) {     // (a warp that gave up still meets the others at the item's two barriers)
+    for (int k = 0, u; (u = ft_item(k)) < n_items && ok; k++) {
       const int4 e = ahead;
       ahead = entry(k + 1);
       const int hq = u % Hq;
       const FtSpan sp = ft_span(e, window);
       const int qp = e.z + min(r, e.y - 1);      // rows past the portion's end are computed, never stored
       const float r1 = EX && r1p ? r1p[hq] : 0.f, r2 = EX && r1p ? r2p[hq] : 0.f;
+      const uint32_t tmem_o = tmem + 256 + (k & 1) * 128 + lane_base;
       float m_run = -INFINITY, l_run = 0.f;
-      const int i0 = (sp.kt_lo ^ c) & 1;         // the chain's first tile
-      for (int i = i0; i < sp.n && ok; i += 2, cnt++) {
+      for (int i = (t0 ^ c) & 1; i < sp.n; i += 2) {
+        const uint32_t t = t0 + i, ph = (t >> 1) & 1, ph_before = ((t - 1) >> 1) & 1;     // this tile's use, and that of the tile before
         const int k_base = (sp.kt_lo + i) * FT_BN;
         const bool need_mask = k_base + FT_BN - 1 > e.z || (window > 0 && k_base < sp.p_last - window + 1);
-        if (!__all_sync(0xffffffffu, hb_mbar_wait(&bar->s_full[c], cnt & 1, abort_flag))) { ok = false; break; }
+        if (!wait(&bar->s_full[c], ph)) break;
         hb_tc_fence_after();
-        uint32_t sr[128];
-#pragma unroll
-        for (int q = 0; q < 4; q++) ft_ld32(tmem_s + 32 * q, sr + 32 * q);
-        hb_tmem_ld_wait();
-#pragma unroll
-        for (int q = 0; q < 4; q++) ft_ld32_fence(sr + 32 * q);
-        hb_tc_fence_before();
-        __syncwarp();
-        if (lane == 0) hb_mbar_arrive(&bar->s_free[c]);   // the scores of the chain's next tile may overwrite S
-        if (need_mask) {
-          const int hi_j = qp - k_base, lo_j = window > 0 ? qp - window - k_base : -1;  // key j of the tile is visible iff lo_j < j <= hi_j
-#pragma unroll
-          for (int j = 0; j < 128; j++)
-            if (!(j <= hi_j && j > lo_j)) sr[j] = __float_as_uint(-INFINITY);
-        }
+        // a row of S in one read; in two with a bias (EX), whose chains are longer and want registers of their own: the second half stays, the first is read again
+        constexpr int H = EX ? 64 : 128;
+        uint32_t sr[H];
         float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        const int hi_j = qp - k_base, lo_j = window > 0 ? qp - window - k_base : -1;  // key j of the tile is visible iff lo_j < j <= hi_j
+        auto read = [&](int at) {
 #pragma unroll
-        for (int j = 0; j < 128; j += 2) mx[(j >> 1) & 3] = fmaxf(fmaxf(mx[(j >> 1) & 3], __uint_as_float(sr[j])), __uint_as_float(sr[j + 1]));
+          for (int q = 0; q < H; q += 32) ft_ld32(tmem_s + at + q, sr + q);
+          hb_tmem_ld_wait();
+#pragma unroll
+          for (int q = 0; q < H; q += 32) ft_ld32_fence(sr + q);
+        };
+        auto mask = [&](int at) {
+          if (need_mask) {
+#pragma unroll
+            for (int j = 0; j < H; j++)
+              if (!(j + at <= hi_j && j + at > lo_j)) sr[j] = __float_as_uint(-INFINITY);
+          }
+        };
+        auto free_s = [&] {        // the scores of the warpgroup's next tile may overwrite S
+          hb_tc_fence_before();
+          __syncwarp();
+          if (lane == 0) hb_mbar_arrive(&bar->s_free[c]);
+        };
+#pragma unroll
+        for (int at = 0; at < 128; at += H) {
+          read(at);
+          if (!EX) free_s();
+          mask(at);
+#pragma unroll
+          for (int j = 0; j < H; j += 2) mx[(j >> 1) & 3] = fmaxf(fmaxf(mx[(j >> 1) & 3], __uint_as_float(sr[j])), __uint_as_float(sr[j + 1]));
+        }
         float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2;
         const float dist0 = (float)(qp - k_base);                     // of the tile's first key
         if (EX) m_tile -= r1 * __log2f(fmaf(r2, fmaxf(dist0 - (FT_BN - 1), 0.f), 1.f));
+        if (i > 0) {       // the maximum so far, from the other warpgroup's tile
+          if (!wait(&bar->m_full[c ^ 1][w], ph_before)) break;
+          m_run = bar->m[r];
+        }
         const bool grow = m_tile > m_run + FT_SLACK;   // also the first tile with a visible key: m_run is -inf
         float corr = 1.f;
         if (grow) {
           corr = hb_exp2(m_run - m_tile);   // 0 while nothing has been summed
           m_run = m_tile;
         }
+        bar->m[r] = m_run;
+        __syncwarp();
+        if (lane == 0) hb_mbar_arrive(&bar->m_full[c][w]);
         const float sub = m_run == -INFINITY ? 0.f : m_run;
         const uint64_t scale2 = ft_pack2(__float_as_uint(scale_log2), __float_as_uint(scale_log2)), sub2 = ft_pack2(__float_as_uint(-sub), __float_as_uint(-sub));
-        uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};
+        uint64_t sum2[2] = {0ull, 0ull};   // four sums of pairs, of keys 64-127 first (the order that one warpgroup with half a row in registers has)
 #pragma unroll
-        for (int j = 0; j < 128; j += 2)   // masked scores are -inf: 2^-inf = 0
-          sr[j >> 1] = ft_prob<EX>(sr[j], sr[j + 1], scale2, sub2, r1, r2, dist0 - (float)j, sum2[(j >> 1) & 3]);
-        float s0, s1;
-        ft_unpack2(ft_add2(ft_add2(sum2[0], sum2[1]), ft_add2(sum2[2], sum2[3])), s0, s1);
-        l_run = l_run * corr + (s0 + s1);
-        // the chain's product before this one has read its P and written its O
-        if (cnt > 0 && !__all_sync(0xffffffffu, hb_mbar_wait(&bar->pv_done[c], (cnt - 1) & 1, abort_flag))) { ok = false; break; }
-        // the row: eight 16-byte chunks in each of the two K blocks of P
+        for (int hh = 1; hh >= 0; hh--) {
+          if (EX && hh == 0) {
+            read(0);
+            free_s();
+            mask(0);
+          }
+          uint32_t* x = sr + (EX ? 0 : hh * 64);
 #pragma unroll
-        for (int cc = 0; cc < 16; cc++) {
-          const uint32_t dst = hb_smem_u32(sP + (2 * c + (cc >> 3)) * FT_TILE) + r * 128 + (((cc & 7) ^ (r & 7)) << 4);
-          asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(sr[4 * cc]), "r"(sr[4 * cc + 1]),
-                       "r"(sr[4 * cc + 2]), "r"(sr[4 * cc + 3]) : "memory");
+          for (int j = 0; j < 64; j += 4) {  // masked scores are -inf: 2^-inf = 0
+            float p0, p1, p2, p3;
+            ft_exp<EX>(x[j], x[j + 1], scale2, sub2, r1, r2, dist0 - (float)(j + hh * 64), p0, p1);
+            ft_exp<EX>(x[j + 2], x[j + 3], scale2, sub2, r1, r2, dist0 - (float)(j + 2 + hh * 64), p2, p3);
+            sum2[(j >> 2) & 1] = ft_add2(sum2[(j >> 2) & 1], ft_pack2(__float_as_uint(p0 + p1), __float_as_uint(p2 + p3)));
+            x[j >> 1] = hb_pack_bf16(p0, p1);
+            x[(j >> 1) + 1] = hb_pack_bf16(p2, p3);
+          }
+          // (without a bias the exponentials of the whole row come first: half by half they were 10 % slower)
+          if (EX || hh == 0) {
+            // the product of the tile two before has read P
+            if ((!EX || hh == 1) && t >= 2 && !wait(&bar->pv_done[c], ph ^ 1)) break;
+            // 64 keys = eight 16-byte chunks of this row in K block hh of P
+#pragma unroll
+            for (int cc = EX ? hh * 8 : 0; cc < (EX ? hh * 8 + 8 : 16); cc++) {
+              const uint32_t dst = hb_smem_u32(sP + (2 * c + (cc >> 3)) * FT_TILE) + r * 128 + (((cc & 7) ^ (r & 7)) << 4);
+              const uint32_t* y = sr + (EX ? 0 : (cc >> 3) * 64) + 4 * (cc & 7);
+              asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]) : "memory");
+            }
+          }
         }
-        if (i > i0 && __any_sync(0xffffffffu, grow)) {   // a raised maximum: the chain's rows of O so far
+        if (!ok) break;
+        if (i > 0) {       // the sum so far
+          if (!wait(&bar->l_full[c ^ 1][w], ph_before)) break;
+          l_run = bar->l[r];
+        }
+        float s0, s1, s2, s3;
+        ft_unpack2(sum2[0], s0, s1);
+        ft_unpack2(sum2[1], s2, s3);
+        l_run = l_run * corr + ((s0 + s1) + (s2 + s3));
+        bar->l[r] = l_run;
+        __syncwarp();
+        if (lane == 0) hb_mbar_arrive(&bar->l_full[c][w]);
+        if (i > 0 && __any_sync(0xffffffffu, grow)) {   // a raised maximum: the rows of O so far, when the product of the tile before has written them
+          if (!wait(&bar->pv_done[c ^ 1], ph_before)) break;   // (its warpgroup's sum came behind the use before)
           hb_tc_fence_after();
 #pragma unroll
           for (int q = 0; q < FT_D / 32; q++) {
             uint32_t o[32];
-            ft_ld32(tmem_o + c * 128 + q * 32, o);
+            ft_ld32(tmem_o + q * 32, o);
             hb_tmem_ld_wait();
             ft_ld32_fence(o);
 #pragma unroll
             for (int d = 0; d < 32; d++) o[d] = __float_as_uint(__uint_as_float(o[d]) * corr);
-            ft_st32(tmem_o + c * 128 + q * 32, o);
+            ft_st32(tmem_o + q * 32, o);
           }
           hb_tmem_st_wait();
         }
@@ -471,47 +515,38 @@ __global__ void __launch_bounds__(FT_THREADS, 1) flash_prefill_tc_kernel(
         __syncwarp();
         if (lane == 0) hb_mbar_arrive(&bar->p_full[c]);
       }
-      // ---- the two chains joined
-      if (ok && i0 < sp.n) ok = __all_sync(0xffffffffu, hb_mbar_wait(&bar->pv_done[c], (cnt - 1) & 1, abort_flag));
-      float2* ml = (float2*)(sP + 2 * c * FT_TILE);      // where P lay: the chain's products are done
-      ml[r] = make_float2(m_run, l_run);
-      hb_tc_fence_before();
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      hb_tc_fence_after();
-      if (ok) {
-        const float2 a = ((const float2*)sP)[r], b = ((const float2*)(sP + 2 * FT_TILE))[r];
-        const float top = fmaxf(a.x, b.x), m = top == -INFINITY ? 0.f : top;   // (no score above -inf: with a sink the row is 0)
-        const float fa = hb_exp2(a.x - m), fb = hb_exp2(b.x - m);   // a chain without a visible key: 2^-inf = 0
-        float l = a.y * fa + b.y * fb;
-        if (EX && sink) l += hb_exp2(fmaf(sink[hq], 1.4426950408889634f, -m));
-        const float inv = 1.f / l, ga = fa * inv, gb = fb * inv;
-        const bool both = sp.n > 1, even = !(sp.kt_lo & 1);         // (with one tile, the other chain's accumulator is not of this item)
+      // ---- the item's end: each warpgroup writes half of the columns; the next item's products go to the other accumulator
+      const uint32_t last = t0 + sp.n - 1, cl = last & 1, ph_last = (last >> 1) & 1;
+      t0 += sp.n;
+      if (ok && cl != c && wait(&bar->m_full[cl][w], ph_last) && wait(&bar->l_full[cl][w], ph_last)) {
+        m_run = bar->m[r];
+        l_run = bar->l[r];
+      }
+      if (ok && wait(&bar->pv_done[cl], ph_last)) {
+        hb_tc_fence_after();
+        if (EX && sink) l_run += hb_exp2(fmaf(sink[hq], 1.4426950408889634f, -m_run));
+        const float inv = 1.f / l_run;
         constexpr int HC = FT_D / 2;                                 // this warpgroup's columns: c * HC ..
-        __nv_bfloat16* dst = out + ((size_t)(e.x + r) * Hq + hq) * FT_D + c * HC;
+        uint32_t o[HC];
+        hb_tmem_ld64_nowait(tmem_o + c * HC, o);
+        hb_tmem_ld_wait();
+        hb_tmem_ld_fence64(o);
+        hb_tc_fence_before();
+        __syncwarp();
+        if (lane == 0) hb_mbar_arrive(&bar->o_free[k & 1]);
+        if (r < e.y) {
+          __nv_bfloat16* dst = out + ((size_t)(e.x + r) * Hq + hq) * FT_D + c * HC;
 #pragma unroll
-        for (int q = 0; q < HC; q += 32) {
-          float v[32], w[32];
-          hb_tmem_ld32(tmem_o + (both || even ? 0 : 128) + c * HC + q, v);
-          if (both) {
-            hb_tmem_ld32(tmem_o + 128 + c * HC + q, w);
-#pragma unroll
-            for (int d = 0; d < 32; d++) v[d] = fmaf(w[d], gb, v[d] * ga);
-          } else {
-            const float g = even ? ga : gb;
-#pragma unroll
-            for (int d = 0; d < 32; d++) v[d] *= g;
-          }
-          if (r < e.y) {
-#pragma unroll
-            for (int d = 0; d < 32; d += 8)
-              *(uint4*)(dst + q + d) = make_uint4(hb_pack_bf16(v[d], v[d + 1]), hb_pack_bf16(v[d + 2], v[d + 3]),
-                                                  hb_pack_bf16(v[d + 4], v[d + 5]), hb_pack_bf16(v[d + 6], v[d + 7]));
+          for (int d = 0; d < HC; d += 8) {
+            uint4 v;
+            v.x = hb_pack_bf16(__uint_as_float(o[d]) * inv, __uint_as_float(o[d + 1]) * inv);
+            v.y = hb_pack_bf16(__uint_as_float(o[d + 2]) * inv, __uint_as_float(o[d + 3]) * inv);
+            v.z = hb_pack_bf16(__uint_as_float(o[d + 4]) * inv, __uint_as_float(o[d + 5]) * inv);
+            v.w = hb_pack_bf16(__uint_as_float(o[d + 6]) * inv, __uint_as_float(o[d + 7]) * inv);
+            *(uint4*)(dst + d) = v;
           }
         }
       }
-      hb_tc_fence_before();
-      asm volatile("bar.sync 2, 256;" ::: "memory");   // both accumulators and the chains' numbers may be overwritten
-      hb_tc_fence_after();
     }
   }
 

@@ -366,3 +366,34 @@ def test_attention_of_more_pairs_than_a_launch_takes(D, requests, tokens, heads)
     torch.cuda.synchronize()
     f.check_status()
     assert bool((out.view(T, heads, D) == vc.transpose(1, 2).reshape(T, 1, D)).all())
+
+
+@pytest.mark.parametrize("ctx,rows,window,extras", [
+    ([0, 0, 700, 5], [700, 16, 300, 1300], 0, False),        # items of one to eleven key tiles
+    ([900, 130], [300, 40], 200, False),
+    ([0, 1000], [600, 128], 0, True),
+])
+def test_both_head_sizes_sum_in_the_same_order(ctx, rows, window, extras):
+    """A head of 64 padded with zeros to 128: the scores, the values and with them every bit are those of the kernel for 64, whose tiles
+    go through one chain. The scores grow along the keys, so that the maximum is raised again and again."""
+    from types import SimpleNamespace
+
+    f = fast()
+    Hq, Hkv, ps = 4, 2, 16
+    q, kc, vc, bt, T, _ = attention_case(Hq, Hkv, 64, ps, ctx, rows, window, 91)
+    for r, n in enumerate(c + m for c, m in zip(ctx, rows)):
+        pages = bt[r, :-(-n // ps)].long()
+        kc[pages] *= torch.linspace(0.5, 12, len(pages), device=DEV, dtype=torch.bfloat16).view(-1, 1, 1, 1)
+    pad = lambda t: torch.cat([t, torch.zeros_like(t)], -1)
+    meta = (i32([sum(rows[:i]) for i in range(len(rows))]), i32(rows), i32(ctx))
+    kw = {}
+    if extras:
+        kw = dict(distance=SimpleNamespace(r1=torch.linspace(0, 1, Hq, device=DEV), r2=torch.linspace(0.1, 1, Hq, device=DEV)), sink=torch.linspace(-1, 1, Hq, device=DEV))
+    outs = []
+    for D, args in ((64, (q, kc, vc)), (128, (pad(q.view(T, Hq, 64)).view(T, -1), pad(kc), pad(vc)))):
+        out = torch.zeros(T, Hq * D, dtype=torch.bfloat16, device=DEV)
+        f.flash_prefill_tc(*(t.contiguous() for t in args), bt, *meta, out, max(rows), Hq, Hkv, D, ps, window, 0.125, 16, **kw)
+        torch.cuda.synchronize()
+        f.check_status()
+        outs.append(out.view(T, Hq, D))
+    assert torch.equal(outs[0], outs[1][:, :, :64]) and bool((outs[1][:, :, 64:] == 0).all())
