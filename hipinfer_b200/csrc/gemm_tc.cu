@@ -655,7 +655,7 @@ HB_EXPORT int hb_gemm_tc(const void* A, long lda, const void* W, long ldw, void*
   if (!status) HB_FAIL("hb_gemm_tc: no status word");
   if (tile_n == 0) {
     // 128 x 256 tiles feed the tensor cores best (a narrower tile reads more operand bytes per flop: measured
-    // 1.1 times the time per column at 192, 1.35 times at 128); a narrower one is taken when it fills the
+    // 1.06 times the time per column at 192, counted as 1.1, and 1.37 times at 128); a narrower one is taken when it fills the
     // SMs' rounds better. An output's value is the same for every tile width.
     const long mt = (M + BM - 1) / BM, sms = sm_count();
     auto cost = [&](int bn, double per_col) { return (double)((mt * ((N + bn - 1) / bn) + sms - 1) / sms) * bn * per_col; };
@@ -664,7 +664,8 @@ HB_EXPORT int hb_gemm_tc(const void* A, long lda, const void* W, long ldw, void*
     if ((epi == EPI_F32 || epi == EPI_ADD_F32) && cost(192, 1.1) < best) { tile_n = 192; best = cost(192, 1.1); }
     if (cost(128, 1.35) < best) tile_n = 128;
     // where the 256-wide tile is the choice, CTA pairs on 256 x 256 tiles do the same work with a third less
-    // operand traffic per CTA (measured 0 to 14 % faster, never slower), given two row halves and a C that TMA can store to
+    // operand traffic per CTA, given two row halves and a C that TMA can store to: faster where there are several rounds (512 x 16,384 x 2,048 30.7 us,
+    // 32.8 by single CTAs), up to 9 % slower in one round (2,048 x 2,048 x 2,048 17.2, 15.6)
     const bool c_ok = !((uintptr_t)C & 15) && (ldc & ((epi == EPI_F32 || epi == EPI_ADD_F32) ? 3 : 7)) == 0;
     if (HB_GEMM_PAIR && tile_n == 256 && M > 128 && c_ok) tile_n = 512;
   }

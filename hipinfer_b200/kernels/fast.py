@@ -244,8 +244,11 @@ def rope_kv_slices(sl: Slices, positions, slot_map, table, q_out, k_cache, v_cac
 def slices_pay(M, N, K) -> bool:
     """Whether a portion's product is better cut along K (csrc/gemm_tc.cu) than run whole on narrower tiles. What a cut saves grows with
     K, what it costs (the partial sums out and in again) with the number of slices. Product and norm, us whole / in slices: K = 2,048
-    in four 16.2 / 13.0 (512 x 2,048), in three 17.4 / 15.4 (700 rows), in two 17.7 / 18.1 (1,000 rows); K = 3,072 in three 22.7 / 20.3
-    (512 x 3,072), in two 22.5 / 24.4 (700 rows); K = 4,096 in two 28.0 / 25.2; K = 1,024 in two 9.8 / 10.0, at 1,000 rows 11.1 / 13.7."""
+    in four 12.0 / 11.1 (256 x 2,048) and 12.8 / 13.3 (512), in three 13.8 / 14.5 (700 rows), in two 14.3 / 17.4 (1,000 rows); K = 3,072 in three
+    16.9 / 15.3 (400 x 3,072) and 17.5 / 17.4 (512), in two 18.1 / 20.3 (700 rows); K = 8,192 in three 33.1 / 28.2, in eight 29.1 / 16.4 (256 x 2,048);
+    K = 4,096 in two 21.5 / 21.3 (400 x 4,096) and 21.4 / 24.1 (512); K = 1,024 in two 8.8 / 10.6. (The line was drawn when whole products of
+    narrow tiles took a third longer; with them as they are, K = 2,048 in three and K = 4,096 in two are up to 12 % better whole. A row's bits are a matter
+    of the line, so it has been left where it was.)"""
     n = _fn("hb_gemm_tc_splits")(M, N, K)
     return n > 2 and K >= 2048 or n == 2 and K >= 4096
 
@@ -323,10 +326,8 @@ def linear32(a, w, out, accumulate) -> bool:
 
 
 def linear(a, w, out, accumulate) -> bool:
-    if a.dtype == torch.float32:
-        return linear32(a, w.t, out, accumulate)
     if not _tc_ok(a, w.t):
-        return False
+        return a.dtype == torch.float32 and linear32(a, w.t, out, accumulate)
     if out.dtype == torch.float32:
         epi = EPI_ADD_F32 if accumulate else EPI_F32
     elif out.dtype == torch.bfloat16 and not accumulate:

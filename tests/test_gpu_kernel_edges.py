@@ -397,3 +397,22 @@ def test_both_head_sizes_sum_in_the_same_order(ctx, rows, window, extras):
         f.check_status()
         outs.append(out.view(T, Hq, D))
     assert torch.equal(outs[0], outs[1][:, :, :64]) and bool((outs[1][:, :, 64:] == 0).all())
+
+
+@pytest.mark.parametrize("tile_n", [128, 192, 256])
+def test_single_cta_tiles_with_an_odd_number_of_boxes(tile_n):
+    """More tiles than SMs for the kernel without pairs, the last column's of a single box: a box leaves before the next tile fills its place."""
+    f = fast()
+    M, N, K = 128 * 160, 288, 64
+    a, w = rnd(M, K, seed=5), rnd(N, K, seed=6, scale=0.1)
+    ref = a.double() @ w.double().T
+    tol = 2e-5 * max(1.0, float(ref.abs().max())) * math.sqrt(K)       # 32-bit sums of K products
+    for epi in (f.EPI_F32, f.EPI_BF16):
+        if epi == f.EPI_BF16 and tile_n == 192:      # 32-bit results only
+            continue
+        out = torch.full((M, N), 7.0, dtype=torch.float32 if epi == f.EPI_F32 else torch.bfloat16, device=DEV)
+        f.gemm_tc(a, w, out, epi, tile_n)
+        torch.cuda.synchronize()
+        f.check_status()
+        rounding = 0.0 if epi == f.EPI_F32 else 2.0 ** -8              # and one rounding to bfloat16
+        assert bool(((out.double() - ref).abs() <= tol + rounding * ref.abs()).all())
